@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "aux_kernels.cuh"
+#include "dense_rhs.h"
 #include "hex_fused.cuh"
 #include "hex_kernels.cuh"
 #include "mlp_kernels.cuh"
@@ -83,6 +84,10 @@ struct dgb_plan {
   size_t force_partials_n = 0;
   ElemLaunch launch_tr, launch_vol, launch_fin, launch_tr64;
   size_t smem_tr = 0, smem_vol = 0, smem_fin = 0, smem_tr64 = 0;
+  // two-launch inviscid right-hand side of the dense path (dense_rhs.cu); faces_regular: every local
+  // face of the block has the face type its element type gives it
+  DenseTables dense = {};
+  bool faces_regular[DGB_MAX_BLOCKS] = {false, false, false};
   size_t smem_pos[DGB_MAX_BLOCKS], smem_troubled[DGB_MAX_BLOCKS];
   // sum-factorised hexahedron path (single hexahedron block)
   bool hex = false;
@@ -268,6 +273,60 @@ int dense_width(const dgb_plan* p, const BlockDev& B) {
   return w;
 }
 
+// Table of the dense kernels in the plan's arithmetic type.
+int upload_real(dgb_plan* p, const std::vector<double>& v, const void** out) {
+  int rc;
+  if (p->prm.precision == 1) {
+    const std::vector<float> f(v.begin(), v.end());
+    const float* d = nullptr;
+    rc = upload(p, f.data(), f.size(), &d);
+    *out = d;
+  } else {
+    const double* d = nullptr;
+    rc = upload(p, v.data(), v.size(), &d);
+    *out = d;
+  }
+  return rc;
+}
+
+// The face-node tables of one block and face type (DenseBlock) from its trace table B
+// [codes][nq][np]: the nodes whose basis does not vanish on the face.  Left empty (and with it the
+// two-launch form off) when the shapes or the number of such nodes are not those of the element type.
+int dense_trace_tables(dgb_plan* p, int b, int ft, int ncodes, int nq, int np, const double* B) {
+  const BlockDev& blk = p->dev.blk[b];
+  if (p->dev.degree < 1 || p->dev.degree > 3 || blk.type < 0 || blk.type > 2 || !B) return DGB_OK;
+  const DenseShape s = dense_shape(p->dev.degree, blk.type);
+  if (np != s.Np || nq != s.nq[ft]) return DGB_OK;
+  const int nfn = s.nfn[ft];
+  std::vector<uint8_t> node((size_t)ncodes * nfn);
+  std::vector<int8_t> inv((size_t)ncodes * np, -1);
+  std::vector<double> cb((size_t)ncodes * nq * nfn), cbt(cb.size());
+  for (int c = 0; c < ncodes; ++c) {
+    int n = 0;
+    for (int i = 0; i < np; ++i) {
+      double most = 0.0;
+      for (int q = 0; q < nq; ++q) most = std::max(most, fabs(B[((size_t)c * nq + q) * np + i]));
+      if (!(most > 1.0e-12)) continue;
+      if (n == nfn) return DGB_OK;
+      node[(size_t)c * nfn + n] = (uint8_t)i;
+      inv[(size_t)c * np + i] = (int8_t)n++;
+    }
+    if (n != nfn) return DGB_OK;
+    for (int q = 0; q < nq; ++q)
+      for (int j = 0; j < nfn; ++j) {
+        const double v = B[((size_t)c * nq + q) * np + node[(size_t)c * nfn + j]];
+        cb[((size_t)c * nq + q) * nfn + j] = v;
+        cbt[((size_t)c * nfn + j) * nq + q] = v;
+      }
+  }
+  DenseBlock& X = p->dense.b[b];
+  int rc;
+  if ((rc = upload(p, node.data(), node.size(), &X.fnode[ft]))) return rc;
+  if ((rc = upload(p, inv.data(), inv.size(), &X.finv[ft]))) return rc;
+  if ((rc = upload_real(p, cb, &X.cB[ft]))) return rc;
+  return upload_real(p, cbt, &X.cBt[ft]);
+}
+
 // Per-element shared-memory slots (bytes, 16-aligned) for one kernel kind and real size.
 void dense_slots(const dgb_plan* p, ElemLaunch& L, DenseKind kind, size_t rs) {
   const int NV = p->dev.nv;
@@ -295,6 +354,43 @@ size_t dense_layout(const dgb_plan* p, ElemLaunch& L, DenseKind kind, size_t rs)
   for (int b = 0; b < p->dev.nblocks; ++b)
     most = std::max(most, (size_t)(kThreads / L.W[b]) * (size_t)L.slot[b]);
   return most;
+}
+
+// Completes the two-launch inviscid form (dense_rhs.cu) where every block has its shapes and tables.
+int dense_finish(dgb_plan* p) {
+  p->dense.ready = false;
+  if (p->hex || p->dev.viscous || p->dev.nv != 5 || p->dev.degree < 1 || p->dev.degree > 3) return DGB_OK;
+  const bool f32 = p->prm.precision == 1;
+  for (int b = 0; b < p->dev.nblocks; ++b) {
+    const BlockDev& B = p->dev.blk[b];
+    DenseBlock& X = p->dense.b[b];
+    if (B.type < 0 || B.type > 2) return DGB_OK;
+    if (B.E == 0) continue;
+    const DenseShape s = dense_shape(p->dev.degree, B.type);
+    const bool tri = B.type != 0, quad = B.type != 2;
+    if (B.Np != s.Np || B.Nq != s.Nq || B.nlf != s.nlf || !p->faces_regular[b] || !B.Bt || !B.dBi || !B.jinv ||
+        !B.wdet || (tri && !X.cB[0]) || (quad && !X.cB[1]))
+      return DGB_OK;
+    X.chunks = volume_chunks(B.Np, dense_width(p, B));
+    X.Bt = B.Bt;
+    X.dBi = B.dBi;
+    X.minv = B.minv;
+    X.mref = B.mref_inv;
+    if (f32) {
+      float* f;
+      int rc;
+      if ((rc = to_float32(p, B.Bt, (size_t)B.Np * B.Nq, &f))) return rc;
+      X.Bt = f;
+      if ((rc = to_float32(p, B.dBi, (size_t)B.Nq * 3 * B.Np, &f))) return rc;
+      X.dBi = f;
+      if ((rc = to_float32(p, B.minv, (size_t)B.E * B.Np * B.Np, &f))) return rc;
+      X.minv = f;
+      if ((rc = to_float32(p, B.mref_inv, (size_t)B.Np * B.Np, &f))) return rc;
+      X.mref = f;
+    }
+  }
+  p->dense.ready = true;
+  return DGB_OK;
 }
 
 size_t dense_smem(const dgb_plan* p, ElemLaunch& L, DenseKind kind, size_t rs) {
@@ -444,6 +540,20 @@ template <int NV, typename R>
 int run_rhs_dense(dgb_plan* p, const StatePtrs& S, const FinalizeArgs& A, cudaStream_t st, cudaEvent_t* ev) {
   const DevPlan& P = p->dev;
   int rc;
+  if (NV == 5 && p->dense.ready) {
+    constexpr bool f32 = sizeof(R) == sizeof(float);
+    auto record = [&](int k) { return ev ? cudaEventRecord(ev[k], st) : cudaSuccess; };
+    CK(record(0));
+    CK(record(1));                             // the face kernel forms the traces itself
+    CK(dense_face_flux(P, S, p->dense, f32, p->prm.limiter == 2, st));
+    CK(record(2));
+    CK(record(3));
+    for (int b = 0; b < P.nblocks; ++b)
+      if (p->tc_on[b]) CK(tc_volume(P, S, b, p->tc[b], p->tc_image[b], p->dev_err, p->sm_count, st));
+    CK(dense_update(P, S, A, p->dense, f32, p->tc_on, st));
+    for (int k = 4; k <= 6; ++k) CK(record(k));
+    return DGB_OK;
+  }
   if (ev) CK(cudaEventRecord(ev[0], st));
   if ((rc = prepare(k_traces<NV, R>, p->smem_tr))) return rc;
   k_traces<NV, R><<<p->launch_tr.cta0[P.nblocks], kThreads, p->smem_tr, st>>>(P, S, p->launch_tr);
@@ -495,6 +605,12 @@ int autotune_dense(dgb_plan* p, const StatePtrs& S, int reps, cudaStream_t st, i
   FinalizeArgs A;
   memset(&A, 0, sizeof(A));
   int rc;
+  if (NV == 5 && p->dense.ready) {            // the two-launch form's work split is fixed
+    const ElemLaunch* fixed[3] = {&p->launch_tr, &p->launch_vol, &p->launch_fin};
+    for (int k = 0; widths && k < 3; ++k)
+      for (int b = 0; b < DGB_MAX_BLOCKS; ++b) widths[k * DGB_MAX_BLOCKS + b] = b < P.nblocks ? fixed[k]->W[b] : 0;
+    return DGB_OK;
+  }
   if ((rc = run_rhs_dense<NV, R>(p, S, A, st, nullptr))) return rc;
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));
@@ -1100,6 +1216,11 @@ int dgb_plan_set_block(dgb_plan* p, int b, const dgb_block_desc* d) {
   if ((rc = upload(p, d->face_sample_basis, (size_t)B.Ns * Np, &B.fsB))) return rc;
   if ((rc = upload(p, d->p1_projector, Np * Np, &B.p1proj))) return rc;
   if ((rc = upload(p, d->elem_face, E * B.nlf, &B.elem_face))) return rc;
+  // triangles come first in every element type's local faces
+  const int ntri = B.type == 0 ? 0 : B.type == 1 ? 2 : 4;
+  p->faces_regular[b] = true;
+  for (size_t k = 0; k < E * B.nlf; ++k)
+    p->faces_regular[b] &= ((d->elem_face[k] >> 30) & 1) == ((int)(k % B.nlf) < ntri ? 0 : 1);
   p->block_set[b] = true;
   return DGB_OK;
 }
@@ -1148,6 +1269,7 @@ int dgb_plan_set_trace(dgb_plan* p, int etype, int ftype, int ncodes, int nq, in
       if ((rc = upload(p, bt.data(), bt.size(), &blk.trBt[ftype]))) return rc;
       if ((rc = upload(p, dt.data(), dt.size(), &blk.trdBt[ftype]))) return rc;
     }
+    if ((rc = dense_trace_tables(p, b, ftype, ncodes, nq, np, B))) return rc;
     found = 1;
   }
   if (!found) return fail(DGB_ERR_ARGUMENT, "trace table for an element type without a block");
@@ -1431,6 +1553,7 @@ int dgb_plan_finalize(dgb_plan* p) {
     p->smem_tr64 = dense_smem(p, p->launch_tr64, traces_kind, sizeof(double));
     if (p->smem_tr > 227 * 1024 || p->smem_vol > 227 * 1024 || p->smem_fin > 227 * 1024)
       return fail(DGB_ERR_UNSUPPORTED, "element too large for the shared-memory kernels");
+    if ((rc = dense_finish(p))) return rc;
   }
   {
     void* d = nullptr;

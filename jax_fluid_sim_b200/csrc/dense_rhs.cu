@@ -1,0 +1,572 @@
+// Inviscid right-hand side of the dense path (hybrid meshes: hexahedra, wedges, tetrahedra) in two
+// launches per evaluation (hybrid/spatial.py:47-72,137-249):
+//
+//   k_dense_faces    face traces and HLLC flux: one thread per face point.  The traces are formed from
+//                    the nodes on the face (the basis of every other node is zero there), read
+//                    from the element states, so no trace buffer goes through memory.
+//   k_dense_update   one CTA per NE elements: volume residual, face terms, M^-1 and the stage update,
+//                    with everything between them in shared memory.
+//
+// The element kernel is bound by the operand loads of its contractions, not by their arithmetic: with
+// one accumulator row per table value and broadcast operand (one element per CTA, one value per
+// load) the load pipe runs at three times the FP64 pipe's time.  So a thread keeps a tile: EB elements x
+// NV variables of one point while it interpolates, IB nodes x EB2 elements x NV variables of one chunk
+// of points while it sums the residual, with 16-byte shared-memory loads; a table value from L1/L2 then
+// serves EB * NV products instead of NV.  NE is chosen so that both phases fill kThreads.
+// Sums run in the order of the one-value-per-thread form: per output the nodes (points) ascend, and
+// the residual is summed per chunk of points, then over the chunks.
+#include "dense_rhs.h"
+
+namespace dgb {
+
+namespace {
+
+// Shapes of an element of type T (0 hexahedron, 1 wedge, 2 tetrahedron) at degree P.
+template <int P, int T>
+struct Shape {
+  static constexpr int N1 = P + 1, TRI = (P + 1) * (P + 2) / 2, QUAD = N1 * N1;
+  static constexpr int Np = T == 0 ? N1 * N1 * N1 : T == 1 ? TRI * N1 : (P + 1) * (P + 2) * (P + 3) / 6;
+  static constexpr int Nq = T == 0 ? (P == 1 ? 8 : P == 2 ? 27 : 125) : T == 1 ? (P == 1 ? 6 : 125) : (P == 1 ? 4 : 125);
+  static constexpr int nlf = T == 0 ? 6 : T == 1 ? 5 : 4;
+  static constexpr int ntri = T == 0 ? 0 : T == 1 ? 2 : 4;         // the triangles come first
+  static constexpr int NQT = P == 1 ? 3 : P == 2 ? 16 : 25, NQQ = (P + 1) * (P + 1);
+  static constexpr int Nf = ntri * NQT + (nlf - ntri) * NQQ;        // face points
+  static constexpr int Nj = ntri * TRI + (nlf - ntri) * QUAD;       // face nodes, per face
+  __host__ __device__ static constexpr int nq(int lf) { return lf < ntri ? NQT : NQQ; }
+  __host__ __device__ static constexpr int nfn(int lf) { return lf < ntri ? TRI : QUAD; }
+  __host__ __device__ static constexpr int poff(int lf) { return lf <= ntri ? lf * NQT : ntri * NQT + (lf - ntri) * NQQ; }
+  __host__ __device__ static constexpr int joff(int lf) { return lf <= ntri ? lf * TRI : ntri * TRI + (lf - ntri) * QUAD; }
+};
+
+// Work split: NE elements per CTA; EB elements per thread while interpolating, IB nodes x EB2
+// elements per thread in the residual sum.  P2 and P3 volume rules of 125 points take one thread per
+// point over four elements; the 27 points of a P2 hexahedron leave room for four pairs; P1 elements
+// are one thread per (element, point).
+template <int P, int T>
+struct Split {
+  static constexpr bool one = P == 1;
+  static constexpr int NE = one ? (T == 0 ? 16 : T == 1 ? 20 : 32) : (P == 2 && T == 0 ? 8 : 4);
+  static constexpr int EB = one ? 1 : (P == 2 && T == 0 ? 2 : 4);
+  static constexpr int EB2 = one ? 1 : 2;
+  static constexpr int IB = one || Shape<P, T>::Np % 2 ? 1 : 2;
+};
+
+__host__ __device__ constexpr int round_up(int a, int b) { return (a + b - 1) / b * b; }
+
+// Shared memory of k_dense_update in units of R.
+template <int P, int T, int NV, typename R>
+struct Smem {
+  using S = Shape<P, T>;
+  using W = Split<P, T>;
+  static constexpr int VA = 16 / (int)sizeof(R);
+  static constexpr int UE = round_up(W::EB * NV, VA);                  // one node of EB elements
+  static constexpr int UG = S::Np * UE;                                 // one group of EB elements
+  static constexpr int GP = round_up(W::EB2 * 3 * NV, VA);             // one point of EB2 elements
+  // point stride of a group: an odd number of 16-byte units, so that a warp's stores (one point per
+  // lane) fall on distinct banks
+  static constexpr int GQ0 = W::EB / W::EB2 * GP, GQ = (GQ0 / VA) % 2 ? GQ0 : GQ0 + VA;
+  static constexpr int GG0 = S::Nq * GQ, GG = (GG0 / VA) % 2 ? GG0 : GG0 + VA;
+  static constexpr int U = 0, Gs = U + W::NE / W::EB * UG;
+  static constexpr int G = W::NE / W::EB * GG;
+  // over G once it is dead: chunk sums, fluxes, face sums, totals, results
+  static constexpr int FS = round_up(NV, VA);                          // one row of NV values
+  static constexpr int chunk_max = kThreads / S::Np > 0 ? kThreads / S::Np : 1;
+  static constexpr int Pc = W::one ? W::NE * S::Np * FS : chunk_max * W::NE * S::Np * FS;
+  static constexpr int Fl = Gs + round_up(Pc, VA), Fp = Fl + W::NE * S::Nf * FS;
+  static constexpr int Tt = Fl;                                        // the fluxes are dead by then
+  static constexpr int End = Fp + W::NE * S::Nj * FS;
+  static_assert(S::Np <= S::Nf, "the totals take the fluxes' place");
+  static constexpr int total = Gs + G > End ? Gs + G : End;
+};
+
+// n values at p (16-byte aligned)
+template <int K, typename R>
+__device__ __forceinline__ void lds16(const R* p, R* r) {
+  constexpr int VA = 16 / (int)sizeof(R);
+  if constexpr (sizeof(R) == 8) {
+#pragma unroll
+    for (int k = 0; k < K / VA; ++k) {
+      const double2 v = reinterpret_cast<const double2*>(p)[k];
+      r[2 * k] = v.x, r[2 * k + 1] = v.y;
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < K / VA; ++k) {
+      const float4 v = reinterpret_cast<const float4*>(p)[k];
+      r[4 * k] = v.x, r[4 * k + 1] = v.y, r[4 * k + 2] = v.z, r[4 * k + 3] = v.w;
+    }
+  }
+#pragma unroll
+  for (int k = K / VA * VA; k < K; ++k) r[k] = p[k];
+}
+template <int K, typename R>
+__device__ __forceinline__ void sts16(R* p, const R* r) {
+  constexpr int VA = 16 / (int)sizeof(R);
+  if constexpr (sizeof(R) == 8) {
+#pragma unroll
+    for (int k = 0; k < K / VA; ++k) reinterpret_cast<double2*>(p)[k] = make_double2(r[2 * k], r[2 * k + 1]);
+  } else {
+#pragma unroll
+    for (int k = 0; k < K / VA; ++k)
+      reinterpret_cast<float4*>(p)[k] = make_float4(r[4 * k], r[4 * k + 1], r[4 * k + 2], r[4 * k + 3]);
+  }
+#pragma unroll
+  for (int k = K / VA * VA; k < K; ++k) p[k] = r[k];
+}
+
+// ------------------------------------------------------------------------------------ element kernel
+template <int P, int T, int NV, typename R>
+__device__ __forceinline__ void update_body(const DevPlan& D, const StatePtrs& St, const FinalizeArgs& A,
+                                            const DenseBlock& X, int b, int cta, bool volume_done, R* sm) {
+  using S = Shape<P, T>;
+  using W = Split<P, T>;
+  using L = Smem<P, T, NV, R>;
+  constexpr int Np = S::Np, Nq = S::Nq, nlf = S::nlf, NE = W::NE, EB = W::EB, EB2 = W::EB2, IB = W::IB;
+  __shared__ int fslot[NE * nlf], fcode[NE * nlf];
+  __shared__ double anchor[NE * NV];
+  __shared__ R Fanc[NE * 3 * NV];                                      // flux of the anchor states
+  const BlockDev& B = D.blk[b];
+  const int e0 = cta * NE, ne = B.E - e0 < NE ? B.E - e0 : NE;     // elements of this CTA
+  const double* Ug = St.b[b] + (size_t)e0 * Np * NV;
+  const int C = X.chunks;
+  for (int t = threadIdx.x; t < ne * nlf; t += kThreads) {
+    int ft, f, side;
+    decode_face(B.elem_face[(size_t)(e0 + t / nlf) * nlf + t % nlf], ft, f, side);
+    fslot[t] = (f << 1) | side;
+    fcode[t] = side == 0 ? D.face[ft].oc[f] : D.face[ft].nc[f];
+  }
+  if (!volume_done) {
+    for (int t = threadIdx.x; t < NE * NV; t += kThreads)
+      anchor[t] = t / NV < ne ? Ug[(size_t)(t / NV) * Np * NV + t % NV] : 1.0;
+    R* U = sm + L::U;
+    R* G = sm + L::Gs;
+    // U minus the anchor; the slots past the last element hold zeros (and unit anchors), so that their
+    // points stay finite
+    for (int t = threadIdx.x; t < NE * Np * NV; t += kThreads) {
+      const int e = t / (Np * NV), i = (t / NV) % Np, v = t % NV;
+      R x = (R)0;
+      if (e < ne) x = (R)(Ug[t] - Ug[(size_t)e * Np * NV + v]);
+      U[(e / EB) * L::UG + i * L::UE + (e % EB) * NV + v] = x;
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < NE * 3; t += kThreads) {
+      const int d = t % 3;
+      const R n[3] = {(R)(d == 0), (R)(d == 1), (R)(d == 2)};
+      R a[NV], F[NV];
+#pragma unroll
+      for (int v = 0; v < NV; ++v) a[v] = (R)anchor[t / 3 * NV + v];
+      normal_flux<NV>(D.ph, a, n, F);
+#pragma unroll
+      for (int v = 0; v < NV; ++v) Fanc[t * NV + v] = F[v];
+    }
+    __syncthreads();
+    // ---- fluxes at the volume points: thread = (point, group of EB elements)
+    const R* Bt = static_cast<const R*>(X.Bt);
+    for (int t = threadIdx.x; t < NE / EB * Nq; t += kThreads) {
+      const int q = t % Nq, g = t / Nq;
+      R acc[EB * NV];
+#pragma unroll
+      for (int k = 0; k < EB * NV; ++k) acc[k] = (R)0;
+      const R* Ur = U + g * L::UG;
+#pragma unroll 4
+      for (int i = 0; i < Np; ++i) {
+        const R bq = __ldg(Bt + i * Nq + q);
+        R x[EB * NV];
+        lds16<EB * NV>(Ur + i * L::UE, x);
+#pragma unroll
+        for (int k = 0; k < EB * NV; ++k) acc[k] += bq * x[k];
+      }
+      R* Gq = G + g * L::GG + q * L::GQ;
+#pragma unroll
+      for (int h = 0; h < EB / EB2; ++h) {
+        R out[EB2 * 3 * NV];                                         // [r][element][v]
+#pragma unroll
+        for (int k = 0; k < EB2; ++k) {
+          const int el = g * EB + h * EB2 + k;
+          const size_t e = (size_t)e0 + (el < ne ? el : 0);
+          const bool aff = B.affine != nullptr && B.affine[e];
+          const double* Jd = aff ? B.ajinv + e * 9 : B.jinv + (e * Nq + q) * 9;
+          R J[9];
+#pragma unroll
+          for (int m = 0; m < 9; ++m) J[m] = (R)Jd[m];
+          const R wq = aff ? (R)(B.wref[q] * B.adet[e]) : (R)(B.wdet[e * Nq + q] * 1.0);
+          R Uq[NV], F[3][NV];
+#pragma unroll
+          for (int v = 0; v < NV; ++v) Uq[v] = (R)(anchor[el * NV + v] + (double)acc[(h * EB2 + k) * NV + v]);
+          const R* Fa = Fanc + el * 3 * NV;
+          const R ex[3] = {(R)1, (R)0, (R)0}, ey[3] = {(R)0, (R)1, (R)0}, ez[3] = {(R)0, (R)0, (R)1};
+          normal_flux<NV>(D.ph, Uq, ex, F[0]);
+          normal_flux<NV>(D.ph, Uq, ey, F[1]);
+          normal_flux<NV>(D.ph, Uq, ez, F[2]);
+#pragma unroll
+          for (int r = 0; r < 3; ++r)
+#pragma unroll
+            for (int v = 0; v < NV; ++v)
+              out[(r * EB2 + k) * NV + v] = (J[r * 3 + 0] * (F[0][v] - Fa[v]) + J[r * 3 + 1] * (F[1][v] - Fa[NV + v]) +
+                                             J[r * 3 + 2] * (F[2][v] - Fa[2 * NV + v])) * wq;
+        }
+        sts16<EB2 * 3 * NV>(Gq + h * L::GP, out);
+      }
+    }
+    __syncthreads();
+    // ---- residual: thread = (IB nodes, chunk of points, EB2 elements); P1 elements keep the chunks
+    // in one thread.  At most ROUNDS items per thread, kept in registers until G is dead.
+    const R* dBi = static_cast<const R*>(X.dBi);
+    constexpr int NI = Np / IB;
+    constexpr int items_max = (W::one ? 1 : L::chunk_max) * NI * (NE / EB2);
+    constexpr int ROUNDS = (items_max + kThreads - 1) / kThreads;
+    const int items = (W::one ? 1 : C) * NI * (NE / EB2);
+    R sum[ROUNDS][IB * EB2 * NV];
+#pragma unroll
+    for (int rd = 0; rd < ROUNDS; ++rd) {
+      const int t = rd * kThreads + threadIdx.x;
+#pragma unroll
+      for (int k = 0; k < IB * EB2 * NV; ++k) sum[rd][k] = (R)0;
+      if (t >= items) continue;
+      const int i = t % NI * IB, ep = (t / NI) % (NE / EB2), c0 = t / (NI * (NE / EB2));
+      const R* Gr = G + (ep * EB2 / EB) * L::GG + (ep % (EB / EB2)) * L::GP;
+      const int clo = W::one ? 0 : c0, chi = W::one ? C : c0 + 1;
+      for (int c = clo; c < chi; ++c) {
+        const int q0 = c * Nq / C, q1 = (c + 1) * Nq / C;
+        R s[IB * EB2 * NV];
+#pragma unroll
+        for (int k = 0; k < IB * EB2 * NV; ++k) s[k] = (R)0;
+#pragma unroll 1
+        for (int q = q0; q < q1; ++q) {
+          R g0[IB], g1[IB], g2[IB];
+#pragma unroll
+          for (int n = 0; n < IB; ++n) {
+            const R* gd = dBi + q * 3 * Np + i + n;
+            g0[n] = __ldg(gd), g1[n] = __ldg(gd + Np), g2[n] = __ldg(gd + 2 * Np);
+          }
+          R x[EB2 * 3 * NV];
+          lds16<EB2 * 3 * NV>(Gr + q * L::GQ, x);
+#pragma unroll
+          for (int n = 0; n < IB; ++n)
+#pragma unroll
+            for (int k = 0; k < EB2 * NV; ++k)
+              s[n * EB2 * NV + k] += g0[n] * x[k] + g1[n] * x[EB2 * NV + k] + g2[n] * x[2 * EB2 * NV + k];
+        }
+#pragma unroll
+        for (int k = 0; k < IB * EB2 * NV; ++k) sum[rd][k] += s[k];
+      }
+    }
+    __syncthreads();                                                   // G is dead
+    R* Pc = sm + L::Gs;                                                // [C][NE][Np][FS]
+#pragma unroll
+    for (int rd = 0; rd < ROUNDS; ++rd) {
+      const int t = rd * kThreads + threadIdx.x;
+      if (t >= items) continue;
+      const int i = t % NI * IB, ep = (t / NI) % (NE / EB2), c0 = t / (NI * (NE / EB2));
+#pragma unroll
+      for (int n = 0; n < IB; ++n)
+#pragma unroll
+        for (int k = 0; k < EB2; ++k)
+          sts16<NV>(Pc + ((c0 * NE + ep * EB2 + k) * Np + i + n) * L::FS, &sum[rd][(n * EB2 + k) * NV]);
+    }
+  } else {
+    __syncthreads();
+  }
+  // ---- face terms: the fluxes of the element's face points, then thread = (element, face, face node)
+  R* Fl = sm + L::Fl;                                                  // [NE][Nf][FS]
+  for (int t = threadIdx.x; t < ne * S::Nf; t += kThreads) {
+    const int e = t / S::Nf, pt = t % S::Nf;
+    int lf = 0;
+    while (lf + 1 < nlf && pt >= S::poff(lf + 1)) ++lf;
+    const FaceDev& fd = D.face[lf < S::ntri ? 0 : 1];
+    const double* src = fd.fluxI + ((size_t)fslot[e * nlf + lf] * S::nq(lf) + pt - S::poff(lf)) * NV;
+    R x[NV];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) x[v] = (R)src[v];
+    sts16<NV>(Fl + (e * S::Nf + pt) * L::FS, x);
+  }
+  __syncthreads();
+  R* Fp = sm + L::Fp;                                                  // [NE][Nj][FS]
+  for (int t = threadIdx.x; t < ne * S::Nj; t += kThreads) {
+    const int e = t / S::Nj, jt = t % S::Nj;
+    int lf = 0;
+    while (lf + 1 < nlf && jt >= S::joff(lf + 1)) ++lf;
+    const int ft = lf < S::ntri ? 0 : 1, nq = S::nq(lf), nfn = S::nfn(lf), j = jt - S::joff(lf);
+    const R* cB = static_cast<const R*>(X.cB[ft]) + (size_t)fcode[e * nlf + lf] * nq * nfn + j;
+    const R* fl = Fl + (e * S::Nf + S::poff(lf)) * L::FS;
+    R s[NV];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) s[v] = (R)0;
+#pragma unroll 4
+    for (int q = 0; q < nq; ++q) {
+      const R bt = __ldg(cB + q * nfn);
+      R x[NV];
+      lds16<NV>(fl + q * L::FS, x);
+#pragma unroll
+      for (int v = 0; v < NV; ++v) s[v] += bt * x[v];
+    }
+    const R sgn = (fslot[e * nlf + lf] & 1) == 0 ? (R)-1 : (R)1;
+#pragma unroll
+    for (int v = 0; v < NV; ++v) s[v] = sgn * s[v];
+    sts16<NV>(Fp + t * L::FS, s);
+  }
+  __syncthreads();
+  // ---- totals: chunk sums, then the faces in local order; thread = (element, node)
+  R* Tt = sm + L::Tt;                                                  // [NE][Np][FS]
+  {
+    const R* Pc = sm + L::Gs;
+    const int nc = W::one ? 1 : C;
+    for (int t = threadIdx.x; t < ne * Np; t += kThreads) {
+      const int e = t / Np, i = t % Np;
+      R s[NV];
+      if (volume_done) {
+        const double* Ri = B.Rinv + ((size_t)(e0 + e) * Np + i) * NV;
+#pragma unroll
+        for (int v = 0; v < NV; ++v) s[v] = (R)Ri[v];
+      } else {
+#pragma unroll
+        for (int v = 0; v < NV; ++v) s[v] = (R)0;
+        for (int c = 0; c < nc; ++c) {
+          R x[NV];
+          lds16<NV>(Pc + ((c * NE + e) * Np + i) * L::FS, x);
+#pragma unroll
+          for (int v = 0; v < NV; ++v) s[v] += x[v];
+        }
+      }
+#pragma unroll
+      for (int lf = 0; lf < nlf; ++lf) {
+        const int j = X.finv[lf < S::ntri ? 0 : 1][fcode[e * nlf + lf] * Np + i];
+        if (j < 0) continue;
+        R x[NV];
+        lds16<NV>(Fp + (e * S::Nj + S::joff(lf) + j) * L::FS, x);
+#pragma unroll
+        for (int v = 0; v < NV; ++v) s[v] += x[v];
+      }
+      sts16<NV>(Tt + t * L::FS, s);
+    }
+  }
+  __syncthreads();
+  // ---- M^-1 (symmetric: read by columns, one node per lane); the results go over the chunk sums
+  R* Rs = sm + L::Gs;                                                  // [NE][Np][NV]
+  for (int t = threadIdx.x; t < ne * Np; t += kThreads) {
+    const int e = t / Np, i = t % Np;
+    const bool aff = B.affine != nullptr && B.affine[e0 + e];
+    const R* Mi = (aff ? static_cast<const R*>(X.mref) : static_cast<const R*>(X.minv) + (size_t)(e0 + e) * Np * Np) + i;
+    const R ms = (R)(aff ? B.acoef[e0 + e] : 1.0);
+    R r[NV];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) r[v] = (R)0;
+#pragma unroll 8
+    for (int j = 0; j < Np; ++j) {
+      const R m = __ldg(Mi + j * Np);
+      R x[NV];
+      lds16<NV>(Tt + (e * Np + j) * L::FS, x);
+#pragma unroll
+      for (int v = 0; v < NV; ++v) r[v] += m * x[v];
+    }
+#pragma unroll
+    for (int v = 0; v < NV; ++v) Rs[t * NV + v] = ms * r[v];
+  }
+  __syncthreads();
+  // ---- stage update or outputs, along the elements' contiguous values
+  const size_t base = (size_t)e0 * Np * NV;
+  for (int t = threadIdx.x; t < ne * Np * NV; t += kThreads) {
+    const double rid = (double)Rs[t];
+    if (!A.stage) {
+      if (A.out_inv[b]) A.out_inv[b][base + t] = rid;
+      if (A.out_vis[b]) A.out_vis[b][base + t] = 0.0;
+    } else {
+      const double eul = Ug[t] + A.dt * rid;
+      if (A.out_vis[b]) A.out_vis[b][base + t] = 0.0;
+      if (A.euler[b]) A.euler[b][base + t] = eul;
+      A.dst[b][base + t] = A.alpha * A.base[b][base + t] + A.beta * eul;
+    }
+  }
+}
+
+struct UpdateGrid {
+  int cta0[DGB_MAX_BLOCKS + 1];
+  bool volume_done[DGB_MAX_BLOCKS];
+};
+
+template <int P, int NV, typename R>
+__global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 5 : 3)
+    k_dense_update(const __grid_constant__ DevPlan D, const StatePtrs St, const __grid_constant__ FinalizeArgs A,
+                   const __grid_constant__ DenseTables X, const UpdateGrid L) {
+  extern __shared__ __align__(16) unsigned char dyn_smem[];
+  R* sm = reinterpret_cast<R*>(dyn_smem);
+  int b = 0;
+  while (b + 1 < D.nblocks && (int)blockIdx.x >= L.cta0[b + 1]) ++b;
+  const int cta = blockIdx.x - L.cta0[b];
+  if (D.blk[b].type == 0) update_body<P, 0, NV, R>(D, St, A, X.b[b], b, cta, L.volume_done[b], sm);
+  else if (D.blk[b].type == 1) update_body<P, 1, NV, R>(D, St, A, X.b[b], b, cta, L.volume_done[b], sm);
+  else update_body<P, 2, NV, R>(D, St, A, X.b[b], b, cta, L.volume_done[b], sm);
+}
+
+// --------------------------------------------------------------------------------------- face kernel
+// One face type's CTA: kThreads / nq faces, one thread per face point.  The face's nodes on both
+// sides come from the element states into shared memory (minus the side's anchor, node 0).
+template <int P, int FT, int NV, typename R>
+__device__ __forceinline__ void faces_body(const DevPlan& D, const StatePtrs& St, const DenseTables& X, int cta,
+                                           bool store_traces, R* sm) {
+  constexpr int nq = FT == 0 ? Shape<P, 1>::NQT : Shape<P, 1>::NQQ, nfn = FT == 0 ? Shape<P, 1>::TRI : Shape<P, 1>::QUAD;
+  constexpr int FPC = kThreads / nq, FS = round_up(NV, 16 / (int)sizeof(R));
+  __shared__ double anc[FPC * 2 * NV];
+  const FaceDev& fd = D.face[FT];
+  const int f0 = cta * FPC, nf = fd.F - f0 < FPC ? fd.F - f0 : FPC;
+  for (int t = threadIdx.x; t < nf * 2 * nfn; t += kThreads) {
+    const int side = (t / nfn) & 1, f = f0 + t / (2 * nfn), j = t % nfn;
+    const int blk = side ? fd.nb[f] : fd.ob[f];
+    if (blk < 0) continue;
+    const int el = side ? fd.nl[f] : fd.ol[f], code = side ? fd.nc[f] : fd.oc[f];
+    const double* u = St.b[blk] + (size_t)el * D.blk[blk].Np * NV;
+    const double* un = u + (int)X.b[blk].fnode[FT][code * nfn + j] * NV;
+    R x[NV];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+      const double a = u[v];
+      if (j == 0) anc[(t / nfn) * NV + v] = a;
+      x[v] = (R)(un[v] - a);
+    }
+    sts16<NV>(sm + t * FS, x);
+  }
+  __syncthreads();
+  const int slot = threadIdx.x / nq, q = threadIdx.x % nq;
+  const int f = f0 + slot;
+  if (slot >= nf) return;
+  const int nb = fd.nb[f];
+  auto trace = [&](int side, int blk, int code, double* out) {
+    const R* cBt = static_cast<const R*>(X.b[blk].cBt[FT]) + (size_t)code * nfn * nq + q;
+    const R* row = sm + (slot * 2 + side) * nfn * FS;
+    R acc[NV];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) acc[v] = (R)0;
+#pragma unroll
+    for (int j = 0; j < nfn; ++j) {
+      const R bt = __ldg(cBt + j * nq);
+      R x[NV];
+      lds16<NV>(row + j * FS, x);
+#pragma unroll
+      for (int v = 0; v < NV; ++v) acc[v] += bt * x[v];
+    }
+#pragma unroll
+    for (int v = 0; v < NV; ++v) out[v] = anc[(slot * 2 + side) * NV + v] + (double)acc[v];
+  };
+  const double* np_ = fd.n + ((size_t)f * nq + q) * 3;
+  const double n[3] = {np_[0], np_[1], np_[2]};
+  const double w = fd.w[(size_t)f * nq + q];
+  const size_t so = ((size_t)f * 2 + 0) * nq + q, sn = ((size_t)f * 2 + 1) * nq + q;
+  double UL[NV], UR[NV], Fh[NV], Fa[NV];
+  trace(0, fd.ob[f], fd.oc[f], UL);
+  if (nb >= 0) {
+    trace(1, nb, fd.nc[f], UR);
+  } else if (D.ph.has_boundary) {
+    ghost_state<NV>(D.ph, case_view(D.ph, D.blk[fd.ob[f]].ecase, fd.ol[f]).far, UL, n, fd.tag[f], UR);
+  } else {
+#pragma unroll
+    for (int v = 0; v < NV; ++v) UR[v] = UL[v];
+  }
+  if (store_traces) {
+#pragma unroll
+    for (int v = 0; v < NV; ++v) fd.trA[so * NV + v] = UL[v];
+    if (nb >= 0)
+#pragma unroll
+      for (int v = 0; v < NV; ++v) fd.trA[sn * NV + v] = UR[v];
+  }
+  hllc<NV>(D.ph, UL, UR, n, Fh);
+#pragma unroll
+  for (int side = 0; side < 2; ++side) {
+    if (side == 1 && nb < 0) break;
+    double a[NV];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) a[v] = anc[(slot * 2 + side) * NV + v];
+    normal_flux<NV>(D.ph, a, n, Fa);
+    double* out = fd.fluxI + (side ? sn : so) * NV;
+#pragma unroll
+    for (int v = 0; v < NV; ++v) out[v] = (Fh[v] - Fa[v]) * w;
+  }
+}
+
+template <int P, typename R, int NV>
+__host__ __device__ constexpr int faces_smem() {
+  constexpr int FS = round_up(NV, 16 / (int)sizeof(R));
+  constexpr int t = kThreads / Shape<P, 1>::NQT * 2 * Shape<P, 1>::TRI * FS;
+  constexpr int q = kThreads / Shape<P, 1>::NQQ * 2 * Shape<P, 1>::QUAD * FS;
+  return t > q ? t : q;
+}
+
+template <int P, int NV, typename R>
+__global__ void __launch_bounds__(kThreads, 4)
+    k_dense_faces(const __grid_constant__ DevPlan D, const StatePtrs St, const __grid_constant__ DenseTables X,
+                  int tri_ctas, bool store_traces) {
+  __shared__ __align__(16) R sm[faces_smem<P, R, NV>()];
+  if ((int)blockIdx.x < tri_ctas) faces_body<P, 0, NV, R>(D, St, X, blockIdx.x, store_traces, sm);
+  else faces_body<P, 1, NV, R>(D, St, X, blockIdx.x - tri_ctas, store_traces, sm);
+}
+
+// -------------------------------------------------------------------------------------------- launch
+template <int P, int NV, typename R>
+cudaError_t launch_faces(const DevPlan& D, const StatePtrs& S, const DenseTables& T, bool store_traces, cudaStream_t st) {
+  constexpr int ft = kThreads / Shape<P, 1>::NQT, fq = kThreads / Shape<P, 1>::NQQ;
+  const int tri = (D.face[0].F + ft - 1) / ft, quad = (D.face[1].F + fq - 1) / fq;
+  if (tri + quad > 0) k_dense_faces<P, NV, R><<<tri + quad, kThreads, 0, st>>>(D, S, T, tri, store_traces);
+  return cudaGetLastError();
+}
+
+template <int P, int NV, typename R>
+cudaError_t launch_update(const DevPlan& D, const StatePtrs& S, const FinalizeArgs& A, const DenseTables& T,
+                          const bool* volume_done, cudaStream_t st) {
+  UpdateGrid L;
+  L.cta0[0] = 0;
+  size_t smem = 0;
+  for (int b = 0; b < D.nblocks; ++b) {
+    const int type = D.blk[b].type;
+    const int ne = type == 0 ? Split<P, 0>::NE : type == 1 ? Split<P, 1>::NE : Split<P, 2>::NE;
+    const size_t need = sizeof(R) * (size_t)(type == 0   ? Smem<P, 0, NV, R>::total
+                                             : type == 1 ? Smem<P, 1, NV, R>::total
+                                                         : Smem<P, 2, NV, R>::total);
+    smem = need > smem ? need : smem;
+    L.cta0[b + 1] = L.cta0[b] + (D.blk[b].E + ne - 1) / ne;
+    L.volume_done[b] = volume_done != nullptr && volume_done[b];
+  }
+  if (L.cta0[D.nblocks] == 0) return cudaSuccess;
+  if (smem > 24 * 1024) {                    // the kernel has static shared memory too
+    const cudaError_t e = cudaFuncSetAttribute(k_dense_update<P, NV, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+  }
+  k_dense_update<P, NV, R><<<L.cta0[D.nblocks], kThreads, smem, st>>>(D, S, A, T, L);
+  return cudaGetLastError();
+}
+
+template <int P>
+DenseShape shape_of(int type) {
+  auto make = [](auto s) {
+    using S = decltype(s);
+    return DenseShape{S::Np, S::Nq, S::nlf, {S::NQT, S::NQQ}, {S::TRI, S::QUAD}};
+  };
+  return type == 0 ? make(Shape<P, 0>()) : type == 1 ? make(Shape<P, 1>()) : make(Shape<P, 2>());
+}
+
+}  // namespace
+
+DenseShape dense_shape(int P, int type) {
+  return P == 1 ? shape_of<1>(type) : P == 2 ? shape_of<2>(type) : shape_of<3>(type);
+}
+
+#define DGB_DENSE_DISPATCH(CALL)                                                                       \
+  if (D.nv == 5) {                                                                                     \
+    if (f32) return D.degree == 1 ? CALL(1, 5, float) : D.degree == 2 ? CALL(2, 5, float) : CALL(3, 5, float);     \
+    return D.degree == 1 ? CALL(1, 5, double) : D.degree == 2 ? CALL(2, 5, double) : CALL(3, 5, double);           \
+  }                                                                                                    \
+  return cudaErrorInvalidValue
+
+cudaError_t dense_face_flux(const DevPlan& D, const StatePtrs& S, const DenseTables& T, bool f32, bool store_traces,
+                            cudaStream_t st) {
+#define DGB_CALL(P, NV, R) (launch_faces<P, NV, R>(D, S, T, store_traces, st))
+  DGB_DENSE_DISPATCH(DGB_CALL);
+#undef DGB_CALL
+}
+
+cudaError_t dense_update(const DevPlan& D, const StatePtrs& S, const FinalizeArgs& A, const DenseTables& T, bool f32,
+                         const bool* volume_done, cudaStream_t st) {
+#define DGB_CALL(P, NV, R) (launch_update<P, NV, R>(D, S, A, T, volume_done, st))
+  DGB_DENSE_DISPATCH(DGB_CALL);
+#undef DGB_CALL
+}
+
+}  // namespace dgb
