@@ -1243,6 +1243,13 @@ int dgb_plan_set_faces(dgb_plan* p, const dgb_face_desc* d) {
   if ((rc = upload(p, d->normals, n * nq * 3, &F.n))) return rc;
   if ((rc = upload(p, d->weights, n * nq, &F.w))) return rc;
   if ((rc = upload(p, d->side_inv_jacobian, n * 2 * nq * 9, &F.jinv))) return rc;
+  // the two sides of each face in one record (dense_rhs.cu)
+  std::vector<int3> side(2 * n);
+  for (size_t f = 0; f < n; ++f) {
+    side[2 * f] = make_int3(d->owner_block[f], d->owner_local[f], d->owner_code[f]);
+    side[2 * f + 1] = make_int3(d->nbr_block[f], d->nbr_local[f], d->nbr_code[f]);
+  }
+  if ((rc = upload(p, side.data(), side.size(), &p->dense.side[d->face_type]))) return rc;
   p->face_present[d->face_type] = n > 0;
   return DGB_OK;
 }

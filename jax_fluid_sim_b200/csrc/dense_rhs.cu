@@ -66,15 +66,20 @@ struct Smem {
   // lane) fall on distinct banks
   static constexpr int GQ0 = W::EB / W::EB2 * GP, GQ = (GQ0 / VA) % 2 ? GQ0 : GQ0 + VA;
   static constexpr int GG0 = S::Nq * GQ, GG = (GG0 / VA) % 2 ? GG0 : GG0 + VA;
-  static constexpr int U = 0, Gs = U + W::NE / W::EB * UG;
+  // at the front: anchors (double), their fluxes, and two ints per (element, face)
+  static constexpr int AN = W::NE * NV * (8 / (int)sizeof(R)), FA = W::NE * 3 * NV;
+  static constexpr int FI = (2 * W::NE * S::nlf * 4 + (int)sizeof(R) - 1) / (int)sizeof(R);
+  static constexpr int U = round_up(AN + FA + FI, VA), Gs = U + W::NE / W::EB * UG;
   static constexpr int G = W::NE / W::EB * GG;
   // over G once it is dead: chunk sums, fluxes, face sums, totals, results
   static constexpr int FS = round_up(NV, VA);                          // one row of NV values
   static constexpr int chunk_max = kThreads / S::Np > 0 ? kThreads / S::Np : 1;
   static constexpr int Pc = W::one ? W::NE * S::Np * FS : chunk_max * W::NE * S::Np * FS;
   static constexpr int Fl = Gs + round_up(Pc, VA), Fp = Fl + W::NE * S::Nf * FS;
-  static constexpr int Tt = Fl;                                        // the fluxes are dead by then
-  static constexpr int End = Fp + W::NE * S::Nj * FS;
+  // totals: over the fluxes, which are dead by then, except at P1 (in the chunk sums' place: each
+  // thread reads its own sums before it writes its total)
+  static constexpr int Tt = W::one ? Gs : Fl;
+  static constexpr int End = Fp + (W::one ? 0 : W::NE * S::Nj * FS);   // P1: no face sums
   static_assert(S::Np <= S::Nf, "the totals take the fluxes' place");
   static constexpr int total = Gs + G > End ? Gs + G : End;
 };
@@ -122,19 +127,25 @@ __device__ __forceinline__ void update_body(const DevPlan& D, const StatePtrs& S
   using W = Split<P, T>;
   using L = Smem<P, T, NV, R>;
   constexpr int Np = S::Np, Nq = S::Nq, nlf = S::nlf, NE = W::NE, EB = W::EB, EB2 = W::EB2, IB = W::IB;
-  __shared__ int fslot[NE * nlf], fcode[NE * nlf];
-  __shared__ double anchor[NE * NV];
-  __shared__ R Fanc[NE * 3 * NV];                                      // flux of the anchor states
+  double* anchor = reinterpret_cast<double*>(sm);
+  R* Fanc = sm + L::AN;                                                // flux of the anchor states
+  int* fslot = reinterpret_cast<int*>(Fanc + L::FA);
+  int* fcode = fslot + NE * nlf;
   const BlockDev& B = D.blk[b];
   const int e0 = cta * NE, ne = B.E - e0 < NE ? B.E - e0 : NE;     // elements of this CTA
   const double* Ug = St.b[b] + (size_t)e0 * Np * NV;
   const int C = X.chunks;
-  for (int t = threadIdx.x; t < ne * nlf; t += kThreads) {
-    int ft, f, side;
-    decode_face(B.elem_face[(size_t)(e0 + t / nlf) * nlf + t % nlf], ft, f, side);
-    fslot[t] = (f << 1) | side;
-    fcode[t] = side == 0 ? D.face[ft].oc[f] : D.face[ft].nc[f];
-  }
+  // every load of a phase is issued before its first use: at three CTAs per SM a loop of dependent
+  // load and store pairs waits out each latency in turn
+  auto faces = [&]() {
+    for (int t = threadIdx.x; t < ne * nlf; t += kThreads) {
+      int ft, f, side;
+      decode_face(B.elem_face[(size_t)e0 * nlf + t], ft, f, side);
+      fslot[t] = (f << 1) | side;
+      fcode[t] = side == 0 ? D.face[ft].oc[f] : D.face[ft].nc[f];
+    }
+  };
+  constexpr int VALS = NE * Np * NV, VR = (VALS + kThreads - 1) / kThreads;
   if (!volume_done) {
     for (int t = threadIdx.x; t < NE * NV; t += kThreads)
       anchor[t] = t / NV < ne ? Ug[(size_t)(t / NV) * Np * NV + t % NV] : 1.0;
@@ -142,11 +153,18 @@ __device__ __forceinline__ void update_body(const DevPlan& D, const StatePtrs& S
     R* G = sm + L::Gs;
     // U minus the anchor; the slots past the last element hold zeros (and unit anchors), so that their
     // points stay finite
-    for (int t = threadIdx.x; t < NE * Np * NV; t += kThreads) {
+    R x[VR];
+#pragma unroll
+    for (int k = 0; k < VR; ++k) {
+      const int t = k * kThreads + threadIdx.x, e = t / (Np * NV);
+      x[k] = t < VALS && e < ne ? (R)(Ug[t] - Ug[(size_t)e * Np * NV + t % NV]) : (R)0;
+    }
+    faces();
+#pragma unroll
+    for (int k = 0; k < VR; ++k) {
+      const int t = k * kThreads + threadIdx.x;
       const int e = t / (Np * NV), i = (t / NV) % Np, v = t % NV;
-      R x = (R)0;
-      if (e < ne) x = (R)(Ug[t] - Ug[(size_t)e * Np * NV + v]);
-      U[(e / EB) * L::UG + i * L::UE + (e % EB) * NV + v] = x;
+      if (t < VALS) U[(e / EB) * L::UG + i * L::UE + (e % EB) * NV + v] = x[k];
     }
     __syncthreads();
     for (int t = threadIdx.x; t < NE * 3; t += kThreads) {
@@ -231,21 +249,35 @@ __device__ __forceinline__ void update_body(const DevPlan& D, const StatePtrs& S
         R s[IB * EB2 * NV];
 #pragma unroll
         for (int k = 0; k < IB * EB2 * NV; ++k) s[k] = (R)0;
+        // the next point's table values are loaded before this point's products: they come from L2 (a
+        // block's dBi is 12 to 192 KB), whose latency the few warps do not cover by themselves
+        R g[3 * IB];
+        const R* gd = dBi + q0 * 3 * Np + i;
+#pragma unroll
+        for (int m = 0; m < 3 * IB; ++m) g[m] = __ldg(gd + m / IB * Np + m % IB);
 #pragma unroll 1
         for (int q = q0; q < q1; ++q) {
-          R g0[IB], g1[IB], g2[IB];
+          R gn[3 * IB];
+          gd += q + 1 < q1 ? 3 * Np : 0;
 #pragma unroll
-          for (int n = 0; n < IB; ++n) {
-            const R* gd = dBi + q * 3 * Np + i + n;
-            g0[n] = __ldg(gd), g1[n] = __ldg(gd + Np), g2[n] = __ldg(gd + 2 * Np);
-          }
+          for (int m = 0; m < 3 * IB; ++m) gn[m] = __ldg(gd + m / IB * Np + m % IB);
           R x[EB2 * 3 * NV];
           lds16<EB2 * 3 * NV>(Gr + q * L::GQ, x);
 #pragma unroll
           for (int n = 0; n < IB; ++n)
 #pragma unroll
-            for (int k = 0; k < EB2 * NV; ++k)
-              s[n * EB2 * NV + k] += g0[n] * x[k] + g1[n] * x[EB2 * NV + k] + g2[n] * x[2 * EB2 * NV + k];
+            for (int k = 0; k < EB2 * NV; ++k) {
+              R& acc = s[n * EB2 * NV + k];
+              if constexpr (sizeof(R) == sizeof(double)) {
+                acc += g[n] * x[k];
+                acc += g[IB + n] * x[EB2 * NV + k];
+                acc += g[2 * IB + n] * x[2 * EB2 * NV + k];
+              } else {
+                acc += g[n] * x[k] + g[IB + n] * x[EB2 * NV + k] + g[2 * IB + n] * x[2 * EB2 * NV + k];
+              }
+            }
+#pragma unroll
+          for (int m = 0; m < 3 * IB; ++m) g[m] = gn[m];
         }
 #pragma unroll
         for (int k = 0; k < IB * EB2 * NV; ++k) sum[rd][k] += s[k];
@@ -265,31 +297,43 @@ __device__ __forceinline__ void update_body(const DevPlan& D, const StatePtrs& S
           sts16<NV>(Pc + ((c0 * NE + ep * EB2 + k) * Np + i + n) * L::FS, &sum[rd][(n * EB2 + k) * NV]);
     }
   } else {
+    faces();
     __syncthreads();
   }
   // ---- face terms: the fluxes of the element's face points, then thread = (element, face, face node)
   R* Fl = sm + L::Fl;                                                  // [NE][Nf][FS]
-  for (int t = threadIdx.x; t < ne * S::Nf; t += kThreads) {
-    const int e = t / S::Nf, pt = t % S::Nf;
-    int lf = 0;
-    while (lf + 1 < nlf && pt >= S::poff(lf + 1)) ++lf;
-    const FaceDev& fd = D.face[lf < S::ntri ? 0 : 1];
-    const double* src = fd.fluxI + ((size_t)fslot[e * nlf + lf] * S::nq(lf) + pt - S::poff(lf)) * NV;
-    R x[NV];
+  {
+    constexpr int FR = (NE * S::Nf + kThreads - 1) / kThreads;
+    double x[FR][NV];
 #pragma unroll
-    for (int v = 0; v < NV; ++v) x[v] = (R)src[v];
-    sts16<NV>(Fl + (e * S::Nf + pt) * L::FS, x);
+    for (int k = 0; k < FR; ++k) {
+      const int t = k * kThreads + threadIdx.x, e = t / S::Nf, pt = t % S::Nf;
+      if (t >= ne * S::Nf) continue;
+      int lf = 0;
+#pragma unroll
+      for (int m = 1; m < nlf; ++m) lf += pt >= S::poff(m);
+      const FaceDev& fd = D.face[lf < S::ntri ? 0 : 1];
+      const double* src = fd.fluxI + ((size_t)fslot[e * nlf + lf] * S::nq(lf) + pt - S::poff(lf)) * NV;
+#pragma unroll
+      for (int v = 0; v < NV; ++v) x[k][v] = src[v];
+    }
+#pragma unroll
+    for (int k = 0; k < FR; ++k) {
+      const int t = k * kThreads + threadIdx.x;
+      if (t >= ne * S::Nf) continue;
+      R y[NV];
+#pragma unroll
+      for (int v = 0; v < NV; ++v) y[v] = (R)x[k][v];
+      sts16<NV>(Fl + t * L::FS, y);
+    }
   }
   __syncthreads();
   R* Fp = sm + L::Fp;                                                  // [NE][Nj][FS]
-  for (int t = threadIdx.x; t < ne * S::Nj; t += kThreads) {
-    const int e = t / S::Nj, jt = t % S::Nj;
-    int lf = 0;
-    while (lf + 1 < nlf && jt >= S::joff(lf + 1)) ++lf;
-    const int ft = lf < S::ntri ? 0 : 1, nq = S::nq(lf), nfn = S::nfn(lf), j = jt - S::joff(lf);
+  // face lf's contribution to its node j: the points in order, then the side's sign
+  auto face_sum = [&](int e, int lf, int j, R* s) {
+    const int ft = lf < S::ntri ? 0 : 1, nq = S::nq(lf), nfn = S::nfn(lf);
     const R* cB = static_cast<const R*>(X.cB[ft]) + (size_t)fcode[e * nlf + lf] * nq * nfn + j;
     const R* fl = Fl + (e * S::Nf + S::poff(lf)) * L::FS;
-    R s[NV];
 #pragma unroll
     for (int v = 0; v < NV; ++v) s[v] = (R)0;
 #pragma unroll 4
@@ -303,9 +347,19 @@ __device__ __forceinline__ void update_body(const DevPlan& D, const StatePtrs& S
     const R sgn = (fslot[e * nlf + lf] & 1) == 0 ? (R)-1 : (R)1;
 #pragma unroll
     for (int v = 0; v < NV; ++v) s[v] = sgn * s[v];
-    sts16<NV>(Fp + t * L::FS, s);
+  };
+  if constexpr (!W::one) {             // P1 sums a node's faces in the totals pass (three faces a node)
+    for (int t = threadIdx.x; t < ne * S::Nj; t += kThreads) {
+      const int e = t / S::Nj, jt = t % S::Nj;
+      int lf = 0;
+#pragma unroll
+      for (int m = 1; m < nlf; ++m) lf += jt >= S::joff(m);
+      R s[NV];
+      face_sum(e, lf, jt - S::joff(lf), s);
+      sts16<NV>(Fp + t * L::FS, s);
+    }
+    __syncthreads();
   }
-  __syncthreads();
   // ---- totals: chunk sums, then the faces in local order; thread = (element, node)
   R* Tt = sm + L::Tt;                                                  // [NE][Np][FS]
   {
@@ -333,7 +387,8 @@ __device__ __forceinline__ void update_body(const DevPlan& D, const StatePtrs& S
         const int j = X.finv[lf < S::ntri ? 0 : 1][fcode[e * nlf + lf] * Np + i];
         if (j < 0) continue;
         R x[NV];
-        lds16<NV>(Fp + (e * S::Nj + S::joff(lf) + j) * L::FS, x);
+        if constexpr (W::one) face_sum(e, lf, j, x);
+        else lds16<NV>(Fp + (e * S::Nj + S::joff(lf) + j) * L::FS, x);
 #pragma unroll
         for (int v = 0; v < NV; ++v) s[v] += x[v];
       }
@@ -342,7 +397,7 @@ __device__ __forceinline__ void update_body(const DevPlan& D, const StatePtrs& S
   }
   __syncthreads();
   // ---- M^-1 (symmetric: read by columns, one node per lane); the results go over the chunk sums
-  R* Rs = sm + L::Gs;                                                  // [NE][Np][NV]
+  R* Rs = sm + (W::one ? L::Fl : L::Gs);                               // [NE][Np][NV]
   for (int t = threadIdx.x; t < ne * Np; t += kThreads) {
     const int e = t / Np, i = t % Np;
     const bool aff = B.affine != nullptr && B.affine[e0 + e];
@@ -365,16 +420,31 @@ __device__ __forceinline__ void update_body(const DevPlan& D, const StatePtrs& S
   __syncthreads();
   // ---- stage update or outputs, along the elements' contiguous values
   const size_t base = (size_t)e0 * Np * NV;
-  for (int t = threadIdx.x; t < ne * Np * NV; t += kThreads) {
-    const double rid = (double)Rs[t];
-    if (!A.stage) {
-      if (A.out_inv[b]) A.out_inv[b][base + t] = rid;
+  const int vals = ne * Np * NV;
+  if (!A.stage) {
+    for (int t = threadIdx.x; t < vals; t += kThreads) {
+      if (A.out_inv[b]) A.out_inv[b][base + t] = (double)Rs[t];
       if (A.out_vis[b]) A.out_vis[b][base + t] = 0.0;
-    } else {
-      const double eul = Ug[t] + A.dt * rid;
+    }
+    return;
+  }
+  double u[VR], w[VR];
+#pragma unroll
+  for (int k = 0; k < VR; ++k) {
+    const int t = k * kThreads + threadIdx.x;
+    if (t < vals) {
+      u[k] = Ug[t];
+      w[k] = A.base[b][base + t];
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < VR; ++k) {
+    const int t = k * kThreads + threadIdx.x;
+    if (t < vals) {
+      const double eul = u[k] + A.dt * (double)Rs[t];
       if (A.out_vis[b]) A.out_vis[b][base + t] = 0.0;
       if (A.euler[b]) A.euler[b][base + t] = eul;
-      A.dst[b][base + t] = A.alpha * A.base[b][base + t] + A.beta * eul;
+      A.dst[b][base + t] = A.alpha * w[k] + A.beta * eul;
     }
   }
 }
@@ -385,7 +455,7 @@ struct UpdateGrid {
 };
 
 template <int P, int NV, typename R>
-__global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 5 : 3)
+__global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) || P == 1 ? 5 : 3)
     k_dense_update(const __grid_constant__ DevPlan D, const StatePtrs St, const __grid_constant__ FinalizeArgs A,
                    const __grid_constant__ DenseTables X, const UpdateGrid L) {
   extern __shared__ __align__(16) unsigned char dyn_smem[];
@@ -410,11 +480,11 @@ __device__ __forceinline__ void faces_body(const DevPlan& D, const StatePtrs& St
   const FaceDev& fd = D.face[FT];
   const int f0 = cta * FPC, nf = fd.F - f0 < FPC ? fd.F - f0 : FPC;
   for (int t = threadIdx.x; t < nf * 2 * nfn; t += kThreads) {
-    const int side = (t / nfn) & 1, f = f0 + t / (2 * nfn), j = t % nfn;
-    const int blk = side ? fd.nb[f] : fd.ob[f];
+    const int j = t % nfn;
+    const int3 side = X.side[FT][f0 * 2 + t / nfn];
+    const int blk = side.x, code = side.z;
     if (blk < 0) continue;
-    const int el = side ? fd.nl[f] : fd.ol[f], code = side ? fd.nc[f] : fd.oc[f];
-    const double* u = St.b[blk] + (size_t)el * D.blk[blk].Np * NV;
+    const double* u = St.b[blk] + (size_t)side.y * D.blk[blk].Np * NV;
     const double* un = u + (int)X.b[blk].fnode[FT][code * nfn + j] * NV;
     R x[NV];
 #pragma unroll

@@ -25,6 +25,7 @@ struct DenseBlock {
 struct DenseTables {
   bool ready;                // every block has the shapes and the face-node structure below
   DenseBlock b[DGB_MAX_BLOCKS];
+  const int3* side[2];       // per face type [F][2]: block (-1: none), element, trace code of each side
 };
 
 // Expected shapes of a block at degree P: 0 hexahedron, 1 wedge, 2 tetrahedron.
