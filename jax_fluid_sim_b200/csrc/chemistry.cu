@@ -15,13 +15,20 @@
 // analytically from the reaction structure, with JAX's convention at ties of max/clip
 // (the derivative is split evenly between the two arguments).
 //
-// Layout: the mechanism travels as one __grid_constant__ kernel parameter (about 12 KB),
-// so every warp-uniform table read is a constant-cache broadcast.  Per thread, the
-// augmented Newton matrix [I - dt J | -R] (ns x ns+1) and the species vectors that the
-// reaction loops index through the stoichiometry lists live in shared memory with a
-// stride of one thread, so a warp's accesses fall in distinct banks.  The net rates
-// accumulate in the matrix's last column.  At 176 doubles a node, a CTA of one warp takes
-// 45 KB, and five CTAs share an SM.
+// Layout of the advance (k_react): four lanes per node, eight nodes per warp.  The Newton matrix and
+// its right-hand side stay in registers, up to three rows a lane; a twelfth row of the same kind
+// holds the mass-weighted sum over the species, which the mass-conserving correction needs.  Each
+// lane evaluates every fourth reaction and writes that reaction's row [dq/drho_j | q] to shared
+// memory, kPass reactions at a time; a lane then adds to its rows the reactions that they take part
+// in (host-built lists, the longest rows of the four lanes side by side).  Elimination is by lanes,
+// the pivot row going round by shuffles.  With a thread per node, the matrix in shared memory let five
+// warps share an SM and every addition to it waited out a shared-memory round trip; now twelve warps do
+// and the chains are register arithmetic: 54,000 nodes of 12 iterations took 4.7 ms before and
+// take @NOW@ ms.
+//
+// The rates alone (k_rates) take one thread per sample: the mechanism is one __grid_constant__ kernel
+// parameter, and the matrix and the species vectors that the reaction loops index live in shared memory
+// with a stride of one thread.
 //
 // Work saved against a literal evaluation, each with the same result up to rounding:
 //  - a reaction whose stoichiometric coefficients are all whole numbers up to 3 forms
@@ -29,12 +36,20 @@
 //    applied to the product);
 //  - the temperature inversion stops once an update moves T by at most 1e-13 T: Newton on
 //    e(T) converges quadratically, so the remaining iterations of the fixed count change T
-//    only in its last bits.
+//    only in its last bits;
+//  - a node keeps its state once a Newton iteration has moved no density by more than two units in the
+//    last place and T by at most 1e-13 T: further iterations of the fixed count could only repeat
+//    that.  A warp stops when its eight nodes have.  Nodes whose iterations have not settled to
+//    rounding run the whole count;
+//  - with one temperature (T_v = T) the three controlling temperatures of a reaction, floored at 10 K,
+//    are the same number (sqrt(T T) is T in binary floating point).
 #include <cuda_runtime.h>
 #include <math.h>
 #include <string.h>
 
+#include <algorithm>
 #include <string>
+#include <vector>
 
 #include "dgb200.h"
 
@@ -52,6 +67,11 @@ constexpr double kExpLo = 9.8597628436862264e-305, kExpHi = 1.0142320547350045e3
 // the temperature inversion's convergence test (relative step)
 constexpr double kTStop = 1.0e-13;
 constexpr double kRUniv = 8.31446261815324, kPStd = 101325.0;
+// k_react: lanes per node, CTA size, reactions per pass, rows
+constexpr int kLanes = 4, kReactThreads = 128, kPass = 8, kRows = 12;
+constexpr int kPasses = (DGB_CHEM_MAX_REACTIONS + kPass - 1) / kPass;
+// a Newton update below this share of a density is rounding
+constexpr double kSettled = 4.5e-16;
 
 struct Reaction {
   double A, b, theta, dn;                 // Arrhenius; sum of net stoichiometry
@@ -75,6 +95,12 @@ struct Tables {
   double s[DGB_CHEM_MAX_SPECIES][2][6];       // a0, a1, a2/2, a3/3, a4/4, a6
   double alpha[DGB_CHEM_MAX_REACTIONS][DGB_CHEM_MAX_SPECIES];
   Reaction rx[DGB_CHEM_MAX_REACTIONS];
+  // k_react: species of row slot * 4 + lane (-1: none, ns: the mass-weighted sum), and per pass of
+  // kPass reactions the row's entries [ptr, ptr of the next row): reaction in the pass, weight
+  int row_of[kRows];
+  int list_ptr[kPasses * kRows + 1];
+  short list_rx[DGB_CHEM_MAX_REACTIONS * (kMaxList + 1)];
+  double list_w[DGB_CHEM_MAX_REACTIONS * (kMaxList + 1)];
   // coupler (coupling.py:26-71)
   int iters, dimensionless;
   double T_ref, rho_ref, e_ref, t_ref, gamma;
@@ -96,8 +122,7 @@ struct Slots {
   __device__ double& C(int q) const { return base[(NS * (NS + 1) + q) * stride]; }     // max(C, 1e-100)
   __device__ double& dlog(int q) const { return base[(NS * (NS + 2) + q) * stride]; }
   __device__ double& g(int q) const { return base[(NS * (NS + 3) + q) * stride]; }
-  __device__ double& r0(int q) const { return base[(NS * (NS + 4) + q) * stride]; }    // Newton's rho0
-  static constexpr int kDoubles = NS * (NS + 5);
+  static constexpr int kDoubles = NS * (NS + 4);
 };
 
 // Temperature powers shared by every species at one temperature T: ln T and 1/T.  A species
@@ -119,22 +144,6 @@ __device__ __forceinline__ int nasa_range(const Tables& M, int q, const TPow& t,
   return Tc < M.trange[q][1] ? 0 : 1;
 }
 
-__device__ __forceinline__ double h_RT(const Tables& M, int q, const TPow& t) {
-  double Tc, lnTc, invTc;
-  const int r = nasa_range(M, q, t, Tc, lnTc, invTc);
-  const double* a = M.h[q][r];
-  const double T2 = Tc * Tc;
-  return a[0] + a[1] * Tc + a[2] * T2 + a[3] * (T2 * Tc) + a[4] * (T2 * T2) + a[5] * invTc;
-}
-
-__device__ __forceinline__ double cp_R(const Tables& M, int q, const TPow& t) {
-  double Tc, lnTc, invTc;
-  const int r = nasa_range(M, q, t, Tc, lnTc, invTc);
-  const double* a = M.cp[q][r];
-  const double T2 = Tc * Tc;
-  return a[0] + a[1] * Tc + a[2] * T2 + a[3] * (T2 * Tc) + a[4] * (T2 * T2);
-}
-
 __device__ __forceinline__ double g_RT(const Tables& M, int q, const TPow& t) {
   double Tc, lnTc, invTc;
   const int r = nasa_range(M, q, t, Tc, lnTc, invTc);
@@ -150,49 +159,6 @@ __device__ __forceinline__ double g_RT(const Tables& M, int q, const TPow& t) {
 __device__ __forceinline__ double select_T(int mode, double T, double Tv) {
   if (mode == 1) return sqrt(jmax(T * Tv, 1.0));
   return mode == 2 ? Tv : T;
-}
-
-// mixture_properties()["internal_energy"], mechanism.py:222-260
-template <int NS>
-__device__ double internal_energy(const Tables& M, const double (&rho)[NS], double T) {
-  double S = 0.0;
-#pragma unroll
-  for (int q = 0; q < NS; ++q) S += rho[q];
-  S = jmax(S, 1.0e-14);
-  const TPow t{T, 0.0, 1.0 / T};     // the energy fits need no logarithm
-  double e = 0.0;
-#pragma unroll
-  for (int q = 0; q < NS; ++q) e += (jmax(rho[q], 0.0) / S) * ((h_RT(M, q, t) - 1.0) * (T * M.RW[q]));
-  return e;
-}
-
-// recover_temperature_from_energy, mechanism.py:262-287
-template <int NS>
-__device__ double recover_T(const Tables& M, const double (&rho)[NS], double target, double T, int iters) {
-  double S = 0.0;
-#pragma unroll
-  for (int q = 0; q < NS; ++q) S += rho[q];
-  S = jmax(S, 1.0e-14);
-  double Y[NS];
-#pragma unroll
-  for (int q = 0; q < NS; ++q) Y[q] = jmax(rho[q], 0.0) / S;
-  for (int it = 0; it < iters; ++it) {
-    const double Ts = jclip(T, 50.0, 50000.0);
-    // 1/Ts is the only temperature power the energy fits need (no logarithm)
-    const TPow t{Ts, 0.0, 1.0 / Ts};
-    double e = 0.0, cv = 0.0;
-#pragma unroll
-    for (int q = 0; q < NS; ++q) {
-      e += Y[q] * ((h_RT(M, q, t) - 1.0) * (Ts * M.RW[q]));
-      cv += Y[q] * ((cp_R(M, q, t) - 1.0) * M.RW[q]);
-    }
-    const double dT = -(e - target) / jmax(cv, 1.0e-5);
-    const double Tn = jclip(T + jclip(dT, -0.5 * T, 0.5 * T), 100.0, 50000.0);
-    const bool done = fabs(Tn - T) <= kTStop * T;
-    T = Tn;
-    if (done) break;
-  }
-  return T;
 }
 
 // prod_k C[sp[k]]^pw[k] for whole exponents, clipped to [exp(-700), exp(700)] as the
@@ -300,11 +266,9 @@ __device__ void rates(const Tables& M, const Slots<NS>& sl, const double (&rho)[
 }
 
 // Mass-conserving correction (mechanism.py:214-218): w = W omega - Y sum(W omega) replaces
-// omega in sl.om, and its Jacobian J = dwd - dY sum(wd) - Y colsum(dwd) replaces sl.A
-// (newton: sl.A becomes [I - dt J | -res] with res = rho - rho0 - dt w).
+// omega in sl.om, and its Jacobian J = dwd - dY sum(wd) - Y colsum(dwd) replaces sl.A.
 template <int NS>
-__device__ void finish(const Tables& M, const Slots<NS>& sl, const double (&rho)[NS], double dt, bool jac,
-                       bool newton) {
+__device__ void finish(const Tables& M, const Slots<NS>& sl, const double (&rho)[NS], bool jac) {
   double Sraw = 0.0;
 #pragma unroll
   for (int q = 0; q < NS; ++q) Sraw += rho[q];
@@ -339,136 +303,384 @@ __device__ void finish(const Tables& M, const Slots<NS>& sl, const double (&rho)
 #pragma unroll
     for (int i = 0; i < NS; ++i) {
       const double dY = i == j ? dmax_tie(rho[i], 0.0) / S + dYo[i] : dYo[i];
-      const double J = sl.A(i, j) - dY * sw - Yr[i] * col;
-      sl.A(i, j) = newton ? (i == j ? 1.0 : 0.0) - dt * J : J;
+      sl.A(i, j) = sl.A(i, j) - dY * sw - Yr[i] * col;
     }
-  }
-  if (newton) {
-#pragma unroll
-    for (int i = 0; i < NS; ++i) sl.A(i, NS) = -(rho[i] - sl.r0(i) - dt * sl.om(i));
   }
 }
 
-// Solve [A | b] in place by LU with partial pivoting (the first largest |pivot|, as
-// LAPACK's getrf); x receives the solution.
+// ------------------------------------------------------------------------------------ point-implicit step
+// Node arrays in shared memory (doubles): the species vectors [C | dlog | c | dC | g], kRows each, then
+// kPass reaction rows.  The reaction rows and the nodes are an odd number of 16-byte units apart, so that
+// the lanes of a warp, which read rows of their own, spread over the banks.
+constexpr int kVec = 5 * kRows, kRxRow = kRows + 2;
+constexpr int kNodeDoubles = kVec + kPass * kRxRow + 2;
+static_assert((kNodeDoubles / 2) % 2 == 1 && (kRxRow / 2) % 2 == 1, "odd strides");
+
+__device__ __forceinline__ double quad_sum(double x) {
+  x += __shfl_xor_sync(0xffffffffu, x, 1);
+  x += __shfl_xor_sync(0xffffffffu, x, 2);
+  return x;
+}
+
+// NASA-7 fits of species q at T (lnT and 1/T given): the temperature clamped to the fit's range.
+__device__ __forceinline__ double species_energy(const Tables& M, int q, double T, double invT, double& cv) {
+  const TPow t{T, 0.0, invT};
+  double Tc, lnTc, invTc;
+  const int r = nasa_range(M, q, t, Tc, lnTc, invTc);
+  const double* a = M.h[q][r];
+  const double* c = M.cp[q][r];
+  const double T2 = Tc * Tc, T3 = T2 * Tc, T4 = T2 * T2;
+  const double h = a[0] + a[1] * Tc + a[2] * T2 + a[3] * T3 + a[4] * T4 + a[5] * invTc;
+  const double cp = c[0] + c[1] * Tc + c[2] * T2 + c[3] * T3 + c[4] * T4;
+  cv = (cp - 1.0) * M.RW[q];
+  return (h - 1.0) * (T * M.RW[q]);
+}
+
+// The species of each of a lane's rows (NS and above: none), as kept in registers.
+template <int SLOTS>
+struct RowSpecies {
+  int q[SLOTS];
+};
+
+// recover_temperature_from_energy, mechanism.py:262-287, the species spread over the node's lanes
+template <int NS, int SLOTS>
+__device__ double recover_T(const Tables& M, const RowSpecies<SLOTS>& row, const double (&rho)[SLOTS], double target,
+                            double T, int iters) {
+  double S = 0.0;
+#pragma unroll
+  for (int s = 0; s < SLOTS; ++s) S += row.q[s] < NS ? rho[s] : 0.0;
+  S = jmax(quad_sum(S), 1.0e-14);
+  double Y[SLOTS];
+#pragma unroll
+  for (int s = 0; s < SLOTS; ++s) Y[s] = row.q[s] < NS ? jmax(rho[s], 0.0) / S : 0.0;
+  bool done = false;
+  for (int it = 0; it < iters; ++it) {
+    const double Ts = jclip(T, 50.0, 50000.0);
+    const double invT = 1.0 / Ts;
+    double e = 0.0, cv = 0.0;
+#pragma unroll
+    for (int s = 0; s < SLOTS; ++s) {
+      double c;
+      const double es = species_energy(M, row.q[s] < NS ? row.q[s] : 0, Ts, invT, c);
+      e += Y[s] * es;
+      cv += Y[s] * c;
+    }
+    e = quad_sum(e);
+    cv = quad_sum(cv);
+    const double dT = -(e - target) / jmax(cv, 1.0e-5);
+    const double Tn = jclip(T + jclip(dT, -0.5 * T, 0.5 * T), 100.0, 50000.0);
+    const bool now = fabs(Tn - T) <= kTStop * T;
+    if (!done) T = Tn;
+    done = done || now;
+    if (__all_sync(0xffffffffu, done)) break;
+  }
+  return T;
+}
+
+// prod_k C[sp[k]]^pw[k] from the node's concentrations, clipped as mass_action above
+__device__ __forceinline__ double node_mass_action(const double* C, int n, const int* sp, const int* pw, double& ok) {
+  double v = 1.0;
+  for (int k = 0; k < n; ++k) {
+    const double c = C[sp[k]];
+    v *= pw[k] == 1 ? c : (pw[k] == 2 ? c * c : c * c * c);
+  }
+  ok = (v > kExpLo && v < kExpHi) ? 1.0 : ((v == kExpLo || v == kExpHi) ? 0.5 : 0.0);
+  return jclip(v, kExpLo, kExpHi);
+}
+
+// Reaction r's row [dq/drho_j | q] at the node's concentrations (the vectors of node) and temperature.
 template <int NS>
-__device__ void lu_solve(const Slots<NS>& sl, double (&x)[NS]) {
-#pragma unroll
-  for (int k = 0; k < NS; ++k) {
-    int p = k;
-    double amax = fabs(sl.A(k, k));
-#pragma unroll
-    for (int i = k + 1; i < NS; ++i) {
-      const double v = fabs(sl.A(i, k));
-      if (v > amax) {
-        amax = v;
-        p = i;
-      }
-    }
-    if (p != k) {
-#pragma unroll
-      for (int j = k; j <= NS; ++j) {
-        const double t = sl.A(k, j);
-        sl.A(k, j) = sl.A(p, j);
-        sl.A(p, j) = t;
-      }
-    }
-    const double rp = 1.0 / sl.A(k, k);
-#pragma unroll
-    for (int i = k + 1; i < NS; ++i) {
-      const double f = sl.A(i, k) * rp;
-#pragma unroll
-      for (int j = k + 1; j <= NS; ++j) sl.A(i, j) -= f * sl.A(k, j);
-    }
+__device__ __forceinline__ void reaction_row(const Tables& M, int r, const double* node, const TPow& tg, double base,
+                                             double* out) {
+  const double *C = node, *dlog = node + kRows, *cpos = node + 2 * kRows, *dC = node + 3 * kRows, *g = node + 4 * kRows;
+  const Reaction& R = M.rx[r];
+  const double kf = R.A * exp(R.b * tg.lnT - R.theta * tg.invT);
+  double dG = 0.0;
+  for (int k = 0; k < R.nd; ++k) dG += R.d_nu[k] * g[R.d_sp[k]];
+  const double conv = R.dn == 0.0 ? 1.0 : (R.dn == 1.0 ? base : (R.dn == -1.0 ? 1.0 / base : pow(base, R.dn)));
+  const double Kc = exp(-jclip(dG, -kClipExp, kClipExp)) * conv;
+  const double kr = kf / jmax(Kc, kMinKc);
+  double fwd, rev, okf, okr;
+  if (R.whole) {
+    fwd = node_mass_action(C, R.nf, R.f_sp, R.f_pw, okf);
+    rev = node_mass_action(C, R.nr, R.r_sp, R.r_pw, okr);
+  } else {
+    double lf = 0.0, lr = 0.0;
+    for (int k = 0; k < R.nf; ++k) lf += R.f_nu[k] * log(C[R.f_sp[k]]);
+    for (int k = 0; k < R.nr; ++k) lr += R.r_nu[k] * log(C[R.r_sp[k]]);
+    fwd = exp(jclip(lf, -kClipExp, kClipExp));
+    rev = exp(jclip(lr, -kClipExp, kClipExp));
+    okf = fabs(lf) < kClipExp ? 1.0 : (fabs(lf) == kClipExp ? 0.5 : 0.0);
+    okr = fabs(lr) < kClipExp ? 1.0 : (fabs(lr) == kClipExp ? 0.5 : 0.0);
   }
+  const double F = kf * fwd, B = kr * rev;
+  double coll = 1.0;
+  if (R.third) {
+    coll = 0.0;
 #pragma unroll
-  for (int i = NS - 1; i >= 0; --i) {
-    double acc = sl.A(i, NS);
+    for (int q = 0; q < NS; ++q) coll += M.alpha[r][q] * cpos[q];
+    const double qc = F - B;
 #pragma unroll
-    for (int j = i + 1; j < NS; ++j) acc -= sl.A(i, j) * x[j];
-    x[i] = acc / sl.A(i, i);
+    for (int q = 0; q < NS; ++q) out[q] = qc * M.alpha[r][q] * dC[q];
+  } else {
+#pragma unroll
+    for (int q = 0; q < NS; ++q) out[q] = 0.0;
   }
+  const double a = F * okf * coll, b = B * okr * coll;
+  for (int m = 0; m < R.nf; ++m) out[R.f_sp[m]] += a * R.f_nu[m] * dlog[R.f_sp[m]];
+  for (int m = 0; m < R.nr; ++m) out[R.r_sp[m]] -= b * R.r_nu[m] * dlog[R.r_sp[m]];
+  out[NS] = F * coll - B * coll;
 }
 
 // ReactingFlowCoupler._react_single_cell for every node of a block.
 template <int NS>
-__global__ void __launch_bounds__(kThreads) k_react(const __grid_constant__ Tables M, const double* U, double* out,
-                                                    long long nodes, int num_nodes, int nvars, double dt,
-                                                    const double* __restrict__ dt_elem) {
-  extern __shared__ double smem[];
-  const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= nodes) return;
-  const Slots<NS> sl{smem + threadIdx.x, (int)blockDim.x};
+__global__ void __launch_bounds__(kReactThreads, 3)
+    k_react(const __grid_constant__ Tables params, const double* U, double* out, long long nodes, int num_nodes, int nvars,
+            double dt, const double* __restrict__ dt_elem) {
+  constexpr int SLOTS = (NS + 1 + kLanes - 1) / kLanes, NC = NS + 1;   // rows a lane; columns with the right side
+  constexpr unsigned kAll = 0xffffffffu;
+  extern __shared__ __align__(16) double smem[];
+  // the mechanism in shared memory: the lanes of a node read different reactions and species
+  constexpr int kTableDoubles = (int)((sizeof(Tables) + 15) / 16 * 2);
+  {
+    const int* src = reinterpret_cast<const int*>(&params);
+    int* dst = reinterpret_cast<int*>(smem);
+    for (int i = threadIdx.x; i < (int)(sizeof(Tables) / sizeof(int)); i += kReactThreads) dst[i] = src[i];
+  }
+  __syncthreads();
+  const Tables& M = *reinterpret_cast<const Tables*>(smem);
+  const int lane = threadIdx.x % kLanes;
+  const long long want = ((long long)blockIdx.x * kReactThreads + threadIdx.x) / kLanes;
+  const bool live = want < nodes;
+  const long long n = live ? want : nodes - 1;          // spare lanes repeat the last node and store nothing
+  double* node = smem + kTableDoubles + (threadIdx.x / kLanes) * kNodeDoubles;
   const double* u = U + n * nvars;
   const double step = dt_elem ? dt_elem[n / num_nodes] : dt;
+  RowSpecies<SLOTS> row;
+#pragma unroll
+  for (int s = 0; s < SLOTS; ++s) {
+    const int q = M.row_of[s * kLanes + lane];
+    row.q[s] = q < 0 ? NS + 1 : q;                       // NS: the mass-weighted sum, NS + 1: no row
+  }
 
   const double rho_t = jmax(u[0], 1.0e-14);
-  double rs[NS], ssum = 0.0;
+  double rs[SLOTS], ssum = 0.0;
 #pragma unroll
-  for (int q = 0; q < NS; ++q) {
-    rs[q] = jmax(u[5 + q], 0.0);
-    ssum += rs[q];
+  for (int s = 0; s < SLOTS; ++s) {
+    rs[s] = row.q[s] < NS ? jmax(u[5 + row.q[s]], 0.0) : 0.0;
+    ssum += rs[s];
   }
+  ssum = quad_sum(ssum);
   const double scale = rho_t / jmax(ssum, 1.0e-20);
 #pragma unroll
-  for (int q = 0; q < NS; ++q) rs[q] *= scale;
+  for (int s = 0; s < SLOTS; ++s) rs[s] *= scale;
   const double ek = 0.5 * (u[1] * u[1] + u[2] * u[2] + u[3] * u[3]) / (rho_t * rho_t);
 
-  double rp[NS], T0, dtp;
+  double T0, dtp;
   if (M.dimensionless) {
     const double es = jmax(u[4] / rho_t - ek, 1.0e-4);
 #pragma unroll
-    for (int q = 0; q < NS; ++q) rp[q] = rs[q] * M.rho_ref;
+    for (int s = 0; s < SLOTS; ++s) rs[s] *= M.rho_ref;
     const double Tg = jmax((M.gamma - 1.0) * es * M.T_ref, 200.0);
-    T0 = recover_T<NS>(M, rp, es * M.e_ref, Tg, 8);
+    T0 = recover_T<NS, SLOTS>(M, row, rs, es * M.e_ref, Tg, 8);
     dtp = step * M.t_ref;
   } else {
     const double e = jmax(u[4] / rho_t - ek, 1.0e3);
-#pragma unroll
-    for (int q = 0; q < NS; ++q) rp[q] = rs[q];
-    T0 = recover_T<NS>(M, rp, e, 1000.0, 8);
+    T0 = recover_T<NS, SLOTS>(M, row, rs, e, 1000.0, 8);
     dtp = step;
   }
 
   // PointImplicitIntegrator.step, constant_temperature=False
-  double rho[NS], total = 0.0;
+  double rho[SLOTS], r0[SLOTS], total = 0.0;
 #pragma unroll
-  for (int q = 0; q < NS; ++q) {
-    rho[q] = jmax(rp[q], 1.0e-20);
-    sl.r0(q) = rho[q];
-    total += rho[q];
+  for (int s = 0; s < SLOTS; ++s) {
+    rho[s] = r0[s] = row.q[s] < NS ? jmax(rs[s], 1.0e-20) : 0.0;
+    total += rho[s];
   }
-  const double e_init = internal_energy<NS>(M, rho, T0);
-  double Tk = T0;
-  for (int it = 0; it < M.iters; ++it) {
-    double d[NS];
-    rates<NS>(M, sl, rho, Tk, true);
-    finish<NS>(M, sl, rho, dtp, true, true);
-    lu_solve<NS>(sl, d);
+  total = quad_sum(total);
+  double e_init = 0.0;
+  {
+    const double S = jmax(total, 1.0e-14), invT = 1.0 / T0;
 #pragma unroll
-    for (int q = 0; q < NS; ++q) rho[q] = jmax(rho[q] + d[q], 0.0);
-    Tk = recover_T<NS>(M, rho, e_init, Tk, 10);
+    for (int s = 0; s < SLOTS; ++s) {
+      double c;
+      const double es = species_energy(M, row.q[s] < NS ? row.q[s] : 0, T0, invT, c);
+      e_init += row.q[s] < NS ? (jmax(rho[s], 0.0) / S) * es : 0.0;
+    }
+    e_init = quad_sum(e_init);
+  }
+  double Tk = T0;
+  bool settled = false;
+  for (int it = 0; it < M.iters; ++it) {
+    // ---- the node's species vectors
+    const double Tg = jmax(Tk, 10.0);
+    const TPow tg = tpow(Tg);
+    __syncwarp();
+#pragma unroll
+    for (int s = 0; s < SLOTS; ++s) {
+      const int q = row.q[s];
+      if (q >= NS) continue;
+      const double craw = rho[s] * M.iW[q];
+      const double c = jmax(craw, 0.0);
+      const double dC = dmax_tie(craw, 0.0) * M.iW[q];
+      const double cc = jmax(c, kMinC);
+      node[q] = cc;
+      node[kRows + q] = dmax_tie(c, kMinC) * dC / cc;
+      node[2 * kRows + q] = c;
+      node[3 * kRows + q] = dC;
+      node[4 * kRows + q] = g_RT(M, q, tg);
+    }
+    __syncwarp();
+    // ---- rows of d omega/d rho and omega (last column), and their mass-weighted sum
+    const double base = kPStd / (kRUniv * Tg);
+    double a[SLOTS][NC];
+#pragma unroll
+    for (int s = 0; s < SLOTS; ++s)
+#pragma unroll
+      for (int j = 0; j < NC; ++j) a[s][j] = 0.0;
+    for (int pass = 0; pass * kPass < M.nr; ++pass) {
+      for (int r = lane; r < kPass; r += kLanes)
+        if (pass * kPass + r < M.nr)
+          reaction_row<NS>(M, pass * kPass + r, node, tg, base, node + kVec + r * kRxRow);
+      __syncwarp();
+#pragma unroll
+      for (int s = 0; s < SLOTS; ++s) {
+        const int* ptr = M.list_ptr + pass * kRows + s * kLanes + lane;
+        const int end = ptr[1];
+        for (int k = ptr[0]; k < end; ++k) {
+          const double w = M.list_w[k];
+          const double* x = node + kVec + M.list_rx[k] * kRxRow;
+#pragma unroll
+          for (int j = 0; j + 1 < NC; j += 2) {
+            const double2 v = *reinterpret_cast<const double2*>(x + j);
+            a[s][j] += w * v.x;
+            a[s][j + 1] += w * v.y;
+          }
+          if (NC % 2) a[s][NC - 1] += w * x[NC - 1];
+        }
+      }
+      __syncwarp();
+    }
+    // ---- mass-conserving correction and the Newton system [I - dt J | -res]
+    double S = 0.0;
+#pragma unroll
+    for (int s = 0; s < SLOTS; ++s) S += row.q[s] < NS ? rho[s] : 0.0;
+    const double Sraw = quad_sum(S);
+    S = jmax(Sraw, 1.0e-14);
+    const double dS = dmax_tie(Sraw, 1.0e-14);
+    // the mass-weighted sum is the last slot of the last lane
+    double col[NC];
+#pragma unroll
+    for (int j = 0; j < NC; ++j) col[j] = __shfl_sync(kAll, a[SLOTS - 1][j], (threadIdx.x & 28) | (kLanes - 1));
+    const double sw = col[NS];
+#pragma unroll
+    for (int s = 0; s < SLOTS; ++s) {
+      const int q = row.q[s];
+      const double W = q < NS ? M.W[q] : 0.0;
+      const double Y = jmax(rho[s], 0.0) / S;
+      const double dYo = -(jmax(rho[s], 0.0) / (S * S)) * dS, dYd = dmax_tie(rho[s], 0.0) / S;
+      const double w = W * a[s][NS] - Y * sw;
+#pragma unroll
+      for (int j = 0; j < NS; ++j) {
+        const double dY = j == q ? dYd + dYo : dYo;
+        const double J = W * a[s][j] - dY * sw - Y * col[j];
+        a[s][j] = (j == q ? 1.0 : 0.0) - dtp * J;
+      }
+      a[s][NS] = -(rho[s] - r0[s] - dtp * w);
+    }
+    // ---- LU with partial pivoting: the pivot is the largest entry of the column to 16 bits
+    unsigned used = 0;                                   // slots of this lane that have been pivot rows
+#pragma unroll
+    for (int s = 0; s < SLOTS; ++s) used |= row.q[s] < NS ? 0u : 1u << s;
+    unsigned long long order = 0;                        // 4 bits a column: its pivot row
+#pragma unroll
+    for (int k = 0; k < NS; ++k) {
+      unsigned key = 0;
+#pragma unroll
+      for (int s = 0; s < SLOTS; ++s) {
+        const unsigned hi = (unsigned)__double2hiint(a[s][k]) & 0x7ffffff0u;
+        const unsigned mine = (used >> s) & 1 ? 0u : hi | (15u - (unsigned)(s * kLanes + lane));
+        key = mine > key ? mine : key;
+      }
+      key = max(key, __shfl_xor_sync(kAll, key, 1));
+      key = max(key, __shfl_xor_sync(kAll, key, 2));
+      const int p = 15 - (int)(key & 15u), ps = p / kLanes, pl = p % kLanes;
+      order |= (unsigned long long)p << (4 * k);
+      double pv[NC];
+#pragma unroll
+      for (int j = k; j < NC; ++j) {
+        double v = a[0][j];
+#pragma unroll
+        for (int s = 1; s < SLOTS; ++s) v = ps == s ? a[s][j] : v;
+        pv[j] = __shfl_sync(kAll, v, (threadIdx.x & 28) | pl);
+      }
+      if (lane == pl) used |= 1u << ps;
+      const double rp = 1.0 / pv[k];
+#pragma unroll
+      for (int s = 0; s < SLOTS; ++s) {
+        const double f = (used >> s) & 1 ? 0.0 : a[s][k] * rp;
+#pragma unroll
+        for (int j = k + 1; j < NC; ++j) a[s][j] -= f * pv[j];
+      }
+    }
+    double d[SLOTS];
+#pragma unroll
+    for (int s = 0; s < SLOTS; ++s) d[s] = 0.0;
+#pragma unroll
+    for (int k = NS - 1; k >= 0; --k) {
+      const int p = (int)((order >> (4 * k)) & 15u), ps = p / kLanes, pl = p % kLanes;
+      double num = a[0][NS], den = a[0][k];
+#pragma unroll
+      for (int s = 1; s < SLOTS; ++s) {
+        num = ps == s ? a[s][NS] : num;
+        den = ps == s ? a[s][k] : den;
+      }
+      const double x = __shfl_sync(kAll, num / den, (threadIdx.x & 28) | pl);
+#pragma unroll
+      for (int s = 0; s < SLOTS; ++s) {
+        a[s][NS] -= a[s][k] * x;
+        d[s] = row.q[s] == k ? x : d[s];
+      }
+    }
+    // ---- update; a node that has settled keeps its state
+    bool still = true;
+    double next[SLOTS];
+#pragma unroll
+    for (int s = 0; s < SLOTS; ++s) {
+      next[s] = jmax(rho[s] + d[s], 0.0);
+      if (row.q[s] >= NS) next[s] = 0.0;
+      still = still && fabs(next[s] - rho[s]) <= kSettled * rho[s];
+      if (!settled) rho[s] = next[s];
+    }
+    const double Tn = recover_T<NS, SLOTS>(M, row, rho, e_init, Tk, 10);
+    still = still && fabs(Tn - Tk) <= kTStop * Tk;
+    if (!settled) Tk = Tn;
+    const unsigned votes = __ballot_sync(kAll, still) >> (threadIdx.x & 28) & 15u;
+    settled = settled || votes == 15u;
+    if (__all_sync(kAll, settled)) break;
   }
   double fsum = 0.0;
 #pragma unroll
-  for (int q = 0; q < NS; ++q) fsum += rho[q];
-  const double fs = total / fsum;
+  for (int s = 0; s < SLOTS; ++s) fsum += row.q[s] < NS ? rho[s] : 0.0;
+  const double fs = total / quad_sum(fsum);
   double nsum = 0.0;
 #pragma unroll
-  for (int q = 0; q < NS; ++q) {
-    double v = rho[q] * fs;
+  for (int s = 0; s < SLOTS; ++s) {
+    double v = rho[s] * fs;
     if (M.dimensionless) v = v / M.rho_ref;
-    rho[q] = jmax(v, 0.0);
-    nsum += rho[q];
+    rho[s] = row.q[s] < NS ? jmax(v, 0.0) : 0.0;
+    nsum += rho[s];
   }
-  const double back = rho_t / jmax(nsum, 1.0e-20);
+  const double back = rho_t / jmax(quad_sum(nsum), 1.0e-20);
+  if (!live) return;
   double* o = out + n * nvars;
   if (o != u) {
-    for (int v = 0; v < 5; ++v) o[v] = u[v];
-    for (int v = 5 + NS; v < nvars; ++v) o[v] = u[v];
+    for (int v = lane; v < 5; v += kLanes) o[v] = u[v];
+    for (int v = 5 + NS + lane; v < nvars; v += kLanes) o[v] = u[v];
   }
 #pragma unroll
-  for (int q = 0; q < NS; ++q) o[5 + q] = rho[q] * back;
+  for (int s = 0; s < SLOTS; ++s)
+    if (row.q[s] < NS) o[5 + row.q[s]] = rho[s] * back;
 }
 
 // ReactionMechanism.net_production_rates (and its Jacobian) for independent samples.
@@ -489,7 +701,7 @@ __global__ void __launch_bounds__(kThreads) k_rates(const __grid_constant__ Tabl
 #pragma unroll
   for (int q = 0; q < NS; ++q)
     if (omega) omega[n * NS + q] = sl.om(q);
-  finish<NS>(M, sl, rho, 0.0, want, false);
+  finish<NS>(M, sl, rho, want);
 #pragma unroll
   for (int q = 0; q < NS; ++q)
     if (wdot) wdot[n * NS + q] = sl.om(q);
@@ -511,15 +723,16 @@ size_t smem_bytes() {
 template <int NS>
 int launch_react(const Tables& M, const double* U, double* out, long long nodes, int num_nodes, int nvars, double dt,
                  const double* dt_elem, cudaStream_t st) {
-  const size_t sm = smem_bytes<NS>();
+  constexpr int per = kReactThreads / kLanes;
+  const size_t sm = (sizeof(Tables) + 15) / 16 * 16 + sizeof(double) * (size_t)per * kNodeDoubles;
   cudaError_t err = cudaFuncSetAttribute(k_react<NS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  // the largest shared-memory carve-out, so that five one-warp CTAs share an SM
+  // the largest shared-memory carve-out, so that three CTAs share an SM
   if (err == cudaSuccess)
     err = cudaFuncSetAttribute(k_react<NS>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                cudaSharedmemCarveoutMaxShared);
   if (err != cudaSuccess) return fail(DGB_ERR_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(err));
-  const unsigned grid = (unsigned)((nodes + kThreads - 1) / kThreads);
-  k_react<NS><<<grid, kThreads, sm, st>>>(M, U, out, nodes, num_nodes, nvars, dt, dt_elem);
+  const unsigned grid = (unsigned)((nodes + per - 1) / per);
+  k_react<NS><<<grid, kReactThreads, sm, st>>>(M, U, out, nodes, num_nodes, nvars, dt, dt_elem);
   err = cudaGetLastError();
   if (err != cudaSuccess) return fail(DGB_ERR_CUDA, std::string("k_react: ") + cudaGetErrorString(err));
   return DGB_OK;
@@ -637,6 +850,36 @@ int dgb_chem_create(const dgb_chem_mechanism* m, const dgb_chem_params* prm, dgb
       R.r_pw[k] = (int)v;
     }
   }
+  // k_react's rows: the species by falling number of reactions, four side by side, so that the lanes
+  // of a node walk lists of similar length; the mass-weighted sum is the last row of NS + 1
+  {
+    const int rows = (ns + 1 + kLanes - 1) / kLanes * kLanes;
+    std::vector<int> sp(ns), count(ns, 0);
+    for (int q = 0; q < ns; ++q) sp[q] = q;
+    for (int r = 0; r < nr; ++r)
+      for (int k = 0; k < M.rx[r].nd; ++k) ++count[M.rx[r].d_sp[k]];
+    std::stable_sort(sp.begin(), sp.end(), [&](int a, int b) { return count[a] > count[b]; });
+    for (int i = 0; i < kRows; ++i) M.row_of[i] = i < ns ? sp[i] : -1;
+    M.row_of[rows - 1] = ns;
+    int n = 0;
+    for (int pass = 0; pass < kPasses; ++pass)
+      for (int i = 0; i < kRows; ++i) {
+        M.list_ptr[pass * kRows + i] = n;
+        const int q = M.row_of[i];
+        if (q < 0) continue;
+        for (int r = pass * kPass; r < nr && r < (pass + 1) * kPass; ++r) {
+          const Reaction& R = M.rx[r];
+          double w = 0.0;
+          for (int k = 0; k < R.nd; ++k)
+            if (q == ns) w += M.W[R.d_sp[k]] * R.d_nu[k];
+            else if (R.d_sp[k] == q) w = R.d_nu[k];
+          if (w == 0.0) continue;
+          M.list_rx[n] = (short)(r - pass * kPass);
+          M.list_w[n++] = w;
+        }
+      }
+    M.list_ptr[kPasses * kRows] = n;
+  }
   // coupling.py:55-67
   M.iters = prm->max_newton_iters;
   M.dimensionless = prm->dimensionless ? 1 : 0;
@@ -669,7 +912,7 @@ int dgb_react_block(dgb_chem* chem, const double* U, double* out, int64_t num_el
   const long long nodes = (long long)num_elements * num_nodes;
   if (nodes == 0) return DGB_OK;                    // an empty block needs no buffers
   if (!U || !out) return fail(DGB_ERR_ARGUMENT, "null argument");
-  if ((nodes + kThreads - 1) / kThreads > 0x7fffffffLL) return fail(DGB_ERR_ARGUMENT, "block too large");
+  if (nodes / (kReactThreads / kLanes) >= 0x7fffffffLL) return fail(DGB_ERR_ARGUMENT, "block too large");
   cudaStream_t st = (cudaStream_t)stream;
   return M.ns == 11 ? launch_react<11>(M, U, out, nodes, num_nodes, nvars, dt, dt_per_element, st)
                     : launch_react<3>(M, U, out, nodes, num_nodes, nvars, dt, dt_per_element, st);
