@@ -535,7 +535,7 @@ __global__ void __launch_bounds__(kThreads) k_rate(const DevPlan P, const StateP
   }
 }
 
-__global__ void k_dt(const Partial* partials, int n, double cfl, double* dt_out) {
+static __global__ void k_dt(const Partial* partials, int n, double cfl, double* dt_out) {
   __shared__ double red[kThreads];
   double m = -INFINITY;
   for (int i = threadIdx.x; i < n; i += blockDim.x) m = fmax(m, partials[i].a);
@@ -600,7 +600,7 @@ __global__ void __launch_bounds__(kThreads) k_adm(const DevPlan P, const StatePt
 // kAdmFinalThreads reduces the partials (a serial loop over thousands of them took 0.3 ms).
 constexpr int kAdmFinalThreads = 256;
 
-__global__ void __launch_bounds__(kAdmFinalThreads) k_adm_final(const Partial* partials, int n, double rho_floor,
+static __global__ void __launch_bounds__(kAdmFinalThreads) k_adm_final(const Partial* partials, int n, double rho_floor,
                                                                double p_floor, int combine, dgb_status* status) {
   __shared__ double sr[kAdmFinalThreads], sp[kAdmFinalThreads];
   double rmin = INFINITY, pmin = INFINITY;

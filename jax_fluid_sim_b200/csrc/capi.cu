@@ -12,10 +12,16 @@
 #include "dense_rhs.h"
 #include "hex_fused.cuh"
 #include "hex_kernels.cuh"
+#include "hex_launch.h"
 #include "mlp_kernels.cuh"
 #include "mood_kernels.cuh"
 #include "subcell_build.cuh"
 #include "tc_volume.h"
+
+namespace dgb {
+DGB_HEX_LAUNCHES(extern, double)
+DGB_HEX_LAUNCHES_F32(extern)
+}  // namespace dgb
 
 using namespace dgb;
 
@@ -92,13 +98,14 @@ struct dgb_plan {
   // sum-factorised hexahedron path (single hexahedron block)
   bool hex = false;
   HexTables hex_tables;
+  HexTablesT<float> hex_tables32;   // the same, rounded, for the float32 kernels
   // hexahedron positivity: elements the certificate pre-pass did not clear, and the grid that
   // works through them (resident CTAs of k_hex_positivity)
   int* cert_list = nullptr;
   int* cert_count = nullptr;
   int pos_grid = 0;
   int trb_grid = 0;   // the same for k_hex_troubled, which shares the list
-  HexCodes hex_codes = {nullptr, nullptr};
+  HexCodes hex_codes = {nullptr, nullptr, nullptr};
   double* hex_lift = nullptr;     // [E][12][N3] nodal BR2 lift scratch
   // fused right-hand side (hex_fused.cuh): on by default, dgb_plan_set_fused
   bool fused = true;
@@ -407,17 +414,23 @@ int launch_face_flux(dgb_plan* p, const StatePtrs& S, int ft, cudaStream_t st) {
   return DGB_OK;
 }
 
+template <typename R>
+const HexTablesT<R>& hex_tables(const dgb_plan* p);
+template <>
+const HexTablesT<double>& hex_tables<double>(const dgb_plan* p) { return p->hex_tables; }
+template <>
+const HexTablesT<float>& hex_tables<float>(const dgb_plan* p) { return p->hex_tables32; }
+
 template <int P, int NV, bool SPLIT, typename R>
 int run_rhs_hex(dgb_plan* p, const StatePtrs& S, const FinalizeArgs& A, cudaStream_t st, cudaEvent_t* ev) {
   using LR = HexSmem<P, NV, R>;
   const DevPlan& D = p->dev;
   const int E = D.blk[0].E;
-  const size_t sm_tr = sizeof(R) * (size_t)LR::TRACES, sm_li = sizeof(R) * (size_t)LR::LIFT;
+  const size_t sm_li = sizeof(R) * (size_t)LR::LIFT;
   const size_t sm_vo = sizeof(R) * (size_t)LR::template VOLUME<SPLIT>, sm_fi = sizeof(R) * (size_t)LR::FINAL;
   int rc;
   if (ev) CK(cudaEventRecord(ev[0], st));
-  if ((rc = prepare(k_hex_traces<P, NV, R>, sm_tr))) return rc;
-  k_hex_traces<P, NV, R><<<E, kThreads, sm_tr, st>>>(D, S, 0, p->hex_tables, p->hex_codes);
+  CK((launch_hex_traces<P, NV, R, false>(D, S, hex_tables<R>(p), p->hex_codes, st)));
   if (ev) CK(cudaEventRecord(ev[1], st));
   if ((rc = launch_face_flux<NV>(p, S, 1, st))) return rc;
   if (ev) CK(cudaEventRecord(ev[2], st));
@@ -444,56 +457,33 @@ int run_rhs_hex(dgb_plan* p, const StatePtrs& S, const FinalizeArgs& A, cudaStre
 // kernels (zero-length).
 template <int P, int NV, bool SPLIT, typename R>
 int run_rhs_hex_fused(dgb_plan* p, const StatePtrs& S, const FinalizeArgs& A, cudaStream_t st, cudaEvent_t* ev) {
-  using LR = HexSmem<P, NV, R>;
-  using LE = HexElemSmem<P, NV, SPLIT, R>;
   const DevPlan& D = p->dev;
-  const int E = D.blk[0].E;
-  const size_t sm_tr = sizeof(R) * (size_t)LR::TRACES, sm_el = sizeof(R) * (size_t)LE::TOTAL;
-  int rc;
   if (ev) CK(cudaEventRecord(ev[0], st));
   // mixed precision: the viscous traces travel to the face kernel in float32
   constexpr bool MIXED = sizeof(R) == sizeof(float);
   const bool f32 = MIXED && D.face[1].trV32 != nullptr && p->f32_traces;
-  constexpr int FPC = kThreads / HexDims<P>::QF2;
-  const int fgrid = blocks_for(D.face[1].F, FPC);
-  if (f32) {
-    if ((rc = prepare(k_hex_traces<P, NV, R, MIXED>, sm_tr))) return rc;
-    k_hex_traces<P, NV, R, MIXED><<<E, kThreads, sm_tr, st>>>(D, S, 0, p->hex_tables, p->hex_codes);
-  } else {
-    if ((rc = prepare(k_hex_traces<P, NV, R>, sm_tr))) return rc;
-    k_hex_traces<P, NV, R><<<E, kThreads, sm_tr, st>>>(D, S, 0, p->hex_tables, p->hex_codes);
-  }
+  if (f32) CK((launch_hex_traces<P, NV, R, MIXED>(D, S, hex_tables<R>(p), p->hex_codes, st)));
+  else CK((launch_hex_traces<P, NV, R, false>(D, S, hex_tables<R>(p), p->hex_codes, st)));
   if (ev) CK(cudaEventRecord(ev[1], st));
-  if (D.face[1].F > 0) {
-    if (f32)
-      k_hex_face<P, NV, R, MIXED><<<fgrid, kThreads, 0, st>>>(D, p->hex_tables, p->hex_codes, p->hex_face);
-    else
-      k_hex_face<P, NV, R><<<fgrid, kThreads, 0, st>>>(D, p->hex_tables, p->hex_codes, p->hex_face);
-  }
+  if (f32) CK((launch_hex_face<P, NV, R, MIXED>(D, p->hex_tables, p->hex_codes, p->hex_face, st)));
+  else CK((launch_hex_face<P, NV, R, false>(D, p->hex_tables, p->hex_codes, p->hex_face, st)));
   if (ev) {
     CK(cudaEventRecord(ev[2], st));
     CK(cudaEventRecord(ev[3], st));
   }
-  if ((rc = prepare(k_hex_element<P, NV, SPLIT, R>, sm_el))) return rc;
-  k_hex_element<P, NV, SPLIT, R><<<E, kThreads, sm_el, st>>>(D, S, p->hex_tables, p->hex_codes, A);
+  CK((launch_hex_element<P, NV, SPLIT, R>(D, S, hex_tables<R>(p), p->hex_codes, A, st)));
   if (ev) {
     CK(cudaEventRecord(ev[4], st));
     CK(cudaEventRecord(ev[5], st));
     CK(cudaEventRecord(ev[6], st));
   }
-  CK(cudaGetLastError());
   return DGB_OK;
 }
 
 // The fused element kernel alone, split residuals, on the face buffers of the last right-hand side.
 template <int P, int NV, typename R>
 int run_hex_element_pass(dgb_plan* p, const StatePtrs& S, const FinalizeArgs& A, cudaStream_t st) {
-  using LE = HexElemSmem<P, NV, true, R>;
-  const size_t sm_el = sizeof(R) * (size_t)LE::TOTAL;
-  int rc;
-  if ((rc = prepare(k_hex_element<P, NV, true, R>, sm_el))) return rc;
-  k_hex_element<P, NV, true, R><<<p->dev.blk[0].E, kThreads, sm_el, st>>>(p->dev, S, p->hex_tables, p->hex_codes, A);
-  CK(cudaGetLastError());
+  CK((launch_hex_element<P, NV, true, R>(p->dev, S, hex_tables<R>(p), p->hex_codes, A, st)));
   return DGB_OK;
 }
 
@@ -1060,21 +1050,15 @@ int run_subcell_api(dgb_plan* p, const dgb_state* base, const dgb_state* cand, d
   if (p->hex) {
     switch (P.degree) {
       case 1: {
-        const size_t sm = sizeof(double) * (size_t)HexSmem<1, NV>::TRACES;
-        if ((rc = prepare(k_hex_traces<1, NV>, sm))) return rc;
-        k_hex_traces<1, NV><<<P.blk[0].E, kThreads, sm, st>>>(P, S, 0, p->hex_tables, p->hex_codes);
+        CK((launch_hex_traces<1, NV, double, false>(P, S, p->hex_tables, p->hex_codes, st)));
         break;
       }
       case 2: {
-        const size_t sm = sizeof(double) * (size_t)HexSmem<2, NV>::TRACES;
-        if ((rc = prepare(k_hex_traces<2, NV>, sm))) return rc;
-        k_hex_traces<2, NV><<<P.blk[0].E, kThreads, sm, st>>>(P, S, 0, p->hex_tables, p->hex_codes);
+        CK((launch_hex_traces<2, NV, double, false>(P, S, p->hex_tables, p->hex_codes, st)));
         break;
       }
       default: {
-        const size_t sm = sizeof(double) * (size_t)HexSmem<3, NV>::TRACES;
-        if ((rc = prepare(k_hex_traces<3, NV>, sm))) return rc;
-        k_hex_traces<3, NV><<<P.blk[0].E, kThreads, sm, st>>>(P, S, 0, p->hex_tables, p->hex_codes);
+        CK((launch_hex_traces<3, NV, double, false>(P, S, p->hex_tables, p->hex_codes, st)));
       }
     }
   } else {
@@ -1326,6 +1310,10 @@ int dgb_plan_set_hex(dgb_plan* p, const double* line_tables, const int32_t* lex2
   }
   int rc;
   if ((rc = upload(p, perm, (size_t)num_codes * face_points, &p->hex_codes.perm))) return rc;
+  if ((rc = upload(p, lex2node, 64, &p->hex_codes.lex2node))) return rc;
+  for (int k = 0; k < kHexTableValues; ++k)
+    reinterpret_cast<float*>(&p->hex_tables32)[k] = (float)reinterpret_cast<const double*>(&t)[k];
+  memcpy(p->hex_tables32.lex2node, t.lex2node, sizeof(t.lex2node));
   p->hex = true;
   return DGB_OK;
 }

@@ -26,7 +26,7 @@
 namespace dgb {
 
 // Local face of each face side of the hexahedron block: face_lf[f * 2 + side] (set-up).
-__global__ void k_hex_face_lf(const DevPlan P_, int8_t* face_lf) {
+static __global__ void k_hex_face_lf(const DevPlan P_, int8_t* face_lf) {
   const BlockDev& B = P_.blk[0];
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= B.E * 6) return;
@@ -337,12 +337,6 @@ __global__ void __launch_bounds__(kThreads, NV <= 5 ? 6 : 1) k_hex_face(const De
   }
 }
 
-// Rotation of the thread <-> line assignment of a pencil pass, so that passes issued back to back
-// without a barrier between them start on different threads.
-__device__ __forceinline__ int rotated(int offset) {
-  return (int)((threadIdx.x + kThreads - (unsigned)offset % kThreads) % kThreads);
-}
-
 // K consecutive shared-memory values at p (16-byte aligned) into r: 16-byte loads, then an 8-byte
 // load of a float pair, then single values.
 template <int K, typename T>
@@ -363,121 +357,155 @@ __device__ __forceinline__ void lds_vec(const T* p, T* r) {
 // The three reference-gradient fields of C nodal channels at the Q^3 volume points,
 // g[r][c][Q3] = (d/dxi_r of the interpolant), by the sum-factorised passes with the intermediates
 // shared between directions: x (bq, dq), y (bq, dq on the bq branch; bq on the dq branch), z.  Each
-// output goes through the same three 1-D products as a separate tensor3 per direction, so the values
-// are the same; the barriers are three instead of nine.  s: 2 C N^2 Q + 3 C N Q^2 values of scratch.
+// output goes through the same three 1-D products as a separate contraction per direction, so the values
+// are the same; the barriers are three instead of nine.  X: 2 C N P1 values of scratch, Y: 3 C N P2.
 template <int C, int N, int Q, typename T>
-__device__ __forceinline__ void grad3(const T* V, T* g, T* s, const T* bq, const T* dq) {
-  T* Bx = s;
-  T* Dx = Bx + C * N * N * Q;
-  T* BB = Dx + C * N * N * Q;
-  T* BD = BB + C * N * Q * Q;
-  T* DB = BD + C * N * Q * Q;
-  constexpr int L1 = C * N * N, L2 = C * N * Q, L3 = C * Q * Q, Q3 = Q * Q * Q;
-  const int st = kThreads;
+struct Grad3 {
+  static constexpr int P1 = plane<T>(N * Q), P2 = plane<T>(Q * Q), X = 2 * C * N * P1, Y = 3 * C * N * P2;
+};
+
+template <int C, int N, int Q, typename T>
+__device__ __forceinline__ void grad3(const T* V, T* g, T* X, T* Y, const T* bq, const T* dq) {
+  using G = Grad3<C, N, Q, T>;
+  constexpr int P1 = G::P1, P2 = G::P2, L1 = C * N * N, L2 = C * N * Q, L3 = C * Q * Q, Q3 = Q * Q * Q, QQ = Q * Q;
+  T* Bx = X;
+  T* Dx = Bx + C * N * P1;
+  T* BB = Y;
+  T* BD = BB + C * N * P2;
+  T* DB = BD + C * N * P2;
+  constexpr bool VI = (N * (int)sizeof(T)) % 16 == 0, VO = (Q * (int)sizeof(T)) % 16 == 0 && (P1 * (int)sizeof(T)) % 16 == 0;
   auto i1 = [](int l) { return l * N; };
-  auto o1 = [](int l) { return l * Q; };
-  pencil<N, Q, false>(V, Bx, bq, L1, 1, 1, i1, o1, rotated(0), st);
-  pencil<N, Q, false>(V, Dx, dq, L1, 1, 1, i1, o1, rotated(L1), st);
+  auto o1 = [](int l) { return (l / N) * P1 + (l % N) * Q; };
+  pass<N, Q, L1, 1, 1, VI, VO>(V, Bx, bq, i1, o1, rotated(0));
+  pass<N, Q, L1, 1, 1, VI, VO>(V, Dx, dq, i1, o1, rotated(L1));
   __syncthreads();
-  auto i2 = [](int l) { return (l / Q) * N * Q + l % Q; };
-  auto o2 = [](int l) { return (l / Q) * Q * Q + l % Q; };
-  pencil<N, Q, false>(Bx, BB, bq, L2, Q, Q, i2, o2, rotated(0), st);
-  pencil<N, Q, false>(Bx, BD, dq, L2, Q, Q, i2, o2, rotated(L2), st);
-  pencil<N, Q, false>(Dx, DB, bq, L2, Q, Q, i2, o2, rotated(2 * L2), st);
+  auto i2 = [](int l) { return (l / Q) * P1 + l % Q; };
+  auto o2 = [](int l) { return (l / Q) * P2 + l % Q; };
+  pass<N, Q, L2, Q, Q, false, false>(Bx, BB, bq, i2, o2, rotated(0));
+  pass<N, Q, L2, Q, Q, false, false>(Bx, BD, dq, i2, o2, rotated(L2));
+  pass<N, Q, L2, Q, Q, false, false>(Dx, DB, bq, i2, o2, rotated(2 * L2));
   __syncthreads();
-  auto i3 = [](int l) { return (l / (Q * Q)) * N * Q * Q + l % (Q * Q); };
-  auto o3 = [](int l) { return (l / (Q * Q)) * Q * Q * Q + l % (Q * Q); };
-  pencil<N, Q, false>(DB, g + 0 * C * Q3, bq, L3, Q * Q, Q * Q, i3, o3, rotated(0), st);
-  pencil<N, Q, false>(BD, g + 1 * C * Q3, bq, L3, Q * Q, Q * Q, i3, o3, rotated(L3), st);
-  pencil<N, Q, false>(BB, g + 2 * C * Q3, dq, L3, Q * Q, Q * Q, i3, o3, rotated(2 * L3), st);
+  auto i3 = [](int l) { return (l / QQ) * N * P2 + l % QQ; };
+  auto o3 = [](int l) { return (l / QQ) * Q * QQ + l % QQ; };
+  pass<N, Q, L3, P2, QQ, false, false>(DB, g + 0 * C * Q3, bq, i3, o3, rotated(0));
+  pass<N, Q, L3, P2, QQ, false, false>(BD, g + 1 * C * Q3, bq, i3, o3, rotated(L3));
+  pass<N, Q, L3, P2, QQ, false, false>(BB, g + 2 * C * Q3, dq, i3, o3, rotated(2 * L3));
   __syncthreads();
 }
 
 // The weak divergence R[c][N3] = sum_r (transposed gradient of direction r) G[r][c][Q3], by three
-// passes (x, y with three inputs each, then z summing the three terms in the order of three
-// accumulating tensor3 calls: (t0 + t1) + t2), so the values match that form with three barriers
-// instead of nine.  A: 3 C Q^2 N values of scratch; the y-pass results overwrite G.
+// passes (x, y with three inputs each, then z summing the three terms as (t0 + t1) + t2).  A: 3 C Q P1
+// values of scratch; the y-pass results overwrite G (3 C Q P2 values, at most its 3 C Q3).
+template <int C, int N, int Q, typename T>
+struct Div3 {
+  static constexpr int P1 = Q * N == 16 ? 20 : Q * N, P2 = Q * plane<T>(N * N) <= Q * Q * Q ? plane<T>(N * N) : N * N;
+  static constexpr int A = 3 * C * Q * P1;
+};
+
 template <int C, int N, int Q, typename T>
 __device__ __forceinline__ void div3(T* G, T* R, T* A, const T* bqT, const T* dqT) {
-  constexpr int Q3 = Q * Q * Q, LX = C * Q * Q, LY = C * Q * N, LZ = C * N * N;
-  constexpr int AS = C * Q * Q * N, BS = C * Q * N * N;
-  const int st = kThreads;
+  using X = Div3<C, N, Q, T>;
+  constexpr int P1 = X::P1, P2 = X::P2, Q3 = Q * Q * Q, NN = N * N, LX = C * Q * Q, LY = C * Q * N, LZ = C * NN;
+  constexpr int AS = C * Q * P1, BS = C * Q * P2;
+  constexpr bool VO = (N * (int)sizeof(T)) % 16 == 0 && (P1 * (int)sizeof(T)) % 16 == 0;
   auto ix = [](int l) { return l * Q; };
-  auto ox = [](int l) { return l * N; };
-  pencil<Q, N, false>(G + 0 * C * Q3, A + 0 * AS, dqT, LX, 1, 1, ix, ox, rotated(0), st);
-  pencil<Q, N, false>(G + 1 * C * Q3, A + 1 * AS, bqT, LX, 1, 1, ix, ox, rotated(LX), st);
-  pencil<Q, N, false>(G + 2 * C * Q3, A + 2 * AS, bqT, LX, 1, 1, ix, ox, rotated(2 * LX), st);
+  auto ox = [](int l) { return (l / Q) * P1 + (l % Q) * N; };
+  pass<Q, N, LX, 1, 1, false, VO>(G + 0 * C * Q3, A + 0 * AS, dqT, ix, ox, rotated(0));
+  pass<Q, N, LX, 1, 1, false, VO>(G + 1 * C * Q3, A + 1 * AS, bqT, ix, ox, rotated(LX));
+  pass<Q, N, LX, 1, 1, false, VO>(G + 2 * C * Q3, A + 2 * AS, bqT, ix, ox, rotated(2 * LX));
   __syncthreads();
-  T* B = G;                                    // [3][C][Q][N][N]
-  auto iy = [](int l) { return (l / N) * Q * N + l % N; };
-  auto oy = [](int l) { return (l / N) * N * N + l % N; };
-  pencil<Q, N, false>(A + 0 * AS, B + 0 * BS, bqT, LY, N, N, iy, oy, rotated(0), st);
-  pencil<Q, N, false>(A + 1 * AS, B + 1 * BS, dqT, LY, N, N, iy, oy, rotated(LY), st);
-  pencil<Q, N, false>(A + 2 * AS, B + 2 * BS, bqT, LY, N, N, iy, oy, rotated(2 * LY), st);
+  T* B = G;                                    // [3][C][Q][P2]
+  auto iy = [](int l) { return (l / N) * P1 + l % N; };
+  auto oy = [](int l) { return (l / N) * P2 + l % N; };
+  pass<Q, N, LY, N, N, false, false>(A + 0 * AS, B + 0 * BS, bqT, iy, oy, rotated(0));
+  pass<Q, N, LY, N, N, false, false>(A + 1 * AS, B + 1 * BS, dqT, iy, oy, rotated(LY));
+  pass<Q, N, LY, N, N, false, false>(A + 2 * AS, B + 2 * BS, bqT, iy, oy, rotated(2 * LY));
   __syncthreads();
-  const T* mb = bqT;                           // read from shared memory (broadcast)
-  const T* md = dqT;
-  for (int line = threadIdx.x; line < LZ; line += st) {
-    const int ib = (line / (N * N)) * Q * N * N + line % (N * N);
-    const int ob = (line / (N * N)) * N * N * N + line % (N * N);
+  for (int line = threadIdx.x; line < LZ; line += kThreads) {
+    const int ib = (line / NN) * Q * P2 + line % NN;
+    const int ob = (line / NN) * N * NN + line % NN;
     T x0[Q], x1[Q], x2[Q];
 #pragma unroll
     for (int i = 0; i < Q; ++i) {
-      x0[i] = B[0 * BS + ib + i * N * N];
-      x1[i] = B[1 * BS + ib + i * N * N];
-      x2[i] = B[2 * BS + ib + i * N * N];
+      x0[i] = B[0 * BS + ib + i * P2];
+      x1[i] = B[1 * BS + ib + i * P2];
+      x2[i] = B[2 * BS + ib + i * P2];
     }
 #pragma unroll
     for (int o = 0; o < N; ++o) {
       T s0 = T(0), s1 = T(0), s2 = T(0);
 #pragma unroll
-      for (int i = 0; i < Q; ++i) s0 += mb[o * Q + i] * x0[i];
+      for (int i = 0; i < Q; ++i) s0 += bqT[o * Q + i] * x0[i];
 #pragma unroll
-      for (int i = 0; i < Q; ++i) s1 += mb[o * Q + i] * x1[i];
+      for (int i = 0; i < Q; ++i) s1 += bqT[o * Q + i] * x1[i];
 #pragma unroll
-      for (int i = 0; i < Q; ++i) s2 += md[o * Q + i] * x2[i];
+      for (int i = 0; i < Q; ++i) s2 += dqT[o * Q + i] * x2[i];
       T acc = s0;
       acc += s1;
       acc += s2;
-      R[ob + o * N * N] = acc;
+      R[ob + o * NN] = acc;
     }
   }
   __syncthreads();
 }
 
-// Shared-memory layout of k_hex_element, in units of R.
+__host__ __device__ constexpr int up4(int n) { return (n + 3) / 4 * 4; }
+
+// Shared-memory layout of k_hex_element, in units of R.  The nodal arrays come first (U, V, LF the nodal
+// lift, RR the residuals), then the scratch W, which each phase lays out for itself; phases also use nodal
+// arrays that are not yet written or already dead.
 template <int P, int NV, bool SPLIT, typename R>
 struct HexElemSmem {
   using D = HexDims<P>;
   static constexpr int N = D::N, Q = D::Q, QF = D::QF, N2 = D::N2, N3 = D::N3, Q3 = D::Q3, QF2 = D::QF2;
-  // table size in R, rounded up to 16 bytes so that the arrays after the tables stay 16-byte aligned
-  static constexpr int T = (int)((sizeof(HexTablesT<R>) + 15) / 16 * 16 / sizeof(R));
   static constexpr int C = SPLIT ? 2 * NV : NV;          // residual channels
-  static constexpr int U = T, V = U + NV * N3, LF = V + 4 * N3, RR = LF + 12 * N3;
-  // the phase scratch starts on a 16-byte boundary (N3 = 27 leaves RR + C N3 odd)
-  static constexpr int W = (RR + C * N3 + 3) / 4 * 4;
-  // phase scratch (aliased)
-  // jc, tmp, bs, ball, then the affine elements' tensor3 scratch (two [12][N3] passes)
-  static constexpr int LIFT = 72 * QF2 + 72 * QF * N + 72 * N2 + 12 * N3 + 2 * 12 * N3;
-  // phase C: uq [NV][Q3], gq [12][Q3], then the lift at the points lq [12][Q3] (later Gi, Gv [3][NV][Q3]
-  // each), then contraction scratch
-  static constexpr int VOL_G = cmax(12 * Q3, (SPLIT ? 6 : 3) * NV * Q3);
-  static constexpr int VOL_S = cmax(cmax(NV * N * N * Q + NV * N * Q * Q, 12 * N * N * Q + 12 * N * Q * Q),
-                                    2 * 4 * N * N * Q + 3 * 4 * N * Q * Q);
-  // the scratch lives beyond lq while Gi/Gv are not yet written; div3's x-pass results go to the
-  // dead uq/gq region when they fit there, otherwise beyond Gi/Gv
-  static constexpr int DIV_A = 3 * NV * Q * Q * N;
-  static constexpr int DIV_AT = DIV_A <= NV * Q3 + 12 * Q3 ? 0 : NV * Q3 + 12 * Q3 + VOL_G;
-  static constexpr int VOL2 = cmax(NV * Q3 + 12 * Q3 + cmax(VOL_G, 12 * Q3 + VOL_S), DIV_AT + DIV_A);
-  static constexpr int FIN = 6 * C * (QF2 + QF * N) + cmax(6 * C * N2, 4 * NV * N3);
-  static constexpr int TOTAL = W + cmax(LIFT, cmax(VOL2, FIN));
+  static constexpr int U = 0, V = up4(U + NV * N3), LF = up4(V + 4 * N3), RR = up4(LF + 12 * N3);
+  static constexpr int W = up4(RR + C * N3);
+  // phase B: jumps jc, x-pass results tmp, face sums bs, nodal sums ball (or the non-affine elements' rows);
+  // the affine M^-1 product's scratch goes over jc and tmp
+  static constexpr int PT = plane<R>(QF * N), PB = plane<R>(N2);
+  static constexpr int LR = (6 * (int)sizeof(R) + 15) / 16 * 16 / (int)sizeof(R);
+  static constexpr int B_TMP = up4(72 * QF2), B_BS = up4(B_TMP + 72 * PT), B_BALL = up4(B_BS + 72 * PB);
+  using M3 = Contract3<12, N, N, R>;
+  static constexpr int LIFT = cmax(B_BALL + cmax(12 * N3, 2 * LR * N3), 0);
+  static_assert(up4(M3::T1) + M3::T2 <= B_BALL, "the affine product's scratch ends before its input");
+  // phase C: uq [NV][Q3], gq [12][Q3], lq [12][Q3] (later Gi, Gv [3][NV][Q3] each).  The lift is
+  // interpolated first, with its scratch over RR, uq and gq where that is large enough; then U, with its scratch
+  // in gq; then the gradients of v, their x-passes over LF and RR (dead by then), their y-passes beyond lq.
+  using I12 = Contract3<12, N, Q, R>;
+  using IU = Contract3<NV, N, Q, R>;
+  using GV = Grad3<4, N, Q, R>;
+  using DV = Div3<NV, N, Q, R>;
+  static constexpr int UQ = W, GQ = UQ + NV * Q3, LQ = GQ + 12 * Q3;
+  static constexpr int LQ_SCRATCH = up4(I12::T1) + I12::T2;
+  static constexpr int L_AT = LQ - RR >= LQ_SCRATCH ? RR : LQ + 12 * Q3;
+  static constexpr int IU_SCRATCH = up4(IU::T1) + IU::T2;
+  static constexpr int U_AT = 12 * Q3 >= IU_SCRATCH ? GQ : LQ + 12 * Q3;
+  static constexpr int X_AT = W - LF >= GV::X ? LF : LQ + 12 * Q3 + GV::Y;
+  static constexpr int Y_AT = LQ + 12 * Q3;
+  static constexpr int GI = LQ, GVI = GI + 3 * NV * Q3, G_END = GI + (SPLIT ? 6 : 3) * NV * Q3;
+  // div3's x-pass results go to the dead uq/gq region when they fit there, otherwise beyond Gi/Gv
+  static constexpr int A_AT = DV::A <= LQ - UQ ? UQ : G_END;
+  static constexpr int VOL = cmax(cmax(cmax(L_AT == RR ? 0 : L_AT + LQ_SCRATCH, U_AT == GQ ? 0 : U_AT + IU_SCRATCH),
+                                       cmax(Y_AT + GV::Y, X_AT == LF ? 0 : X_AT + GV::X)),
+                                  cmax(G_END, A_AT == UQ ? 0 : A_AT + DV::A));
+  // phase D: hc [6][C][QF2] face fluxes (later the M^-1 result or the residual rows), tmp, face sums hs (later
+  // the M^-1 partial sums); the affine product's scratch goes over hc and tmp, its result to hs
+  static constexpr int CSH = (NV + 16 / (int)sizeof(R) - 1) / (16 / (int)sizeof(R)) * (16 / (int)sizeof(R));
+  static constexpr int CS = SPLIT ? 2 * CSH : CSH;
+  using MC = Contract3<C, N, N, R>;
+  static constexpr int D_TMP = up4(6 * C * QF2);
+  static constexpr int D_HS = up4(cmax(cmax(D_TMP + 6 * C * PT, up4(MC::T1) + MC::T2), CS * N3));
+  static constexpr int FIN = D_HS + cmax(6 * C * PB, 4 * NV * N3);
+  static constexpr int TOTAL = cmax(W + LIFT, cmax(VOL, W + FIN));
 };
 
 // Lift + volume + finalize of one hexahedron (see the file comment).  SPLIT keeps the inviscid
 // and viscous residuals apart (right-hand-side outputs, the MOOD step's viscous residual).
 template <int P, int NV, bool SPLIT, typename R = double>
-__global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) k_hex_element(const DevPlan P_, const StatePtrs S, const HexTables tables,
-                                                         const HexCodes codes, const FinalizeArgs A) {
+__global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) k_hex_element(const __grid_constant__ DevPlan P_, const StatePtrs S,
+                                                         const __grid_constant__ HexTablesT<R> tables,
+                                                         const HexCodes codes, const __grid_constant__ FinalizeArgs A) {
   using D = HexDims<P>;
   using L = HexElemSmem<P, NV, SPLIT, R>;
   constexpr int N = D::N, Q = D::Q, QF = D::QF, N2 = D::N2, N3 = D::N3, Q3 = D::Q3, QF2 = D::QF2;
@@ -485,26 +513,23 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) 
   constexpr int b = 0;
   extern __shared__ __align__(16) unsigned char dyn_smem[];
   R* smem = reinterpret_cast<R*>(dyn_smem);
-  HexTablesT<R>* tb = reinterpret_cast<HexTablesT<R>*>(smem);
   R* U = smem + L::U;            // [NV][N3] minus anchor
   R* V = smem + L::V;            // [4][N3]
   R* Lf = smem + L::LF;          // [12][N3] nodal lift
   R* Rr = smem + L::RR;          // [C][N3] residuals (inviscid, then viscous)
   R* W = smem + L::W;
-  __shared__ int node2lex[64], fslot[6], fperm[6], fface[6];
-  __shared__ double anchor_d[NV];
-  __shared__ R anchor[NV];
+  __shared__ int node2lex[64], lex2node[64], fslot[6], fperm[6], fface[6];
+  __shared__ R anchor[NV], w1[Q];
   const BlockDev& B = P_.blk[b];
   const FaceDev& fd = P_.face[1];
   const int e = blockIdx.x;
   if ((A.only && !A.only[e]) || (A.skip && A.skip[e])) return;     // uniform across the CTA
   const CaseView cv = case_view(P_.ph, B.ecase, e);
-  load_tables<P>(tables, tb);
   const double* Ug = S.b[b] + (size_t)e * N3 * NV;
-  if (threadIdx.x < NV) {
-    anchor_d[threadIdx.x] = Ug[threadIdx.x];
-    anchor[threadIdx.x] = (R)Ug[threadIdx.x];
-  }
+  // the state arrives in one coalesced sweep (raw: the head of the scratch) and is spread from shared memory
+  double* raw = reinterpret_cast<double*>(W);
+  static_assert((L::TOTAL - L::W) * (int)sizeof(R) >= N3 * NV * (int)sizeof(double) && L::W * sizeof(R) % 8 == 0, "raw state");
+  for (int idx = threadIdx.x; idx < N3 * NV; idx += kThreads) raw[idx] = Ug[idx];
   if (threadIdx.x < 6) {
     int ft, f, side;
     decode_face(B.elem_face[e * 6 + threadIdx.x], ft, f, side);
@@ -512,12 +537,16 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) 
     fperm[threadIdx.x] = (side == 0 ? fd.oc[f] : fd.nc[f]) * QF2;
     fface[threadIdx.x] = (f << 1) | side;
   }
-  __syncthreads();
-  for (int l = threadIdx.x; l < N3; l += kThreads) node2lex[tb->lex2node[l]] = l;
-  for (int idx = threadIdx.x; idx < NV * N3; idx += kThreads) {
-    const int v = idx / N3, l = idx % N3;
-    U[idx] = (R)(Ug[tb->lex2node[l] * NV + v] - anchor_d[v]);
+  for (int l = threadIdx.x; l < N3; l += kThreads) {
+    const int node = codes.lex2node[l];
+    lex2node[l] = node;
+    node2lex[node] = l;
   }
+  __syncthreads();
+  if (threadIdx.x < NV) anchor[threadIdx.x] = (R)raw[threadIdx.x];
+  if (threadIdx.x == 0)
+#pragma unroll
+    for (int k = 0; k < Q; ++k) w1[k] = tables.w1[k];
   const bool visc = P_.viscous;
   const bool aff = B.affine && B.affine[e];
   // a predicted troubled element: only its viscous residual is used (the subcell scheme replaces
@@ -525,27 +554,31 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) 
   const bool skip_inv = SPLIT && A.skip_inviscid && A.skip_inviscid[e];
   const double* MT = B.minv + (size_t)e * N3 * N3;
   const float* MT32 = (sizeof(R) == sizeof(float) && B.minv32) ? B.minv32 + (size_t)e * N3 * N3 : nullptr;
-  if (visc) {
-    for (int l = threadIdx.x; l < N3; l += kThreads) {
-      const int node = tb->lex2node[l];
-      double u[NV], vv[4];
+  for (int l = threadIdx.x; l < N3; l += kThreads) {
+    const double* un = raw + lex2node[l] * NV;
+    double u[NV];
 #pragma unroll
-      for (int v = 0; v < NV; ++v) u[v] = Ug[node * NV + v];
+    for (int v = 0; v < NV; ++v) {
+      u[v] = un[v];
+      U[v * N3 + l] = (R)(u[v] - raw[v]);
+    }
+    if (visc) {
+      double vv[4];
       viscous_vars<NV>(P_.ph, u, vv);
 #pragma unroll
       for (int m = 0; m < 4; ++m) V[m * N3 + l] = (R)vv[m];
     }
+  }
+  if (visc) {
+    __syncthreads();                    // raw is dead
     // ---- phase B: nodal lift M^-1 sum_f B_f^T jump_f
     constexpr int CH = 72;
     R* jc = W;                        // [6][12][QF2] jumps at the canonical face points
-    R* tmp = jc + CH * QF2;           // [72][QF][N]
-    R* bs = tmp + CH * QF * N;        // [6][12][N2]
-    R* ball = bs + CH * N2;           // [12][N3]
-    R* ax = ball + 12 * N3;           // affine scratch [2][12][N3]
-    // dense-lift row groups of the non-affine elements: 6 channels padded to 16 bytes; the rows
-    // (2 LR N3 values) reach into ax, which only affine elements use
-    constexpr int LR = (6 * (int)sizeof(R) + 15) / 16 * 16 / (int)sizeof(R);
-    static_assert(2 * LR <= 36, "the dense-lift rows must fit in ball and ax");
+    R* tmp = W + L::B_TMP;            // [72][PT]
+    R* bs = W + L::B_BS;              // [6][12][PB]
+    R* ball = W + L::B_BALL;          // [12][N3]
+    // dense-lift row groups of the non-affine elements: 6 channels padded to 16 bytes
+    constexpr int LR = L::LR, PB = L::PB;
     // one face point per thread: its 12 jump components (contiguous) to the canonical point
     for (int it = threadIdx.x; it < 6 * QF2; it += kThreads) {
       const int lf = it / QF2, q = it % QF2;
@@ -572,7 +605,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) 
       }
     }
     __syncthreads();
-    tensor2<CH, QF, QF, N, N>(jc, bs, tmp, tb->bfT, tb->bfT);
+    contract2<CH, QF, N>(jc, bs, tmp, tables.bfT);
     for (int idx = threadIdx.x; idx < 12 * N3; idx += kThreads) {
       const int c = idx / N3, l = idx % N3;
       const int xyz[3] = {l % N, (l / N) % N, l / N2};
@@ -581,15 +614,15 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) 
       for (int lf = 0; lf < 6; ++lf) {
         int a0, end, a1, a2;
         hex_face_axes(lf, a0, end, a1, a2);
-        if (xyz[a0] == end) acc += bs[(lf * 12 + c) * N2 + xyz[a2] * N + xyz[a1]];
+        if (xyz[a0] == end) acc += bs[(lf * 12 + c) * PB + xyz[a2] * N + xyz[a1]];
       }
       // non-affine elements: rows of two 16-byte aligned groups of 6 channels (LR apart) in element
       // node order, for 16-byte loads in the dense M^-1 (summed in node order)
-      ball[aff ? idx : tb->lex2node[l] * 2 * LR + (c / 6) * LR + c % 6] = acc;
+      ball[aff ? idx : lex2node[l] * 2 * LR + (c / 6) * LR + c % 6] = acc;
     }
     __syncthreads();
     if (aff) {
-      tensor3<12, N, N, N, N, N, N, false>(ball, Lf, ax, ax + 12 * N3, tb->m1i, tb->m1i, tb->m1i);
+      contract3<12, N, N>(ball, Lf, W, W + up4(L::M3::T1), tables.m1i);
       const R cf = (R)B.acoef[e];
       for (int idx = threadIdx.x; idx < 12 * N3; idx += kThreads) Lf[idx] *= cf;
     } else {
@@ -617,11 +650,17 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) 
   // ---- phase C: volume terms (k_hex_volume's arithmetic with the lift from shared memory; the
   // gradient and divergence contractions share their intermediate passes, grad3 / div3)
   {
-    R* uq = W;                           // [NV][Q3]   U - anchor at volume points
-    R* gq = uq + NV * Q3;                // [12][Q3]   gradients of v: reference (3 x 4), then physical + lift
-    R* lq = gq + 12 * Q3;                // [12][Q3]   nodal lift at the points; Gi, Gv reuse this region
-    R* sc = lq + 12 * Q3;                // contraction scratch (before Gi, Gv are written)
-    tensor3<NV, N, N, N, Q, Q, Q, false>(U, uq, sc, sc + NV * N * N * Q, tb->bq, tb->bq, tb->bq);
+    R* uq = smem + L::UQ;                // [NV][Q3]   U - anchor at volume points
+    R* gq = smem + L::GQ;                // [12][Q3]   gradients of v: reference (3 x 4), then physical + lift
+    R* lq = smem + L::LQ;                // [12][Q3]   nodal lift at the points; Gi, Gv reuse this region
+    if (visc) {
+      R* sc = smem + L::L_AT;
+      contract3<12, N, Q>(Lf, lq, sc, sc + up4(L::I12::T1), tables.bq);
+    }
+    {
+      R* sc = smem + L::U_AT;
+      contract3<NV, N, Q>(U, uq, sc, sc + up4(L::IU::T1), tables.bq);
+    }
     const double* jinv = B.jinv + (size_t)e * Q3 * 9;
     const float* jinv32 = (sizeof(R) == sizeof(float) && B.jinv32) ? B.jinv32 + (size_t)e * Q3 * 9 : nullptr;
     const double* wdet = B.wdet + (size_t)e * Q3;
@@ -632,8 +671,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) 
       deta = (R)B.adet[e];
     }
     if (visc) {
-      tensor3<12, N, N, N, Q, Q, Q, false>(Lf, lq, sc, sc + 12 * N * N * Q, tb->bq, tb->bq, tb->bq);
-      grad3<4, N, Q>(V, gq, sc, tb->bq, tb->dq);
+      grad3<4, N, Q>(V, gq, smem + L::X_AT, smem + L::Y_AT, tables.bq, tables.dq);
       // reference -> physical gradient per point, plus the lift at the point
       for (int q = threadIdx.x; q < Q3; q += kThreads) {
         R J[9], gr[12];
@@ -665,7 +703,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) 
       R J[9];
 #pragma unroll
       for (int k = 0; k < 9; ++k) J[k] = aff ? Ja[k] : (jinv32 ? (R)jinv32[q * 9 + k] : (R)jinv[q * 9 + k]);
-      const R wq = aff ? tb->w1[q / (Q * Q)] * tb->w1[(q / Q) % Q] * tb->w1[q % Q] * deta : (R)wdet[q];
+      const R wq = aff ? w1[q / (Q * Q)] * w1[(q / Q) % Q] * w1[q % Q] * deta : (R)wdet[q];
       R Uq[NV], F[3][NV];
 #pragma unroll
       for (int v = 0; v < NV; ++v) Uq[v] = anchor[v] + uq[v * Q3 + q];
@@ -708,16 +746,16 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) 
     __syncthreads();
     R* Ri = Rr;
     R* Rv = Rr + NV * N3;
-    R* A = W + L::DIV_AT;                 // uq and gq are dead: the x-pass results go there if they fit
+    R* A = smem + L::A_AT;                // uq and gq are dead: the x-pass results go there if they fit
     if (skip_inv) {
       for (int idx = threadIdx.x; idx < NV * N3; idx += kThreads) Ri[idx] = R(0);
       __syncthreads();
     } else {
-      div3<NV, N, Q>(Gi, Ri, A, tb->bqT, tb->dqT);
+      div3<NV, N, Q>(Gi, Ri, A, tables.bqT, tables.dqT);
     }
     if (SPLIT) {
       if (visc) {
-        div3<NV, N, Q>(Gv, Rv, A, tb->bqT, tb->dqT);
+        div3<NV, N, Q>(Gv, Rv, A, tables.bqT, tables.dqT);
       } else {
         for (int idx = threadIdx.x; idx < NV * N3; idx += kThreads) Rv[idx] = R(0);
         __syncthreads();
@@ -726,8 +764,8 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) 
   }
   // ---- phase D: face terms, M^-1, stage update (k_hex_finalize with the residuals in shared memory)
   R* hc = W;                                    // [6][C][QF2] face flux at canonical points
-  R* tmp = hc + 6 * C * QF2;                    // [6][C][QF][N]
-  R* hs = tmp + 6 * C * QF * N;                 // [6][C][N2]; reused for the M^-1 partial sums
+  R* tmp = W + L::D_TMP;                        // [6][C][PT]
+  R* hs = W + L::D_HS;                          // [6][C][PB]; reused for the M^-1 partial sums
   const size_t base = (size_t)e * N3 * NV;
   // one face point per thread: its NV inviscid and NV viscous flux values (contiguous)
   for (int it = threadIdx.x; it < 6 * QF2; it += kThreads) {
@@ -761,13 +799,11 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) 
     }
   }
   __syncthreads();
-  tensor2<6 * C, QF, QF, N, N>(hc, hs, tmp, tb->bfT, tb->bfT);
+  contract2<6 * C, QF, N>(hc, hs, tmp, tables.bfT);
   // non-affine elements: the residuals go to rows RrT [N3][CS] in element node order (inviscid
   // channels, then from CSH the viscous ones) in the dead hc/tmp region, for pair loads in the
   // dense M^-1
-  constexpr int CSH = (NV + 16 / (int)sizeof(R) - 1) / (16 / (int)sizeof(R)) * (16 / (int)sizeof(R));
-  constexpr int CS = SPLIT ? 2 * CSH : CSH;
-  static_assert(CS * N3 <= 6 * C * (QF2 + QF * N), "the residual rows must end before hs");
+  constexpr int CSH = L::CSH, CS = L::CS;
   R* RrT = W;
   for (int idx = threadIdx.x; idx < C * N3; idx += kThreads) {
     const int c = idx / N3, l = idx % N3;
@@ -777,35 +813,41 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) 
     for (int lf = 0; lf < 6; ++lf) {
       int a0, end, a1, a2;
       hex_face_axes(lf, a0, end, a1, a2);
-      if (xyz[a0] == end) acc += hs[(lf * C + c) * N2 + xyz[a2] * N + xyz[a1]];
+      if (xyz[a0] == end) acc += hs[(lf * C + c) * L::PB + xyz[a2] * N + xyz[a1]];
     }
     if (aff)
       Rr[idx] = acc;
     else
-      RrT[tb->lex2node[l] * CS + (c < NV ? c : CSH + c - NV)] = acc;
+      RrT[lex2node[l] * CS + (c < NV ? c : CSH + c - NV)] = acc;
   }
   __syncthreads();
-  auto emit = [&](size_t o, double ri, double rv) {
-    if (!A.stage) {
-      if (A.out_inv[b]) A.out_inv[b][o] = ri;
-      if (SPLIT && A.out_vis[b]) A.out_vis[b][o] = rv;
-    } else {
-      const double total = SPLIT ? ri + rv : ri;
-      const double eul = S.b[b][o] + A.dt * total;
-      if (SPLIT && A.out_vis[b]) A.out_vis[b][o] = rv;
-      if (A.euler[b]) A.euler[b][o] = eul;
-      A.dst[b][o] = A.alpha * A.base[b][o] + A.beta * eul;
+  // values idx (node-major, as in memory) of the residuals, inviscid and viscous: coalesced stores
+  auto emit = [&](const R* inv, const R* vis, R cf) {
+    for (int idx = threadIdx.x; idx < NV * N3; idx += kThreads) {
+      const size_t o = base + idx;
+      const double ri = (double)(cf * inv[idx]), rv = SPLIT ? (double)(cf * vis[idx]) : 0.0;
+      if (!A.stage) {
+        if (A.out_inv[b]) A.out_inv[b][o] = ri;
+        if (SPLIT && A.out_vis[b]) A.out_vis[b][o] = rv;
+      } else {
+        const double total = SPLIT ? ri + rv : ri;
+        const double eul = S.b[b][o] + A.dt * total;
+        if (SPLIT && A.out_vis[b]) A.out_vis[b][o] = rv;
+        if (A.euler[b]) A.euler[b][o] = eul;
+        A.dst[b][o] = A.alpha * A.base[b][o] + A.beta * eul;
+      }
     }
   };
+  R* rows = U;                                        // [C / NV][N3][NV] results in memory order (U, V, LF are dead)
+  static_assert(2 * NV * N3 <= L::RR, "the results must fit in the dead nodal arrays");
   if (aff) {
-    tensor3<C, N, N, N, N, N, N, false>(Rr, hs, tmp, hc, tb->m1i, tb->m1i, tb->m1i);
-    const R cf = (R)B.acoef[e];
-    for (int idx = threadIdx.x; idx < NV * N3; idx += kThreads) {
-      const int v = idx / N3, l = idx % N3;
-      const double ri = (double)(cf * hs[v * N3 + l]);
-      const double rv = SPLIT ? (double)(cf * hs[(NV + v) * N3 + l]) : 0.0;
-      emit(base + (size_t)tb->lex2node[l] * NV + v, ri, rv);
+    contract3<C, N, N>(Rr, hs, W, W + up4(L::MC::T1), tables.m1i);
+    for (int idx = threadIdx.x; idx < C * N3; idx += kThreads) {
+      const int c = idx / N3, l = idx % N3;
+      rows[(c / NV) * NV * N3 + lex2node[l] * NV + c % NV] = hs[idx];
     }
+    __syncthreads();
+    emit(rows, rows + NV * N3, (R)B.acoef[e]);
     return;
   }
   constexpr int VB = NV < 8 ? NV : 8;
@@ -852,8 +894,11 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) 
       si += part[(2 * NV + v) * N3 + i];
       sv += part[(3 * NV + v) * N3 + i];
     }
-    emit(base + (size_t)i * NV + v, (double)si, (double)sv);
+    rows[i * NV + v] = si;
+    if (SPLIT) rows[NV * N3 + i * NV + v] = sv;
   }
+  __syncthreads();
+  emit(rows, rows + NV * N3, R(1));
 }
 
 // Predictor statistics of the hexahedron block (the layout of k_elem_stats), one warp per element:

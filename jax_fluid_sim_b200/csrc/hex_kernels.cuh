@@ -42,6 +42,7 @@ static_assert(offsetof(HexTablesT<float>, lex2node) == kHexTableValues * sizeof(
 struct HexCodes {
   const uint8_t* perm;   // [codes][QF*QF]: owner face-point order -> canonical face grid index
   const int8_t* face;    // [codes]: local face of the code
+  const int32_t* lex2node;   // [N3] as in the tables (lanes read it at their own indices)
 };
 
 template <int P>
@@ -185,6 +186,95 @@ __device__ __forceinline__ void warp_tensor3(const T* in, T* out, T* t1, T* t2, 
   __syncwarp();
 }
 
+// ------------------------------------------------------------------------------------------
+// Contraction passes of the fused kernels (traces, element).  They differ from pencil above in where
+// their operands come from, which is what bounds these kernels (profiled: 70 to 85 % of the shared-memory
+// pipe's wavefronts, a quarter of them the matrices' own loads and up to half of them bank conflicts):
+//  - the matrix is read from the kernel's parameters (constant bank), not from shared memory;
+//  - planes of 16 values between passes are laid out 20 apart and, in float64, planes of 20
+//    values 21 apart: a pass reads and writes one value of every line at a time, 4 (5) lines to a plane,
+//    and those strides put the planes of a half warp (float64) or warp (float32) on distinct banks;
+//  - alignment and strides are known at compile time.
+// The sums are pencil's, value for value.
+template <typename T>
+__host__ __device__ constexpr int plane(int n) { return n == 16 ? 20 : (n == 20 && sizeof(T) == 8 ? 21 : n); }
+
+// Rotation of the thread <-> line assignment of a pass, so that passes issued back to back without a
+// barrier between them start on different threads.
+__device__ __forceinline__ int rotated(int offset) {
+  return (int)((threadIdx.x + kThreads - (unsigned)offset % kThreads) % kThreads);
+}
+
+template <int IN, int OUT, int LINES, int IST, int OST, bool VIN, bool VOUT, typename T, typename InBase, typename OutBase>
+__device__ __forceinline__ void pass(const T* in, T* out, const T* M, InBase in_base, OutBase out_base, int first) {
+  constexpr int VW = 16 / sizeof(T);
+  for (int line = first; line < LINES; line += kThreads) {
+    const T* src = in + in_base(line);
+    T x[IN];
+    if constexpr (VIN && IST == 1 && IN % VW == 0) {
+#pragma unroll
+      for (int i = 0; i < IN; i += VW) load16(src + i, &x[i]);
+    } else {
+#pragma unroll
+      for (int i = 0; i < IN; ++i) x[i] = src[i * IST];
+    }
+    T y[OUT];
+#pragma unroll
+    for (int o = 0; o < OUT; ++o) {
+      T s = T(0);
+#pragma unroll
+      for (int i = 0; i < IN; ++i) s += M[o * IN + i] * x[i];
+      y[o] = s;
+    }
+    T* dst = out + out_base(line);
+    if constexpr (VOUT && OST == 1 && OUT % VW == 0) {
+#pragma unroll
+      for (int o = 0; o < OUT; o += VW) store16(dst + o, &y[o]);
+    } else {
+#pragma unroll
+      for (int o = 0; o < OUT; ++o) dst[o * OST] = y[o];
+    }
+  }
+}
+
+// Scratch of contract3: t1 then t2.
+template <int C, int I, int O, typename T>
+struct Contract3 {
+  static constexpr int P1 = plane<T>(I * O), P2 = plane<T>(O * O);
+  static constexpr int T1 = C * I * P1, T2 = C * I * P2;
+};
+
+// out[c][oz][oy][ox] = sum M[oz][iz] M[oy][iy] M[ox][ix] in[c][iz][iy][ix]; in and out are dense, in 16-byte
+// aligned; ends with a barrier.
+template <int C, int I, int O, typename T>
+__device__ __forceinline__ void contract3(const T* in, T* out, T* t1, T* t2, const T* M) {
+  using X = Contract3<C, I, O, T>;
+  constexpr int P1 = X::P1, P2 = X::P2, OO = O * O;
+  pass<I, O, C * I * I, 1, 1, (I * (int)sizeof(T)) % 16 == 0, (O * (int)sizeof(T)) % 16 == 0 && (P1 * (int)sizeof(T)) % 16 == 0>(
+      in, t1, M, [](int l) { return l * I; }, [](int l) { return (l / I) * P1 + (l % I) * O; }, rotated(0));
+  __syncthreads();
+  pass<I, O, C * I * O, O, O, false, false>(
+      t1, t2, M, [](int l) { return (l / O) * P1 + l % O; }, [](int l) { return (l / O) * P2 + l % O; }, rotated(0));
+  __syncthreads();
+  pass<I, O, C * OO, P2, OO, false, false>(
+      t2, out, M, [](int l) { return (l / OO) * I * P2 + l % OO; }, [](int l) { return (l / OO) * O * OO + l % OO; },
+      rotated(0));
+  __syncthreads();
+}
+
+// 2-D: out[c][k2][k1] (channel stride plane(K K)) = sum M[k2][j2] M[k1][j1] in[c][j2][j1]; t: C plane(J K)
+// values of scratch; in dense and 16-byte aligned; ends with a barrier.
+template <int C, int J, int K, typename T>
+__device__ __forceinline__ void contract2(const T* in, T* out, T* t, const T* M) {
+  constexpr int PT = plane<T>(J * K), PO = plane<T>(K * K);
+  pass<J, K, C * J, 1, 1, (J * (int)sizeof(T)) % 16 == 0, (K * (int)sizeof(T)) % 16 == 0 && (PT * (int)sizeof(T)) % 16 == 0>(
+      in, t, M, [](int l) { return l * J; }, [](int l) { return (l / J) * PT + (l % J) * K; }, rotated(0));
+  __syncthreads();
+  pass<J, K, C * K, K, K, false, false>(
+      t, out, M, [](int l) { return (l / K) * PT + l % K; }, [](int l) { return (l / K) * PO + l % K; }, rotated(0));
+  __syncthreads();
+}
+
 // 2-D: out[c][k2][k1] = sum M2[k2][j2] M1[k1][j1] in[c][j2][j1]
 template <int C, int J1, int J2, int K1, int K2, typename T>
 __device__ __forceinline__ void tensor2(const T* in, T* out, T* t, const T* M1, const T* M2) {
@@ -220,11 +310,15 @@ struct HexSmem {
   static constexpr int T = (int)((sizeof(HexTablesT<R>) + 15) / 16 * 16 / sizeof(R));
   static constexpr int MS = N3 + 1;                 // padded row stride of the staged M^-1 (transposed)
   // traces: U, v, then the six faces' slabs, contraction scratch, face values and tangential derivatives
-  static constexpr int TR_U = T, TR_V = TR_U + NV * N3, TR_W = TR_V + 4 * N3;
-  // The face values alias the slabs when the three face contractions run as one merged pass (every read of
-  // the slabs comes before the barrier after which the face values are written); N2 == QF2 at P1-P3.
-  static constexpr bool TR_ALIAS = (NV + 4) * N3 >= 24 * N * QF && N2 == QF2;
-  static constexpr int TRACES = TR_W + 6 * (NV + 8) * (N2 + N * QF + (TR_ALIAS ? 0 : QF2)) + 2 * 24 * QF2;
+  static constexpr int TR_U = 0, TR_V = TR_U + NV * N3, TR_W = (TR_V + 4 * N3 + 3) / 4 * 4;
+  // slabs [CH][N2], then the x-passes' results [CH][plane] and the df pass [24][plane], then the derivatives
+  // g1, g2 [24][QF2] each.  The face values alias the slabs: every read of the slabs comes before the
+  // barrier after which the face values are written; N2 == QF2 at P1-P3.
+  static constexpr int TR_CH = 6 * (NV + 8), TR_PL = plane<R>(N * QF);
+  static_assert(N2 == QF2, "the face values take the slabs' place");
+  static constexpr int TR_T = TR_W + (TR_CH * N2 + 3) / 4 * 4, TR_D = TR_T + TR_CH * TR_PL;
+  static constexpr int TR_G = (NV + 4) * N3 >= 24 * TR_PL ? TR_D : TR_D + 24 * TR_PL;   // the df pass goes over U, V if it fits
+  static constexpr int TRACES = TR_G + 2 * 24 * QF2;
   // lift: staged M^-T, b per face on its slab, b on all nodes, scratch
   static constexpr int LI_BS = T, LI_B = LI_BS + 6 * 12 * N2, LI_W = LI_B + 12 * N3;
   static constexpr int LI_X = LI_W + 72 * QF2 + 72 * QF * N + 72 * N2 + 72 * QF2;   // affine scratch
@@ -274,33 +368,35 @@ __device__ __forceinline__ void stage_minv(const double* Mg, const int* lex2node
 // gradients, for each of the six faces, in the owner's face-point order.
 // F32: the viscous traces go to the float32 buffers trV32 / trG32 (fused form, mixed precision).
 template <int P, int NV, typename R = double, bool F32 = false>
-__global__ void __launch_bounds__(kThreads) k_hex_traces(const DevPlan P_, const StatePtrs S, int b,
-                                                        const HexTables tables, const HexCodes codes) {
+__global__ void __launch_bounds__(kThreads) k_hex_traces(const __grid_constant__ DevPlan P_, const StatePtrs S, int b,
+                                                        const __grid_constant__ HexTablesT<R> tables,
+                                                        const HexCodes codes) {
   using D = HexDims<P>;
   using L = HexSmem<P, NV, R>;
   constexpr int N = D::N, QF = D::QF, N2 = D::N2, N3 = D::N3, QF2 = D::QF2;
   extern __shared__ __align__(16) unsigned char dyn_smem[];
   R* smem = reinterpret_cast<R*>(dyn_smem);
-  HexTablesT<R>* tb = reinterpret_cast<HexTablesT<R>*>(smem);
   R* U = smem + L::TR_U;             // [NV][N3], minus anchor
   R* V = smem + L::TR_V;             // [4][N3]
   // all six faces at once, channel blocks [U: 6*NV][v: 6*4][dv/dn: 6*4], each of N2 (slabs)
   // or QF2 (face points) values
-  constexpr int CH = 6 * (NV + 8);
+  constexpr int CH = L::TR_CH, PL = L::TR_PL;
   R* slabs = smem + L::TR_W;
-  R* ftmp = slabs + CH * N2;         // tensor2 scratch [CH][N][QF]
-  // [CH][QF2] values at the canonical face points (over the slabs when the layout aliases them)
-  R* fo = L::TR_ALIAS ? slabs : ftmp + CH * N * QF;
-  R* g1 = L::TR_ALIAS ? ftmp + CH * N * QF : fo + CH * QF2;   // [6*4][QF2] derivative of v along a1
+  R* ftmp = smem + L::TR_T;          // x-passes [CH][PL]
+  // [CH][QF2] values at the canonical face points, the second face axis fastest (a pass then stores whole lines)
+  R* fo = slabs;
+  R* g1 = smem + L::TR_G;            // [6*4][QF2] derivative of v along a1 (same order)
   R* g2 = g1 + 24 * QF2;             // [6*4][QF2] derivative of v along a2
   __shared__ int fslot[6], fperm[6];
   const BlockDev& B = P_.blk[b];
   const FaceDev& fd = P_.face[1];
   const int e = blockIdx.x;
-  load_tables<P>(tables, tb);
   const double* Ug = S.b[b] + (size_t)e * N3 * NV;
   __shared__ double anchor[NV];
-  if (threadIdx.x < NV) anchor[threadIdx.x] = Ug[threadIdx.x];
+  // the state arrives in one coalesced sweep (raw takes the place of ftmp) and is spread from shared memory
+  double* raw = reinterpret_cast<double*>(ftmp);
+  static_assert(CH * PL * (int)sizeof(R) >= N3 * NV * (int)sizeof(double) && L::TR_T * sizeof(R) % 8 == 0, "raw state");
+  for (int idx = threadIdx.x; idx < N3 * NV; idx += kThreads) raw[idx] = Ug[idx];
   if (threadIdx.x < 6) {
     int ft, f, side;
     decode_face(B.elem_face[e * 6 + threadIdx.x], ft, f, side);
@@ -308,17 +404,18 @@ __global__ void __launch_bounds__(kThreads) k_hex_traces(const DevPlan P_, const
     fperm[threadIdx.x] = (side == 0 ? fd.oc[f] : fd.nc[f]) * QF2;
   }
   __syncthreads();
-  for (int idx = threadIdx.x; idx < NV * N3; idx += kThreads) {
-    const int v = idx / N3, l = idx % N3;
-    U[idx] = (R)(Ug[tb->lex2node[l] * NV + v] - anchor[v]);
-  }
+  if (threadIdx.x < NV) anchor[threadIdx.x] = raw[threadIdx.x];
   const bool visc = P_.viscous;
-  if (visc) {
-    for (int l = threadIdx.x; l < N3; l += kThreads) {
-      const int node = tb->lex2node[l];
-      double u[NV], vv[4];
+  for (int l = threadIdx.x; l < N3; l += kThreads) {
+    const double* un = raw + codes.lex2node[l] * NV;
+    double u[NV];
 #pragma unroll
-      for (int v = 0; v < NV; ++v) u[v] = Ug[node * NV + v];
+    for (int v = 0; v < NV; ++v) {
+      u[v] = un[v];
+      U[v * N3 + l] = (R)(u[v] - raw[v]);
+    }
+    if (visc) {
+      double vv[4];
       viscous_vars<NV>(P_.ph, u, vv);
 #pragma unroll
       for (int m = 0; m < 4; ++m) V[m * N3 + l] = (R)vv[m];
@@ -335,7 +432,9 @@ __global__ void __launch_bounds__(kThreads) k_hex_traces(const DevPlan P_, const
 #pragma unroll
     for (int m = 0; m < NV; ++m) slabs[(lf * NV + m) * N2 + j] = U[m * N3 + at];
     if (visc) {
-      const R* dn = end ? tb->d1 : tb->d0;
+      R dn[N];
+#pragma unroll
+      for (int j0 = 0; j0 < N; ++j0) dn[j0] = end ? tables.d1[j0] : tables.d0[j0];
 #pragma unroll
       for (int m = 0; m < 4; ++m) {
         slabs[(6 * NV + lf * 4 + m) * N2 + j] = V[m * N3 + at];
@@ -347,40 +446,39 @@ __global__ void __launch_bounds__(kThreads) k_hex_traces(const DevPlan P_, const
     }
   }
   __syncthreads();
-  if (visc) {
-    if constexpr ((NV + 4) * N3 >= 24 * N * QF) {
-      // The three face contractions with two barriers instead of six: the x-passes (bf on every
-      // channel; df on the 24 v channels, into the U/V region, dead after the slab gather), then the
-      // y-passes (bf -> fo; bf on the df pass -> g1; df on the bf pass of the v channels -> g2).  Each
-      // output goes through the same two 1-D products as in three tensor2 calls.  Consecutive passes
-      // start on rotated threads so that the lines spread evenly.
-      R* xd = U;                                   // [24][N][QF]
+  // The face contractions with two barriers: the x-passes (bf on every channel; df on the 24 v channels,
+  // into the U/V region, dead after the slab gather, where it fits), then the y-passes (bf -> fo; bf on the
+  // df pass -> g1; df on the bf pass of the v channels -> g2).  Consecutive passes start on rotated
+  // threads so that the lines spread evenly.
+  {
+    auto i1 = [](int l) { return l * N; };
+    auto o1 = [](int l) { return (l / N) * PL + (l % N) * QF; };
+    constexpr bool VI = (N * (int)sizeof(R)) % 16 == 0, VO = (QF * (int)sizeof(R)) % 16 == 0 && (PL * (int)sizeof(R)) % 16 == 0;
+    auto i2 = [](int l) { return (l / QF) * PL + l % QF; };
+    auto o2 = [](int l) { return l * QF; };
+    constexpr bool VQ = (QF * (int)sizeof(R)) % 16 == 0;
+    if (visc) {
+      R* xd = L::TR_G == L::TR_D ? U : smem + L::TR_D;                 // [24][PL]
       const R* vsl = slabs + 6 * NV * N2;
-      const int st = kThreads;
-      auto rot = [st](int off) { return (int)((threadIdx.x + st - off % st) % st); };
-      auto i1 = [](int l) { return l * N; };
-      auto o1 = [](int l) { return l * QF; };
-      pencil<N, QF, false>(slabs, ftmp, tb->bf, CH * N, 1, 1, i1, o1, rot(0), st);
-      pencil<N, QF, false>(vsl, xd, tb->df, 24 * N, 1, 1, i1, o1, rot(CH * N), st);
+      pass<N, QF, CH * N, 1, 1, VI, VO>(slabs, ftmp, tables.bf, i1, o1, rotated(0));
+      pass<N, QF, 24 * N, 1, 1, VI, VO>(vsl, xd, tables.df, i1, o1, rotated(CH * N));
       __syncthreads();
-      auto i2 = [](int l) { return (l / QF) * N * QF + l % QF; };
-      auto o2 = [](int l) { return (l / QF) * QF * QF + l % QF; };
-      pencil<N, QF, false>(ftmp, fo, tb->bf, CH * QF, QF, QF, i2, o2, rot(0), st);
-      pencil<N, QF, false>(xd, g1, tb->bf, 24 * QF, QF, QF, i2, o2, rot(CH * QF), st);
-      pencil<N, QF, false>(ftmp + 6 * NV * N * QF, g2, tb->df, 24 * QF, QF, QF, i2, o2, rot(CH * QF + 24 * QF), st);
-      __syncthreads();
+      pass<N, QF, CH * QF, QF, 1, false, VQ>(ftmp, fo, tables.bf, i2, o2, rotated(0));
+      pass<N, QF, 24 * QF, QF, 1, false, VQ>(xd, g1, tables.bf, i2, o2, rotated(CH * QF));
+      pass<N, QF, 24 * QF, QF, 1, false, VQ>(ftmp + 6 * NV * PL, g2, tables.df, i2, o2, rotated(CH * QF + 24 * QF));
     } else {
-      tensor2<CH, N, N, QF, QF>(slabs, fo, ftmp, tb->bf, tb->bf);
-      tensor2<24, N, N, QF, QF>(slabs + 6 * NV * N2, g1, ftmp, tb->df, tb->bf);
-      tensor2<24, N, N, QF, QF>(slabs + 6 * NV * N2, g2, ftmp, tb->bf, tb->df);
+      pass<N, QF, 6 * NV * N, 1, 1, VI, VO>(slabs, ftmp, tables.bf, i1, o1, rotated(0));
+      __syncthreads();
+      pass<N, QF, 6 * NV * QF, QF, 1, false, VQ>(ftmp, fo, tables.bf, i2, o2, rotated(0));
     }
-  } else {
-    tensor2<6 * NV, N, N, QF, QF>(slabs, fo, ftmp, tb->bf, tb->bf);
   }
+  __syncthreads();
+  // canonical face point c = c2 QF + c1 is at c1 QF + c2 in fo, g1 and g2
+  auto swapped = [](int c) { return (c % QF) * QF + c / QF; };
   // one face point per thread from here on: its values are contiguous in the face buffers
   for (int it = threadIdx.x; it < 6 * QF2; it += kThreads) {
     const int lf = it / QF2, q = it % QF2;
-    const int c = codes.perm[fperm[lf] + q];
+    const int c = swapped(codes.perm[fperm[lf] + q]);
     double* dst = fd.trA + ((size_t)fslot[lf] + q) * NV;
 #pragma unroll
     for (int v = 0; v < NV; ++v) dst[v] = anchor[v] + (double)fo[(lf * NV + v) * QF2 + c];
@@ -393,7 +491,7 @@ __global__ void __launch_bounds__(kThreads) k_hex_traces(const DevPlan P_, const
     const R* gn = fv + 24 * QF2;              // [6][4][QF2]
     for (int it = threadIdx.x; it < 6 * QF2; it += kThreads) {
       const int lf = it / QF2, q = it % QF2;
-      const int c = codes.perm[fperm[lf] + q];
+      const int c = swapped(codes.perm[fperm[lf] + q]);
       const size_t pt = (size_t)fslot[lf] + q;
       // a point's 4 values and 12 gradients are contiguous: 16-byte stores
       R tv[4];

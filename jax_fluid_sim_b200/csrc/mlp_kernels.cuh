@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(kThreads) k_elem_stats(const DevPlan P, const 
 
 // One thread per element: neighbour means through the element's faces -> 8 features.
 // stats_all[b] points at block b's stats; features are written for block b at feat.
-__global__ void __launch_bounds__(kThreads) k_mlp_features(const DevPlan P, int b, const float* const* stats_all,
+static __global__ void __launch_bounds__(kThreads) k_mlp_features(const DevPlan P, int b, const float* const* stats_all,
                                                           float* __restrict__ feat) {
   const BlockDev& B = P.blk[b];
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(kThreads) k_mlp_features(const DevPlan P, int 
 // One thread per sample: normalised features -> probability; float16 weights staged in shared
 // memory (every thread reads the same weight: broadcast), float32 accumulation.
 // norm = [mean[8], inv_std[8]].  prob and/or flag (prob > threshold) may be null.
-__global__ void __launch_bounds__(128) k_mlp_infer(const __half* __restrict__ w16, const float* __restrict__ norm,
+static __global__ void __launch_bounds__(128) k_mlp_infer(const __half* __restrict__ w16, const float* __restrict__ norm,
                                                    const float* __restrict__ X, long long n, float threshold,
                                                    float* __restrict__ prob, uint8_t* __restrict__ flag) {
   __shared__ __half w[kMlpParams];
@@ -183,7 +183,7 @@ constexpr int kMlpTrainSmemFloats =
     kMlpIn * kWS + 2 * kMlpH * kWS + 4 * kMlpH + 1 + kMlpChunk * kMlpIn + 2 * kMlpChunk +
     3 * kMlpChunk * kMlpH + 2 * kMlpChunk * kMlpH + 2 * kMlpChunk;
 
-__global__ void __launch_bounds__(kMlpTrainThreads) k_mlp_train(const float* __restrict__ wts,
+static __global__ void __launch_bounds__(kMlpTrainThreads) k_mlp_train(const float* __restrict__ wts,
                                                                const float* __restrict__ norm,
                                                                const float* __restrict__ X,
                                                                const uint8_t* __restrict__ y,
@@ -327,7 +327,7 @@ __global__ void __launch_bounds__(kMlpTrainThreads) k_mlp_train(const float* __r
 }
 
 // Adam (Kingma & Ba 2015) on the float32 master weights; clears grad; refreshes the float16 copy.
-__global__ void k_mlp_adam(float* __restrict__ w, float* __restrict__ grad, float* __restrict__ m,
+static __global__ void k_mlp_adam(float* __restrict__ w, float* __restrict__ grad, float* __restrict__ m,
                            float* __restrict__ v, __half* __restrict__ w16, float lr, float b1, float b2,
                            float eps, float c1, float c2) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;

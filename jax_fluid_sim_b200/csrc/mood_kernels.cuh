@@ -421,7 +421,7 @@ __global__ void __launch_bounds__(kThreads) k_mood_update(const DevPlan P, const
   }
 }
 
-__global__ void k_blend(const double* base, const double* x, double alpha, double beta, double* out, size_t n) {
+static __global__ void k_blend(const double* base, const double* x, double alpha, double beta, double* out, size_t n) {
   const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (i < n) out[i] = alpha * base[i] + beta * x[i];
 }

@@ -124,7 +124,7 @@ __device__ __forceinline__ void subface_metrics(const double* pv, const int32_t*
 
 // One element per CTA; *bad receives 1 + the first element whose Gram matrix is not positive
 // definite.
-__global__ void __launch_bounds__(256) k_subcell_build(const SubcellRefDev r, const double* __restrict__ xyz_all,
+static __global__ void __launch_bounds__(256) k_subcell_build(const SubcellRefDev r, const double* __restrict__ xyz_all,
                                                        SubcellBuildOut o, int* bad) {
   extern __shared__ double sm[];
   const int S = r.S, Qs = r.Qs, ng = r.ng, V = r.V, Np = r.Np, cs = r.cs;
@@ -229,7 +229,7 @@ struct SubcellCentres {
 // matched to the owner's 16 (osub) by the nearest centre, both taken relative to their side's
 // mean; *bad receives 1 + the first face whose match is not a permutation or is farther than
 // 2e-6 of max(1, largest owner centre norm).
-__global__ void __launch_bounds__(256) k_subcell_match(const FaceDev fd, const SubcellCentres C,
+static __global__ void __launch_bounds__(256) k_subcell_match(const FaceDev fd, const SubcellCentres C,
                                                        const int32_t* __restrict__ osub,
                                                        const int32_t* __restrict__ ncand, int32_t* __restrict__ nsub,
                                                        int* bad) {
