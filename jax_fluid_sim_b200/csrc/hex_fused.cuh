@@ -354,150 +354,40 @@ __device__ __forceinline__ void lds_vec(const T* p, T* r) {
   for (int k = K8; k < K; ++k) r[k] = p[k];
 }
 
-// The three reference-gradient fields of C nodal channels at the Q^3 volume points,
-// g[r][c][Q3] = (d/dxi_r of the interpolant), by the sum-factorised passes with the intermediates
-// shared between directions: x (bq, dq), y (bq, dq on the bq branch; bq on the dq branch), z.  Each
-// output goes through the same three 1-D products as a separate contraction per direction, so the values
-// are the same; the barriers are three instead of nine.  X: 2 C N P1 values of scratch, Y: 3 C N P2.
-template <int C, int N, int Q, typename T>
-struct Grad3 {
-  static constexpr int P1 = plane<T>(N * Q), P2 = plane<T>(Q * Q), X = 2 * C * N * P1, Y = 3 * C * N * P2;
-};
-
-template <int C, int N, int Q, typename T>
-__device__ __forceinline__ void grad3(const T* V, T* g, T* X, T* Y, const T* bq, const T* dq) {
-  using G = Grad3<C, N, Q, T>;
-  constexpr int P1 = G::P1, P2 = G::P2, L1 = C * N * N, L2 = C * N * Q, L3 = C * Q * Q, Q3 = Q * Q * Q, QQ = Q * Q;
-  T* Bx = X;
-  T* Dx = Bx + C * N * P1;
-  T* BB = Y;
-  T* BD = BB + C * N * P2;
-  T* DB = BD + C * N * P2;
-  constexpr bool VI = (N * (int)sizeof(T)) % 16 == 0, VO = (Q * (int)sizeof(T)) % 16 == 0 && (P1 * (int)sizeof(T)) % 16 == 0;
-  auto i1 = [](int l) { return l * N; };
-  auto o1 = [](int l) { return (l / N) * P1 + (l % N) * Q; };
-  pass<N, Q, L1, 1, 1, VI, VO>(V, Bx, bq, i1, o1, rotated(0));
-  pass<N, Q, L1, 1, 1, VI, VO>(V, Dx, dq, i1, o1, rotated(L1));
-  __syncthreads();
-  auto i2 = [](int l) { return (l / Q) * P1 + l % Q; };
-  auto o2 = [](int l) { return (l / Q) * P2 + l % Q; };
-  pass<N, Q, L2, Q, Q, false, false>(Bx, BB, bq, i2, o2, rotated(0));
-  pass<N, Q, L2, Q, Q, false, false>(Bx, BD, dq, i2, o2, rotated(L2));
-  pass<N, Q, L2, Q, Q, false, false>(Dx, DB, bq, i2, o2, rotated(2 * L2));
-  __syncthreads();
-  auto i3 = [](int l) { return (l / QQ) * N * P2 + l % QQ; };
-  auto o3 = [](int l) { return (l / QQ) * Q * QQ + l % QQ; };
-  pass<N, Q, L3, P2, QQ, false, false>(DB, g + 0 * C * Q3, bq, i3, o3, rotated(0));
-  pass<N, Q, L3, P2, QQ, false, false>(BD, g + 1 * C * Q3, bq, i3, o3, rotated(L3));
-  pass<N, Q, L3, P2, QQ, false, false>(BB, g + 2 * C * Q3, dq, i3, o3, rotated(2 * L3));
-  __syncthreads();
-}
-
-// The weak divergence R[c][N3] = sum_r (transposed gradient of direction r) G[r][c][Q3], by three
-// passes (x, y with three inputs each, then z summing the three terms as (t0 + t1) + t2).  A: 3 C Q P1
-// values of scratch; the y-pass results overwrite G (3 C Q P2 values, at most its 3 C Q3).
-template <int C, int N, int Q, typename T>
-struct Div3 {
-  static constexpr int P1 = Q * N == 16 ? 20 : Q * N, P2 = Q * plane<T>(N * N) <= Q * Q * Q ? plane<T>(N * N) : N * N;
-  static constexpr int A = 3 * C * Q * P1;
-};
-
-template <int C, int N, int Q, typename T>
-__device__ __forceinline__ void div3(T* G, T* R, T* A, const T* bqT, const T* dqT) {
-  using X = Div3<C, N, Q, T>;
-  constexpr int P1 = X::P1, P2 = X::P2, Q3 = Q * Q * Q, NN = N * N, LX = C * Q * Q, LY = C * Q * N, LZ = C * NN;
-  constexpr int AS = C * Q * P1, BS = C * Q * P2;
-  constexpr bool VO = (N * (int)sizeof(T)) % 16 == 0 && (P1 * (int)sizeof(T)) % 16 == 0;
-  auto ix = [](int l) { return l * Q; };
-  auto ox = [](int l) { return (l / Q) * P1 + (l % Q) * N; };
-  pass<Q, N, LX, 1, 1, false, VO>(G + 0 * C * Q3, A + 0 * AS, dqT, ix, ox, rotated(0));
-  pass<Q, N, LX, 1, 1, false, VO>(G + 1 * C * Q3, A + 1 * AS, bqT, ix, ox, rotated(LX));
-  pass<Q, N, LX, 1, 1, false, VO>(G + 2 * C * Q3, A + 2 * AS, bqT, ix, ox, rotated(2 * LX));
-  __syncthreads();
-  T* B = G;                                    // [3][C][Q][P2]
-  auto iy = [](int l) { return (l / N) * P1 + l % N; };
-  auto oy = [](int l) { return (l / N) * P2 + l % N; };
-  pass<Q, N, LY, N, N, false, false>(A + 0 * AS, B + 0 * BS, bqT, iy, oy, rotated(0));
-  pass<Q, N, LY, N, N, false, false>(A + 1 * AS, B + 1 * BS, dqT, iy, oy, rotated(LY));
-  pass<Q, N, LY, N, N, false, false>(A + 2 * AS, B + 2 * BS, bqT, iy, oy, rotated(2 * LY));
-  __syncthreads();
-  for (int line = threadIdx.x; line < LZ; line += kThreads) {
-    const int ib = (line / NN) * Q * P2 + line % NN;
-    const int ob = (line / NN) * N * NN + line % NN;
-    T x0[Q], x1[Q], x2[Q];
-#pragma unroll
-    for (int i = 0; i < Q; ++i) {
-      x0[i] = B[0 * BS + ib + i * P2];
-      x1[i] = B[1 * BS + ib + i * P2];
-      x2[i] = B[2 * BS + ib + i * P2];
-    }
-#pragma unroll
-    for (int o = 0; o < N; ++o) {
-      T s0 = T(0), s1 = T(0), s2 = T(0);
-#pragma unroll
-      for (int i = 0; i < Q; ++i) s0 += bqT[o * Q + i] * x0[i];
-#pragma unroll
-      for (int i = 0; i < Q; ++i) s1 += bqT[o * Q + i] * x1[i];
-#pragma unroll
-      for (int i = 0; i < Q; ++i) s2 += dqT[o * Q + i] * x2[i];
-      T acc = s0;
-      acc += s1;
-      acc += s2;
-      R[ob + o * NN] = acc;
-    }
-  }
-  __syncthreads();
-}
-
 __host__ __device__ constexpr int up4(int n) { return (n + 3) / 4 * 4; }
 
-// Shared-memory layout of k_hex_element, in units of R.  The nodal arrays come first (U, V, LF the nodal
-// lift, RR the residuals), then the scratch W, which each phase lays out for itself; phases also use nodal
-// arrays that are not yet written or already dead.
+// Shared-memory layout of k_hex_element, in units of R.  Nodal arrays hold N planes of PS values a channel, the
+// point arrays Q3 values a channel.  The nodal U, V and lift LF stand side by side, so that their planes are
+// one list; the point arrays come over them once the planes have been read.
 template <int P, int NV, bool SPLIT, typename R>
 struct HexElemSmem {
   using D = HexDims<P>;
   static constexpr int N = D::N, Q = D::Q, QF = D::QF, N2 = D::N2, N3 = D::N3, Q3 = D::Q3, QF2 = D::QF2;
   static constexpr int C = SPLIT ? 2 * NV : NV;          // residual channels
-  static constexpr int U = 0, V = up4(U + NV * N3), LF = up4(V + 4 * N3), RR = up4(LF + 12 * N3);
-  static constexpr int W = up4(RR + C * N3);
-  // phase B: jumps jc, x-pass results tmp, face sums bs, nodal sums ball (or the non-affine elements' rows);
-  // the affine M^-1 product's scratch goes over jc and tmp
-  static constexpr int PT = plane<R>(QF * N), PB = plane<R>(N2);
+  static constexpr int PS = plane_stride<R>(N2), NS = N * PS, FP = plane_stride<R>(QF2), QQ = Q * Q;
+  static constexpr int U = 0, V = U + NV * NS, LF = V + 4 * NS, NODAL = up4(LF + 12 * NS);
+  // phase B, beyond the nodal arrays: face planes of the jumps (contracted in place), the nodal sums (or the
+  // non-affine elements' rows of two groups of 6 channels, LR apart)
   static constexpr int LR = (6 * (int)sizeof(R) + 15) / 16 * 16 / (int)sizeof(R);
-  static constexpr int B_TMP = up4(72 * QF2), B_BS = up4(B_TMP + 72 * PT), B_BALL = up4(B_BS + 72 * PB);
-  using M3 = Contract3<12, N, N, R>;
-  static constexpr int LIFT = cmax(B_BALL + cmax(12 * N3, 2 * LR * N3), 0);
-  static_assert(up4(M3::T1) + M3::T2 <= B_BALL, "the affine product's scratch ends before its input");
-  // phase C: uq [NV][Q3], gq [12][Q3], lq [12][Q3] (later Gi, Gv [3][NV][Q3] each).  The lift is
-  // interpolated first, with its scratch over RR, uq and gq where that is large enough; then U, with its scratch
-  // in gq; then the gradients of v, their x-passes over LF and RR (dead by then), their y-passes beyond lq.
-  using I12 = Contract3<12, N, Q, R>;
-  using IU = Contract3<NV, N, Q, R>;
-  using GV = Grad3<4, N, Q, R>;
-  using DV = Div3<NV, N, Q, R>;
-  static constexpr int UQ = W, GQ = UQ + NV * Q3, LQ = GQ + 12 * Q3;
-  static constexpr int LQ_SCRATCH = up4(I12::T1) + I12::T2;
-  static constexpr int L_AT = LQ - RR >= LQ_SCRATCH ? RR : LQ + 12 * Q3;
-  static constexpr int IU_SCRATCH = up4(IU::T1) + IU::T2;
-  static constexpr int U_AT = 12 * Q3 >= IU_SCRATCH ? GQ : LQ + 12 * Q3;
-  static constexpr int X_AT = W - LF >= GV::X ? LF : LQ + 12 * Q3 + GV::Y;
-  static constexpr int Y_AT = LQ + 12 * Q3;
-  static constexpr int GI = LQ, GVI = GI + 3 * NV * Q3, G_END = GI + (SPLIT ? 6 : 3) * NV * Q3;
-  // div3's x-pass results go to the dead uq/gq region when they fit there, otherwise beyond Gi/Gv
-  static constexpr int A_AT = DV::A <= LQ - UQ ? UQ : G_END;
-  static constexpr int VOL = cmax(cmax(cmax(L_AT == RR ? 0 : L_AT + LQ_SCRATCH, U_AT == GQ ? 0 : U_AT + IU_SCRATCH),
-                                       cmax(Y_AT + GV::Y, X_AT == LF ? 0 : X_AT + GV::X)),
-                                  cmax(G_END, A_AT == UQ ? 0 : A_AT + DV::A));
-  // phase D: hc [6][C][QF2] face fluxes (later the M^-1 result or the residual rows), tmp, face sums hs (later
-  // the M^-1 partial sums); the affine product's scratch goes over hc and tmp, its result to hs
+  static constexpr int JC = NODAL, BALL = up4(JC + 72 * FP), B_END = BALL + cmax(12 * NS, 2 * LR * N3);
+  // phase C: U - anchor uq [NV][Q3], gradients of v gq [12][Q3] and the lift lq [12][Q3] (later Gi, Gv [3][NV][Q3]
+  // each) at the points; half-contracted planes beyond them: U, V, LF (T2), then the two y and x derivatives of v
+  static constexpr int UQ = 0, GQ = UQ + NV * Q3, LQ = GQ + 12 * Q3;
+  static constexpr int T2 = up4(cmax(LQ + 12 * Q3, NODAL)), TBD = T2 + (NV + 16) * N * QQ, TDB = TBD + 4 * N * QQ;
+  static constexpr int T_END = TDB + 4 * N * QQ;
+  static constexpr int GI = LQ, GVI = GI + 3 * NV * Q3, G_END = up4(GI + (SPLIT ? 6 : 3) * NV * Q3);
+  // residuals [C][NS]: over uq and gq, dead by then, where they fit
+  static constexpr bool RR_IN = C * NS <= LQ;
+  // phase D: face planes hc [6][C][FP] (later the results in memory order), then the non-affine elements' rows
+  // of residuals and the M^-1 partial sums
   static constexpr int CSH = (NV + 16 / (int)sizeof(R) - 1) / (16 / (int)sizeof(R)) * (16 / (int)sizeof(R));
   static constexpr int CS = SPLIT ? 2 * CSH : CSH;
-  using MC = Contract3<C, N, N, R>;
-  static constexpr int D_TMP = up4(6 * C * QF2);
-  static constexpr int D_HS = up4(cmax(cmax(D_TMP + 6 * C * PT, up4(MC::T1) + MC::T2), CS * N3));
-  static constexpr int FIN = D_HS + cmax(6 * C * PB, 4 * NV * N3);
-  static constexpr int TOTAL = cmax(W + LIFT, cmax(VOL, W + FIN));
+  static constexpr int D_SIZE = up4(6 * C * FP) + up4(CS * N3) + 4 * NV * N3;
+  static constexpr int RR = RR_IN ? 0 : up4(cmax(G_END, D_SIZE)), RR_END = RR + up4(C * NS);
+  static constexpr int HC = RR_IN ? RR_END : 0, RT = HC + up4(6 * C * FP), PART = RT + up4(CS * N3);
+  static constexpr int D_END = cmax(HC + D_SIZE, RR_END);
+  static_assert(C * N3 <= 6 * C * FP, "the results take the face planes' place");
+  static constexpr int TOTAL = up4(cmax(cmax(B_END, T_END), cmax(G_END, D_END)));
 };
 
 // Lift + volume + finalize of one hexahedron (see the file comment).  SPLIT keeps the inviscid
@@ -513,11 +403,12 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) 
   constexpr int b = 0;
   extern __shared__ __align__(16) unsigned char dyn_smem[];
   R* smem = reinterpret_cast<R*>(dyn_smem);
-  R* U = smem + L::U;            // [NV][N3] minus anchor
-  R* V = smem + L::V;            // [4][N3]
-  R* Lf = smem + L::LF;          // [12][N3] nodal lift
-  R* Rr = smem + L::RR;          // [C][N3] residuals (inviscid, then viscous)
-  R* W = smem + L::W;
+  constexpr int PS = L::PS, NS = L::NS, FP = L::FP, QQ = L::QQ;
+  R* U = smem + L::U;            // [NV][NS] minus anchor
+  R* V = smem + L::V;            // [4][NS]
+  R* Lf = smem + L::LF;          // [12][NS] nodal lift
+  R* Rr = smem + L::RR;          // [C][NS] residuals (inviscid, then viscous)
+  auto nod = [](int l) { return l / N2 * PS + l % N2; };      // node l of a channel
   __shared__ int node2lex[64], lex2node[64], fslot[6], fperm[6], fface[6];
   __shared__ R anchor[NV], w1[Q];
   const BlockDev& B = P_.blk[b];
@@ -526,9 +417,10 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) 
   if ((A.only && !A.only[e]) || (A.skip && A.skip[e])) return;     // uniform across the CTA
   const CaseView cv = case_view(P_.ph, B.ecase, e);
   const double* Ug = S.b[b] + (size_t)e * N3 * NV;
-  // the state arrives in one coalesced sweep (raw: the head of the scratch) and is spread from shared memory
-  double* raw = reinterpret_cast<double*>(W);
-  static_assert((L::TOTAL - L::W) * (int)sizeof(R) >= N3 * NV * (int)sizeof(double) && L::W * sizeof(R) % 8 == 0, "raw state");
+  // the state arrives in one coalesced sweep (raw: beyond the nodal arrays) and is spread from shared memory
+  double* raw = reinterpret_cast<double*>(smem + L::NODAL);
+  static_assert((L::TOTAL - L::NODAL) * (int)sizeof(R) >= N3 * NV * (int)sizeof(double) && L::NODAL * sizeof(R) % 8 == 0,
+                "raw state");
   for (int idx = threadIdx.x; idx < N3 * NV; idx += kThreads) raw[idx] = Ug[idx];
   if (threadIdx.x < 6) {
     int ft, f, side;
@@ -560,25 +452,21 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) 
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
       u[v] = un[v];
-      U[v * N3 + l] = (R)(u[v] - raw[v]);
+      U[v * NS + nod(l)] = (R)(u[v] - raw[v]);
     }
     if (visc) {
       double vv[4];
       viscous_vars<NV>(P_.ph, u, vv);
 #pragma unroll
-      for (int m = 0; m < 4; ++m) V[m * N3 + l] = (R)vv[m];
+      for (int m = 0; m < 4; ++m) V[m * NS + nod(l)] = (R)vv[m];
     }
   }
   if (visc) {
     __syncthreads();                    // raw is dead
     // ---- phase B: nodal lift M^-1 sum_f B_f^T jump_f
-    constexpr int CH = 72;
-    R* jc = W;                        // [6][12][QF2] jumps at the canonical face points
-    R* tmp = W + L::B_TMP;            // [72][PT]
-    R* bs = W + L::B_BS;              // [6][12][PB]
-    R* ball = W + L::B_BALL;          // [12][N3]
-    // dense-lift row groups of the non-affine elements: 6 channels padded to 16 bytes
-    constexpr int LR = L::LR, PB = L::PB;
+    R* jc = smem + L::JC;             // [6][12][FP] jumps at the canonical face points, then their sums at the face nodes
+    R* ball = smem + L::BALL;         // [12][NS]
+    constexpr int LR = L::LR;
     // one face point per thread: its 12 jump components (contiguous) to the canonical point
     for (int it = threadIdx.x; it < 6 * QF2; it += kThreads) {
       const int lf = it / QF2, q = it % QF2;
@@ -589,23 +477,24 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) 
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
           const float4 v = src[k];
-          jc[(lf * 12 + 4 * k) * QF2 + cp] = v.x;
-          jc[(lf * 12 + 4 * k + 1) * QF2 + cp] = v.y;
-          jc[(lf * 12 + 4 * k + 2) * QF2 + cp] = v.z;
-          jc[(lf * 12 + 4 * k + 3) * QF2 + cp] = v.w;
+          jc[(lf * 12 + 4 * k) * FP + cp] = v.x;
+          jc[(lf * 12 + 4 * k + 1) * FP + cp] = v.y;
+          jc[(lf * 12 + 4 * k + 2) * FP + cp] = v.z;
+          jc[(lf * 12 + 4 * k + 3) * FP + cp] = v.w;
         }
       } else {
         const double2* src = reinterpret_cast<const double2*>(fd.jumpW + jo);
 #pragma unroll
         for (int k = 0; k < 6; ++k) {
           const double2 v = src[k];
-          jc[(lf * 12 + 2 * k) * QF2 + cp] = (R)v.x;
-          jc[(lf * 12 + 2 * k + 1) * QF2 + cp] = (R)v.y;
+          jc[(lf * 12 + 2 * k) * FP + cp] = (R)v.x;
+          jc[(lf * 12 + 2 * k + 1) * FP + cp] = (R)v.y;
         }
       }
     }
     __syncthreads();
-    contract2<CH, QF, N>(jc, bs, tmp, tables.bfT);
+    planes<QF, N, FP, FP, kThreads>(jc, jc, 72, tables.bfT, tables.bfT, threadIdx.x);
+    __syncthreads();
     for (int idx = threadIdx.x; idx < 12 * N3; idx += kThreads) {
       const int c = idx / N3, l = idx % N3;
       const int xyz[3] = {l % N, (l / N) % N, l / N2};
@@ -614,17 +503,28 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) 
       for (int lf = 0; lf < 6; ++lf) {
         int a0, end, a1, a2;
         hex_face_axes(lf, a0, end, a1, a2);
-        if (xyz[a0] == end) acc += bs[(lf * 12 + c) * PB + xyz[a2] * N + xyz[a1]];
+        if (xyz[a0] == end) acc += jc[(lf * 12 + c) * FP + xyz[a2] * N + xyz[a1]];
       }
       // non-affine elements: rows of two 16-byte aligned groups of 6 channels (LR apart) in element
       // node order, for 16-byte loads in the dense M^-1 (summed in node order)
-      ball[aff ? idx : lex2node[l] * 2 * LR + (c / 6) * LR + c % 6] = acc;
+      ball[aff ? c * NS + nod(l) : lex2node[l] * 2 * LR + (c / 6) * LR + c % 6] = acc;
     }
     __syncthreads();
     if (aff) {
-      contract3<12, N, N>(ball, Lf, W, W + up4(L::M3::T1), tables.m1i);
+      planes<N, N, PS, PS, kThreads>(ball, ball, 12 * N, tables.m1i, tables.m1i, threadIdx.x);
+      __syncthreads();
       const R cf = (R)B.acoef[e];
-      for (int idx = threadIdx.x; idx < 12 * N3; idx += kThreads) Lf[idx] *= cf;
+      for (int line = threadIdx.x; line < 12 * N2; line += kThreads) {
+        R x[N];
+        line_load<N, N2, PS, NS>(ball, line, x);
+#pragma unroll
+        for (int o = 0; o < N; ++o) {
+          R acc = R(0);
+#pragma unroll
+          for (int i = 0; i < N; ++i) acc += tables.m1i[o * N + i] * x[i];
+          Lf[line / N2 * NS + o * PS + line % N2] = acc * cf;
+        }
+      }
     } else {
       auto dense_lift = [&](const auto* M) {
         for (int idx = threadIdx.x; idx < 2 * N3; idx += kThreads) {
@@ -638,29 +538,40 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) 
 #pragma unroll
             for (int k = 0; k < 6; ++k) sacc[k] += m * bj[k];
           }
-          const int li = node2lex[i];
+          const int li = nod(node2lex[i]);
 #pragma unroll
-          for (int k = 0; k < 6; ++k) Lf[(c0 + k) * N3 + li] = sacc[k];
+          for (int k = 0; k < 6; ++k) Lf[(c0 + k) * NS + li] = sacc[k];
         }
       };
       if (MT32) dense_lift(MT32); else dense_lift(MT);
     }
   }
   __syncthreads();
-  // ---- phase C: volume terms (k_hex_volume's arithmetic with the lift from shared memory; the
-  // gradient and divergence contractions share their intermediate passes, grad3 / div3)
+  // ---- phase C: volume terms (k_hex_volume's arithmetic with the lift from shared memory)
   {
     R* uq = smem + L::UQ;                // [NV][Q3]   U - anchor at volume points
-    R* gq = smem + L::GQ;                // [12][Q3]   gradients of v: reference (3 x 4), then physical + lift
+    R* gq = smem + L::GQ;                // [3][4][Q3] reference gradients of v
     R* lq = smem + L::LQ;                // [12][Q3]   nodal lift at the points; Gi, Gv reuse this region
+    R* t2 = smem + L::T2;                // planes of U, V, LF contracted along x and y
+    R* tbd = smem + L::TBD;              // the same of V with the y derivative, and with the x derivative
+    R* tdb = smem + L::TDB;
+    // U, V and the lift as one list of planes, then V's derivatives; three directions share the planes:
+    // each gradient goes through the same three 1-D products as a contraction of its own
+    planes<N, Q, PS, QQ, kThreads>(U, t2, (visc ? NV + 16 : NV) * N, tables.bq, tables.bq, rotated(0));
     if (visc) {
-      R* sc = smem + L::L_AT;
-      contract3<12, N, Q>(Lf, lq, sc, sc + up4(L::I12::T1), tables.bq);
+      planes<N, Q, PS, QQ, kThreads>(V, tbd, 4 * N, tables.bq, tables.dq, rotated((NV + 16) * N));
+      planes<N, Q, PS, QQ, kThreads>(V, tdb, 4 * N, tables.dq, tables.bq, rotated((NV + 20) * N));
     }
-    {
-      R* sc = smem + L::U_AT;
-      contract3<NV, N, Q>(U, uq, sc, sc + up4(L::IU::T1), tables.bq);
+    __syncthreads();
+    constexpr int CQ = N * QQ;
+    lines<N, Q, QQ, QQ, CQ, QQ, Q3, kThreads>(t2, uq, NV * QQ, tables.bq, rotated(0));
+    if (visc) {
+      lines<N, Q, QQ, QQ, CQ, QQ, Q3, kThreads>(t2 + (NV + 4) * CQ, lq, 12 * QQ, tables.bq, rotated(NV * QQ));
+      lines<N, Q, QQ, QQ, CQ, QQ, Q3, kThreads>(tdb, gq, 4 * QQ, tables.bq, rotated((NV + 12) * QQ));
+      lines<N, Q, QQ, QQ, CQ, QQ, Q3, kThreads>(tbd, gq + 4 * Q3, 4 * QQ, tables.bq, rotated((NV + 16) * QQ));
+      lines<N, Q, QQ, QQ, CQ, QQ, Q3, kThreads>(t2 + NV * CQ, gq + 8 * Q3, 4 * QQ, tables.dq, rotated((NV + 20) * QQ));
     }
+    __syncthreads();
     const double* jinv = B.jinv + (size_t)e * Q3 * 9;
     const float* jinv32 = (sizeof(R) == sizeof(float) && B.jinv32) ? B.jinv32 + (size_t)e * Q3 * 9 : nullptr;
     const double* wdet = B.wdet + (size_t)e * Q3;
@@ -670,28 +581,9 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) 
       for (int k = 0; k < 9; ++k) Ja[k] = (R)B.ajinv[(size_t)e * 9 + k];
       deta = (R)B.adet[e];
     }
-    if (visc) {
-      grad3<4, N, Q>(V, gq, smem + L::X_AT, smem + L::Y_AT, tables.bq, tables.dq);
-      // reference -> physical gradient per point, plus the lift at the point
-      for (int q = threadIdx.x; q < Q3; q += kThreads) {
-        R J[9], gr[12];
-#pragma unroll
-        for (int k = 0; k < 9; ++k) J[k] = aff ? Ja[k] : (jinv32 ? (R)jinv32[q * 9 + k] : (R)jinv[q * 9 + k]);
-#pragma unroll
-        for (int k = 0; k < 12; ++k) gr[k] = gq[k * Q3 + q];
-#pragma unroll
-        for (int m = 0; m < 4; ++m)
-#pragma unroll
-          for (int d = 0; d < 3; ++d) {
-            R x = gr[0 * 4 + m] * J[0 * 3 + d] + gr[1 * 4 + m] * J[1 * 3 + d] + gr[2 * 4 + m] * J[2 * 3 + d];
-            x += lq[(m * 3 + d) * Q3 + q];
-            gq[(m * 3 + d) * Q3 + q] = x;
-          }
-      }
-      __syncthreads();
-    }
-    R* Gi = lq;                          // [3][NV][Q3]
-    R* Gv = Gi + 3 * NV * Q3;            // [3][NV][Q3] (SPLIT only)
+    // a point's Gi and Gv take the place of its own lift (and later channels): no other thread reads there
+    R* Gi = smem + L::GI;                // [3][NV][Q3]
+    R* Gv = smem + L::GVI;               // [3][NV][Q3] (SPLIT only)
     R Fa[3][NV];
     {
       const R ex[3] = {R(1), R(0), R(0)}, ey[3] = {R(0), R(1), R(0)}, ez[3] = {R(0), R(0), R(1)};
@@ -722,9 +614,18 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) 
 #pragma unroll
       for (int k = 0; k < 3 * NV; ++k) Fv[k] = R(0);
       if (visc) {
+        // reference -> physical gradient, plus the lift
         R grad[12];
 #pragma unroll
-        for (int k = 0; k < 12; ++k) grad[k] = gq[k * Q3 + q];
+        for (int m = 0; m < 4; ++m) {
+          const R g0 = gq[m * Q3 + q], g1 = gq[(4 + m) * Q3 + q], g2 = gq[(8 + m) * Q3 + q];
+#pragma unroll
+          for (int d = 0; d < 3; ++d) {
+            R x = g0 * J[0 * 3 + d] + g1 * J[1 * 3 + d] + g2 * J[2 * 3 + d];
+            x += lq[(m * 3 + d) * Q3 + q];
+            grad[m * 3 + d] = x;
+          }
+        }
         viscous_flux<NV>(P_.ph, cv.mu, cv.kappa, Uq, grad, Fv);
       }
 #pragma unroll
@@ -744,28 +645,53 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) 
         }
     }
     __syncthreads();
-    R* Ri = Rr;
-    R* Rv = Rr + NV * N3;
-    R* A = smem + L::A_AT;                // uq and gq are dead: the x-pass results go there if they fit
+    // weak divergence: planes along x and y in place (dqT along the direction of the component), then along z,
+    // where the three components' terms are summed as (t0 + t1) + t2
+    auto divergence = [&](R* G, R* out) {
+      planes<Q, N, QQ, QQ, kThreads>(G, G, NV * Q, tables.dqT, tables.bqT, rotated(0));
+      planes<Q, N, QQ, QQ, kThreads>(G + NV * Q3, G + NV * Q3, NV * Q, tables.bqT, tables.dqT, rotated(NV * Q));
+      planes<Q, N, QQ, QQ, kThreads>(G + 2 * NV * Q3, G + 2 * NV * Q3, NV * Q, tables.bqT, tables.bqT, rotated(2 * NV * Q));
+      __syncthreads();
+      for (int line = threadIdx.x; line < NV * N2; line += kThreads) {
+        R x0[Q], x1[Q], x2[Q];
+        line_load<Q, N2, QQ, Q3>(G, line, x0);
+        line_load<Q, N2, QQ, Q3>(G + NV * Q3, line, x1);
+        line_load<Q, N2, QQ, Q3>(G + 2 * NV * Q3, line, x2);
+#pragma unroll
+        for (int o = 0; o < N; ++o) {
+          R s0 = R(0), s1 = R(0), s2 = R(0);
+#pragma unroll
+          for (int i = 0; i < Q; ++i) s0 += tables.bqT[o * Q + i] * x0[i];
+#pragma unroll
+          for (int i = 0; i < Q; ++i) s1 += tables.bqT[o * Q + i] * x1[i];
+#pragma unroll
+          for (int i = 0; i < Q; ++i) s2 += tables.dqT[o * Q + i] * x2[i];
+          R acc = s0;
+          acc += s1;
+          acc += s2;
+          out[line / N2 * NS + o * PS + line % N2] = acc;
+        }
+      }
+      __syncthreads();
+    };
+    R* Rv = Rr + NV * NS;
     if (skip_inv) {
-      for (int idx = threadIdx.x; idx < NV * N3; idx += kThreads) Ri[idx] = R(0);
+      for (int idx = threadIdx.x; idx < NV * NS; idx += kThreads) Rr[idx] = R(0);
       __syncthreads();
     } else {
-      div3<NV, N, Q>(Gi, Ri, A, tables.bqT, tables.dqT);
+      divergence(Gi, Rr);
     }
     if (SPLIT) {
       if (visc) {
-        div3<NV, N, Q>(Gv, Rv, A, tables.bqT, tables.dqT);
+        divergence(Gv, Rv);
       } else {
-        for (int idx = threadIdx.x; idx < NV * N3; idx += kThreads) Rv[idx] = R(0);
+        for (int idx = threadIdx.x; idx < NV * NS; idx += kThreads) Rv[idx] = R(0);
         __syncthreads();
       }
     }
   }
   // ---- phase D: face terms, M^-1, stage update (k_hex_finalize with the residuals in shared memory)
-  R* hc = W;                                    // [6][C][QF2] face flux at canonical points
-  R* tmp = W + L::D_TMP;                        // [6][C][PT]
-  R* hs = W + L::D_HS;                          // [6][C][PB]; reused for the M^-1 partial sums
+  R* hc = smem + L::HC;                         // [6][C][FP] face flux at canonical points, then at the face nodes
   const size_t base = (size_t)e * N3 * NV;
   // one face point per thread: its NV inviscid and NV viscous flux values (contiguous)
   for (int it = threadIdx.x; it < 6 * QF2; it += kThreads) {
@@ -781,42 +707,43 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) 
         const R hi = skip_inv ? R(0) : (R)si * fd.fluxI32[ki + v];
         const R hv = visc ? -(R)si * fd.fluxV32[kv + v] : R(0);
         if (SPLIT) {
-          hc[(lf * C + v) * QF2 + c] = hi;
-          hc[(lf * C + NV + v) * QF2 + c] = hv;
+          hc[(lf * C + v) * FP + c] = hi;
+          hc[(lf * C + NV + v) * FP + c] = hv;
         } else {
-          hc[(lf * C + v) * QF2 + c] = hi + hv;
+          hc[(lf * C + v) * FP + c] = hi + hv;
         }
       } else {
         const double hi = skip_inv ? 0.0 : si * fd.fluxI[ki + v];
         const double hv = visc ? -si * fd.fluxV[kv + v] : 0.0;
         if (SPLIT) {
-          hc[(lf * C + v) * QF2 + c] = (R)hi;
-          hc[(lf * C + NV + v) * QF2 + c] = (R)hv;
+          hc[(lf * C + v) * FP + c] = (R)hi;
+          hc[(lf * C + NV + v) * FP + c] = (R)hv;
         } else {
-          hc[(lf * C + v) * QF2 + c] = (R)(hi + hv);
+          hc[(lf * C + v) * FP + c] = (R)(hi + hv);
         }
       }
     }
   }
   __syncthreads();
-  contract2<6 * C, QF, N>(hc, hs, tmp, tables.bfT);
+  planes<QF, N, FP, FP, kThreads>(hc, hc, 6 * C, tables.bfT, tables.bfT, threadIdx.x);
+  __syncthreads();
   // non-affine elements: the residuals go to rows RrT [N3][CS] in element node order (inviscid
-  // channels, then from CSH the viscous ones) in the dead hc/tmp region, for pair loads in the
+  // channels, then from CSH the viscous ones) beyond hc, for pair loads in the
   // dense M^-1
   constexpr int CSH = L::CSH, CS = L::CS;
-  R* RrT = W;
+  R* RrT = smem + L::RT;
   for (int idx = threadIdx.x; idx < C * N3; idx += kThreads) {
     const int c = idx / N3, l = idx % N3;
     const int xyz[3] = {l % N, (l / N) % N, l / N2};
-    R acc = Rr[idx];
+    R acc = Rr[c * NS + nod(l)];
 #pragma unroll
     for (int lf = 0; lf < 6; ++lf) {
       int a0, end, a1, a2;
       hex_face_axes(lf, a0, end, a1, a2);
-      if (xyz[a0] == end) acc += hs[(lf * C + c) * L::PB + xyz[a2] * N + xyz[a1]];
+      if (xyz[a0] == end) acc += hc[(lf * C + c) * FP + xyz[a2] * N + xyz[a1]];
     }
     if (aff)
-      Rr[idx] = acc;
+      Rr[c * NS + nod(l)] = acc;
     else
       RrT[lex2node[l] * CS + (c < NV ? c : CSH + c - NV)] = acc;
   }
@@ -838,13 +765,21 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) 
       }
     }
   };
-  R* rows = U;                                        // [C / NV][N3][NV] results in memory order (U, V, LF are dead)
-  static_assert(2 * NV * N3 <= L::RR, "the results must fit in the dead nodal arrays");
+  R* rows = hc;                                       // [C / NV][N3][NV] results in memory order (hc is dead)
   if (aff) {
-    contract3<C, N, N>(Rr, hs, W, W + up4(L::MC::T1), tables.m1i);
-    for (int idx = threadIdx.x; idx < C * N3; idx += kThreads) {
-      const int c = idx / N3, l = idx % N3;
-      rows[(c / NV) * NV * N3 + lex2node[l] * NV + c % NV] = hs[idx];
+    planes<N, N, PS, PS, kThreads>(Rr, Rr, C * N, tables.m1i, tables.m1i, threadIdx.x);
+    __syncthreads();
+    for (int line = threadIdx.x; line < C * N2; line += kThreads) {
+      R x[N];
+      line_load<N, N2, PS, NS>(Rr, line, x);
+      const int c = line / N2;
+#pragma unroll
+      for (int o = 0; o < N; ++o) {
+        R acc = R(0);
+#pragma unroll
+        for (int i = 0; i < N; ++i) acc += tables.m1i[o * N + i] * x[i];
+        rows[(c / NV) * NV * N3 + lex2node[o * N2 + line % N2] * NV + c % NV] = acc;
+      }
     }
     __syncthreads();
     emit(rows, rows + NV * N3, (R)B.acoef[e]);
@@ -854,7 +789,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) 
   constexpr int NG = (NV + VB - 1) / VB;
   constexpr int HALVES = NG * N3 * 2 <= kThreads ? 2 : 1;
   constexpr int JH = (N3 + HALVES - 1) / HALVES;
-  R* part = hs;                                       // [HALVES][2][NV][N3]
+  R* part = smem + L::PART;                           // [HALVES][2][NV][N3]
   auto apply = [&](const auto* M) {
     for (int idx = threadIdx.x; idx < HALVES * NG * N3; idx += kThreads) {
       const int i = idx % N3, g = (idx / N3) % NG, h = idx / (NG * N3);

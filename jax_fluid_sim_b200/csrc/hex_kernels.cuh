@@ -187,92 +187,102 @@ __device__ __forceinline__ void warp_tensor3(const T* in, T* out, T* t1, T* t2, 
 }
 
 // ------------------------------------------------------------------------------------------
-// Contraction passes of the fused kernels (traces, element).  They differ from pencil above in where
-// their operands come from, which is what bounds these kernels (profiled: 70 to 85 % of the shared-memory
-// pipe's wavefronts, a quarter of them the matrices' own loads and up to half of them bank conflicts):
-//  - the matrix is read from the kernel's parameters (constant bank), not from shared memory;
-//  - planes of 16 values between passes are laid out 20 apart and, in float64, planes of 20
-//    values 21 apart: a pass reads and writes one value of every line at a time, 4 (5) lines to a plane,
-//    and those strides put the planes of a half warp (float64) or warp (float32) on distinct banks;
-//  - alignment and strides are known at compile time.
-// The sums are pencil's, value for value.
+// Contraction passes of the fused kernels (traces, element).  These kernels are bound by the wavefronts of
+// the shared-memory pipe (profiled with one pencil pass per axis: 70 to 85 % of it, a quarter of them the
+// matrices' own loads, up to half bank conflicts), so:
+//  - a thread contracts a whole plane along both its axes in registers (plane_item): the values between
+//    the two axes never go through shared memory, and the barrier between them goes too;
+//  - the matrices are read from the kernel's parameters (constant bank), not from shared memory;
+//  - planes of 16 values are laid out 18 (float64) or 20 (float32) apart, an odd number of 16-byte units:
+//    lanes on consecutive planes then fall on distinct banks, with 16-byte accesses; planes of 25 and 9 values
+//    are odd as they are.
+// Per value the sums are those of the pencil form.  P3 element kernel, per element: 8,626 wavefronts with
+// pencil passes, 5,976 with the matrices and paddings alone, @EL@ now.
 template <typename T>
-__host__ __device__ constexpr int plane(int n) { return n == 16 ? 20 : (n == 20 && sizeof(T) == 8 ? 21 : n); }
+__host__ __device__ constexpr int plane_stride(int n) { return n == 16 ? (sizeof(T) == 8 ? 18 : 20) : n; }
 
-// Rotation of the thread <-> line assignment of a pass, so that passes issued back to back without a
-// barrier between them start on different threads.
+// Rotation of the thread <-> item assignment, so that loops issued back to back without a barrier between
+// them start on different threads.
+template <int NT = kThreads>
 __device__ __forceinline__ int rotated(int offset) {
-  return (int)((threadIdx.x + kThreads - (unsigned)offset % kThreads) % kThreads);
+  return (int)((threadIdx.x + NT - (unsigned)offset % NT) % NT);
 }
 
-template <int IN, int OUT, int LINES, int IST, int OST, bool VIN, bool VOUT, typename T, typename InBase, typename OutBase>
-__device__ __forceinline__ void pass(const T* in, T* out, const T* M, InBase in_base, OutBase out_base, int first) {
+// One plane: out[oy][ox] = sum My[oy][iy] (sum Mx[ox][ix] in[iy][ix]).  Every input is read before the first
+// output is written, so out may be in.  16-byte accesses where a row is a multiple of 16 bytes (both
+// planes must then be 16-byte aligned).
+template <int I, int O, typename T>
+__device__ __forceinline__ void plane_item(const T* in, T* out, const T* Mx, const T* My) {
   constexpr int VW = 16 / sizeof(T);
-  for (int line = first; line < LINES; line += kThreads) {
-    const T* src = in + in_base(line);
-    T x[IN];
-    if constexpr (VIN && IST == 1 && IN % VW == 0) {
+  constexpr bool VI = I == 4, VO = O == 4;               // the strides of 16-value planes keep rows aligned
+  T t[I][O];
 #pragma unroll
-      for (int i = 0; i < IN; i += VW) load16(src + i, &x[i]);
+  for (int iy = 0; iy < I; ++iy) {
+    T x[I];
+    if constexpr (VI) {
+#pragma unroll
+      for (int i = 0; i < I; i += VW) load16(in + iy * I + i, &x[i]);
     } else {
 #pragma unroll
-      for (int i = 0; i < IN; ++i) x[i] = src[i * IST];
+      for (int i = 0; i < I; ++i) x[i] = in[iy * I + i];
     }
-    T y[OUT];
 #pragma unroll
-    for (int o = 0; o < OUT; ++o) {
-      T s = T(0);
+    for (int o = 0; o < O; ++o) {
+      T acc = T(0);
 #pragma unroll
-      for (int i = 0; i < IN; ++i) s += M[o * IN + i] * x[i];
-      y[o] = s;
+      for (int i = 0; i < I; ++i) acc += Mx[o * I + i] * x[i];
+      t[iy][o] = acc;
     }
-    T* dst = out + out_base(line);
-    if constexpr (VOUT && OST == 1 && OUT % VW == 0) {
+  }
 #pragma unroll
-      for (int o = 0; o < OUT; o += VW) store16(dst + o, &y[o]);
+  for (int oy = 0; oy < O; ++oy) {
+    T y[O];
+#pragma unroll
+    for (int o = 0; o < O; ++o) {
+      T acc = T(0);
+#pragma unroll
+      for (int i = 0; i < I; ++i) acc += My[oy * I + i] * t[i][o];
+      y[o] = acc;
+    }
+    if constexpr (VO && I == O) {
+#pragma unroll
+      for (int o = 0; o < O; o += VW) store16(out + oy * O + o, &y[o]);
     } else {
 #pragma unroll
-      for (int o = 0; o < OUT; ++o) dst[o * OST] = y[o];
+      for (int o = 0; o < O; ++o) out[oy * O + o] = y[o];
     }
   }
 }
 
-// Scratch of contract3: t1 then t2.
-template <int C, int I, int O, typename T>
-struct Contract3 {
-  static constexpr int P1 = plane<T>(I * O), P2 = plane<T>(O * O);
-  static constexpr int T1 = C * I * P1, T2 = C * I * P2;
-};
-
-// out[c][oz][oy][ox] = sum M[oz][iz] M[oy][iy] M[ox][ix] in[c][iz][iy][ix]; in and out are dense, in 16-byte
-// aligned; ends with a barrier.
-template <int C, int I, int O, typename T>
-__device__ __forceinline__ void contract3(const T* in, T* out, T* t1, T* t2, const T* M) {
-  using X = Contract3<C, I, O, T>;
-  constexpr int P1 = X::P1, P2 = X::P2, OO = O * O;
-  pass<I, O, C * I * I, 1, 1, (I * (int)sizeof(T)) % 16 == 0, (O * (int)sizeof(T)) % 16 == 0 && (P1 * (int)sizeof(T)) % 16 == 0>(
-      in, t1, M, [](int l) { return l * I; }, [](int l) { return (l / I) * P1 + (l % I) * O; }, rotated(0));
-  __syncthreads();
-  pass<I, O, C * I * O, O, O, false, false>(
-      t1, t2, M, [](int l) { return (l / O) * P1 + l % O; }, [](int l) { return (l / O) * P2 + l % O; }, rotated(0));
-  __syncthreads();
-  pass<I, O, C * OO, P2, OO, false, false>(
-      t2, out, M, [](int l) { return (l / OO) * I * P2 + l % OO; }, [](int l) { return (l / OO) * O * OO + l % OO; },
-      rotated(0));
-  __syncthreads();
+// count planes at strides IS and OS
+template <int I, int O, int IS, int OS, int NT, typename T>
+__device__ __forceinline__ void planes(const T* in, T* out, int count, const T* Mx, const T* My, int first) {
+  for (int p = first; p < count; p += NT) plane_item<I, O>(in + p * IS, out + p * OS, Mx, My);
 }
 
-// 2-D: out[c][k2][k1] (channel stride plane(K K)) = sum M[k2][j2] M[k1][j1] in[c][j2][j1]; t: C plane(J K)
-// values of scratch; in dense and 16-byte aligned; ends with a barrier.
-template <int C, int J, int K, typename T>
-__device__ __forceinline__ void contract2(const T* in, T* out, T* t, const T* M) {
-  constexpr int PT = plane<T>(J * K), PO = plane<T>(K * K);
-  pass<J, K, C * J, 1, 1, (J * (int)sizeof(T)) % 16 == 0, (K * (int)sizeof(T)) % 16 == 0 && (PT * (int)sizeof(T)) % 16 == 0>(
-      in, t, M, [](int l) { return l * J; }, [](int l) { return (l / J) * PT + (l % J) * K; }, rotated(0));
-  __syncthreads();
-  pass<J, K, C * K, K, K, false, false>(
-      t, out, M, [](int l) { return (l / K) * PT + l % K; }, [](int l) { return (l / K) * PO + l % K; }, rotated(0));
-  __syncthreads();
+// The third axis: lines of I values at stride IS (one per plane) of channels CI apart; L lines to a channel.
+template <int I, int L, int IS, int CI, typename T>
+__device__ __forceinline__ void line_load(const T* in, int line, T (&x)[I]) {
+  const T* src = in + line / L * CI + line % L;
+#pragma unroll
+  for (int i = 0; i < I; ++i) x[i] = src[i * IS];
+}
+
+// out[c][o][l] = sum M[o][i] in[c][i][l] for count lines; outputs OS apart, channels CO apart
+template <int I, int O, int L, int IS, int CI, int OS, int CO, int NT, typename T>
+__device__ __forceinline__ void lines(const T* in, T* out, int count, const T* M, int first) {
+  for (int line = first; line < count; line += NT) {
+    T x[I];
+    line_load<I, L, IS, CI>(in, line, x);
+    T* dst = out + line / L * CO + line % L;
+#pragma unroll
+    for (int o = 0; o < O; ++o) {
+      T acc = T(0);
+#pragma unroll
+      for (int i = 0; i < I; ++i) acc += M[o * I + i] * x[i];
+      dst[o * OS] = acc;
+    }
+  }
 }
 
 // 2-D: out[c][k2][k1] = sum M2[k2][j2] M1[k1][j1] in[c][j2][j1]
@@ -311,14 +321,12 @@ struct HexSmem {
   static constexpr int MS = N3 + 1;                 // padded row stride of the staged M^-1 (transposed)
   // traces: U, v, then the six faces' slabs, contraction scratch, face values and tangential derivatives
   static constexpr int TR_U = 0, TR_V = TR_U + NV * N3, TR_W = (TR_V + 4 * N3 + 3) / 4 * 4;
-  // slabs [CH][N2], then the x-passes' results [CH][plane] and the df pass [24][plane], then the derivatives
-  // g1, g2 [24][QF2] each.  The face values alias the slabs: every read of the slabs comes before the
-  // barrier after which the face values are written; N2 == QF2 at P1-P3.
-  static constexpr int TR_CH = 6 * (NV + 8), TR_PL = plane<R>(N * QF);
-  static_assert(N2 == QF2, "the face values take the slabs' place");
-  static constexpr int TR_T = TR_W + (TR_CH * N2 + 3) / 4 * 4, TR_D = TR_T + TR_CH * TR_PL;
-  static constexpr int TR_G = (NV + 4) * N3 >= 24 * TR_PL ? TR_D : TR_D + 24 * TR_PL;   // the df pass goes over U, V if it fits
-  static constexpr int TRACES = TR_G + 2 * 24 * QF2;
+  // slabs [CH][FP] (the face values of U and dv/dn take their place), the face values of v [24][FP] and the
+  // tangential derivatives g1, g2 [24][FP] each; N2 == QF2 at P1-P3
+  static constexpr int TR_CH = 6 * (NV + 8), FP = plane_stride<R>(QF2);
+  static_assert(N2 == QF2, "face planes of nodes and points have one size");
+  static constexpr int TR_F = (TR_W + TR_CH * FP + 3) / 4 * 4, TR_G = TR_F + 24 * FP;
+  static constexpr int TRACES = TR_G + 48 * FP;
   // lift: staged M^-T, b per face on its slab, b on all nodes, scratch
   static constexpr int LI_BS = T, LI_B = LI_BS + 6 * 12 * N2, LI_W = LI_B + 12 * N3;
   static constexpr int LI_X = LI_W + 72 * QF2 + 72 * QF * N + 72 * N2 + 72 * QF2;   // affine scratch
@@ -378,24 +386,23 @@ __global__ void __launch_bounds__(kThreads) k_hex_traces(const __grid_constant__
   R* smem = reinterpret_cast<R*>(dyn_smem);
   R* U = smem + L::TR_U;             // [NV][N3], minus anchor
   R* V = smem + L::TR_V;             // [4][N3]
-  // all six faces at once, channel blocks [U: 6*NV][v: 6*4][dv/dn: 6*4], each of N2 (slabs)
-  // or QF2 (face points) values
-  constexpr int CH = L::TR_CH, PL = L::TR_PL;
+  // all six faces at once, channel blocks [U: 6*NV][v: 6*4][dv/dn: 6*4], each a plane of N2 nodes, later of
+  // QF2 canonical face points (v: at fv)
+  constexpr int FP = L::FP;
   R* slabs = smem + L::TR_W;
-  R* ftmp = smem + L::TR_T;          // x-passes [CH][PL]
-  // [CH][QF2] values at the canonical face points, the second face axis fastest (a pass then stores whole lines)
-  R* fo = slabs;
-  R* g1 = smem + L::TR_G;            // [6*4][QF2] derivative of v along a1 (same order)
-  R* g2 = g1 + 24 * QF2;             // [6*4][QF2] derivative of v along a2
+  R* fv = smem + L::TR_F;            // [6*4][FP] v at the face points
+  R* g1 = smem + L::TR_G;            // [6*4][FP] derivative of v along a1
+  R* g2 = g1 + 24 * FP;              // [6*4][FP] derivative of v along a2
   __shared__ int fslot[6], fperm[6];
   const BlockDev& B = P_.blk[b];
   const FaceDev& fd = P_.face[1];
   const int e = blockIdx.x;
   const double* Ug = S.b[b] + (size_t)e * N3 * NV;
   __shared__ double anchor[NV];
-  // the state arrives in one coalesced sweep (raw takes the place of ftmp) and is spread from shared memory
-  double* raw = reinterpret_cast<double*>(ftmp);
-  static_assert(CH * PL * (int)sizeof(R) >= N3 * NV * (int)sizeof(double) && L::TR_T * sizeof(R) % 8 == 0, "raw state");
+  // the state arrives in one coalesced sweep (raw, where the slabs go) and is spread from shared memory
+  double* raw = reinterpret_cast<double*>(slabs);
+  static_assert((L::TRACES - L::TR_W) * (int)sizeof(R) >= N3 * NV * (int)sizeof(double) && L::TR_W * sizeof(R) % 8 == 0,
+                "raw state");
   for (int idx = threadIdx.x; idx < N3 * NV; idx += kThreads) raw[idx] = Ug[idx];
   if (threadIdx.x < 6) {
     int ft, f, side;
@@ -430,73 +437,54 @@ __global__ void __launch_bounds__(kThreads) k_hex_traces(const __grid_constant__
     const int st0 = axis_stride<N>(a0), off = j1 * axis_stride<N>(a1) + j2 * axis_stride<N>(a2);
     const int at = end * st0 + off;
 #pragma unroll
-    for (int m = 0; m < NV; ++m) slabs[(lf * NV + m) * N2 + j] = U[m * N3 + at];
+    for (int m = 0; m < NV; ++m) slabs[(lf * NV + m) * FP + j] = U[m * N3 + at];
     if (visc) {
       R dn[N];
 #pragma unroll
       for (int j0 = 0; j0 < N; ++j0) dn[j0] = end ? tables.d1[j0] : tables.d0[j0];
 #pragma unroll
       for (int m = 0; m < 4; ++m) {
-        slabs[(6 * NV + lf * 4 + m) * N2 + j] = V[m * N3 + at];
+        slabs[(6 * NV + lf * 4 + m) * FP + j] = V[m * N3 + at];
         R val = R(0);
 #pragma unroll
         for (int j0 = 0; j0 < N; ++j0) val += dn[j0] * V[m * N3 + j0 * st0 + off];
-        slabs[(6 * NV + 24 + lf * 4 + m) * N2 + j] = val;
+        slabs[(6 * NV + 24 + lf * 4 + m) * FP + j] = val;
       }
     }
   }
   __syncthreads();
-  // The face contractions with two barriers: the x-passes (bf on every channel; df on the 24 v channels,
-  // into the U/V region, dead after the slab gather, where it fits), then the y-passes (bf -> fo; bf on the
-  // df pass -> g1; df on the bf pass of the v channels -> g2).  Consecutive passes start on rotated
-  // threads so that the lines spread evenly.
-  {
-    auto i1 = [](int l) { return l * N; };
-    auto o1 = [](int l) { return (l / N) * PL + (l % N) * QF; };
-    constexpr bool VI = (N * (int)sizeof(R)) % 16 == 0, VO = (QF * (int)sizeof(R)) % 16 == 0 && (PL * (int)sizeof(R)) % 16 == 0;
-    auto i2 = [](int l) { return (l / QF) * PL + l % QF; };
-    auto o2 = [](int l) { return l * QF; };
-    constexpr bool VQ = (QF * (int)sizeof(R)) % 16 == 0;
-    if (visc) {
-      R* xd = L::TR_G == L::TR_D ? U : smem + L::TR_D;                 // [24][PL]
-      const R* vsl = slabs + 6 * NV * N2;
-      pass<N, QF, CH * N, 1, 1, VI, VO>(slabs, ftmp, tables.bf, i1, o1, rotated(0));
-      pass<N, QF, 24 * N, 1, 1, VI, VO>(vsl, xd, tables.df, i1, o1, rotated(CH * N));
-      __syncthreads();
-      pass<N, QF, CH * QF, QF, 1, false, VQ>(ftmp, fo, tables.bf, i2, o2, rotated(0));
-      pass<N, QF, 24 * QF, QF, 1, false, VQ>(xd, g1, tables.bf, i2, o2, rotated(CH * QF));
-      pass<N, QF, 24 * QF, QF, 1, false, VQ>(ftmp + 6 * NV * PL, g2, tables.df, i2, o2, rotated(CH * QF + 24 * QF));
-    } else {
-      pass<N, QF, 6 * NV * N, 1, 1, VI, VO>(slabs, ftmp, tables.bf, i1, o1, rotated(0));
-      __syncthreads();
-      pass<N, QF, 6 * NV * QF, QF, 1, false, VQ>(ftmp, fo, tables.bf, i2, o2, rotated(0));
-    }
+  // the face contractions, all in one phase: U and dv/dn in place, v to fv and its derivatives (df along one
+  // face axis, bf along the other) to g1 and g2
+  planes<N, QF, FP, FP, kThreads>(slabs, slabs, 6 * NV, tables.bf, tables.bf, rotated(0));
+  if (visc) {
+    R* v = slabs + 6 * NV * FP;
+    planes<N, QF, FP, FP, kThreads>(v + 24 * FP, v + 24 * FP, 24, tables.bf, tables.bf, rotated(6 * NV));
+    planes<N, QF, FP, FP, kThreads>(v, fv, 24, tables.bf, tables.bf, rotated(6 * NV + 24));
+    planes<N, QF, FP, FP, kThreads>(v, g1, 24, tables.df, tables.bf, rotated(6 * NV + 48));
+    planes<N, QF, FP, FP, kThreads>(v, g2, 24, tables.bf, tables.df, rotated(6 * NV + 72));
   }
   __syncthreads();
-  // canonical face point c = c2 QF + c1 is at c1 QF + c2 in fo, g1 and g2
-  auto swapped = [](int c) { return (c % QF) * QF + c / QF; };
   // one face point per thread from here on: its values are contiguous in the face buffers
   for (int it = threadIdx.x; it < 6 * QF2; it += kThreads) {
     const int lf = it / QF2, q = it % QF2;
-    const int c = swapped(codes.perm[fperm[lf] + q]);
+    const int c = codes.perm[fperm[lf] + q];
     double* dst = fd.trA + ((size_t)fslot[lf] + q) * NV;
 #pragma unroll
-    for (int v = 0; v < NV; ++v) dst[v] = anchor[v] + (double)fo[(lf * NV + v) * QF2 + c];
+    for (int v = 0; v < NV; ++v) dst[v] = anchor[v] + (double)slabs[(lf * NV + v) * FP + c];
   }
   // the anchor state per face side, for the face kernel's anchor flux
   for (int idx = threadIdx.x; idx < 6 * NV; idx += kThreads)
     fd.anc[(size_t)(fslot[idx / NV] / QF2) * NV + idx % NV] = anchor[idx % NV];
   if (visc) {
-    const R* fv = fo + 6 * NV * QF2;          // [6][4][QF2]
-    const R* gn = fv + 24 * QF2;              // [6][4][QF2]
+    const R* gn = slabs + (6 * NV + 24) * FP;      // [6][4][FP] derivative along the face normal's axis
     for (int it = threadIdx.x; it < 6 * QF2; it += kThreads) {
       const int lf = it / QF2, q = it % QF2;
-      const int c = swapped(codes.perm[fperm[lf] + q]);
+      const int c = codes.perm[fperm[lf] + q];
       const size_t pt = (size_t)fslot[lf] + q;
       // a point's 4 values and 12 gradients are contiguous: 16-byte stores
       R tv[4];
 #pragma unroll
-      for (int m = 0; m < 4; ++m) tv[m] = fv[(lf * 4 + m) * QF2 + c];
+      for (int m = 0; m < 4; ++m) tv[m] = fv[(lf * 4 + m) * FP + c];
       if (F32) {
         *reinterpret_cast<float4*>(fd.trV32 + pt * 4) = make_float4((float)tv[0], (float)tv[1], (float)tv[2], (float)tv[3]);
       } else {
@@ -517,7 +505,7 @@ __global__ void __launch_bounds__(kThreads) k_hex_traces(const __grid_constant__
       R gout[12];
 #pragma unroll
       for (int m = 0; m < 4; ++m) {
-        const int k = (lf * 4 + m) * QF2 + c;
+        const int k = (lf * 4 + m) * FP + c;
         const R gnv = gn[k], g1v = g1[k], g2v = g2[k];
         // reference gradient component along axis r: normal (a0) or tangential (a1 < a2)
         const R gx = a0 == 0 ? gnv : g1v;
