@@ -393,12 +393,12 @@ struct HexElemSmem {
 // Lift + volume + finalize of one hexahedron (see the file comment).  SPLIT keeps the inviscid
 // and viscous residuals apart (right-hand-side outputs, the MOOD step's viscous residual).
 template <int P, int NV, bool SPLIT, typename R = double>
-__global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) k_hex_element(const __grid_constant__ DevPlan P_, const StatePtrs S,
+__global__ void __launch_bounds__(HexDims<P>::NT, sizeof(R) == sizeof(float) ? 6 * kThreads / HexDims<P>::NT : 1) k_hex_element(const __grid_constant__ DevPlan P_, const StatePtrs S,
                                                          const __grid_constant__ HexTablesT<R> tables,
                                                          const HexCodes codes, const __grid_constant__ FinalizeArgs A) {
   using D = HexDims<P>;
   using L = HexElemSmem<P, NV, SPLIT, R>;
-  constexpr int N = D::N, Q = D::Q, QF = D::QF, N2 = D::N2, N3 = D::N3, Q3 = D::Q3, QF2 = D::QF2;
+  constexpr int N = D::N, Q = D::Q, QF = D::QF, N2 = D::N2, N3 = D::N3, Q3 = D::Q3, QF2 = D::QF2, NT = D::NT;
   constexpr int C = L::C;
   constexpr int b = 0;
   extern __shared__ __align__(16) unsigned char dyn_smem[];
@@ -421,7 +421,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) 
   double* raw = reinterpret_cast<double*>(smem + L::NODAL);
   static_assert((L::TOTAL - L::NODAL) * (int)sizeof(R) >= N3 * NV * (int)sizeof(double) && L::NODAL * sizeof(R) % 8 == 0,
                 "raw state");
-  for (int idx = threadIdx.x; idx < N3 * NV; idx += kThreads) raw[idx] = Ug[idx];
+  for (int idx = threadIdx.x; idx < N3 * NV; idx += NT) raw[idx] = Ug[idx];
   if (threadIdx.x < 6) {
     int ft, f, side;
     decode_face(B.elem_face[e * 6 + threadIdx.x], ft, f, side);
@@ -429,7 +429,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) 
     fperm[threadIdx.x] = (side == 0 ? fd.oc[f] : fd.nc[f]) * QF2;
     fface[threadIdx.x] = (f << 1) | side;
   }
-  for (int l = threadIdx.x; l < N3; l += kThreads) {
+  for (int l = threadIdx.x; l < N3; l += NT) {
     const int node = codes.lex2node[l];
     lex2node[l] = node;
     node2lex[node] = l;
@@ -446,7 +446,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) 
   const bool skip_inv = SPLIT && A.skip_inviscid && A.skip_inviscid[e];
   const double* MT = B.minv + (size_t)e * N3 * N3;
   const float* MT32 = (sizeof(R) == sizeof(float) && B.minv32) ? B.minv32 + (size_t)e * N3 * N3 : nullptr;
-  for (int l = threadIdx.x; l < N3; l += kThreads) {
+  for (int l = threadIdx.x; l < N3; l += NT) {
     const double* un = raw + lex2node[l] * NV;
     double u[NV];
 #pragma unroll
@@ -468,7 +468,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) 
     R* ball = smem + L::BALL;         // [12][NS]
     constexpr int LR = L::LR;
     // one face point per thread: its 12 jump components (contiguous) to the canonical point
-    for (int it = threadIdx.x; it < 6 * QF2; it += kThreads) {
+    for (int it = threadIdx.x; it < 6 * QF2; it += NT) {
       const int lf = it / QF2, q = it % QF2;
       const int cp = codes.perm[fperm[lf] + q];
       const size_t jo = ((size_t)(fface[lf] >> 1) * QF2 + q) * 12;
@@ -493,9 +493,9 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) 
       }
     }
     __syncthreads();
-    planes<QF, N, FP, FP, kThreads>(jc, jc, 72, tables.bfT, tables.bfT, threadIdx.x);
+    planes<QF, N, FP, FP, NT>(jc, jc, 72, tables.bfT, tables.bfT, threadIdx.x);
     __syncthreads();
-    for (int idx = threadIdx.x; idx < 12 * N3; idx += kThreads) {
+    for (int idx = threadIdx.x; idx < 12 * N3; idx += NT) {
       const int c = idx / N3, l = idx % N3;
       const int xyz[3] = {l % N, (l / N) % N, l / N2};
       R acc = R(0);
@@ -511,10 +511,10 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) 
     }
     __syncthreads();
     if (aff) {
-      planes<N, N, PS, PS, kThreads>(ball, ball, 12 * N, tables.m1i, tables.m1i, threadIdx.x);
+      planes<N, N, PS, PS, NT>(ball, ball, 12 * N, tables.m1i, tables.m1i, threadIdx.x);
       __syncthreads();
       const R cf = (R)B.acoef[e];
-      for (int line = threadIdx.x; line < 12 * N2; line += kThreads) {
+      for (int line = threadIdx.x; line < 12 * N2; line += NT) {
         R x[N];
         line_load<N, N2, PS, NS>(ball, line, x);
 #pragma unroll
@@ -527,7 +527,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) 
       }
     } else {
       auto dense_lift = [&](const auto* M) {
-        for (int idx = threadIdx.x; idx < 2 * N3; idx += kThreads) {
+        for (int idx = threadIdx.x; idx < 2 * N3; idx += NT) {
           const int i = idx % N3, g = idx / N3, c0 = g * 6;
           R sacc[6] = {R(0), R(0), R(0), R(0), R(0), R(0)};
 #pragma unroll 4
@@ -557,19 +557,19 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) 
     R* tdb = smem + L::TDB;
     // U, V and the lift as one list of planes, then V's derivatives; three directions share the planes:
     // each gradient goes through the same three 1-D products as a contraction of its own
-    planes<N, Q, PS, QQ, kThreads>(U, t2, (visc ? NV + 16 : NV) * N, tables.bq, tables.bq, rotated(0));
+    planes<N, Q, PS, QQ, NT>(U, t2, (visc ? NV + 16 : NV) * N, tables.bq, tables.bq, rotated<NT>(0));
     if (visc) {
-      planes<N, Q, PS, QQ, kThreads>(V, tbd, 4 * N, tables.bq, tables.dq, rotated((NV + 16) * N));
-      planes<N, Q, PS, QQ, kThreads>(V, tdb, 4 * N, tables.dq, tables.bq, rotated((NV + 20) * N));
+      planes<N, Q, PS, QQ, NT>(V, tbd, 4 * N, tables.bq, tables.dq, rotated<NT>((NV + 16) * N));
+      planes<N, Q, PS, QQ, NT>(V, tdb, 4 * N, tables.dq, tables.bq, rotated<NT>((NV + 20) * N));
     }
     __syncthreads();
     constexpr int CQ = N * QQ;
-    lines<N, Q, QQ, QQ, CQ, QQ, Q3, kThreads>(t2, uq, NV * QQ, tables.bq, rotated(0));
+    lines<N, Q, QQ, QQ, CQ, QQ, Q3, NT>(t2, uq, NV * QQ, tables.bq, rotated<NT>(0));
     if (visc) {
-      lines<N, Q, QQ, QQ, CQ, QQ, Q3, kThreads>(t2 + (NV + 4) * CQ, lq, 12 * QQ, tables.bq, rotated(NV * QQ));
-      lines<N, Q, QQ, QQ, CQ, QQ, Q3, kThreads>(tdb, gq, 4 * QQ, tables.bq, rotated((NV + 12) * QQ));
-      lines<N, Q, QQ, QQ, CQ, QQ, Q3, kThreads>(tbd, gq + 4 * Q3, 4 * QQ, tables.bq, rotated((NV + 16) * QQ));
-      lines<N, Q, QQ, QQ, CQ, QQ, Q3, kThreads>(t2 + NV * CQ, gq + 8 * Q3, 4 * QQ, tables.dq, rotated((NV + 20) * QQ));
+      lines<N, Q, QQ, QQ, CQ, QQ, Q3, NT>(t2 + (NV + 4) * CQ, lq, 12 * QQ, tables.bq, rotated<NT>(NV * QQ));
+      lines<N, Q, QQ, QQ, CQ, QQ, Q3, NT>(tdb, gq, 4 * QQ, tables.bq, rotated<NT>((NV + 12) * QQ));
+      lines<N, Q, QQ, QQ, CQ, QQ, Q3, NT>(tbd, gq + 4 * Q3, 4 * QQ, tables.bq, rotated<NT>((NV + 16) * QQ));
+      lines<N, Q, QQ, QQ, CQ, QQ, Q3, NT>(t2 + NV * CQ, gq + 8 * Q3, 4 * QQ, tables.dq, rotated<NT>((NV + 20) * QQ));
     }
     __syncthreads();
     const double* jinv = B.jinv + (size_t)e * Q3 * 9;
@@ -591,7 +591,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) 
       normal_flux<NV>(P_.ph, anchor, ey, Fa[1]);
       normal_flux<NV>(P_.ph, anchor, ez, Fa[2]);
     }
-    for (int q = threadIdx.x; q < Q3; q += kThreads) {
+    for (int q = threadIdx.x; q < Q3; q += NT) {
       R J[9];
 #pragma unroll
       for (int k = 0; k < 9; ++k) J[k] = aff ? Ja[k] : (jinv32 ? (R)jinv32[q * 9 + k] : (R)jinv[q * 9 + k]);
@@ -648,11 +648,11 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) 
     // weak divergence: planes along x and y in place (dqT along the direction of the component), then along z,
     // where the three components' terms are summed as (t0 + t1) + t2
     auto divergence = [&](R* G, R* out) {
-      planes<Q, N, QQ, QQ, kThreads>(G, G, NV * Q, tables.dqT, tables.bqT, rotated(0));
-      planes<Q, N, QQ, QQ, kThreads>(G + NV * Q3, G + NV * Q3, NV * Q, tables.bqT, tables.dqT, rotated(NV * Q));
-      planes<Q, N, QQ, QQ, kThreads>(G + 2 * NV * Q3, G + 2 * NV * Q3, NV * Q, tables.bqT, tables.bqT, rotated(2 * NV * Q));
+      planes<Q, N, QQ, QQ, NT>(G, G, NV * Q, tables.dqT, tables.bqT, rotated<NT>(0));
+      planes<Q, N, QQ, QQ, NT>(G + NV * Q3, G + NV * Q3, NV * Q, tables.bqT, tables.dqT, rotated<NT>(NV * Q));
+      planes<Q, N, QQ, QQ, NT>(G + 2 * NV * Q3, G + 2 * NV * Q3, NV * Q, tables.bqT, tables.bqT, rotated<NT>(2 * NV * Q));
       __syncthreads();
-      for (int line = threadIdx.x; line < NV * N2; line += kThreads) {
+      for (int line = threadIdx.x; line < NV * N2; line += NT) {
         R x0[Q], x1[Q], x2[Q];
         line_load<Q, N2, QQ, Q3>(G, line, x0);
         line_load<Q, N2, QQ, Q3>(G + NV * Q3, line, x1);
@@ -676,7 +676,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) 
     };
     R* Rv = Rr + NV * NS;
     if (skip_inv) {
-      for (int idx = threadIdx.x; idx < NV * NS; idx += kThreads) Rr[idx] = R(0);
+      for (int idx = threadIdx.x; idx < NV * NS; idx += NT) Rr[idx] = R(0);
       __syncthreads();
     } else {
       divergence(Gi, Rr);
@@ -685,7 +685,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) 
       if (visc) {
         divergence(Gv, Rv);
       } else {
-        for (int idx = threadIdx.x; idx < NV * NS; idx += kThreads) Rv[idx] = R(0);
+        for (int idx = threadIdx.x; idx < NV * NS; idx += NT) Rv[idx] = R(0);
         __syncthreads();
       }
     }
@@ -694,7 +694,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) 
   R* hc = smem + L::HC;                         // [6][C][FP] face flux at canonical points, then at the face nodes
   const size_t base = (size_t)e * N3 * NV;
   // one face point per thread: its NV inviscid and NV viscous flux values (contiguous)
-  for (int it = threadIdx.x; it < 6 * QF2; it += kThreads) {
+  for (int it = threadIdx.x; it < 6 * QF2; it += NT) {
     const int lf = it / QF2, q = it % QF2;
     const int f = fface[lf] >> 1, side = fface[lf] & 1;
     const double si = side == 0 ? -1.0 : 1.0;
@@ -725,14 +725,14 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) 
     }
   }
   __syncthreads();
-  planes<QF, N, FP, FP, kThreads>(hc, hc, 6 * C, tables.bfT, tables.bfT, threadIdx.x);
+  planes<QF, N, FP, FP, NT>(hc, hc, 6 * C, tables.bfT, tables.bfT, threadIdx.x);
   __syncthreads();
   // non-affine elements: the residuals go to rows RrT [N3][CS] in element node order (inviscid
   // channels, then from CSH the viscous ones) beyond hc, for pair loads in the
   // dense M^-1
   constexpr int CSH = L::CSH, CS = L::CS;
   R* RrT = smem + L::RT;
-  for (int idx = threadIdx.x; idx < C * N3; idx += kThreads) {
+  for (int idx = threadIdx.x; idx < C * N3; idx += NT) {
     const int c = idx / N3, l = idx % N3;
     const int xyz[3] = {l % N, (l / N) % N, l / N2};
     R acc = Rr[c * NS + nod(l)];
@@ -750,7 +750,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) 
   __syncthreads();
   // values idx (node-major, as in memory) of the residuals, inviscid and viscous: coalesced stores
   auto emit = [&](const R* inv, const R* vis, R cf) {
-    for (int idx = threadIdx.x; idx < NV * N3; idx += kThreads) {
+    for (int idx = threadIdx.x; idx < NV * N3; idx += NT) {
       const size_t o = base + idx;
       const double ri = (double)(cf * inv[idx]), rv = SPLIT ? (double)(cf * vis[idx]) : 0.0;
       if (!A.stage) {
@@ -767,9 +767,9 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) 
   };
   R* rows = hc;                                       // [C / NV][N3][NV] results in memory order (hc is dead)
   if (aff) {
-    planes<N, N, PS, PS, kThreads>(Rr, Rr, C * N, tables.m1i, tables.m1i, threadIdx.x);
+    planes<N, N, PS, PS, NT>(Rr, Rr, C * N, tables.m1i, tables.m1i, threadIdx.x);
     __syncthreads();
-    for (int line = threadIdx.x; line < C * N2; line += kThreads) {
+    for (int line = threadIdx.x; line < C * N2; line += NT) {
       R x[N];
       line_load<N, N2, PS, NS>(Rr, line, x);
       const int c = line / N2;
@@ -791,7 +791,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) 
   constexpr int JH = (N3 + HALVES - 1) / HALVES;
   R* part = smem + L::PART;                           // [HALVES][2][NV][N3]
   auto apply = [&](const auto* M) {
-    for (int idx = threadIdx.x; idx < HALVES * NG * N3; idx += kThreads) {
+    for (int idx = threadIdx.x; idx < HALVES * NG * N3; idx += NT) {
       const int i = idx % N3, g = (idx / N3) % NG, h = idx / (NG * N3);
       const int v0 = g * VB;
       R ri[VB], rv[VB];
@@ -822,7 +822,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) 
   };
   if (MT32) apply(MT32); else apply(MT);
   __syncthreads();
-  for (int idx = threadIdx.x; idx < NV * N3; idx += kThreads) {
+  for (int idx = threadIdx.x; idx < NV * N3; idx += NT) {
     const int v = idx / N3, i = idx % N3;
     R si = part[(0 * NV + v) * N3 + i], sv = part[(1 * NV + v) * N3 + i];
     if (HALVES == 2) {

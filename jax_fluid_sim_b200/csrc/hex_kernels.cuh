@@ -51,6 +51,8 @@ struct HexDims {
   static constexpr int Q = P == 1 ? 2 : (P == 2 ? 3 : 5);
   static constexpr int QF = P == 1 ? 2 : (P == 2 ? 3 : 4);
   static constexpr int N3 = N * N * N, Q3 = Q * Q * Q, N2 = N * N, QF2 = QF * QF;
+  // CTA size of the traces and element kernels (one element each)
+  static constexpr int NT = P == 3 ? 128 : P == 2 ? 64 : 32;
 };
 
 // local face -> (normal axis, end) for the reference's hexahedron face list (hybrid/mesh.py:51-58)
@@ -376,12 +378,12 @@ __device__ __forceinline__ void stage_minv(const double* Mg, const int* lex2node
 // gradients, for each of the six faces, in the owner's face-point order.
 // F32: the viscous traces go to the float32 buffers trV32 / trG32 (fused form, mixed precision).
 template <int P, int NV, typename R = double, bool F32 = false>
-__global__ void __launch_bounds__(kThreads) k_hex_traces(const __grid_constant__ DevPlan P_, const StatePtrs S, int b,
+__global__ void __launch_bounds__(HexDims<P>::NT) k_hex_traces(const __grid_constant__ DevPlan P_, const StatePtrs S, int b,
                                                         const __grid_constant__ HexTablesT<R> tables,
                                                         const HexCodes codes) {
   using D = HexDims<P>;
   using L = HexSmem<P, NV, R>;
-  constexpr int N = D::N, QF = D::QF, N2 = D::N2, N3 = D::N3, QF2 = D::QF2;
+  constexpr int N = D::N, QF = D::QF, N2 = D::N2, N3 = D::N3, QF2 = D::QF2, NT = D::NT;
   extern __shared__ __align__(16) unsigned char dyn_smem[];
   R* smem = reinterpret_cast<R*>(dyn_smem);
   R* U = smem + L::TR_U;             // [NV][N3], minus anchor
@@ -403,7 +405,7 @@ __global__ void __launch_bounds__(kThreads) k_hex_traces(const __grid_constant__
   double* raw = reinterpret_cast<double*>(slabs);
   static_assert((L::TRACES - L::TR_W) * (int)sizeof(R) >= N3 * NV * (int)sizeof(double) && L::TR_W * sizeof(R) % 8 == 0,
                 "raw state");
-  for (int idx = threadIdx.x; idx < N3 * NV; idx += kThreads) raw[idx] = Ug[idx];
+  for (int idx = threadIdx.x; idx < N3 * NV; idx += NT) raw[idx] = Ug[idx];
   if (threadIdx.x < 6) {
     int ft, f, side;
     decode_face(B.elem_face[e * 6 + threadIdx.x], ft, f, side);
@@ -413,7 +415,7 @@ __global__ void __launch_bounds__(kThreads) k_hex_traces(const __grid_constant__
   __syncthreads();
   if (threadIdx.x < NV) anchor[threadIdx.x] = raw[threadIdx.x];
   const bool visc = P_.viscous;
-  for (int l = threadIdx.x; l < N3; l += kThreads) {
+  for (int l = threadIdx.x; l < N3; l += NT) {
     const double* un = raw + codes.lex2node[l] * NV;
     double u[NV];
 #pragma unroll
@@ -430,7 +432,7 @@ __global__ void __launch_bounds__(kThreads) k_hex_traces(const __grid_constant__
   }
   __syncthreads();
   // one face node (face, j1, j2) per thread: all its channels
-  for (int it = threadIdx.x; it < 6 * N2; it += kThreads) {
+  for (int it = threadIdx.x; it < 6 * N2; it += NT) {
     const int lf = it / N2, j = it % N2, j1 = j % N, j2 = j / N;
     int a0, end, a1, a2;
     hex_face_axes(lf, a0, end, a1, a2);
@@ -455,17 +457,17 @@ __global__ void __launch_bounds__(kThreads) k_hex_traces(const __grid_constant__
   __syncthreads();
   // the face contractions, all in one phase: U and dv/dn in place, v to fv and its derivatives (df along one
   // face axis, bf along the other) to g1 and g2
-  planes<N, QF, FP, FP, kThreads>(slabs, slabs, 6 * NV, tables.bf, tables.bf, rotated(0));
+  planes<N, QF, FP, FP, NT>(slabs, slabs, 6 * NV, tables.bf, tables.bf, rotated<NT>(0));
   if (visc) {
     R* v = slabs + 6 * NV * FP;
-    planes<N, QF, FP, FP, kThreads>(v + 24 * FP, v + 24 * FP, 24, tables.bf, tables.bf, rotated(6 * NV));
-    planes<N, QF, FP, FP, kThreads>(v, fv, 24, tables.bf, tables.bf, rotated(6 * NV + 24));
-    planes<N, QF, FP, FP, kThreads>(v, g1, 24, tables.df, tables.bf, rotated(6 * NV + 48));
-    planes<N, QF, FP, FP, kThreads>(v, g2, 24, tables.bf, tables.df, rotated(6 * NV + 72));
+    planes<N, QF, FP, FP, NT>(v + 24 * FP, v + 24 * FP, 24, tables.bf, tables.bf, rotated<NT>(6 * NV));
+    planes<N, QF, FP, FP, NT>(v, fv, 24, tables.bf, tables.bf, rotated<NT>(6 * NV + 24));
+    planes<N, QF, FP, FP, NT>(v, g1, 24, tables.df, tables.bf, rotated<NT>(6 * NV + 48));
+    planes<N, QF, FP, FP, NT>(v, g2, 24, tables.bf, tables.df, rotated<NT>(6 * NV + 72));
   }
   __syncthreads();
   // one face point per thread from here on: its values are contiguous in the face buffers
-  for (int it = threadIdx.x; it < 6 * QF2; it += kThreads) {
+  for (int it = threadIdx.x; it < 6 * QF2; it += NT) {
     const int lf = it / QF2, q = it % QF2;
     const int c = codes.perm[fperm[lf] + q];
     double* dst = fd.trA + ((size_t)fslot[lf] + q) * NV;
@@ -473,11 +475,11 @@ __global__ void __launch_bounds__(kThreads) k_hex_traces(const __grid_constant__
     for (int v = 0; v < NV; ++v) dst[v] = anchor[v] + (double)slabs[(lf * NV + v) * FP + c];
   }
   // the anchor state per face side, for the face kernel's anchor flux
-  for (int idx = threadIdx.x; idx < 6 * NV; idx += kThreads)
+  for (int idx = threadIdx.x; idx < 6 * NV; idx += NT)
     fd.anc[(size_t)(fslot[idx / NV] / QF2) * NV + idx % NV] = anchor[idx % NV];
   if (visc) {
     const R* gn = slabs + (6 * NV + 24) * FP;      // [6][4][FP] derivative along the face normal's axis
-    for (int it = threadIdx.x; it < 6 * QF2; it += kThreads) {
+    for (int it = threadIdx.x; it < 6 * QF2; it += NT) {
       const int lf = it / QF2, q = it % QF2;
       const int c = codes.perm[fperm[lf] + q];
       const size_t pt = (size_t)fslot[lf] + q;
