@@ -174,6 +174,28 @@ __global__ void k_to_float32(const double* __restrict__ src, float* __restrict__
     dst[i] = (float)src[i];
 }
 
+// Rows of nq points with K values each become K rows of nq points, in place; one CTA per row.
+__global__ void k_values_by_row(double* data, int nq, int K) {
+  extern __shared__ double row[];
+  double* mine = data + (size_t)blockIdx.x * nq * K;
+  for (int i = threadIdx.x; i < nq * K; i += blockDim.x) row[i] = mine[i];
+  __syncthreads();
+  for (int i = threadIdx.x; i < nq * K; i += blockDim.x) mine[i] = row[i % nq * K + i / nq];
+}
+
+// Uploads a per-point table given point by point [rows][nq][K] as [rows][K][nq].
+int upload_by_value(dgb_plan* p, const double* host, size_t rows, int nq, int K, const double** out) {
+  int rc;
+  if ((rc = upload(p, host, rows * nq * K, out))) return rc;
+  if (rows == 0 || nq == 0) return DGB_OK;
+  const size_t smem = sizeof(double) * nq * K;
+  if (rows > 0x7fffffff || smem > 48 * 1024) return fail(DGB_ERR_UNSUPPORTED, "per-point table too large");
+  k_values_by_row<<<(unsigned)rows, 128, smem>>>(const_cast<double*>(*out), nq, K);
+  CK(cudaGetLastError());
+  CK(cudaDeviceSynchronize());
+  return DGB_OK;
+}
+
 // A float32 copy of n device doubles, owned by the plan (null source: null copy).
 int to_float32(dgb_plan* p, const double* src, size_t n, float** out) {
   *out = nullptr;
@@ -1191,7 +1213,7 @@ int dgb_plan_set_block(dgb_plan* p, int b, const dgb_block_desc* d) {
       B.lebesgue = fmax(B.lebesgue, a);
     }
   }
-  if ((rc = upload(p, d->inv_jacobian, E * Nq * 9, &B.jinv))) return rc;
+  if ((rc = upload_by_value(p, d->inv_jacobian, E, (int)Nq, 9, &B.jinv))) return rc;
   if ((rc = upload(p, d->wdet, E * Nq, &B.wdet))) return rc;
   // the inverse mass matrices may instead be built on the device (dgb_plan_build_inverse_mass)
   B.minv = nullptr;
@@ -1224,9 +1246,9 @@ int dgb_plan_set_faces(dgb_plan* p, const dgb_face_desc* d) {
   if ((rc = upload(p, d->nbr_local, n, &F.nl))) return rc;
   if ((rc = upload(p, d->nbr_code, n, &F.nc))) return rc;
   if ((rc = upload(p, d->tags, n, &F.tag))) return rc;
-  if ((rc = upload(p, d->normals, n * nq * 3, &F.n))) return rc;
+  if ((rc = upload_by_value(p, d->normals, n, (int)nq, 3, &F.n))) return rc;
   if ((rc = upload(p, d->weights, n * nq, &F.w))) return rc;
-  if ((rc = upload(p, d->side_inv_jacobian, n * 2 * nq * 9, &F.jinv))) return rc;
+  if ((rc = upload_by_value(p, d->side_inv_jacobian, n * 2, (int)nq, 9, &F.jinv))) return rc;
   // the two sides of each face in one record (dense_rhs.cu)
   std::vector<int3> side(2 * n);
   for (size_t f = 0; f < n; ++f) {

@@ -203,10 +203,11 @@ __device__ __forceinline__ void update_body(const DevPlan& D, const StatePtrs& S
           const int el = g * EB + h * EB2 + k;
           const size_t e = (size_t)e0 + (el < ne ? el : 0);
           const bool aff = B.affine != nullptr && B.affine[e];
-          const double* Jd = aff ? B.ajinv + e * 9 : B.jinv + (e * Nq + q) * 9;
+          const double* Jd = aff ? B.ajinv + e * 9 : B.jinv + e * 9 * Nq + q;
+          const int js = aff ? 1 : Nq;
           R J[9];
 #pragma unroll
-          for (int m = 0; m < 9; ++m) J[m] = (R)Jd[m];
+          for (int m = 0; m < 9; ++m) J[m] = (R)Jd[m * js];
           const R wq = aff ? (R)(B.wref[q] * B.adet[e]) : (R)(B.wdet[e * Nq + q] * 1.0);
           R Uq[NV], F[3][NV];
 #pragma unroll
@@ -313,9 +314,10 @@ __device__ __forceinline__ void update_body(const DevPlan& D, const StatePtrs& S
 #pragma unroll
       for (int m = 1; m < nlf; ++m) lf += pt >= S::poff(m);
       const FaceDev& fd = D.face[lf < S::ntri ? 0 : 1];
-      const double* src = fd.fluxI + ((size_t)fslot[e * nlf + lf] * S::nq(lf) + pt - S::poff(lf)) * NV;
+      const int nq = S::nq(lf);
+      const double* src = fd.fluxI + face_at((size_t)fslot[e * nlf + lf], NV, 0, nq, pt - S::poff(lf));
 #pragma unroll
-      for (int v = 0; v < NV; ++v) x[k][v] = src[v];
+      for (int v = 0; v < NV; ++v) x[k][v] = src[v * nq];
     }
 #pragma unroll
     for (int k = 0; k < FR; ++k) {
@@ -517,10 +519,9 @@ __device__ __forceinline__ void faces_body(const DevPlan& D, const StatePtrs& St
 #pragma unroll
     for (int v = 0; v < NV; ++v) out[v] = anc[(slot * 2 + side) * NV + v] + (double)acc[v];
   };
-  const double* np_ = fd.n + ((size_t)f * nq + q) * 3;
-  const double n[3] = {np_[0], np_[1], np_[2]};
+  const double n[3] = {fd.n[face_at(f, 3, 0, nq, q)], fd.n[face_at(f, 3, 1, nq, q)], fd.n[face_at(f, 3, 2, nq, q)]};
   const double w = fd.w[(size_t)f * nq + q];
-  const size_t so = ((size_t)f * 2 + 0) * nq + q, sn = ((size_t)f * 2 + 1) * nq + q;
+  const size_t so = (size_t)f * 2, sn = so + 1;
   double UL[NV], UR[NV], Fh[NV], Fa[NV];
   trace(0, fd.ob[f], fd.oc[f], UL);
   if (nb >= 0) {
@@ -533,10 +534,10 @@ __device__ __forceinline__ void faces_body(const DevPlan& D, const StatePtrs& St
   }
   if (store_traces) {
 #pragma unroll
-    for (int v = 0; v < NV; ++v) fd.trA[so * NV + v] = UL[v];
+    for (int v = 0; v < NV; ++v) fd.trA[face_at(so, NV, v, nq, q)] = UL[v];
     if (nb >= 0)
 #pragma unroll
-      for (int v = 0; v < NV; ++v) fd.trA[sn * NV + v] = UR[v];
+      for (int v = 0; v < NV; ++v) fd.trA[face_at(sn, NV, v, nq, q)] = UR[v];
   }
   hllc<NV>(D.ph, UL, UR, n, Fh);
 #pragma unroll
@@ -546,9 +547,9 @@ __device__ __forceinline__ void faces_body(const DevPlan& D, const StatePtrs& St
 #pragma unroll
     for (int v = 0; v < NV; ++v) a[v] = anc[(slot * 2 + side) * NV + v];
     normal_flux<NV>(D.ph, a, n, Fa);
-    double* out = fd.fluxI + (side ? sn : so) * NV;
+    double* out = fd.fluxI + face_at(side ? sn : so, NV, 0, nq, q);
 #pragma unroll
-    for (int v = 0; v < NV; ++v) out[v] = (Fh[v] - Fa[v]) * w;
+    for (int v = 0; v < NV; ++v) out[v * nq] = (Fh[v] - Fa[v]) * w;
   }
 }
 

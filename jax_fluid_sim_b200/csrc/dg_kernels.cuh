@@ -32,7 +32,7 @@ struct BlockDev {
   int type, E, Np, Nq, nlf, Ns;
   const double* B;        // [Nq][Np]
   const double* dB;       // [Nq][Np][3]
-  const double* jinv;     // [E][Nq][9]
+  const double* jinv;     // [E][9][Nq]
   const double* wdet;     // [E][Nq]
   const double* minv;     // [E][Np][Np]
   double lebesgue;        // max over the limiter samples (nodes, volume, face) of sum_i |B_i|
@@ -61,35 +61,42 @@ struct BlockDev {
   const int32_t* ecase;   // [E] case of each element (ensembles; null for one case)
   // float32 copies read by the mixed-precision hexahedron kernels (null in float64 plans)
   const float* minv32;    // [E][Np][Np], same layout as minv
-  const float* jinv32;    // [E][Nq][9]
+  const float* jinv32;    // [E][9][Nq]
 };
 
+// Per-point tables and buffers of a face (side) hold one value of every point side by side, so that a
+// warp, whose lanes take consecutive points, touches whole lines (face_at).
 struct FaceDev {
   int F, nq;
   const int32_t *ob, *ol, *oc, *nb, *nl, *nc, *tag;
-  const double* n;        // [F][nq][3]
+  const double* n;        // [F][3][nq]
   const double* w;        // [F][nq]
-  const double* jinv;     // [F][2][nq][9]
-  double* trA;            // [F][2][nq][NV] anchor-form U traces
+  const double* jinv;     // [F][2][9][nq]
+  double* trA;            // [F][2][NV][nq] anchor-form U traces
   double* anc;            // [F][2][NV] anchor state (node 0) of each side's element
-  double* trP;            // [F][2][nq][NV] plain U traces
-  double* trV;            // [F][2][nq][4]
-  double* trG;            // [F][2][nq][12] raw gradients of the viscous variables
-  double* fluxI;          // [F][2][nq][NV] (F_hat - F(anchor).n) w per side
-  double* jumpW;          // [F][nq][12]    0.5 w [v] (x) n
-  double* liftF;          // [F][2][nq][12] br2 * B_f r_f per side
-  double* fluxV;          // [F][nq][NV]    viscous normal flux times w
+  double* trP;            // [F][2][NV][nq] plain U traces
+  double* trV;            // [F][2][4][nq]
+  double* trG;            // [F][2][12][nq] raw gradients of the viscous variables
+  double* fluxI;          // [F][2][NV][nq] (F_hat - F(anchor).n) w per side
+  double* jumpW;          // [F][12][nq]    0.5 w [v] (x) n
+  double* liftF;          // [F][2][12][nq] br2 * B_f r_f per side
+  double* fluxV;          // [F][NV][nq]    viscous normal flux times w
   const float* jinv32;    // float32 copy of jinv (mixed-precision plans; else null)
   // float32 traces of the viscous variables and their gradients, written and read by the fused
   // hexahedron kernels of mixed-precision plans (else null)
-  float* trV32;           // [F][2][nq][4]
-  float* trG32;           // [F][2][nq][12]
+  float* trV32;           // [F][2][4][nq]
+  float* trG32;           // [F][2][12][nq]
   // float32 face fluxes and BR2 jumps of the fused hexahedron kernels of mixed-precision plans (the
   // element kernel rounds them to float32 anyway)
-  float* fluxI32;         // [F][2][nq][NV]
-  float* fluxV32;         // [F][nq][NV]
-  float* jumpW32;         // [F][nq][12]
+  float* fluxI32;         // [F][2][NV][nq]
+  float* fluxV32;         // [F][NV][nq]
+  float* jumpW32;         // [F][12][nq]
 };
+
+// Value k of K at point q of face (or face side: face * 2 + side) r.
+__host__ __device__ __forceinline__ size_t face_at(size_t r, int K, int k, int nq, int q) {
+  return (r * K + k) * nq + q;
+}
 
 struct DevPlan {
   int nv, nblocks, viscous, degree;
@@ -189,7 +196,7 @@ __global__ void __launch_bounds__(kThreads) k_traces(const DevPlan P, const Stat
     const int ft = Fc.ft[lf], nq = Fc.nq[lf];
     const FaceDev& fd = P.face[ft];
     const double* Bt = B.trBt[ft] + (size_t)Fc.code[lf] * Np * nq + q;    // [i][q]: stride nq
-    const size_t pt = ((size_t)Fc.f[lf] * 2 + Fc.side[lf]) * nq + q;
+    const size_t fs = (size_t)Fc.f[lf] * 2 + Fc.side[lf];
     R acc[NV];
 #pragma unroll
     for (int v = 0; v < NV; ++v) acc[v] = (R)0;
@@ -199,15 +206,15 @@ __global__ void __launch_bounds__(kThreads) k_traces(const DevPlan P, const Stat
       for (int v = 0; v < NV; ++v) acc[v] += bt * U[i * NV + v];
     }
 #pragma unroll
-    for (int v = 0; v < NV; ++v) fd.trA[pt * NV + v] = anchor[g][v] + (double)acc[v];
+    for (int v = 0; v < NV; ++v) fd.trA[face_at(fs, NV, v, nq, q)] = anchor[g][v] + (double)acc[v];
     if (q == 0)
 #pragma unroll
-      for (int v = 0; v < NV; ++v) fd.anc[((size_t)Fc.f[lf] * 2 + Fc.side[lf]) * NV + v] = anchor[g][v];
+      for (int v = 0; v < NV; ++v) fd.anc[fs * NV + v] = anchor[g][v];
     if (P.viscous) {
       const double* dBt = B.trdBt[ft] + (size_t)Fc.code[lf] * Np * 3 * nq + q;   // [i][r][q]
       R J[9];
 #pragma unroll
-      for (int k = 0; k < 9; ++k) J[k] = (R)fd.jinv[pt * 9 + k];
+      for (int k = 0; k < 9; ++k) J[k] = (R)fd.jinv[face_at(fs, 9, k, nq, q)];
       R tv[4], tg[12];
 #pragma unroll
       for (int k = 0; k < 4; ++k) tv[k] = (R)0;
@@ -229,9 +236,9 @@ __global__ void __launch_bounds__(kThreads) k_traces(const DevPlan P, const Stat
         }
       }
 #pragma unroll
-      for (int m = 0; m < 4; ++m) fd.trV[pt * 4 + m] = (double)tv[m];
+      for (int m = 0; m < 4; ++m) fd.trV[face_at(fs, 4, m, nq, q)] = (double)tv[m];
 #pragma unroll
-      for (int k = 0; k < 12; ++k) fd.trG[pt * 12 + k] = (double)tg[k];
+      for (int k = 0; k < 12; ++k) fd.trG[face_at(fs, 12, k, nq, q)] = (double)tg[k];
     }
   }
 }
@@ -248,15 +255,15 @@ __global__ void __launch_bounds__(kThreads, NV <= 5 ? 6 : 1) k_face_flux(const D
   if (t >= fd.F * nq) return;
   const int f = t / nq, q = t % nq;
   const int nb = fd.nb[f];
-  const double* n = fd.n + ((size_t)f * nq + q) * 3;
+  const double n[3] = {fd.n[face_at(f, 3, 0, nq, q)], fd.n[face_at(f, 3, 1, nq, q)], fd.n[face_at(f, 3, 2, nq, q)]};
   const double w = fd.w[(size_t)f * nq + q];
-  const size_t so = ((size_t)f * 2 + 0) * nq + q, sn = ((size_t)f * 2 + 1) * nq + q;
+  const size_t so = (size_t)f * 2, sn = so + 1;
   double UL[NV], UR[NV], Fh[NV], Fa[NV];
 #pragma unroll
-  for (int v = 0; v < NV; ++v) UL[v] = fd.trA[so * NV + v];
+  for (int v = 0; v < NV; ++v) UL[v] = fd.trA[face_at(so, NV, v, nq, q)];
   if (nb >= 0) {
 #pragma unroll
-    for (int v = 0; v < NV; ++v) UR[v] = fd.trA[sn * NV + v];
+    for (int v = 0; v < NV; ++v) UR[v] = fd.trA[face_at(sn, NV, v, nq, q)];
   } else if (P.ph.has_boundary) {
     ghost_state<NV>(P.ph, case_view(P.ph, P.blk[fd.ob[f]].ecase, fd.ol[f]).far, UL, n, fd.tag[f], UR);
   } else {
@@ -270,7 +277,7 @@ __global__ void __launch_bounds__(kThreads, NV <= 5 ? 6 : 1) k_face_flux(const D
     for (int v = 0; v < NV; ++v) a[v] = fd.anc[((size_t)f * 2 + 0) * NV + v];
     normal_flux<NV>(P.ph, a, n, Fa);
 #pragma unroll
-    for (int v = 0; v < NV; ++v) fd.fluxI[so * NV + v] = (Fh[v] - Fa[v]) * w;
+    for (int v = 0; v < NV; ++v) fd.fluxI[face_at(so, NV, v, nq, q)] = (Fh[v] - Fa[v]) * w;
   }
   if (nb >= 0) {
     double a[NV];
@@ -278,26 +285,25 @@ __global__ void __launch_bounds__(kThreads, NV <= 5 ? 6 : 1) k_face_flux(const D
     for (int v = 0; v < NV; ++v) a[v] = fd.anc[((size_t)f * 2 + 1) * NV + v];
     normal_flux<NV>(P.ph, a, n, Fa);
 #pragma unroll
-    for (int v = 0; v < NV; ++v) fd.fluxI[sn * NV + v] = (Fh[v] - Fa[v]) * w;
+    for (int v = 0; v < NV; ++v) fd.fluxI[face_at(sn, NV, v, nq, q)] = (Fh[v] - Fa[v]) * w;
   }
   if (P.viscous) {
     double vo[4], vn[4];
 #pragma unroll
-    for (int m = 0; m < 4; ++m) vo[m] = fd.trV[so * 4 + m];
+    for (int m = 0; m < 4; ++m) vo[m] = fd.trV[face_at(so, 4, m, nq, q)];
     if (nb >= 0) {
 #pragma unroll
-      for (int m = 0; m < 4; ++m) vn[m] = fd.trV[sn * 4 + m];
+      for (int m = 0; m < 4; ++m) vn[m] = fd.trV[face_at(sn, 4, m, nq, q)];
     } else if (P.ph.has_boundary) {
       const CaseView cv = case_view(P.ph, P.blk[fd.ob[f]].ecase, fd.ol[f]);
       viscous_ghost<NV>(P.ph, cv.far, cv.wall_T, UL, n, fd.tag[f], vn);
     } else {
       viscous_vars<NV>(P.ph, UL, vn);
     }
-    double* out = fd.jumpW + ((size_t)f * nq + q) * 12;
 #pragma unroll
     for (int m = 0; m < 4; ++m)
 #pragma unroll
-      for (int d = 0; d < 3; ++d) out[m * 3 + d] = 0.5 * w * (vn[m] - vo[m]) * n[d];
+      for (int d = 0; d < 3; ++d) fd.jumpW[face_at(f, 12, m * 3 + d, nq, q)] = 0.5 * w * (vn[m] - vo[m]) * n[d];
   }
 }
 
@@ -357,7 +363,7 @@ __global__ void __launch_bounds__(kThreads, NV <= 5 ? 4 : 1) k_volume(const DevP
   // affine elements read one inverse Jacobian and |det J| instead of per-point tables
   const bool aff = B.affine != nullptr && B.affine[ee];
   const double* jinv = aff ? B.ajinv + ee * 9 : B.jinv + ee * Nq * 9;
-  const int jstride = aff ? 0 : 9;
+  const int jpoint = aff ? 0 : 1, jvalue = aff ? 1 : Nq;   // strides of jinv between points and between values
   const double* wdet = aff ? B.wref : B.wdet + ee * Nq;
   const double wscale = aff ? B.adet[ee] : 1.0;
   const double* Mi = aff ? B.mref_inv : B.minv + ee * Np * Np;
@@ -382,7 +388,7 @@ __global__ void __launch_bounds__(kThreads, NV <= 5 ? 4 : 1) k_volume(const DevP
         const double* Bt = B.trB[Fc.ft[lf]] + (size_t)Fc.code[lf] * nq * Np;
         const double* Jw = P.face[Fc.ft[lf]].jumpW + (size_t)Fc.f[lf] * nq * 12;
         R acc = (R)0;
-        for (int q = 0; q < nq; ++q) acc += (R)Jw[q * 12 + c] * (R)Bt[q * Np + i];
+        for (int q = 0; q < nq; ++q) acc += (R)Jw[c * nq + q] * (R)Bt[q * Np + i];
         bf[idx] = acc;
       }
     }
@@ -416,7 +422,7 @@ __global__ void __launch_bounds__(kThreads, NV <= 5 ? 4 : 1) k_volume(const DevP
       const double* Bt = B.trB[Fc.ft[lf]] + ((size_t)Fc.code[lf] * nq + q) * Np;
       R acc = (R)0;
       for (int i = 0; i < Np; ++i) acc += (R)Bt[i] * rf[(lf * Np + i) * 12 + c];
-      P.face[Fc.ft[lf]].liftF[(((size_t)Fc.f[lf] * 2 + Fc.side[lf]) * nq + q) * 12 + c] =
+      P.face[Fc.ft[lf]].liftF[face_at((size_t)Fc.f[lf] * 2 + Fc.side[lf], 12, c, nq, q)] =
           P.ph.br2 * (double)acc;
     }
   }
@@ -434,10 +440,10 @@ __global__ void __launch_bounds__(kThreads, NV <= 5 ? 4 : 1) k_volume(const DevP
     }
     for (int q = lane; q < Nq; q += W) {
       const double* Bq = B.Bt + q;                    // [i][q]: stride Nq
-      const double* Jd = jinv + q * jstride;
+      const double* Jd = jinv + q * jpoint;
       R J[9];
 #pragma unroll
-      for (int k = 0; k < 9; ++k) J[k] = (R)Jd[k];
+      for (int k = 0; k < 9; ++k) J[k] = (R)Jd[k * jvalue];
       const R wq = (R)(wdet[q] * wscale);
       R Uq[NV];
 #pragma unroll
@@ -541,23 +547,23 @@ __global__ void __launch_bounds__(kThreads) k_face_visc(const DevPlan P, int ft)
   if (t >= fd.F * nq) return;
   const int f = t / nq, q = t % nq;
   const int nb = fd.nb[f];
-  const double* n = fd.n + ((size_t)f * nq + q) * 3;
+  const double n[3] = {fd.n[face_at(f, 3, 0, nq, q)], fd.n[face_at(f, 3, 1, nq, q)], fd.n[face_at(f, 3, 2, nq, q)]};
   const double w = fd.w[(size_t)f * nq + q];
-  const size_t so = ((size_t)f * 2 + 0) * nq + q, sn = ((size_t)f * 2 + 1) * nq + q;
+  const size_t so = (size_t)f * 2, sn = so + 1;
   // the two sides of a face always belong to one case
   const CaseView cv = case_view(P.ph, P.blk[fd.ob[f]].ecase, fd.ol[f]);
   double U[NV], g[12], Fo[3 * NV];
 #pragma unroll
-  for (int v = 0; v < NV; ++v) U[v] = fd.trP[so * NV + v];
+  for (int v = 0; v < NV; ++v) U[v] = fd.trP[face_at(so, NV, v, nq, q)];
 #pragma unroll
-  for (int c = 0; c < 12; ++c) g[c] = fd.trG[so * 12 + c] + fd.liftF[so * 12 + c];
+  for (int c = 0; c < 12; ++c) g[c] = fd.trG[face_at(so, 12, c, nq, q)] + fd.liftF[face_at(so, 12, c, nq, q)];
   viscous_flux<NV>(P.ph, cv.mu, cv.kappa, U, g, Fo);
   if (nb >= 0) {
     double Fn[3 * NV];
 #pragma unroll
-    for (int v = 0; v < NV; ++v) U[v] = fd.trP[sn * NV + v];
+    for (int v = 0; v < NV; ++v) U[v] = fd.trP[face_at(sn, NV, v, nq, q)];
 #pragma unroll
-    for (int c = 0; c < 12; ++c) g[c] = fd.trG[sn * 12 + c] + fd.liftF[sn * 12 + c];
+    for (int c = 0; c < 12; ++c) g[c] = fd.trG[face_at(sn, 12, c, nq, q)] + fd.liftF[face_at(sn, 12, c, nq, q)];
     viscous_flux<NV>(P.ph, cv.mu, cv.kappa, U, g, Fn);
 #pragma unroll
     for (int k = 0; k < 3 * NV; ++k) Fo[k] = 0.5 * (Fo[k] + Fn[k]);
@@ -567,7 +573,7 @@ __global__ void __launch_bounds__(kThreads) k_face_visc(const DevPlan P, int ft)
   for (int v = 0; v < NV; ++v) out[v] = Fo[0 * NV + v] * n[0] + Fo[1 * NV + v] * n[1] + Fo[2 * NV + v] * n[2];
   if (nb < 0 && P.ph.has_boundary && tag_in(fd.tag[f], P.ph.wall, P.ph.n_wall)) out[4] = 0.0;
 #pragma unroll
-  for (int v = 0; v < NV; ++v) fd.fluxV[((size_t)f * nq + q) * NV + v] = out[v] * w;
+  for (int v = 0; v < NV; ++v) fd.fluxV[face_at(f, NV, v, nq, q)] = out[v] * w;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -596,14 +602,14 @@ __global__ void __launch_bounds__(kThreads) k_wall_forces(const DevPlan P, int f
   if (t < (long)fd.F * nq) {
     const int f = (int)(t / nq), q = (int)(t % nq);
     if (fd.nb[f] < 0 && tag_in(fd.tag[f], walls.tags, walls.n)) {
-      const size_t so = ((size_t)f * 2 + 0) * nq + q;
-      const double* n = fd.n + ((size_t)f * nq + q) * 3;
+      const size_t so = (size_t)f * 2;
+      const double n[3] = {fd.n[face_at(f, 3, 0, nq, q)], fd.n[face_at(f, 3, 1, nq, q)], fd.n[face_at(f, 3, 2, nq, q)]};
       const double w = fd.w[(size_t)f * nq + q];
       const double* x = points + ((size_t)f * nq + q) * 3;
       const double r[3] = {x[0] - walls.center[0], x[1] - walls.center[1], x[2] - walls.center[2]};
       double U[NV], W[NV];
 #pragma unroll
-      for (int v = 0; v < NV; ++v) U[v] = fd.trA[so * NV + v];
+      for (int v = 0; v < NV; ++v) U[v] = fd.trA[face_at(so, NV, v, nq, q)];
       primitive<NV>(P.ph, U, W);
       double F[3];
 #pragma unroll
@@ -617,7 +623,7 @@ __global__ void __launch_bounds__(kThreads) k_wall_forces(const DevPlan P, int f
       if (P.viscous) {
         double g[12], Fv[3 * NV];
 #pragma unroll
-        for (int k = 0; k < 12; ++k) g[k] = fd.trG[so * 12 + k] + fd.liftF[so * 12 + k];
+        for (int k = 0; k < 12; ++k) g[k] = fd.trG[face_at(so, 12, k, nq, q)] + fd.liftF[face_at(so, 12, k, nq, q)];
         const CaseView cv = case_view(P.ph, P.blk[fd.ob[f]].ecase, fd.ol[f]);
         viscous_flux<NV>(P.ph, cv.mu, cv.kappa, U, g, Fv);
 #pragma unroll
@@ -713,7 +719,7 @@ __global__ void __launch_bounds__(kThreads) k_finalize(const DevPlan P, const St
       for (int q = 0; q < nq; ++q) {
         const R bt = (R)Bt[(size_t)q * Np];
 #pragma unroll
-        for (int v = 0; v < NV; ++v) si[v] += bt * (R)fi[q * NV + v];
+        for (int v = 0; v < NV; ++v) si[v] += bt * (R)fi[v * nq + q];
       }
 #pragma unroll
       for (int v = 0; v < NV; ++v) Fp[t * NV + v] = sgn * si[v];
@@ -725,7 +731,7 @@ __global__ void __launch_bounds__(kThreads) k_finalize(const DevPlan P, const St
         for (int q = 0; q < nq; ++q) {
           const R bt = (R)Bt[(size_t)q * Np];
 #pragma unroll
-          for (int v = 0; v < NV; ++v) sv[v] += bt * (R)fv[q * NV + v];
+          for (int v = 0; v < NV; ++v) sv[v] += bt * (R)fv[v * nq + q];
         }
 #pragma unroll
         for (int v = 0; v < NV; ++v) Vp[t * NV + v] = -sgn * sv[v];

@@ -119,17 +119,16 @@ __global__ void __launch_bounds__(kThreads, NV <= 5 ? 6 : 1) k_hex_face(const De
   double UL[NV];
   if (live) {
     nb = fd.nb[f];
-    const double* np_ = fd.n + ((size_t)f * QF2 + q) * 3;
-    n[0] = np_[0], n[1] = np_[1], n[2] = np_[2];
+    n[0] = fd.n[face_at(f, 3, 0, QF2, q)], n[1] = fd.n[face_at(f, 3, 1, QF2, q)], n[2] = fd.n[face_at(f, 3, 2, QF2, q)];
     w = fd.w[(size_t)f * QF2 + q];
-    so = ((size_t)f * 2 + 0) * QF2 + q;
-    sn = ((size_t)f * 2 + 1) * QF2 + q;
+    so = (size_t)f * 2;
+    sn = so + 1;
     double UR[NV], Fh[NV], Fa[NV];
 #pragma unroll
-    for (int v = 0; v < NV; ++v) UL[v] = fd.trA[so * NV + v];
+    for (int v = 0; v < NV; ++v) UL[v] = fd.trA[face_at(so, NV, v, QF2, q)];
     if (nb >= 0) {
 #pragma unroll
-      for (int v = 0; v < NV; ++v) UR[v] = fd.trA[sn * NV + v];
+      for (int v = 0; v < NV; ++v) UR[v] = fd.trA[face_at(sn, NV, v, QF2, q)];
     } else if (P_.ph.has_boundary) {
       ghost_state<NV>(P_.ph, case_view(P_.ph, P_.blk[0].ecase, fd.ol[f]).far, UL, n, fd.tag[f], UR);
     } else {
@@ -144,8 +143,8 @@ __global__ void __launch_bounds__(kThreads, NV <= 5 ? 6 : 1) k_hex_face(const De
       normal_flux<NV>(P_.ph, a, n, Fa);
 #pragma unroll
       for (int v = 0; v < NV; ++v) {
-        if (RF) fd.fluxI32[so * NV + v] = (float)((Fh[v] - Fa[v]) * w);
-        else fd.fluxI[so * NV + v] = (Fh[v] - Fa[v]) * w;
+        if (RF) fd.fluxI32[face_at(so, NV, v, QF2, q)] = (float)((Fh[v] - Fa[v]) * w);
+        else fd.fluxI[face_at(so, NV, v, QF2, q)] = (Fh[v] - Fa[v]) * w;
       }
     }
     if (nb >= 0) {
@@ -155,22 +154,18 @@ __global__ void __launch_bounds__(kThreads, NV <= 5 ? 6 : 1) k_hex_face(const De
       normal_flux<NV>(P_.ph, a, n, Fa);
 #pragma unroll
       for (int v = 0; v < NV; ++v) {
-        if (RF) fd.fluxI32[sn * NV + v] = (float)((Fh[v] - Fa[v]) * w);
-        else fd.fluxI[sn * NV + v] = (Fh[v] - Fa[v]) * w;
+        if (RF) fd.fluxI32[face_at(sn, NV, v, QF2, q)] = (float)((Fh[v] - Fa[v]) * w);
+        else fd.fluxI[face_at(sn, NV, v, QF2, q)] = (Fh[v] - Fa[v]) * w;
       }
     }
   }
   if (!P_.viscous) return;
   double vo[4], vn[4];
-  // a face point's 4 viscous values: one 16-byte load (float32) or two (float64)
-  auto load_v = [&](size_t pt, double* out) {
-    if constexpr (F32) {
-      const float4 t = __ldg(reinterpret_cast<const float4*>(fd.trV32 + pt * 4));
-      out[0] = t.x, out[1] = t.y, out[2] = t.z, out[3] = t.w;
-    } else {
-      const double2* t = reinterpret_cast<const double2*>(fd.trV + pt * 4);
-      const double2 a = t[0], b2 = t[1];
-      out[0] = a.x, out[1] = a.y, out[2] = b2.x, out[3] = b2.y;
+  auto load_v = [&](size_t side, double* out) {
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      if constexpr (F32) out[m] = __ldg(fd.trV32 + face_at(side, 4, m, QF2, q));
+      else out[m] = fd.trV[face_at(side, 4, m, QF2, q)];
     }
   };
   if (live) {
@@ -183,8 +178,7 @@ __global__ void __launch_bounds__(kThreads, NV <= 5 ? 6 : 1) k_hex_face(const De
     } else {
       viscous_vars<NV>(P_.ph, UL, vn);
     }
-    const size_t jo = ((size_t)f * QF2 + q) * 12;
-    // a point's 12 jumps are contiguous in the face buffer and in jmp: 16-byte stores
+    // a point's 12 jumps are a row of jmp: 16-byte stores
     R jr[12];
 #pragma unroll
     for (int m = 0; m < 4; ++m)
@@ -192,23 +186,18 @@ __global__ void __launch_bounds__(kThreads, NV <= 5 ? 6 : 1) k_hex_face(const De
       for (int d = 0; d < 3; ++d) jr[m * 3 + d] = (R)(0.5 * w * (vn[m] - vo[m]) * n[d]);
     R* js = &jmp[slot * JS + q * 12];
     if constexpr (RF) {
-      float4* g4 = reinterpret_cast<float4*>(fd.jumpW32 + jo);
       float4* s4 = reinterpret_cast<float4*>(js);
 #pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        const float4 v = make_float4(jr[4 * k], jr[4 * k + 1], jr[4 * k + 2], jr[4 * k + 3]);
-        g4[k] = v;
-        s4[k] = v;
-      }
+      for (int k = 0; k < 3; ++k) s4[k] = make_float4(jr[4 * k], jr[4 * k + 1], jr[4 * k + 2], jr[4 * k + 3]);
     } else {
-      double2* g2 = reinterpret_cast<double2*>(fd.jumpW + jo);
       double2* s2 = reinterpret_cast<double2*>(js);
 #pragma unroll
-      for (int k = 0; k < 6; ++k) {
-        const double2 v = make_double2(jr[2 * k], jr[2 * k + 1]);
-        g2[k] = v;
-        s2[k] = v;
-      }
+      for (int k = 0; k < 6; ++k) s2[k] = make_double2(jr[2 * k], jr[2 * k + 1]);
+    }
+#pragma unroll
+    for (int k = 0; k < 12; ++k) {
+      if constexpr (RF) fd.jumpW32[face_at(f, 12, k, QF2, q)] = jr[k];
+      else fd.jumpW[face_at(f, 12, k, QF2, q)] = jr[k];
     }
   }
   __syncthreads();
@@ -294,25 +283,14 @@ __global__ void __launch_bounds__(kThreads, NV <= 5 ? 6 : 1) k_hex_face(const De
     // (dgb_wall_forces reads the viscous traction there)
     if (nb < 0)
 #pragma unroll
-      for (int c = 0; c < 12; ++c) fd.liftF[ss * 12 + c] = (double)lift[c];
+      for (int c = 0; c < 12; ++c) fd.liftF[face_at(ss, 12, c, QF2, q)] = (double)lift[c];
     R U[NV], g[12];
 #pragma unroll
-    for (int v = 0; v < NV; ++v) U[v] = (R)fd.trP[ss * NV + v];
-    // the point's 12 gradients: 16-byte loads
-    if constexpr (F32) {
-      const float4* t = reinterpret_cast<const float4*>(fd.trG32 + ss * 12);
+    for (int v = 0; v < NV; ++v) U[v] = (R)fd.trP[face_at(ss, NV, v, QF2, q)];
 #pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        const float4 a = __ldg(t + k);
-        g[4 * k] = (R)a.x, g[4 * k + 1] = (R)a.y, g[4 * k + 2] = (R)a.z, g[4 * k + 3] = (R)a.w;
-      }
-    } else {
-      const double2* t = reinterpret_cast<const double2*>(fd.trG + ss * 12);
-#pragma unroll
-      for (int k = 0; k < 6; ++k) {
-        const double2 a = t[k];
-        g[2 * k] = (R)a.x, g[2 * k + 1] = (R)a.y;
-      }
+    for (int c = 0; c < 12; ++c) {
+      if constexpr (F32) g[c] = (R)__ldg(fd.trG32 + face_at(ss, 12, c, QF2, q));
+      else g[c] = (R)fd.trG[face_at(ss, 12, c, QF2, q)];
     }
 #pragma unroll
     for (int c = 0; c < 12; ++c) g[c] += lift[c];
@@ -332,8 +310,8 @@ __global__ void __launch_bounds__(kThreads, NV <= 5 ? 6 : 1) k_hex_face(const De
   if (nb < 0 && P_.ph.has_boundary && tag_in(fd.tag[f], P_.ph.wall, P_.ph.n_wall)) out[4] = R(0);
 #pragma unroll
   for (int v = 0; v < NV; ++v) {
-    if (RF) fd.fluxV32[((size_t)f * QF2 + q) * NV + v] = (float)(out[v] * (R)w);
-    else fd.fluxV[((size_t)f * QF2 + q) * NV + v] = (double)(out[v] * (R)w);
+    if (RF) fd.fluxV32[face_at(f, NV, v, QF2, q)] = (float)(out[v] * (R)w);
+    else fd.fluxV[face_at(f, NV, v, QF2, q)] = (double)(out[v] * (R)w);
   }
 }
 
@@ -393,12 +371,12 @@ struct HexElemSmem {
 // Lift + volume + finalize of one hexahedron (see the file comment).  SPLIT keeps the inviscid
 // and viscous residuals apart (right-hand-side outputs, the MOOD step's viscous residual).
 template <int P, int NV, bool SPLIT, typename R = double>
-__global__ void __launch_bounds__(HexDims<P>::NT, sizeof(R) == sizeof(float) ? 6 * kThreads / HexDims<P>::NT : 1) k_hex_element(const __grid_constant__ DevPlan P_, const StatePtrs S,
+__global__ void __launch_bounds__(HexDims<P>::NTE, sizeof(R) == sizeof(float) ? 6 * kThreads / HexDims<P>::NTE : 1) k_hex_element(const __grid_constant__ DevPlan P_, const StatePtrs S,
                                                          const __grid_constant__ HexTablesT<R> tables,
                                                          const HexCodes codes, const __grid_constant__ FinalizeArgs A) {
   using D = HexDims<P>;
   using L = HexElemSmem<P, NV, SPLIT, R>;
-  constexpr int N = D::N, Q = D::Q, QF = D::QF, N2 = D::N2, N3 = D::N3, Q3 = D::Q3, QF2 = D::QF2, NT = D::NT;
+  constexpr int N = D::N, Q = D::Q, QF = D::QF, N2 = D::N2, N3 = D::N3, Q3 = D::Q3, QF2 = D::QF2, NT = D::NTE;
   constexpr int C = L::C;
   constexpr int b = 0;
   extern __shared__ __align__(16) unsigned char dyn_smem[];
@@ -467,29 +445,15 @@ __global__ void __launch_bounds__(HexDims<P>::NT, sizeof(R) == sizeof(float) ? 6
     R* jc = smem + L::JC;             // [6][12][FP] jumps at the canonical face points, then their sums at the face nodes
     R* ball = smem + L::BALL;         // [12][NS]
     constexpr int LR = L::LR;
-    // one face point per thread: its 12 jump components (contiguous) to the canonical point
+    // one face point per thread: its 12 jump components to the canonical point
     for (int it = threadIdx.x; it < 6 * QF2; it += NT) {
       const int lf = it / QF2, q = it % QF2;
       const int cp = codes.perm[fperm[lf] + q];
-      const size_t jo = ((size_t)(fface[lf] >> 1) * QF2 + q) * 12;
-      if constexpr (sizeof(R) == sizeof(float)) {
-        const float4* src = reinterpret_cast<const float4*>(fd.jumpW32 + jo);
+      const size_t jo = face_at(fface[lf] >> 1, 12, 0, QF2, q);
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-          const float4 v = src[k];
-          jc[(lf * 12 + 4 * k) * FP + cp] = v.x;
-          jc[(lf * 12 + 4 * k + 1) * FP + cp] = v.y;
-          jc[(lf * 12 + 4 * k + 2) * FP + cp] = v.z;
-          jc[(lf * 12 + 4 * k + 3) * FP + cp] = v.w;
-        }
-      } else {
-        const double2* src = reinterpret_cast<const double2*>(fd.jumpW + jo);
-#pragma unroll
-        for (int k = 0; k < 6; ++k) {
-          const double2 v = src[k];
-          jc[(lf * 12 + 2 * k) * FP + cp] = (R)v.x;
-          jc[(lf * 12 + 2 * k + 1) * FP + cp] = (R)v.y;
-        }
+      for (int k = 0; k < 12; ++k) {
+        if constexpr (sizeof(R) == sizeof(float)) jc[(lf * 12 + k) * FP + cp] = fd.jumpW32[jo + k * QF2];
+        else jc[(lf * 12 + k) * FP + cp] = (R)fd.jumpW[jo + k * QF2];
       }
     }
     __syncthreads();
@@ -594,7 +558,7 @@ __global__ void __launch_bounds__(HexDims<P>::NT, sizeof(R) == sizeof(float) ? 6
     for (int q = threadIdx.x; q < Q3; q += NT) {
       R J[9];
 #pragma unroll
-      for (int k = 0; k < 9; ++k) J[k] = aff ? Ja[k] : (jinv32 ? (R)jinv32[q * 9 + k] : (R)jinv[q * 9 + k]);
+      for (int k = 0; k < 9; ++k) J[k] = aff ? Ja[k] : (jinv32 ? (R)jinv32[k * Q3 + q] : (R)jinv[k * Q3 + q]);
       const R wq = aff ? w1[q / (Q * Q)] * w1[(q / Q) % Q] * w1[q % Q] * deta : (R)wdet[q];
       R Uq[NV], F[3][NV];
 #pragma unroll
@@ -699,13 +663,13 @@ __global__ void __launch_bounds__(HexDims<P>::NT, sizeof(R) == sizeof(float) ? 6
     const int f = fface[lf] >> 1, side = fface[lf] & 1;
     const double si = side == 0 ? -1.0 : 1.0;
     const int c = codes.perm[fperm[lf] + q];
-    const size_t ki = ((size_t)fslot[lf] + q) * NV, kv = ((size_t)f * QF2 + q) * NV;
+    const size_t ki = (size_t)fslot[lf] * NV + q, kv = (size_t)f * QF2 * NV + q;
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
       if constexpr (sizeof(R) == sizeof(float)) {
         // float32 fluxes of the mixed-precision face kernel
-        const R hi = skip_inv ? R(0) : (R)si * fd.fluxI32[ki + v];
-        const R hv = visc ? -(R)si * fd.fluxV32[kv + v] : R(0);
+        const R hi = skip_inv ? R(0) : (R)si * fd.fluxI32[ki + v * QF2];
+        const R hv = visc ? -(R)si * fd.fluxV32[kv + v * QF2] : R(0);
         if (SPLIT) {
           hc[(lf * C + v) * FP + c] = hi;
           hc[(lf * C + NV + v) * FP + c] = hv;
@@ -713,8 +677,8 @@ __global__ void __launch_bounds__(HexDims<P>::NT, sizeof(R) == sizeof(float) ? 6
           hc[(lf * C + v) * FP + c] = hi + hv;
         }
       } else {
-        const double hi = skip_inv ? 0.0 : si * fd.fluxI[ki + v];
-        const double hv = visc ? -si * fd.fluxV[kv + v] : 0.0;
+        const double hi = skip_inv ? 0.0 : si * fd.fluxI[ki + v * QF2];
+        const double hv = visc ? -si * fd.fluxV[kv + v * QF2] : 0.0;
         if (SPLIT) {
           hc[(lf * C + v) * FP + c] = (R)hi;
           hc[(lf * C + NV + v) * FP + c] = (R)hv;

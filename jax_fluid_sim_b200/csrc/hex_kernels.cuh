@@ -52,7 +52,12 @@ struct HexDims {
   static constexpr int QF = P == 1 ? 2 : (P == 2 ? 3 : 4);
   static constexpr int N3 = N * N * N, Q3 = Q * Q * Q, N2 = N * N, QF2 = QF * QF;
   // CTA size of the traces and element kernels (one element each)
-  static constexpr int NT = P == 3 ? 128 : P == 2 ? 64 : 32;
+  // CTA sizes of the traces and element kernels (one element each).  A phase of a P2 element has 9 to 90 items:
+  // at 128 threads the warps mostly waited for one another at the barriers.  Element kernel of 12,776 P2
+  // hexahedra (float64) at 128, 64, 32 threads: 779, 537, 454 us; traces 193, 192, 206.  A P3 element fills
+  // 128 threads, and its shared memory, not its threads, limits the CTAs of an SM: at 64 threads its element
+  // kernel takes 4,964 us where it takes 3,753 at 128 (39,488 hexahedra, float64).
+  static constexpr int NT = P == 3 ? 128 : P == 2 ? 64 : 32, NTE = P == 3 ? 128 : 32;
 };
 
 // local face -> (normal axis, end) for the reference's hexahedron face list (hybrid/mesh.py:51-58)
@@ -470,9 +475,9 @@ __global__ void __launch_bounds__(HexDims<P>::NT) k_hex_traces(const __grid_cons
   for (int it = threadIdx.x; it < 6 * QF2; it += NT) {
     const int lf = it / QF2, q = it % QF2;
     const int c = codes.perm[fperm[lf] + q];
-    double* dst = fd.trA + ((size_t)fslot[lf] + q) * NV;
+    double* dst = fd.trA + (size_t)fslot[lf] * NV + q;
 #pragma unroll
-    for (int v = 0; v < NV; ++v) dst[v] = anchor[v] + (double)slabs[(lf * NV + v) * FP + c];
+    for (int v = 0; v < NV; ++v) dst[v * QF2] = anchor[v] + (double)slabs[(lf * NV + v) * FP + c];
   }
   // the anchor state per face side, for the face kernel's anchor flux
   for (int idx = threadIdx.x; idx < 6 * NV; idx += NT)
@@ -482,27 +487,22 @@ __global__ void __launch_bounds__(HexDims<P>::NT) k_hex_traces(const __grid_cons
     for (int it = threadIdx.x; it < 6 * QF2; it += NT) {
       const int lf = it / QF2, q = it % QF2;
       const int c = codes.perm[fperm[lf] + q];
-      const size_t pt = (size_t)fslot[lf] + q;
-      // a point's 4 values and 12 gradients are contiguous: 16-byte stores
-      R tv[4];
+      const size_t pt = (size_t)fslot[lf];       // (face * 2 + side) * QF2
 #pragma unroll
-      for (int m = 0; m < 4; ++m) tv[m] = fv[(lf * 4 + m) * FP + c];
-      if (F32) {
-        *reinterpret_cast<float4*>(fd.trV32 + pt * 4) = make_float4((float)tv[0], (float)tv[1], (float)tv[2], (float)tv[3]);
-      } else {
-        double2* t2 = reinterpret_cast<double2*>(fd.trV + pt * 4);
-        t2[0] = make_double2((double)tv[0], (double)tv[1]);
-        t2[1] = make_double2((double)tv[2], (double)tv[3]);
+      for (int m = 0; m < 4; ++m) {
+        const R tv = fv[(lf * 4 + m) * FP + c];
+        if (F32) fd.trV32[pt * 4 + m * QF2 + q] = (float)tv;
+        else fd.trV[pt * 4 + m * QF2 + q] = (double)tv;
       }
       int a0, end, a1, a2;
       hex_face_axes(lf, a0, end, a1, a2);
       R J[9];
       if (sizeof(R) == sizeof(float) && fd.jinv32) {
 #pragma unroll
-        for (int k = 0; k < 9; ++k) J[k] = (R)fd.jinv32[pt * 9 + k];
+        for (int k = 0; k < 9; ++k) J[k] = (R)fd.jinv32[pt * 9 + k * QF2 + q];
       } else {
 #pragma unroll
-        for (int k = 0; k < 9; ++k) J[k] = (R)fd.jinv[pt * 9 + k];
+        for (int k = 0; k < 9; ++k) J[k] = (R)fd.jinv[pt * 9 + k * QF2 + q];
       }
       R gout[12];
 #pragma unroll
@@ -516,15 +516,10 @@ __global__ void __launch_bounds__(HexDims<P>::NT) k_hex_traces(const __grid_cons
 #pragma unroll
         for (int d = 0; d < 3; ++d) gout[m * 3 + d] = gx * J[0 * 3 + d] + gy * J[1 * 3 + d] + gz * J[2 * 3 + d];
       }
-      if (F32) {
-        float4* g4 = reinterpret_cast<float4*>(fd.trG32 + pt * 12);
 #pragma unroll
-        for (int k = 0; k < 3; ++k)
-          g4[k] = make_float4((float)gout[4 * k], (float)gout[4 * k + 1], (float)gout[4 * k + 2], (float)gout[4 * k + 3]);
-      } else {
-        double2* g2d = reinterpret_cast<double2*>(fd.trG + pt * 12);
-#pragma unroll
-        for (int k = 0; k < 6; ++k) g2d[k] = make_double2((double)gout[2 * k], (double)gout[2 * k + 1]);
+      for (int k = 0; k < 12; ++k) {
+        if (F32) fd.trG32[pt * 12 + k * QF2 + q] = (float)gout[k];
+        else fd.trG[pt * 12 + k * QF2 + q] = (double)gout[k];
       }
     }
   }
@@ -572,7 +567,7 @@ __global__ void __launch_bounds__(kThreads) k_hex_lift(const DevPlan P_, int b, 
   const float* MT32 = (sizeof(R) == sizeof(float) && B.minv32) ? B.minv32 + (size_t)e * N3 * N3 : nullptr;
   for (int idx = threadIdx.x; idx < 6 * QF2 * 12; idx += kThreads) {
     const int lf = idx / (QF2 * 12), q = (idx / 12) % QF2, c = idx % 12;
-    jc[(lf * 12 + c) * QF2 + codes.perm[fperm[lf] + q]] = (R)fd.jumpW[((size_t)fjump[lf] * QF2 + q) * 12 + c];
+    jc[(lf * 12 + c) * QF2 + codes.perm[fperm[lf] + q]] = (R)fd.jumpW[face_at(fjump[lf], 12, c, QF2, q)];
   }
   __syncthreads();
   tensor2<CH, QF, QF, N, N>(jc, bs, tmp, tb->bfT, tb->bfT);
@@ -652,7 +647,7 @@ __global__ void __launch_bounds__(kThreads) k_hex_lift(const DevPlan P_, int b, 
   tensor2<CH, N, N, QF, QF>(rs, lq, tmp, tb->bf, tb->bf);
   for (int idx = threadIdx.x; idx < 6 * QF2 * 12; idx += kThreads) {
     const int lf = idx / (QF2 * 12), q = (idx / 12) % QF2, c = idx % 12;
-    fd.liftF[((size_t)fslot[lf] + q) * 12 + c] =
+    fd.liftF[(size_t)fslot[lf] * 12 + c * QF2 + q] =
         P_.ph.br2 * (double)lq[(lf * 12 + c) * QF2 + codes.perm[fperm[lf] + q]];
   }
 }
@@ -731,7 +726,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) 
     for (int q = threadIdx.x; q < Q3; q += kThreads) {
       R J[9], gr[12];
 #pragma unroll
-      for (int k = 0; k < 9; ++k) J[k] = aff ? Ja[k] : (jinv32 ? (R)jinv32[q * 9 + k] : (R)jinv[q * 9 + k]);
+      for (int k = 0; k < 9; ++k) J[k] = aff ? Ja[k] : (jinv32 ? (R)jinv32[k * Q3 + q] : (R)jinv[k * Q3 + q]);
 #pragma unroll
       for (int k = 0; k < 12; ++k) gr[k] = gq[k * Q3 + q];      // [r][m]
 #pragma unroll
@@ -756,7 +751,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) ? 6 : 1) 
   for (int q = threadIdx.x; q < Q3; q += kThreads) {
     R J[9];
 #pragma unroll
-    for (int k = 0; k < 9; ++k) J[k] = aff ? Ja[k] : (jinv32 ? (R)jinv32[q * 9 + k] : (R)jinv[q * 9 + k]);
+    for (int k = 0; k < 9; ++k) J[k] = aff ? Ja[k] : (jinv32 ? (R)jinv32[k * Q3 + q] : (R)jinv[k * Q3 + q]);
     const R wq = aff ? tb->w1[q / (Q * Q)] * tb->w1[(q / Q) % Q] * tb->w1[q % Q] * deta : (R)wdet[q];
     R Uq[NV], F[3][NV];
 #pragma unroll
@@ -855,8 +850,8 @@ __global__ void __launch_bounds__(kThreads) k_hex_finalize(const DevPlan P_, con
     const int lf = idx / (QF2 * NV), q = (idx / NV) % QF2, v = idx % NV;
     const int f = fface[lf] >> 1, side = fface[lf] & 1;
     const double si = side == 0 ? -1.0 : 1.0;
-    const double hi = si * fd.fluxI[((size_t)fslot[lf] + q) * NV + v];
-    const double hv = visc ? -si * fd.fluxV[((size_t)f * QF2 + q) * NV + v] : 0.0;
+    const double hi = si * fd.fluxI[(size_t)fslot[lf] * NV + v * QF2 + q];
+    const double hv = visc ? -si * fd.fluxV[face_at(f, NV, v, QF2, q)] : 0.0;
     const int c = codes.perm[fperm[lf] + q];
     if (SPLIT) {
       hc[(lf * C + v) * QF2 + c] = (R)hi;

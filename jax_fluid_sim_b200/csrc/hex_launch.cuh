@@ -34,7 +34,7 @@ cudaError_t launch_hex_element(const DevPlan& D, const StatePtrs& S, const HexTa
   constexpr size_t smem = sizeof(R) * (size_t)HexElemSmem<P, NV, SPLIT, R>::TOTAL;
   const cudaError_t e = allow_smem(k_hex_element<P, NV, SPLIT, R>, smem);
   if (e != cudaSuccess || D.blk[0].E == 0) return e;
-  k_hex_element<P, NV, SPLIT, R><<<D.blk[0].E, HexDims<P>::NT, smem, st>>>(D, S, T, codes, A);
+  k_hex_element<P, NV, SPLIT, R><<<D.blk[0].E, HexDims<P>::NTE, smem, st>>>(D, S, T, codes, A);
   return cudaGetLastError();
 }
 

@@ -253,14 +253,15 @@ __device__ __forceinline__ void mood_face(const DevPlan& P, const MoodDev& M, co
     // DG face flux at the face rule points, integrated (hybrid/subcell.py:690-746); lanes
     // 16-31 stride over the face points.  It enters (new - old) with a minus sign.
     for (int q = lane - kSub; q < fd.nq; q += 32 - kSub) {
-      const size_t so = ((size_t)f * 2 + 0) * fd.nq + q, sn = ((size_t)f * 2 + 1) * fd.nq + q;
-      const double* n = fd.n + ((size_t)f * fd.nq + q) * 3;
+      const int nq = fd.nq;
+      const size_t so = (size_t)f * 2, sn = so + 1;
+      const double n[3] = {fd.n[face_at(f, 3, 0, nq, q)], fd.n[face_at(f, 3, 1, nq, q)], fd.n[face_at(f, 3, 2, nq, q)]};
       double UL[NV], UR[NV], H[NV];
 #pragma unroll
-      for (int v = 0; v < NV; ++v) UL[v] = fd.trA[so * NV + v];
+      for (int v = 0; v < NV; ++v) UL[v] = fd.trA[face_at(so, NV, v, nq, q)];
       if (nb >= 0) {
 #pragma unroll
-        for (int v = 0; v < NV; ++v) UR[v] = fd.trA[sn * NV + v];
+        for (int v = 0; v < NV; ++v) UR[v] = fd.trA[face_at(sn, NV, v, nq, q)];
       } else if (P.ph.has_boundary) {
         ghost_state<NV>(P.ph, case_view(P.ph, P.blk[ob].ecase, ol).far, UL, n, fd.tag[f], UR);
       } else {

@@ -347,7 +347,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_volume(const DevPlan P, co
           } else {
             const size_t pq = ((size_t)e0 + e) * Nq + q;
 #pragma unroll
-            for (int k = 0; k < 9; ++k) J[k] = (float)B.jinv[pq * 9 + k];
+            for (int k = 0; k < 9; ++k) J[k] = (float)B.jinv[(((size_t)e0 + e) * 9 + k) * Nq + q];
             wq = (float)B.wdet[pq];
           }
         } else {
