@@ -5,7 +5,7 @@
 //                   face-point samples (hybrid/limiter.py:69-147).
 //   k_troubled      Persson-type high-mode sensor on (rho, p) plus the MOOD admissibility
 //                   test at samples and the mean (hybrid/limiter.py:165-185, 285-300).
-//   k_rate / k_dt   CFL rate per element, max by warp shuffles then one final CTA
+//   k_rate          CFL rate per element and, by the last CTA, dt
 //                   (hybrid/time_integration.py:93-169).
 //   k_adm / k_adm_final   finite check and min rho / min p over all nodes
 //                   (hybrid/time_integration.py:291-312), combined across stages.
@@ -481,14 +481,41 @@ struct Partial {
   int pad;
 };
 
+// The reductions over the whole state are one launch over all blocks: CTAs [cta0[b], cta0[b + 1]) take block b,
+// every CTA leaves a partial, and the one that finishes last (by the ticket counter, which wraps to zero for
+// the next launch) reduces them.  A launch per block and one for the final reduction cost about 5 us each
+// on states of any size that stays in L2, a tenth of a small step.
+struct ReduceGrid {
+  int cta0[DGB_MAX_BLOCKS + 1];
+};
+
+__device__ __forceinline__ int reduce_block(const ReduceGrid& G, int nblocks) {
+  int b = 0;
+  while (b + 1 < nblocks && (int)blockIdx.x >= G.cta0[b + 1]) ++b;
+  return b;
+}
+
+// Thread 0 has written the CTA's partial: true in every thread of the CTA that is the last to do so.
+__device__ __forceinline__ bool last_cta(unsigned* ticket) {
+  __shared__ bool last;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicInc(ticket, gridDim.x - 1) == gridDim.x - 1;
+  }
+  __syncthreads();
+  return last;
+}
+
+// max over elements of the reference's rate, then dt = clip(cfl / max)
 template <int NV>
-__global__ void __launch_bounds__(kThreads) k_rate(const DevPlan P, const StatePtrs S, int b, double cp,
-                                                  Partial* partials, int offset) {
-  // one warp per element; grid-stride over elements
+__global__ void __launch_bounds__(kThreads) k_rate(const DevPlan P, const StatePtrs S, const ReduceGrid G, double cp,
+                                                  Partial* partials, unsigned* ticket, double cfl, double* dt_out) {
+  // one warp per element; grid-stride over the block's elements
+  const int b = reduce_block(G, P.nblocks);
   const BlockDev& B = P.blk[b];
   const int lane = threadIdx.x & 31;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int nwarps = (gridDim.x * blockDim.x) >> 5;
+  const int warp = ((blockIdx.x - G.cta0[b]) * kThreads + threadIdx.x) >> 5;
+  const int nwarps = ((G.cta0[b + 1] - G.cta0[b]) * kThreads) >> 5;
   const double df = 2.0 * P.degree + 1.0;
   double best = -INFINITY;
   for (int e = warp; e < B.E; e += nwarps) {
@@ -531,34 +558,32 @@ __global__ void __launch_bounds__(kThreads) k_rate(const DevPlan P, const StateP
   if (threadIdx.x == 0) {
     double m = red[0];
     for (int k = 1; k < kThreads / 32; ++k) m = fmax(m, red[k]);
-    partials[offset + blockIdx.x].a = m;
+    __stcg(&partials[blockIdx.x].a, m);
   }
-}
-
-static __global__ void k_dt(const Partial* partials, int n, double cfl, double* dt_out) {
-  __shared__ double red[kThreads];
+  if (!last_cta(ticket)) return;
   double m = -INFINITY;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) m = fmax(m, partials[i].a);
-  red[threadIdx.x] = m;
+  for (int i = threadIdx.x; i < (int)gridDim.x; i += kThreads) m = fmax(m, __ldcg(&partials[i].a));
+  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffff, m, o));
+  if (lane == 0) red[threadIdx.x >> 5] = m;
   __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) red[threadIdx.x] = fmax(red[threadIdx.x], red[threadIdx.x + s]);
-    __syncthreads();
-  }
   if (threadIdx.x == 0) {
-    const double dt = cfl / fmax(red[0], 1.0e-12);
+    for (int k = 0; k < kThreads / 32; ++k) m = fmax(m, red[k]);
+    const double dt = cfl / fmax(m, 1.0e-12);
     *dt_out = fmin(fmax(dt, 1.0e-7), 1.0e-3);
   }
 }
 
 template <int NV>
-__global__ void __launch_bounds__(kThreads) k_adm(const DevPlan P, const StatePtrs S, int b, Partial* partials,
-                                                 int offset) {
+__global__ void __launch_bounds__(kThreads) k_adm(const DevPlan P, const StatePtrs S, const ReduceGrid G,
+                                                 Partial* partials, unsigned* ticket, double rho_floor, double p_floor,
+                                                 int combine, dgb_status* status) {
+  const int b = reduce_block(G, P.nblocks);
   const BlockDev& B = P.blk[b];
   const size_t nodes = (size_t)B.E * B.Np;
   double rmin = INFINITY, pmin = INFINITY;
   int finite = 1, rnan = 0, pnan = 0;
-  for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < nodes; k += (size_t)gridDim.x * blockDim.x) {
+  const size_t stride = (size_t)(G.cta0[b + 1] - G.cta0[b]) * kThreads;
+  for (size_t k = (blockIdx.x - G.cta0[b]) * (size_t)kThreads + threadIdx.x; k < nodes; k += stride) {
     const double* U = S.b[b] + k * NV;
 #pragma unroll
     for (int v = 0; v < NV; ++v) finite &= isfinite(U[v]) ? 1 : 0;
@@ -568,68 +593,49 @@ __global__ void __launch_bounds__(kThreads) k_adm(const DevPlan P, const StatePt
     rmin = fmin(rmin, U[0]);
     pmin = fmin(pmin, p);
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    rmin = fmin(rmin, __shfl_xor_sync(0xffffffff, rmin, o));
-    pmin = fmin(pmin, __shfl_xor_sync(0xffffffff, pmin, o));
-  }
-  finite = __syncthreads_and(finite);
-  rnan = __syncthreads_or(rnan);
-  pnan = __syncthreads_or(pnan);
+  // (rho_min, p_min, finite) over the CTA; fmin drops a NaN where the reference keeps it
   __shared__ double r1[kThreads / 32], r2[kThreads / 32];
-  if ((threadIdx.x & 31) == 0) {
-    r1[threadIdx.x >> 5] = rmin;
-    r2[threadIdx.x >> 5] = pmin;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double a = r1[0], c = r2[0];
-    for (int k = 1; k < kThreads / 32; ++k) {
-      a = fmin(a, r1[k]);
-      c = fmin(c, r2[k]);
+  auto reduce = [&]() {
+    for (int o = 16; o > 0; o >>= 1) {
+      rmin = fmin(rmin, __shfl_xor_sync(0xffffffff, rmin, o));
+      pmin = fmin(pmin, __shfl_xor_sync(0xffffffff, pmin, o));
     }
-    Partial out;
-    out.a = rnan ? NAN : a;
-    out.b = pnan ? NAN : c;
-    out.flag = finite;
-    out.pad = 0;
-    partials[offset + blockIdx.x] = out;
-  }
-}
-
-// combine: first stage overwrites the status, later stages AND / min into it.  One CTA of
-// kAdmFinalThreads reduces the partials (a serial loop over thousands of them took 0.3 ms).
-constexpr int kAdmFinalThreads = 256;
-
-static __global__ void __launch_bounds__(kAdmFinalThreads) k_adm_final(const Partial* partials, int n, double rho_floor,
-                                                               double p_floor, int combine, dgb_status* status) {
-  __shared__ double sr[kAdmFinalThreads], sp[kAdmFinalThreads];
-  double rmin = INFINITY, pmin = INFINITY;
-  int finite = 1, rnan = 0, pnan = 0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    const Partial q = partials[i];
-    rnan |= isnan(q.a);
-    pnan |= isnan(q.b);
-    rmin = fmin(rmin, q.a);
-    pmin = fmin(pmin, q.b);
-    finite &= q.flag;
-  }
-  finite = __syncthreads_and(finite);
-  rnan = __syncthreads_or(rnan);
-  pnan = __syncthreads_or(pnan);
-  sr[threadIdx.x] = rmin;
-  sp[threadIdx.x] = pmin;
-  __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if ((int)threadIdx.x < s) {
-      sr[threadIdx.x] = fmin(sr[threadIdx.x], sr[threadIdx.x + s]);
-      sp[threadIdx.x] = fmin(sp[threadIdx.x], sp[threadIdx.x + s]);
+    finite = __syncthreads_and(finite);
+    rnan = __syncthreads_or(rnan);
+    pnan = __syncthreads_or(pnan);
+    if ((threadIdx.x & 31) == 0) {
+      r1[threadIdx.x >> 5] = rmin;
+      r2[threadIdx.x >> 5] = pmin;
     }
     __syncthreads();
+    for (int k = 0; k < kThreads / 32; ++k) {
+      rmin = fmin(rmin, r1[k]);
+      pmin = fmin(pmin, r2[k]);
+    }
+    rmin = rnan ? NAN : rmin;
+    pmin = pnan ? NAN : pmin;
+  };
+  reduce();
+  if (threadIdx.x == 0) {
+    __stcg(&partials[blockIdx.x].a, rmin);
+    __stcg(&partials[blockIdx.x].b, pmin);
+    __stcg(&partials[blockIdx.x].flag, finite);
   }
+  if (!last_cta(ticket)) return;
+  rmin = pmin = INFINITY;
+  finite = 1, rnan = pnan = 0;
+  for (int i = threadIdx.x; i < (int)gridDim.x; i += kThreads) {
+    const double a = __ldcg(&partials[i].a), c = __ldcg(&partials[i].b);
+    rnan |= isnan(a);
+    pnan |= isnan(c);
+    rmin = fmin(rmin, a);
+    pmin = fmin(pmin, c);
+    finite &= __ldcg(&partials[i].flag);
+  }
+  reduce();
   if (threadIdx.x != 0) return;
-  rmin = rnan ? NAN : sr[0];
-  pmin = pnan ? NAN : sp[0];
   const int valid = finite && (rmin >= rho_floor) && (pmin >= p_floor);
+  // combine: the first stage overwrites the status, later stages AND / min into it
   if (combine) {
     status->valid = status->valid && valid;
     status->rho_min = (isnan(status->rho_min) || isnan(rmin)) ? NAN : fmin(status->rho_min, rmin);

@@ -79,9 +79,8 @@ struct dgb_plan {
   double* stage1[DGB_MAX_BLOCKS] = {nullptr, nullptr, nullptr};
   double* stage2[DGB_MAX_BLOCKS] = {nullptr, nullptr, nullptr};
   Partial* partials = nullptr;
-  int rate_grid[DGB_MAX_BLOCKS] = {0, 0, 0};
-  int adm_grid[DGB_MAX_BLOCKS] = {0, 0, 0};
-  int npartials = 0;
+  ReduceGrid rate_grid = {}, adm_grid = {};
+  unsigned* ticket = nullptr;          // last_cta's counter
   double* dt_scratch = nullptr;
   // batched launches of the dense element kernels (all blocks in one grid) and their shared memory
   int num_cases = 0;   // dgb_plan_set_cases
@@ -798,26 +797,18 @@ int run_positivity(dgb_plan* p, const StatePtrs& S, cudaStream_t st) {
 
 template <int NV>
 int run_admissibility(dgb_plan* p, const StatePtrs& S, dgb_status* status, int combine, cudaStream_t st) {
-  int off = 0;
-  for (int b = 0; b < p->dev.nblocks; ++b) {
-    k_adm<NV><<<p->adm_grid[b], kThreads, 0, st>>>(p->dev, S, b, p->partials, off);
-    off += p->adm_grid[b];
-  }
-  k_adm_final<<<1, kAdmFinalThreads, 0, st>>>(p->partials, off, p->lim.adm_density_floor, p->lim.adm_pressure_floor, combine,
-                                status);
+  const ReduceGrid& G = p->adm_grid;
+  k_adm<NV><<<std::max(1, G.cta0[p->dev.nblocks]), kThreads, 0, st>>>(
+      p->dev, S, G, p->partials, p->ticket, p->lim.adm_density_floor, p->lim.adm_pressure_floor, combine, status);
   CK(cudaGetLastError());
   return DGB_OK;
 }
 
 template <int NV>
 int run_stable_dt(dgb_plan* p, const StatePtrs& S, double cfl, double* dt_out, cudaStream_t st) {
-  int off = 0;
   const double cp = p->prm.gamma * p->prm.gas_constant / (p->prm.gamma - 1.0);
-  for (int b = 0; b < p->dev.nblocks; ++b) {
-    k_rate<NV><<<p->rate_grid[b], kThreads, 0, st>>>(p->dev, S, b, cp, p->partials, off);
-    off += p->rate_grid[b];
-  }
-  k_dt<<<1, kThreads, 0, st>>>(p->partials, off, cfl, dt_out);
+  const ReduceGrid& G = p->rate_grid;
+  k_rate<NV><<<std::max(1, G.cta0[p->dev.nblocks]), kThreads, 0, st>>>(p->dev, S, G, cp, p->partials, p->ticket, cfl, dt_out);
   CK(cudaGetLastError());
   return DGB_OK;
 }
@@ -1537,7 +1528,6 @@ int dgb_plan_finalize(dgb_plan* p) {
                                                               : hex_troubled_grid<3, 16>(p));
     if (rc) return rc;
   }
-  p->npartials = 0;
   for (int b = 0; b < p->dev.nblocks; ++b) {
     BlockDev& B = p->dev.blk[b];
     for (int ft = 0; ft < 2; ++ft) {
@@ -1555,10 +1545,6 @@ int dgb_plan_finalize(dgb_plan* p) {
     (void)max_nq;
     p->smem_pos[b] = sizeof(double) * (size_t)(B.Np + B.Np + B.Nq + B.Ns) * NV;
     p->smem_troubled[b] = sizeof(double) * ((size_t)(B.Np + B.Np + B.Nq + B.Ns) * NV + 2 * B.Np);
-    p->rate_grid[b] = blocks_for(B.E, kThreads / 32) < 2 * 148 * 8 ? blocks_for(B.E, kThreads / 32) : 2 * 148 * 8;
-    const long nodes = (long)B.E * B.Np;
-    p->adm_grid[b] = blocks_for(nodes, kThreads) < 148 * 8 ? blocks_for(nodes, kThreads) : 148 * 8;
-    p->npartials += (p->rate_grid[b] > p->adm_grid[b] ? p->rate_grid[b] : p->adm_grid[b]);
     if (p->smem_pos[b] > 227 * 1024)
       return fail(DGB_ERR_UNSUPPORTED, "element too large for the shared-memory kernels");
   }
@@ -1572,11 +1558,30 @@ int dgb_plan_finalize(dgb_plan* p) {
       return fail(DGB_ERR_UNSUPPORTED, "element too large for the shared-memory kernels");
     if ((rc = dense_finish(p))) return rc;
   }
+  // CTAs of the reductions: one warp per element (rate), one thread per node (admissibility), at most eight
+  // CTAs per SM over all blocks, shared by the blocks' sizes
   {
+    auto split = [&](ReduceGrid& G, auto work, int per) {
+      long total = 0;
+      for (int b = 0; b < p->dev.nblocks; ++b) total += blocks_for(work(p->dev.blk[b]), per);
+      const double share = std::min(1.0, 148.0 * 8 / std::max(1L, total));
+      G.cta0[0] = 0;
+      for (int b = 0; b < p->dev.nblocks; ++b) {
+        const int n = blocks_for(work(p->dev.blk[b]), per);
+        G.cta0[b + 1] = G.cta0[b] + (n > 0 ? std::max(1, (int)(n * share)) : 0);
+      }
+      return G.cta0[p->dev.nblocks];
+    };
+    const int n = std::max(split(p->rate_grid, [](const BlockDev& B) { return (long)B.E; }, kThreads / 32),
+                           split(p->adm_grid, [](const BlockDev& B) { return (long)B.E * B.Np; }, kThreads));
     void* d = nullptr;
-    CK(cudaMalloc(&d, sizeof(Partial) * (size_t)(p->npartials + 1)));
+    CK(cudaMalloc(&d, sizeof(Partial) * (size_t)(n + 1)));
     p->allocations.push_back(d);
     p->partials = static_cast<Partial*>(d);
+    CK(cudaMalloc(&d, sizeof(unsigned)));
+    p->allocations.push_back(d);
+    CK(cudaMemset(d, 0, sizeof(unsigned)));
+    p->ticket = static_cast<unsigned*>(d);
   }
   if ((rc = alloc(p, 1, &p->dt_scratch))) return rc;
   {

@@ -371,7 +371,7 @@ struct HexElemSmem {
 // Lift + volume + finalize of one hexahedron (see the file comment).  SPLIT keeps the inviscid
 // and viscous residuals apart (right-hand-side outputs, the MOOD step's viscous residual).
 template <int P, int NV, bool SPLIT, typename R = double>
-__global__ void __launch_bounds__(HexDims<P>::NTE, sizeof(R) == sizeof(float) ? 6 * kThreads / HexDims<P>::NTE : 1) k_hex_element(const __grid_constant__ DevPlan P_, const StatePtrs S,
+__global__ void __launch_bounds__(HexDims<P>::NTE, sizeof(R) == sizeof(float) ? (SPLIT || NV > 5 ? 6 : 7) * kThreads / HexDims<P>::NTE : 1) k_hex_element(const __grid_constant__ DevPlan P_, const StatePtrs S,
                                                          const __grid_constant__ HexTablesT<R> tables,
                                                          const HexCodes codes, const __grid_constant__ FinalizeArgs A) {
   using D = HexDims<P>;
@@ -424,6 +424,18 @@ __global__ void __launch_bounds__(HexDims<P>::NTE, sizeof(R) == sizeof(float) ? 
   const bool skip_inv = SPLIT && A.skip_inviscid && A.skip_inviscid[e];
   const double* MT = B.minv + (size_t)e * N3 * N3;
   const float* MT32 = (sizeof(R) == sizeof(float) && B.minv32) ? B.minv32 + (size_t)e * N3 * N3 : nullptr;
+  if (!aff) {
+    // the element's M^-1, inverse Jacobians and w|det J| on their way to L2 while the nodal work runs
+    auto prefetch = [&](const void* p, int bytes) {
+      for (int o = threadIdx.x * 128; o < bytes; o += NT * 128)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const char*>(p) + o));
+    };
+    if (MT32) prefetch(MT32, N3 * N3 * 4);
+    else prefetch(MT, N3 * N3 * 8);
+    if (sizeof(R) == sizeof(float) && B.jinv32) prefetch(B.jinv32 + (size_t)e * Q3 * 9, Q3 * 9 * 4);
+    else prefetch(B.jinv + (size_t)e * Q3 * 9, Q3 * 9 * 8);
+    prefetch(B.wdet + (size_t)e * Q3, Q3 * 8);
+  }
   for (int l = threadIdx.x; l < N3; l += NT) {
     const double* un = raw + lex2node[l] * NV;
     double u[NV];
@@ -494,7 +506,7 @@ __global__ void __launch_bounds__(HexDims<P>::NTE, sizeof(R) == sizeof(float) ? 
         for (int idx = threadIdx.x; idx < 2 * N3; idx += NT) {
           const int i = idx % N3, g = idx / N3, c0 = g * 6;
           R sacc[6] = {R(0), R(0), R(0), R(0), R(0), R(0)};
-#pragma unroll 4
+#pragma unroll 8
           for (int j = 0; j < N3; ++j) {
             const R m = (R)__ldg(M + (size_t)j * N3 + i);
             R bj[6];
@@ -762,7 +774,7 @@ __global__ void __launch_bounds__(HexDims<P>::NTE, sizeof(R) == sizeof(float) ? 
 #pragma unroll
       for (int k = 0; k < VB; ++k) ri[k] = rv[k] = R(0);
       const int j1 = (h + 1) * JH < N3 ? (h + 1) * JH : N3;
-#pragma unroll 4
+#pragma unroll 8
       for (int j = h * JH; j < j1; ++j) {
         const R m = (R)__ldg(M + (size_t)j * N3 + i);
         R xi[VB], xv[VB];
