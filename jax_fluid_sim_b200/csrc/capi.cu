@@ -118,6 +118,8 @@ struct dgb_plan {
   double* sub_bdc[DGB_MAX_BLOCKS] = {nullptr, nullptr, nullptr};
   bool sub_face_set[2] = {false, false};
   bool mood_ready = false;
+  MoodLists mood_lists = {};
+  size_t mood_marks = 0;
   uint8_t* flags[DGB_MAX_BLOCKS] = {nullptr, nullptr, nullptr};
   // learned troubled-cell predictor (dgb_plan_set_predictor)
   int pred_mode = 0;
@@ -501,14 +503,16 @@ int run_rhs_hex_fused(dgb_plan* p, const StatePtrs& S, const FinalizeArgs& A, cu
   return DGB_OK;
 }
 
-// The fused element kernel alone, split residuals, on the face buffers of the last right-hand side.
+// The fused element kernel alone, split residuals, of the listed troubled elements, on the face buffers of the
+// last right-hand side.
 template <int P, int NV, typename R>
 int run_hex_element_pass(dgb_plan* p, const StatePtrs& S, const FinalizeArgs& A, cudaStream_t st) {
-  CK((launch_hex_element<P, NV, true, R>(p->dev, S, hex_tables<R>(p), p->hex_codes, A, st)));
+  CK((launch_hex_element_list<P, NV, R>(p->dev, S, hex_tables<R>(p), p->hex_codes, A, p->mood_lists.troubled,
+                                        p->mood_lists.count + kMoodTroubled, p->dev.blk[0].E, st)));
   return DGB_OK;
 }
 
-// The viscous residual of the flagged elements only (p->vis), for the subcell scheme: the fused
+// The viscous residual of the listed troubled elements (p->vis), for the subcell scheme: the fused
 // element kernel with the inviscid terms skipped, on the face data of the stage's right-hand side.
 template <int NV>
 int run_viscous_flagged(dgb_plan* p, const StatePtrs& S, cudaStream_t st) {
@@ -516,7 +520,6 @@ int run_viscous_flagged(dgb_plan* p, const StatePtrs& S, cudaStream_t st) {
   memset(&V, 0, sizeof(V));
   V.out_vis[0] = p->vis[0];
   V.skip_inviscid = p->flags[0];
-  V.only = p->flags[0];
   const bool f32 = p->prm.precision == 1;
   switch (p->dev.degree) {
     case 1: return f32 ? run_hex_element_pass<1, NV, float>(p, S, V, st) : run_hex_element_pass<1, NV, double>(p, S, V, st);
@@ -848,30 +851,44 @@ FlagPtrs flag_ptrs(uint8_t* const* f) {
 
 // Subcell recompute of the candidate `cand` from the base `cur` (traces of `cur` must be in
 // the face buffers): writes `out`.
+// Lists the troubled elements, the active faces and the elements on them.
+int run_mood_screen(dgb_plan* p, const FlagPtrs& F, cudaStream_t st) {
+  const int faces = p->dev.face[0].F + p->dev.face[1].F;
+  if (faces == 0) return DGB_OK;
+  CK(cudaMemsetAsync(p->mood_lists.count, 0, sizeof(unsigned) * (kMoodCounts + p->mood_marks), st));
+  k_mood_screen<<<blocks_for(faces, kThreads), kThreads, 0, st>>>(p->dev, p->mood, F, p->mood_lists);
+  CK(cudaGetLastError());
+  return DGB_OK;
+}
+
+// The subcell recompute of the listed elements, in place on out (the candidate); after run_mood_screen.
 template <int NV>
-int run_subcell(dgb_plan* p, const StatePtrs& cur, double* const* cand, double* const* visc, double dt,
-                const FlagPtrs& F, double* const* out, cudaStream_t st) {
+int run_subcell(dgb_plan* p, const StatePtrs& cur, double* const* visc, double dt, const FlagPtrs& F, double* const* out,
+                cudaStream_t st) {
   const DevPlan& P = p->dev;
   MoodDev M = p->mood;
   M.recon = p->prm.reconstruction;
+  StatePtrs vis, dst;
+  long elements = 0, faces = (long)P.face[0].F + P.face[1].F;
+  size_t sm_fv = 0, sm_up = 0;
+  for (int b = 0; b < DGB_MAX_BLOCKS; ++b) {
+    vis.b[b] = visc ? visc[b] : nullptr;
+    dst.b[b] = out[b];
+    if (b >= P.nblocks) continue;
+    const SubcellBlockDev& C = M.blk[b];
+    elements += P.blk[b].E;
+    sm_fv = std::max(sm_fv, sizeof(double) * (size_t)mood_fv_smem(NV, P.blk[b].Np, C.S, C.NI));
+    sm_up = std::max(sm_up, sizeof(double) * (size_t)mood_update_smem(NV, P.blk[b].Np, C.S));
+  }
+  if (elements == 0 || faces == 0) return DGB_OK;
   int rc;
-  for (int b = 0; b < P.nblocks; ++b) {
-    if (P.blk[b].E == 0) continue;
-    const SubcellBlockDev& C = M.blk[b];
-    const size_t sm = sizeof(double) * ((size_t)P.blk[b].Np * NV + (size_t)C.S * NV * 4 + (size_t)C.NI * NV);
-    if ((rc = prepare(k_mood_fv<NV>, sm))) return rc;
-    k_mood_fv<NV><<<P.blk[b].E, kThreads, sm, st>>>(P, M, cur, b, F);
-  }
-  for (int ft = 0; ft < 2; ++ft)
-    if (p->face_present[ft])
-      k_mood_faces<NV><<<blocks_for((long)P.face[ft].F, kThreads), kThreads, 0, st>>>(P, M, cur, ft, F);
-  for (int b = 0; b < P.nblocks; ++b) {
-    if (P.blk[b].E == 0) continue;
-    const SubcellBlockDev& C = M.blk[b];
-    const size_t sm = sizeof(double) * ((size_t)C.S * NV * 2 + (size_t)P.blk[b].Np * NV);
-    if ((rc = prepare(k_mood_update<NV>, sm))) return rc;
-    k_mood_update<NV><<<P.blk[b].E, kThreads, sm, st>>>(P, M, b, F, cand[b], visc ? visc[b] : nullptr, dt, out[b]);
-  }
+  // about one resident wave of CTAs each
+  const int most = (int)std::min(elements, 148L * 6);
+  if ((rc = prepare(k_mood_fv<NV>, sm_fv))) return rc;
+  k_mood_fv<NV><<<most, kThreads, sm_fv, st>>>(P, M, cur, p->mood_lists);
+  k_mood_faces<NV><<<std::min(blocks_for(faces, kThreads / 32), 148 * 8), kThreads, 0, st>>>(P, M, cur, F, p->mood_lists);
+  if ((rc = prepare(k_mood_update<NV>, sm_up))) return rc;
+  k_mood_update<NV><<<most, kThreads, sm_up, st>>>(P, M, F, vis, dt, dst, p->mood_lists);
   CK(cudaGetLastError());
   return DGB_OK;
 }
@@ -960,10 +977,11 @@ int run_step_mood(dgb_plan* p, const StatePtrs& U0, double dt, dgb_status* statu
     }
     if ((rc = run_rhs<NV>(p, *cur[s], A, st))) return rc;
     if ((rc = run_troubled<NV>(p, UNL, nullptr, p->flags, st, true))) return rc;
+    if ((rc = run_mood_screen(p, F, st))) return rc;
     if (vis_after && (rc = run_viscous_flagged<NV>(p, *cur[s], st))) return rc;
     // the subcell update lands in place in the Euler candidate: elements that are neither
     // troubled nor corrected at a face keep theirs without a copy
-    if ((rc = run_subcell<NV>(p, *cur[s], p->eul, p->vis, dt, F, p->eul, st))) return rc;
+    if ((rc = run_subcell<NV>(p, *cur[s], p->vis, dt, F, p->eul, st))) return rc;
     if ((rc = run_positivity<NV>(p, EUL, st))) return rc;
     if (p->hex) {
       rc = p->dev.degree == 1 ? run_blend_positivity_hex<1, NV>(p, U0.b[0], p->eul[0], alphas[s], betas[s], dst[s]->b[0], st)
@@ -1079,11 +1097,17 @@ int run_subcell_api(dgb_plan* p, const dgb_state* base, const dgb_state* cand, d
     if ((rc = prepare(k_traces<NV, double>, p->smem_tr64))) return rc;
     k_traces<NV, double><<<p->launch_tr64.cta0[P.nblocks], kThreads, p->smem_tr64, st>>>(P, S, p->launch_tr64);
   }
-  double* candp[DGB_MAX_BLOCKS] = {cand->block[0], cand->block[1], cand->block[2]};
   double* visp[DGB_MAX_BLOCKS] = {arhs ? arhs->block[0] : nullptr, arhs ? arhs->block[1] : nullptr,
                                   arhs ? arhs->block[2] : nullptr};
   double* outp[DGB_MAX_BLOCKS] = {out->block[0], out->block[1], out->block[2]};
-  return run_subcell<NV>(p, S, candp, arhs ? visp : nullptr, dt, flag_ptrs(troubled), outp, st);
+  // the update is in place on the candidate's copy
+  for (int b = 0; b < P.nblocks; ++b)
+    if (P.blk[b].E > 0 && cand->block[b] != out->block[b])
+      CK(cudaMemcpyAsync(out->block[b], cand->block[b], sizeof(double) * (size_t)P.blk[b].E * P.blk[b].Np * NV,
+                         cudaMemcpyDeviceToDevice, st));
+  const FlagPtrs F = flag_ptrs(troubled);
+  if ((rc = run_mood_screen(p, F, st))) return rc;
+  return run_subcell<NV>(p, S, arhs ? visp : nullptr, dt, F, outp, st);
 }
 
 }  // namespace
@@ -2008,6 +2032,27 @@ int dgb_plan_enable_mood(dgb_plan* p) {
     p->allocations.push_back(a);
     CK(cudaMemset(a, 0, F));
     p->mood.face[ft].active = static_cast<uint8_t*>(a);
+  }
+  {
+    // work lists: every element and face may be on them
+    size_t E = 0, F = (size_t)p->dev.face[0].F + p->dev.face[1].F;
+    for (int b = 0; b < p->dev.nblocks; ++b) E += p->dev.blk[b].E;
+    unsigned* words = nullptr;
+    const size_t n = 3 * E + F + kMoodCounts;
+    CK(cudaMalloc(&words, sizeof(unsigned) * n));
+    p->allocations.push_back(words);
+    CK(cudaMemset(words, 0, sizeof(unsigned) * n));
+    MoodLists& L = p->mood_lists;
+    L.count = words;
+    L.troubled = words + kMoodCounts + E;
+    L.touched = L.troubled + E;
+    L.faces = L.touched + E;
+    unsigned* mark = words + kMoodCounts;       // cleared together with the counts
+    p->mood_marks = E;
+    for (int b = 0; b < p->dev.nblocks; ++b) {
+      L.mark[b] = mark;
+      mark += p->dev.blk[b].E;
+    }
   }
   for (double*& d : p->sub_bdc) {    // the boundary subface centres were only needed for matching
     cudaFree(d);

@@ -368,12 +368,11 @@ struct HexElemSmem {
   static constexpr int TOTAL = up4(cmax(cmax(B_END, T_END), cmax(G_END, D_END)));
 };
 
-// Lift + volume + finalize of one hexahedron (see the file comment).  SPLIT keeps the inviscid
+// Lift + volume + finalize of hexahedron e by one CTA (see the file comment).  SPLIT keeps the inviscid
 // and viscous residuals apart (right-hand-side outputs, the MOOD step's viscous residual).
-template <int P, int NV, bool SPLIT, typename R = double>
-__global__ void __launch_bounds__(HexDims<P>::NTE, sizeof(R) == sizeof(float) ? (SPLIT || NV > 5 ? 6 : 7) * kThreads / HexDims<P>::NTE : 1) k_hex_element(const __grid_constant__ DevPlan P_, const StatePtrs S,
-                                                         const __grid_constant__ HexTablesT<R> tables,
-                                                         const HexCodes codes, const __grid_constant__ FinalizeArgs A) {
+template <int P, int NV, bool SPLIT, typename R>
+__device__ __forceinline__ void hex_element(const DevPlan& P_, const StatePtrs& S, const HexTablesT<R>& tables,
+                                            const HexCodes& codes, const FinalizeArgs& A, const int e) {
   using D = HexDims<P>;
   using L = HexElemSmem<P, NV, SPLIT, R>;
   constexpr int N = D::N, Q = D::Q, QF = D::QF, N2 = D::N2, N3 = D::N3, Q3 = D::Q3, QF2 = D::QF2, NT = D::NTE;
@@ -391,8 +390,6 @@ __global__ void __launch_bounds__(HexDims<P>::NTE, sizeof(R) == sizeof(float) ? 
   __shared__ R anchor[NV], w1[Q];
   const BlockDev& B = P_.blk[b];
   const FaceDev& fd = P_.face[1];
-  const int e = blockIdx.x;
-  if ((A.only && !A.only[e]) || (A.skip && A.skip[e])) return;     // uniform across the CTA
   const CaseView cv = case_view(P_.ph, B.ecase, e);
   const double* Ug = S.b[b] + (size_t)e * N3 * NV;
   // the state arrives in one coalesced sweep (raw: beyond the nodal arrays) and is spread from shared memory
@@ -810,6 +807,31 @@ __global__ void __launch_bounds__(HexDims<P>::NTE, sizeof(R) == sizeof(float) ? 
   }
   __syncthreads();
   emit(rows, rows + NV * N3, R(1));
+}
+
+template <int P, int NV, bool SPLIT, typename R>
+constexpr int hex_element_ctas() { return sizeof(R) == sizeof(float) ? (SPLIT || NV > 5 ? 6 : 7) * kThreads / HexDims<P>::NTE : 1; }
+
+// Every element, except those flagged in A.skip.
+template <int P, int NV, bool SPLIT, typename R>
+__global__ void __launch_bounds__(HexDims<P>::NTE, hex_element_ctas<P, NV, SPLIT, R>())
+    k_hex_element(const __grid_constant__ DevPlan P_, const StatePtrs S, const __grid_constant__ HexTablesT<R> tables,
+                  const HexCodes codes, const __grid_constant__ FinalizeArgs A) {
+  if (A.skip && A.skip[blockIdx.x]) return;     // uniform across the CTA
+  hex_element<P, NV, SPLIT, R>(P_, S, tables, codes, A, blockIdx.x);
+}
+
+// The listed elements, taken in turn by the CTAs.
+template <int P, int NV, typename R>
+__global__ void __launch_bounds__(HexDims<P>::NTE, hex_element_ctas<P, NV, true, R>())
+    k_hex_element_list(const __grid_constant__ DevPlan P_, const StatePtrs S, const __grid_constant__ HexTablesT<R> tables,
+                       const HexCodes codes, const __grid_constant__ FinalizeArgs A, const unsigned* __restrict__ list,
+                       const unsigned* __restrict__ count) {
+  const unsigned n = *count;
+  for (unsigned i = blockIdx.x; i < n; i += gridDim.x) {
+    hex_element<P, NV, true, R>(P_, S, tables, codes, A, (int)list[i]);
+    __syncthreads();
+  }
 }
 
 // Predictor statistics of the hexahedron block (the layout of k_elem_stats), one warp per element:

@@ -38,4 +38,17 @@ cudaError_t launch_hex_element(const DevPlan& D, const StatePtrs& S, const HexTa
   return cudaGetLastError();
 }
 
+template <int P, int NV, typename R>
+cudaError_t launch_hex_element_list(const DevPlan& D, const StatePtrs& S, const HexTablesT<R>& T, const HexCodes& codes,
+                                    const FinalizeArgs& A, const unsigned* list, const unsigned* count, int most,
+                                    cudaStream_t st) {
+  constexpr size_t smem = sizeof(R) * (size_t)HexElemSmem<P, NV, true, R>::TOTAL;
+  const cudaError_t e = allow_smem(k_hex_element_list<P, NV, R>, smem);
+  if (e != cudaSuccess || most == 0) return e;
+  // about one resident wave
+  const int ctas = 148 * 4 * kThreads / HexDims<P>::NTE;
+  k_hex_element_list<P, NV, R><<<most < ctas ? most : ctas, HexDims<P>::NTE, smem, st>>>(D, S, T, codes, A, list, count);
+  return cudaGetLastError();
+}
+
 }  // namespace dgb

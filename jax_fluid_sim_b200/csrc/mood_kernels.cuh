@@ -4,19 +4,25 @@
 // the subcell scheme on every element and selects with `where`; here only troubled
 // elements (flags from k_troubled on the unlimited candidate) and the parent faces they
 // touch do work:
-//   k_mood_fv      troubled element: subcell means (projection), Green-Gauss gradients,
+//   k_mood_screen  one thread per parent face: lists the faces with a troubled side, the
+//                  troubled elements, and the elements on such faces (troubled or not).
+//   k_mood_fv      troubled elements: subcell means (projection), Green-Gauss gradients,
 //                  constant/TVD/CWENO-Z face states with admissibility clamps, HLLC on the
 //                  internal subfaces, internal residual per subcell (gather, no atomics).
-//   k_mood_faces   each warp screens 32 parent faces, then works those with a troubled side
-//                  one at a time (mood_face): lanes 0-15 the 16
+//   k_mood_faces   listed faces, one warp each (mood_face): lanes 0-15 the 16
 //                  DG-FV coupling subfaces (FV mean on a troubled side, DG value at the
 //                  subface centre otherwise), lanes 16-31 the DG face flux integrated with
 //                  the face rule; stores subface fluxes and (new - old) face flux.
-//   k_mood_update  troubled element: subface fluxes added in local-face order, FV update
-//                  (+ projected viscous rhs), bound-limited reconstruction to DG; other
-//                  elements: the candidate plus the conservative correction from active
-//                  faces on which they are not troubled.
+//   k_mood_update  listed elements, in place.  Troubled: subface fluxes added in local-face order,
+//                  FV update (+ projected viscous rhs), bound-limited reconstruction to DG; others:
+//                  the conservative correction from active faces on which they are not troubled.
+// The lists hold every block's elements (and both face types), so each kernel is one launch whose CTAs
+// take entries in turn.  Before, every kernel was a launch per block with a CTA per element, which on a
+// shocked flow of 202,752 hexahedra (1 % of them troubled) left 99 % of the CTAs to start and return:
+// 532 us a stage for the three and the flagged elements' viscous pass.  The order of the
+// lists changes from run to run; no result depends on it.
 #pragma once
+#include "aux_kernels.cuh"
 #include "dg_kernels.cuh"
 
 namespace dgb {
@@ -62,6 +68,27 @@ struct FlagPtrs {
   const uint8_t* f[DGB_MAX_BLOCKS];
 };
 
+// Work lists of one recompute.  count: troubled elements, touched elements, active faces; the counts and the
+// marks after them are cleared before the faces are screened.
+struct MoodLists {
+  unsigned* troubled;   // block << 28 | element
+  unsigned* touched;    // the same
+  unsigned* faces;      // face type << 30 | face
+  unsigned* mark[DGB_MAX_BLOCKS];   // [E] 1 once an element is on the touched list
+  unsigned* count;
+};
+enum { kMoodTroubled, kMoodTouched, kMoodFaces, kMoodCounts };
+
+// Appends the lanes with want set to list (one atomic per warp).
+__device__ __forceinline__ void append(unsigned* list, unsigned* count, bool want, unsigned entry) {
+  const unsigned votes = __ballot_sync(0xffffffffu, want), lane = threadIdx.x & 31;
+  if (votes == 0) return;
+  unsigned at = 0;
+  if (lane == (unsigned)(__ffs(votes) - 1)) at = atomicAdd(count, __popc(votes));
+  at = __shfl_sync(0xffffffffu, at, __ffs(votes) - 1);
+  if (want) list[at + __popc(votes & ((1u << lane) - 1))] = entry;
+}
+
 // Admissibility clamps of reconstructed subcell traces (hybrid/subcell.py:645-663)
 template <int NV>
 __device__ __forceinline__ void clamp_state(double* U) {
@@ -73,69 +100,105 @@ __device__ __forceinline__ void clamp_state(double* U) {
 }
 
 // --------------------------------------------------------------------------------------------
-template <int NV>
-__global__ void __launch_bounds__(kThreads) k_mood_fv(const DevPlan P, const MoodDev M, const StatePtrs S, int b,
-                                                     const FlagPtrs F) {
-  const int e = blockIdx.x;
-  if (!F.f[b][e]) return;
-  extern __shared__ double smem[];
-  const BlockDev& B = P.blk[b];
-  const SubcellBlockDev& C = M.blk[b];
-  const int Np = B.Np, Sn = C.S, NI = C.NI;
-  double* U = smem;                     // [Np][NV]
-  double* ub = U + Np * NV;             // [S][NV]
-  double* g = ub + Sn * NV;             // [S][3][NV]
-  double* fi = g + Sn * 3 * NV;         // [NI][NV]
-  const double* Ug = S.b[b] + (size_t)e * Np * NV;
-  for (int i = threadIdx.x; i < Np * NV; i += kThreads) U[i] = Ug[i];
-  __syncthreads();
-  const double* Pe = C.P + (size_t)e * Sn * Np;
-  for (int idx = threadIdx.x; idx < Sn * NV; idx += kThreads) {
-    const int s = idx / NV, v = idx % NV;
-    double acc = 0.0;
-    for (int i = 0; i < Np; ++i) acc += Pe[s * Np + i] * U[i * NV + v];
-    ub[idx] = acc;
-    C.ubar[(size_t)e * Sn * NV + idx] = acc;
-  }
-  __syncthreads();
-  const double* nrm = C.in_n + (size_t)e * NI * 3;
-  const double* ar = C.in_a + (size_t)e * NI;
-  const double* vol = C.vol + (size_t)e * Sn;
-  const double* cen = C.cen + (size_t)e * Sn * 3;
-  if (M.recon != 0) {
-    // Green-Gauss gradient per subcell: sum over its internal subfaces of 0.5 n A (U_nbr - U_own) / V
-    for (int idx = threadIdx.x; idx < Sn * 3 * NV; idx += kThreads) {
-      const int s = idx / (3 * NV), d = (idx / NV) % 3, v = idx % NV;
-      double acc = 0.0;
-      for (int k = C.csr_ptr[s]; k < C.csr_ptr[s + 1]; ++k) {
-        const int f = C.csr_face[k];
-        acc += (0.5 * nrm[f * 3 + d] * ar[f]) * (ub[C.inbr[f] * NV + v] - ub[C.iown[f] * NV + v]);
+// One thread per parent face of both types (whole warps).
+static __global__ void __launch_bounds__(kThreads) k_mood_screen(const DevPlan P, const MoodDev M, const FlagPtrs Fl,
+                                                                const MoodLists L) {
+  const int F0 = P.face[0].F, F = F0 + P.face[1].F;
+  const int t = blockIdx.x * kThreads + threadIdx.x;
+  bool active = false, tr[2] = {false, false}, first[2] = {false, false};
+  unsigned entry[2] = {0, 0};
+  const int ft = t >= F0 ? 1 : 0, f = t - (ft ? F0 : 0);
+  if (t < F) {
+    const FaceDev& fd = P.face[ft];
+    const int blk[2] = {fd.ob[f], fd.nb[f]}, el[2] = {fd.ol[f], fd.nl[f]};
+#pragma unroll
+    for (int s = 0; s < 2; ++s)
+      if (blk[s] >= 0) {
+        tr[s] = Fl.f[blk[s]][el[s]] != 0;
+        entry[s] = (unsigned)blk[s] << 28 | (unsigned)el[s];
       }
-      g[idx] = acc / fmax(vol[s], 1.0e-14);
+    active = tr[0] || tr[1];
+    M.face[ft].active[f] = active;
+    if (active)
+#pragma unroll
+      for (int s = 0; s < 2; ++s) first[s] = blk[s] >= 0 && atomicExch(&L.mark[blk[s]][el[s]], 1u) == 0u;
+  }
+  append(L.faces, L.count + kMoodFaces, active, (unsigned)ft << 30 | (unsigned)f);
+#pragma unroll
+  for (int s = 0; s < 2; ++s) {
+    append(L.touched, L.count + kMoodTouched, first[s], entry[s]);
+    append(L.troubled, L.count + kMoodTroubled, first[s] && tr[s], entry[s]);
+  }
+}
+
+// Shared memory of k_mood_fv (doubles): the nodal state, the subcell means, then either the element's projection
+// rows or the gradients and both traces of the internal subfaces.
+__host__ __device__ inline int mood_fv_smem(int NV, int Np, int S, int NI) {
+  const int work = 3 * S * NV + 2 * NI * NV;
+  return Np * NV + S * NV + (S * Np > work ? S * Np : work);
+}
+
+template <int NV>
+__global__ void __launch_bounds__(kThreads) k_mood_fv(const DevPlan P, const MoodDev M, const StatePtrs S,
+                                                     const MoodLists L) {
+  extern __shared__ double smem[];
+  const unsigned n = L.count[kMoodTroubled];
+  for (unsigned item = blockIdx.x; item < n; item += gridDim.x) {
+    const int b = L.troubled[item] >> 28, e = L.troubled[item] & 0xfffffffu;
+    const BlockDev& B = P.blk[b];
+    const SubcellBlockDev& C = M.blk[b];
+    const int Np = B.Np, Sn = C.S, NI = C.NI;
+    double* U = smem;                     // [Np][NV]
+    double* ub = U + Np * NV;             // [S][NV]
+    double* Pr = ub + Sn * NV;            // [S][Np] projection
+    double* g = Pr;                       // [S][3][NV]
+    double* tl = g + 3 * Sn * NV;         // [NI][NV] owner-side trace, later the flux
+    double* tr = tl + NI * NV;            // [NI][NV] neighbour-side trace
+    const double* Ug = S.b[b] + (size_t)e * Np * NV;
+    const double* Pe = C.P + (size_t)e * Sn * Np;
+    for (int i = threadIdx.x; i < Np * NV; i += kThreads) U[i] = Ug[i];
+#pragma unroll 8
+    for (int i = threadIdx.x; i < Sn * Np; i += kThreads) Pr[i] = Pe[i];
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < Sn * NV; idx += kThreads) {
+      const int s = idx / NV, v = idx % NV;
+      double acc = 0.0;
+      for (int i = 0; i < Np; ++i) acc += Pr[s * Np + i] * U[i * NV + v];
+      ub[idx] = acc;
+      C.ubar[(size_t)e * Sn * NV + idx] = acc;
     }
     __syncthreads();
-  }
-  for (int f = threadIdx.x; f < NI; f += kThreads) {
-    const int o = C.iown[f], n = C.inbr[f];
-    double UL[NV], UR[NV], Fl[NV];
-    if (M.recon == 0) {
-#pragma unroll
-      for (int v = 0; v < NV; ++v) {
-        UL[v] = ub[o * NV + v];
-        UR[v] = ub[n * NV + v];
+    const double* nrm = C.in_n + (size_t)e * NI * 3;
+    const double* ar = C.in_a + (size_t)e * NI;
+    const double* vol = C.vol + (size_t)e * Sn;
+    const double* cen = C.cen + (size_t)e * Sn * 3;
+    if (M.recon != 0) {
+      // Green-Gauss gradient per subcell: sum over its internal subfaces of 0.5 n A (U_nbr - U_own) / V
+      for (int idx = threadIdx.x; idx < Sn * 3 * NV; idx += kThreads) {
+        const int s = idx / (3 * NV), d = (idx / NV) % 3, v = idx % NV;
+        double acc = 0.0;
+        for (int k = C.csr_ptr[s]; k < C.csr_ptr[s + 1]; ++k) {
+          const int f = C.csr_face[k];
+          acc += (0.5 * nrm[f * 3 + d] * ar[f]) * (ub[C.inbr[f] * NV + v] - ub[C.iown[f] * NV + v]);
+        }
+        g[idx] = acc / fmax(vol[s], 1.0e-14);
       }
-    } else {
-      double dc[3];
-#pragma unroll
-      for (int d = 0; d < 3; ++d) dc[d] = cen[n * 3 + d] - cen[o * 3 + d];
-#pragma unroll
-      for (int v = 0; v < NV; ++v) {
-        const double dU = ub[n * NV + v] - ub[o * NV + v];
+      __syncthreads();
+    }
+    // both traces of every internal subface, one (subface, variable) per thread
+    for (int idx = threadIdx.x; idx < NI * NV; idx += kThreads) {
+      const int f = idx / NV, v = idx % NV;
+      const int o = C.iown[f], nb = C.inbr[f];
+      const double uo = ub[o * NV + v], un = ub[nb * NV + v];
+      double ul = uo, ur = un;
+      if (M.recon != 0) {
+        const double dU = un - uo;
         double duo = 0.0, dun = 0.0;
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
-          duo += g[(o * 3 + d) * NV + v] * dc[d];
-          dun -= g[(n * 3 + d) * NV + v] * dc[d];
+          const double dc = cen[nb * 3 + d] - cen[o * 3 + d];
+          duo += g[(o * 3 + d) * NV + v] * dc;
+          dun -= g[(nb * 3 + d) * NV + v] * dc;
         }
         if (M.recon == 1) {
           // smooth Venkatakrishnan-type TVD limiter (subcell.py:578-606)
@@ -144,13 +207,13 @@ __global__ void __launch_bounds__(kThreads) k_mood_fv(const DevPlan P, const Moo
           const double rn = (-dU) / (dun + (dun >= 0.0 ? eps : -eps));
           const double po = ro > 0.0 ? (ro * ro + 2.0 * ro) / (ro * ro + ro + 2.0) : 0.0;
           const double pn = rn > 0.0 ? (rn * rn + 2.0 * rn) / (rn * rn + rn + 2.0) : 0.0;
-          UL[v] = ub[o * NV + v] + 0.5 * fmin(fmax(po, 0.0), 1.0) * duo;
-          UR[v] = ub[n * NV + v] + 0.5 * fmin(fmax(pn, 0.0), 1.0) * dun;
+          ul = uo + 0.5 * fmin(fmax(po, 0.0), 1.0) * duo;
+          ur = un + 0.5 * fmin(fmax(pn, 0.0), 1.0) * dun;
         } else {
           // CWENO-Z (subcell.py:608-641)
           const double so = duo, sn = -dun;
-          const double ph = 0.5 * (ub[o * NV + v] + ub[n * NV + v]) + 0.125 * (so - sn);
-          const double po = ub[o * NV + v] + 0.5 * so, pn = ub[n * NV + v] - 0.5 * sn;
+          const double ph = 0.5 * (uo + un) + 0.125 * (so - sn);
+          const double po = uo + 0.5 * so, pn = un - 0.5 * sn;
           const double es = 1.0e-12;
           const double bh = (sn - so) * (sn - so) + 0.1 * dU * dU;
           const double bo = (dU - so) * (dU - so) + 0.1 * dU * dU;
@@ -160,28 +223,42 @@ __global__ void __launch_bounds__(kThreads) k_mood_fv(const DevPlan P, const Moo
           const double th = tau / (bh + es), to = tau / (bo + es), tn = tau / (bn + es), tc = tau / (bc + es);
           const double a0 = 0.70 * (1.0 + th * th), a1 = 0.28 * (1.0 + to * to), a2 = 0.02 * (1.0 + tc * tc);
           const double sl = a0 + a1 + a2;
-          UL[v] = (a0 / sl) * ph + (a1 / sl) * po + (a2 / sl) * ub[o * NV + v];
+          ul = (a0 / sl) * ph + (a1 / sl) * po + (a2 / sl) * uo;
           const double a1r = 0.28 * (1.0 + tn * tn);
           const double sr = a0 + a1r + a2;
-          UR[v] = (a0 / sr) * ph + (a1r / sr) * pn + (a2 / sr) * ub[n * NV + v];
+          ur = (a0 / sr) * ph + (a1r / sr) * pn + (a2 / sr) * un;
         }
       }
-      clamp_state<NV>(UL);
-      clamp_state<NV>(UR);
+      tl[idx] = ul;
+      tr[idx] = ur;
     }
-    hllc<NV>(P.ph, UL, UR, nrm + f * 3, Fl);
+    __syncthreads();
+    for (int f = threadIdx.x; f < NI; f += kThreads) {
+      double UL[NV], UR[NV], Fl[NV];
 #pragma unroll
-    for (int v = 0; v < NV; ++v) fi[f * NV + v] = Fl[v] * ar[f];
-  }
-  __syncthreads();
-  for (int idx = threadIdx.x; idx < Sn * NV; idx += kThreads) {
-    const int s = idx / NV, v = idx % NV;
-    double acc = 0.0;
-    for (int k = C.csr_ptr[s]; k < C.csr_ptr[s + 1]; ++k) {
-      const int f = C.csr_face[k];
-      acc += C.iown[f] == s ? -fi[f * NV + v] : fi[f * NV + v];
+      for (int v = 0; v < NV; ++v) {
+        UL[v] = tl[f * NV + v];
+        UR[v] = tr[f * NV + v];
+      }
+      if (M.recon != 0) {
+        clamp_state<NV>(UL);
+        clamp_state<NV>(UR);
+      }
+      hllc<NV>(P.ph, UL, UR, nrm + f * 3, Fl);
+#pragma unroll
+      for (int v = 0; v < NV; ++v) tl[f * NV + v] = Fl[v] * ar[f];
     }
-    C.rsub[(size_t)e * Sn * NV + idx] = acc;
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < Sn * NV; idx += kThreads) {
+      const int s = idx / NV, v = idx % NV;
+      double acc = 0.0;
+      for (int k = C.csr_ptr[s]; k < C.csr_ptr[s + 1]; ++k) {
+        const int f = C.csr_face[k];
+        acc += C.iown[f] == s ? -tl[f * NV + v] : tl[f * NV + v];
+      }
+      C.rsub[(size_t)e * Sn * NV + idx] = acc;
+    }
+    __syncthreads();
   }
 }
 
@@ -285,140 +362,137 @@ __device__ __forceinline__ void mood_face(const DevPlan& P, const MoodDev& M, co
   }
 }
 
-// Each warp screens 32 parent faces (one per lane) for a troubled side, records which are active,
-// then works its active faces one after another with the whole warp.
+// The listed faces, one warp each.
 template <int NV>
-__global__ void __launch_bounds__(kThreads) k_mood_faces(const DevPlan P, const MoodDev M, const StatePtrs S, int ft,
-                                                        const FlagPtrs Fl) {
-  const FaceDev& fd = P.face[ft];
-  const SubcellFaceDev& sf = M.face[ft];
-  const int lane = threadIdx.x & 31;
-  const long f0 = ((long)blockIdx.x * kThreads + threadIdx.x) & ~31L;
-  if (f0 >= fd.F) return;                       // whole warps leave together
-  const long f = f0 + lane;
-  bool active = false;
-  if (f < fd.F) {
-    const int ob = fd.ob[f], ol = fd.ol[f], nb = fd.nb[f], nl = fd.nl[f];
-    active = Fl.f[ob][ol] != 0 || (nb >= 0 && Fl.f[nb][nl] != 0);
-    sf.active[f] = active;
-  }
-  unsigned todo = __ballot_sync(0xffffffffu, active);
-  while (todo) {
-    const int k = __ffs(todo) - 1;
-    todo &= todo - 1;
-    mood_face<NV>(P, M, S, ft, (int)(f0 + k), Fl, lane);
-  }
+__global__ void __launch_bounds__(kThreads) k_mood_faces(const DevPlan P, const MoodDev M, const StatePtrs S,
+                                                        const FlagPtrs Fl, const MoodLists L) {
+  const unsigned n = L.count[kMoodFaces], warps = gridDim.x * (kThreads / 32);
+  for (unsigned item = (blockIdx.x * kThreads + threadIdx.x) >> 5; item < n; item += warps)
+    mood_face<NV>(P, M, S, L.faces[item] >> 30, (int)(L.faces[item] & 0x3fffffffu), Fl, threadIdx.x & 31);
 }
 
 // --------------------------------------------------------------------------------------------
-// out = troubled ? bound-limited reconstruction of the FV update : candidate + corrections.  out may
-// be cand (in place): a troubled element's update does not read its candidate.
+// Shared memory of k_mood_update (doubles): residuals, FV means, the raw reconstruction, then the element's
+// projection and later its reconstruction rows.
+__host__ __device__ inline int mood_update_smem(int NV, int Np, int S) { return 2 * S * NV + Np * NV + S * Np; }
+
+// The touched elements of out (the candidate): troubled ? bound-limited reconstruction of the FV update :
+// candidate + corrections.
 template <int NV>
-__global__ void __launch_bounds__(kThreads) k_mood_update(const DevPlan P, const MoodDev M, int b, const FlagPtrs Fl,
-                                                         const double* cand, const double* visc, double dt,
-                                                         double* out) {
+__global__ void __launch_bounds__(kThreads) k_mood_update(const DevPlan P, const MoodDev M, const FlagPtrs Fl,
+                                                         const StatePtrs visc, double dt, const StatePtrs out_,
+                                                         const MoodLists L) {
   extern __shared__ double smem[];
-  const BlockDev& B = P.blk[b];
-  const SubcellBlockDev& C = M.blk[b];
-  const int e = blockIdx.x, Np = B.Np, Sn = C.S;
-  const size_t base = (size_t)e * Np * NV;
-  const double* vol = C.vol + (size_t)e * Sn;
-  __shared__ double vtot;
-  if (!Fl.f[b][e]) {
-    // conservative correction from active faces where this element is not troubled; the element
-    // volume is summed only when one is
-    __shared__ double corr[DGB_MAX_VARS];
-    __shared__ int any;
-    if (threadIdx.x == 0) any = 0;
-    __syncthreads();
-    if (threadIdx.x < B.nlf) {
-      int ft, f, side;
-      decode_face(B.elem_face[e * B.nlf + threadIdx.x], ft, f, side);
-      if (M.face[ft].active[f]) atomicOr(&any, 1);
-    }
-    __syncthreads();
-    if (out == cand && !any) return;     // in place: an element without corrections keeps its candidate
-    if (any && threadIdx.x == 0) {
-      double s = 0.0;
-      for (int k = 0; k < Sn; ++k) s += vol[k];
-      vtot = s;
-    }
-    __syncthreads();
-    if (threadIdx.x < NV) {
-      double c = 0.0;
-      for (int lf = 0; lf < B.nlf; ++lf) {
-        int ft, f, side;
-        decode_face(B.elem_face[e * B.nlf + lf], ft, f, side);
-        if (!M.face[ft].active[f]) continue;
-        const double d = M.face[ft].dflux[(size_t)f * NV + threadIdx.x];
-        c += side == 0 ? -dt * d / vtot : dt * d / vtot;
+  __shared__ double vtot, corr[DGB_MAX_VARS];
+  const unsigned n = L.count[kMoodTouched];
+  for (unsigned item = blockIdx.x; item < n; item += gridDim.x) {
+    const int b = L.touched[item] >> 28, e = L.touched[item] & 0xfffffffu;
+    const BlockDev& B = P.blk[b];
+    const SubcellBlockDev& C = M.blk[b];
+    const int Np = B.Np, Sn = C.S;
+    const size_t base = (size_t)e * Np * NV;
+    const double* vol = C.vol + (size_t)e * Sn;
+    double* out = out_.b[b];
+    if (!Fl.f[b][e]) {
+      // conservative correction from the active faces, in local-face order
+      if (threadIdx.x == 0) {
+        double s = 0.0;
+        for (int k = 0; k < Sn; ++k) s += vol[k];
+        vtot = s;
       }
-      corr[threadIdx.x] = c;
+      __syncthreads();
+      if (threadIdx.x < NV) {
+        double c = 0.0;
+        for (int lf = 0; lf < B.nlf; ++lf) {
+          int ft, f, side;
+          decode_face(B.elem_face[e * B.nlf + lf], ft, f, side);
+          if (!M.face[ft].active[f]) continue;
+          const double d = M.face[ft].dflux[(size_t)f * NV + threadIdx.x];
+          c += side == 0 ? -dt * d / vtot : dt * d / vtot;
+        }
+        corr[threadIdx.x] = c;
+      }
+      __syncthreads();
+      for (int idx = threadIdx.x; idx < Np * NV; idx += kThreads) out[base + idx] = out[base + idx] + corr[idx % NV];
+      __syncthreads();
+      continue;
+    }
+    double* res = smem;                    // [S][NV]
+    double* fv = res + Sn * NV;            // [S][NV]
+    double* raw = fv + Sn * NV;            // [Np][NV]
+    double* rows = raw + Np * NV;          // [S][Np] projection, then [Np][S] reconstruction
+    const double* vis = visc.b[b];
+    for (int idx = threadIdx.x; idx < Sn * NV; idx += kThreads) res[idx] = C.rsub[(size_t)e * Sn * NV + idx];
+    if (vis) {
+      const double* Pe = C.P + (size_t)e * Sn * Np;
+#pragma unroll 8
+      for (int i = threadIdx.x; i < Sn * Np; i += kThreads) rows[i] = Pe[i];
+      for (int i = threadIdx.x; i < Np * NV; i += kThreads) raw[i] = vis[base + i];
+    }
+    for (int lf = 0; lf < B.nlf; ++lf) {
+      int ft, f, side;
+      decode_face(B.elem_face[e * B.nlf + lf], ft, f, side);
+      const SubcellFaceDev& sf = M.face[ft];
+      const int32_t* sub = side == 0 ? sf.osub : sf.nsub;
+      __syncthreads();
+      for (int idx = threadIdx.x; idx < kSub * NV; idx += kThreads) {
+        const int j = idx / NV, v = idx % NV;
+        const int sc = C.scatter[sub[f * kSub + j]];
+        if (sc < 0) continue;
+        const double h = sf.fsub[((size_t)f * kSub + j) * NV + v];
+        res[sc * NV + v] += side == 0 ? -h : h;
+      }
     }
     __syncthreads();
-    for (int idx = threadIdx.x; idx < Np * NV; idx += kThreads)
-      out[base + idx] = any ? cand[base + idx] + corr[idx % NV] : cand[base + idx];
-    return;
-  }
-  double* res = smem;                    // [S][NV]
-  double* fv = res + Sn * NV;            // [S][NV]
-  double* raw = fv + Sn * NV;            // [Np][NV]
-  for (int idx = threadIdx.x; idx < Sn * NV; idx += kThreads) res[idx] = C.rsub[(size_t)e * Sn * NV + idx];
-  for (int lf = 0; lf < B.nlf; ++lf) {
-    int ft, f, side;
-    decode_face(B.elem_face[e * B.nlf + lf], ft, f, side);
-    const SubcellFaceDev& sf = M.face[ft];
-    const int32_t* sub = side == 0 ? sf.osub : sf.nsub;
+    for (int idx = threadIdx.x; idx < Sn * NV; idx += kThreads) {
+      const int s = idx / NV, v = idx % NV;
+      double x = C.ubar[(size_t)e * Sn * NV + idx] + dt * res[idx] / vol[s];
+      if (vis) {
+        double pv = 0.0;
+        for (int i = 0; i < Np; ++i) pv += rows[s * Np + i] * raw[i * NV + v];
+        x += dt * pv;
+      }
+      fv[idx] = x;
+    }
     __syncthreads();
-    for (int idx = threadIdx.x; idx < kSub * NV; idx += kThreads) {
-      const int j = idx / NV, v = idx % NV;
-      const int sc = C.scatter[sub[f * kSub + j]];
-      if (sc < 0) continue;
-      const double h = sf.fsub[((size_t)f * kSub + j) * NV + v];
-      res[sc * NV + v] += side == 0 ? -h : h;
+    const double* Re = C.R + (size_t)e * Np * Sn;
+#pragma unroll 8
+    for (int i = threadIdx.x; i < Np * Sn; i += kThreads) rows[i] = Re[i];
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < Np * NV; idx += kThreads) {
+      const int i = idx / NV, v = idx % NV;
+      double acc = 0.0;
+      for (int s = 0; s < Sn; ++s) acc += rows[i * Sn + s] * fv[s * NV + v];
+      raw[idx] = acc;
     }
-  }
-  __syncthreads();
-  const double* Pe = C.P + (size_t)e * Sn * Np;
-  for (int idx = threadIdx.x; idx < Sn * NV; idx += kThreads) {
-    const int s = idx / NV, v = idx % NV;
-    double x = C.ubar[(size_t)e * Sn * NV + idx] + dt * res[idx] / vol[s];
-    if (visc) {
-      double pv = 0.0;
-      for (int i = 0; i < Np; ++i) pv += Pe[s * Np + i] * visc[base + i * NV + v];
-      x += dt * pv;
+    __syncthreads();
+    // Zhang-Shu bound limiting per variable (hybrid/subcell.py:406-439)
+    if (threadIdx.x < NV) {
+      const int v = threadIdx.x;
+      double ms = 0.0, vs = 0.0, smin = INFINITY, smax = -INFINITY, dmin = INFINITY, dmax = -INFINITY;
+      for (int s = 0; s < Sn; ++s) {
+        ms += fv[s * NV + v] * vol[s];
+        vs += vol[s];
+        smin = fmin(smin, fv[s * NV + v]);
+        smax = fmax(smax, fv[s * NV + v]);
+      }
+      const double mean = ms / fmax(vs, 1.0e-14);
+      for (int i = 0; i < Np; ++i) {
+        dmin = fmin(dmin, raw[i * NV + v]);
+        dmax = fmax(dmax, raw[i * NV + v]);
+      }
+      const double eps = 1.0e-12;
+      const double tmax = dmax > mean + eps ? (smax - mean) / (dmax - mean + eps) : 1.0;
+      const double tmin = dmin < mean - eps ? (mean - smin) / (mean - dmin + eps) : 1.0;
+      corr[v] = fmin(fmax(fmin(tmax, tmin), 0.0), 1.0);
+      res[v] = mean;                       // res is dead
     }
-    fv[idx] = x;
-  }
-  __syncthreads();
-  const double* Re = C.R + (size_t)e * Np * Sn;
-  for (int idx = threadIdx.x; idx < Np * NV; idx += kThreads) {
-    const int i = idx / NV, v = idx % NV;
-    double acc = 0.0;
-    for (int s = 0; s < Sn; ++s) acc += Re[i * Sn + s] * fv[s * NV + v];
-    raw[idx] = acc;
-  }
-  __syncthreads();
-  // Zhang-Shu bound limiting per variable (hybrid/subcell.py:406-439)
-  if (threadIdx.x < NV) {
-    const int v = threadIdx.x;
-    double ms = 0.0, vs = 0.0, smin = INFINITY, smax = -INFINITY, dmin = INFINITY, dmax = -INFINITY;
-    for (int s = 0; s < Sn; ++s) {
-      ms += fv[s * NV + v] * vol[s];
-      vs += vol[s];
-      smin = fmin(smin, fv[s * NV + v]);
-      smax = fmax(smax, fv[s * NV + v]);
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < Np * NV; idx += kThreads) {
+      const double mean = res[idx % NV];
+      out[base + idx] = mean + corr[idx % NV] * (raw[idx] - mean);
     }
-    const double mean = ms / fmax(vs, 1.0e-14);
-    for (int i = 0; i < Np; ++i) {
-      dmin = fmin(dmin, raw[i * NV + v]);
-      dmax = fmax(dmax, raw[i * NV + v]);
-    }
-    const double eps = 1.0e-12;
-    const double tmax = dmax > mean + eps ? (smax - mean) / (dmax - mean + eps) : 1.0;
-    const double tmin = dmin < mean - eps ? (mean - smin) / (mean - dmin + eps) : 1.0;
-    const double th = fmin(fmax(fmin(tmax, tmin), 0.0), 1.0);
-    for (int i = 0; i < Np; ++i) out[base + i * NV + v] = mean + th * (raw[i * NV + v] - mean);
+    __syncthreads();
   }
 }
 
