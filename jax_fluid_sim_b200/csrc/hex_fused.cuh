@@ -37,7 +37,7 @@ static __global__ void k_hex_face_lf(const DevPlan P_, int8_t* face_lf) {
 
 // Local-lift operator of every face of the non-affine elements (set-up), in the canonical face-point
 // order of that face: L[c][c'] = sum_{i,j in slab} BF[c][i] M^-1[node i][node j] BF[c'][j], BF the
-// face interpolation bf (x) bf.  One CTA per (listed element, local face).  Mt is M^-1 transposed
+// face interpolation bf (x) bf, stored as [c'][c].  One CTA per (listed element, local face).  Mt is M^-1 transposed
 // in element node order (the hexahedron path's layout).
 template <int P, typename T>
 __global__ void k_hex_lop(const DevPlan P_, const HexTables tables, const int* __restrict__ elems, int count,
@@ -75,7 +75,7 @@ __global__ void k_hex_lop(const DevPlan P_, const HexTables tables, const int* _
     double acc = 0.0;
     for (int si = 0; si < N2; ++si)
       acc += tables.bf[(c % QF) * N + si % N] * tables.bf[(c / QF) * N + si / N] * t1[si][cp];
-    out[idx] = (T)acc;
+    out[cp * QF2 + c] = (T)acc;       // transposed: a face's lanes then read one row together
   }
 }
 
@@ -84,7 +84,7 @@ __global__ void k_hex_lop(const DevPlan P_, const HexTables tables, const int* _
 struct HexFaceArgs {
   const int8_t* face_lf;      // [F][2]
   const int* lop_index;       // [E], -1 for affine elements
-  const double* lop;          // [count][6][QF2][QF2], float64 plans
+  const double* lop;          // [count][6][QF2][QF2] (transposed), float64 plans
   const float* lop32;         // the same in float32, mixed-precision plans
 };
 
@@ -264,12 +264,12 @@ __global__ void __launch_bounds__(kThreads, NV <= 5 ? 6 : 1) k_hex_face(const De
 #pragma unroll
       for (int c = 0; c < 12; ++c) lift[c] *= scale;
     } else {
-      const size_t lo = ((size_t)li * 6 + lf) * QF2 * QF2 + (size_t)cq * QF2;
+      const size_t lo = ((size_t)li * 6 + lf) * QF2 * QF2 + cq;
 #pragma unroll
       for (int qp = 0; qp < QF2; ++qp) {
         R kk;
-        if constexpr (sizeof(R) == sizeof(float)) kk = __ldg(A.lop32 + lo + pm(qp));
-        else kk = (R)__ldg(A.lop + lo + pm(qp));
+        if constexpr (sizeof(R) == sizeof(float)) kk = __ldg(A.lop32 + lo + pm(qp) * QF2);
+        else kk = (R)__ldg(A.lop + lo + pm(qp) * QF2);
         R jv[12];
         jrow(qp, jv);
 #pragma unroll
