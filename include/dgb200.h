@@ -242,6 +242,11 @@ int dgb_plan_update_params(dgb_plan* plan, const dgb_params* params);
  * Either output may be NULL (not computed / not written). */
 int dgb_rhs(dgb_plan* plan, const dgb_state* U, const dgb_state* inviscid_out,
             const dgb_state* viscous_out, void* stream);
+/* HybridNavierStokesOperator.rhs (hybrid/navier_stokes.py:338-343): the whole residual in one output, formed
+ * as one instead of as the sum of the two outputs above (equal to round-off).  float64 plans whose path has that
+ * form: Euler plans, the fused hexahedron form, the two-launch dense form (5 variables); else
+ * DGB_ERR_UNSUPPORTED. */
+int dgb_rhs_total(dgb_plan* plan, const dgb_state* U, const dgb_state* out, void* stream);
 /* Physical coordinates of every face point, [F][nq][3] for one face type (the moment arms of
  * dgb_wall_forces). */
 int dgb_plan_set_face_points(dgb_plan* plan, int face_type, const double* points);

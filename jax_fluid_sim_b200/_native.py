@@ -11,6 +11,7 @@ from pathlib import Path
 import numpy as np
 
 MAX_BLOCKS, MAX_TAGS, MAX_VARS = 3, 8, 16
+UNSUPPORTED = -3                     # DGB_ERR_UNSUPPORTED
 LIB_PATH = Path(__file__).resolve().parent / "libdgb200.so"
 
 c_int, c_double, c_void_p = ctypes.c_int, ctypes.c_double, ctypes.c_void_p
@@ -153,6 +154,7 @@ def lib():
                                 P_double, P_double, P_double, P_double, P_double, P_double],
             "dgb_plan_destroy": [c_void_p],
             "dgb_plan_update_params": [c_void_p, ctypes.POINTER(Params)],
+            "dgb_rhs_total": [c_void_p, ctypes.POINTER(State), ctypes.POINTER(State), c_void_p],
             "dgb_rhs": [c_void_p, ctypes.POINTER(State), ctypes.POINTER(State), ctypes.POINTER(State), c_void_p],
             "dgb_stable_dt": [c_void_p, ctypes.POINTER(State), c_double, c_void_p, c_void_p],
             "dgb_positivity": [c_void_p, ctypes.POINTER(State), c_void_p],

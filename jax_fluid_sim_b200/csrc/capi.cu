@@ -386,10 +386,10 @@ size_t dense_layout(const dgb_plan* p, ElemLaunch& L, DenseKind kind, size_t rs)
   return most;
 }
 
-// Completes the two-launch inviscid form (dense_rhs.cu) where every block has its shapes and tables.
+// Completes the two-launch form (dense_rhs.cu) where every block has its shapes and tables.
 int dense_finish(dgb_plan* p) {
   p->dense.ready = false;
-  if (p->hex || p->dev.viscous || p->dev.nv != 5 || p->dev.degree < 1 || p->dev.degree > 3) return DGB_OK;
+  if (p->hex || p->dev.nv != 5 || p->dev.degree < 1 || p->dev.degree > 3) return DGB_OK;
   const bool f32 = p->prm.precision == 1;
   for (int b = 0; b < p->dev.nblocks; ++b) {
     const BlockDev& B = p->dev.blk[b];
@@ -398,7 +398,7 @@ int dense_finish(dgb_plan* p) {
     if (B.E == 0) continue;
     const DenseShape s = dense_shape(p->dev.degree, B.type);
     const bool tri = B.type != 0, quad = B.type != 2;
-    if (B.Np != s.Np || B.Nq != s.Nq || B.nlf != s.nlf || !p->faces_regular[b] || !B.Bt || !B.dBi || !B.jinv ||
+    if (B.Np != s.Np || B.Nq != s.Nq || B.nlf != s.nlf || !p->faces_regular[b] || !B.Bt || !B.dBi || !B.dBq || !B.jinv ||
         !B.wdet || (tri && !X.cB[0]) || (quad && !X.cB[1]))
       return DGB_OK;
     X.chunks = volume_chunks(B.Np, dense_width(p, B));
@@ -554,7 +554,8 @@ template <int NV, typename R>
 int run_rhs_dense(dgb_plan* p, const StatePtrs& S, const FinalizeArgs& A, cudaStream_t st, cudaEvent_t* ev) {
   const DevPlan& P = p->dev;
   int rc;
-  if (NV == 5 && p->dense.ready) {
+  const bool split = (!A.stage && !A.total) || A.out_vis[0] != nullptr;
+  if (NV == 5 && p->dense.ready && !(P.viscous && (split || sizeof(R) == sizeof(float)))) {
     constexpr bool f32 = sizeof(R) == sizeof(float);
     auto record = [&](int k) { return ev ? cudaEventRecord(ev[k], st) : cudaSuccess; };
     CK(record(0));
@@ -619,7 +620,7 @@ int autotune_dense(dgb_plan* p, const StatePtrs& S, int reps, cudaStream_t st, i
   FinalizeArgs A;
   memset(&A, 0, sizeof(A));
   int rc;
-  if (NV == 5 && p->dense.ready) {            // the two-launch form's work split is fixed
+  if (NV == 5 && p->dense.ready && !P.viscous) {   // the two-launch form's work split is fixed
     const ElemLaunch* fixed[3] = {&p->launch_tr, &p->launch_vol, &p->launch_fin};
     for (int k = 0; widths && k < 3; ++k)
       for (int b = 0; b < DGB_MAX_BLOCKS; ++b) widths[k * DGB_MAX_BLOCKS + b] = b < P.nblocks ? fixed[k]->W[b] : 0;
@@ -689,7 +690,7 @@ int autotune_dense(dgb_plan* p, const StatePtrs& S, int reps, cudaStream_t st, i
 // events: optional array of DGB_RHS_STAGES + 1 events recorded around the stages
 template <int NV>
 int run_rhs(dgb_plan* p, const StatePtrs& S, const FinalizeArgs& A, cudaStream_t st, cudaEvent_t* ev = nullptr) {
-  const bool split = !A.stage || A.out_vis[0] != nullptr;
+  const bool split = (!A.stage && !A.total) || A.out_vis[0] != nullptr;
   if (p->hex) return split ? run_rhs_hex_prec<NV, true>(p, S, A, st, ev) : run_rhs_hex_prec<NV, false>(p, S, A, st, ev);
   return p->prm.precision == 1 ? run_rhs_dense<NV, float>(p, S, A, st, ev) : run_rhs_dense<NV, double>(p, S, A, st, ev);
 }
@@ -1718,6 +1719,21 @@ int dgb_rhs(dgb_plan* p, const dgb_state* U, const dgb_state* inv_out, const dgb
     A.out_inv[b] = inv_out ? inv_out->block[b] : nullptr;
     A.out_vis[b] = vis_out ? vis_out->block[b] : nullptr;
   }
+  const StatePtrs S = to_ptrs(U);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  return p->dev.nv == 5 ? run_rhs<5>(p, S, A, st) : run_rhs<16>(p, S, A, st);
+}
+
+int dgb_rhs_total(dgb_plan* p, const dgb_state* U, const dgb_state* out, void* stream) {
+  int rc;
+  if ((rc = check_ready(p)) || (rc = check_state(p, U, "U")) || (rc = check_state(p, out, "out"))) return rc;
+  if (p->prm.precision == 1) return fail(DGB_ERR_UNSUPPORTED, "mixed plans form the residuals apart (dgb_rhs)");
+  if (p->dev.viscous && !(p->hex ? p->fused : p->dense.ready))
+    return fail(DGB_ERR_UNSUPPORTED, "this plan forms the residuals apart (dgb_rhs)");
+  FinalizeArgs A;
+  memset(&A, 0, sizeof(A));
+  A.total = 1;
+  for (int b = 0; b < DGB_MAX_BLOCKS; ++b) A.out_inv[b] = out->block[b];
   const StatePtrs S = to_ptrs(U);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   return p->dev.nv == 5 ? run_rhs<5>(p, S, A, st) : run_rhs<16>(p, S, A, st);

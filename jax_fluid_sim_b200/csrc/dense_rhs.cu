@@ -1,11 +1,17 @@
-// Inviscid right-hand side of the dense path (hybrid meshes: hexahedra, wedges, tetrahedra) in two
-// launches per evaluation (hybrid/spatial.py:47-72,137-249):
+// Right-hand side of the dense path (hybrid meshes: hexahedra, wedges, tetrahedra) in two launches per
+// evaluation (hybrid/spatial.py:47-72,137-249, hybrid/navier_stokes.py:27-347), as one residual:
 //
 //   k_dense_faces    face traces and HLLC flux: one thread per face point.  The traces are formed from
 //                    the nodes on the face (the basis of every other node is zero there), read
-//                    from the element states, so no trace buffer goes through memory.
-//   k_dense_update   one CTA per NE elements: volume residual, face terms, M^-1 and the stage update,
-//                    with everything between them in shared memory.
+//                    from the element states, so no trace buffer goes through memory.  With viscous
+//                    terms also the gradients, the BR2 jump, both sides' local lifts (M^-1 over the face's
+//                    nodes alone, 9 to 16 times fewer products than over all nodes) and the viscous flux.
+//   k_dense_update   one CTA per NE elements: (nodal lift,) volume residual, face terms, M^-1 and the
+//                    stage update, with everything between them in shared memory.
+//
+// The residual of a 4^3 P2 hybrid box with viscous terms took nine launches and three additions of the
+// split residuals, 122 us, and takes these two, 49 us.  Split residuals (MOOD, the separate right-hand
+// sides) and mixed viscous plans keep the general kernels of dg_kernels.cuh.
 //
 // The element kernel is bound by the operand loads of its contractions, not by their arithmetic: with
 // one accumulator row per table value and broadcast operand (one element per CTA, one value per
@@ -42,22 +48,25 @@ struct Shape {
 // elements per thread in the residual sum.  P2 and P3 volume rules of 125 points take one thread per
 // point over four elements; the 27 points of a P2 hexahedron leave room for four pairs; P1 elements
 // are one thread per (element, point).
-template <int P, int T>
+// With viscous terms an element has about four times the work and shared memory: one P2 or P3 element per CTA
+// (two 27-point hexahedra), tiles of one element.
+template <int P, int T, bool VISC>
 struct Split {
   static constexpr bool one = P == 1;
-  static constexpr int NE = one ? (T == 0 ? 16 : T == 1 ? 20 : 32) : (P == 2 && T == 0 ? 8 : 4);
-  static constexpr int EB = one ? 1 : (P == 2 && T == 0 ? 2 : 4);
-  static constexpr int EB2 = one ? 1 : 2;
-  static constexpr int IB = one || Shape<P, T>::Np % 2 ? 1 : 2;
+  static constexpr int NE = VISC ? (one ? (T == 0 ? 8 : T == 1 ? 10 : 16) : (P == 2 && T == 0 ? 2 : 1))
+                                 : (one ? (T == 0 ? 16 : T == 1 ? 20 : 32) : (P == 2 && T == 0 ? 8 : 4));
+  static constexpr int EB = one || VISC ? 1 : (P == 2 && T == 0 ? 2 : 4);
+  static constexpr int EB2 = one || VISC ? 1 : 2;
+  static constexpr int IB = one || VISC || Shape<P, T>::Np % 2 ? 1 : 2;
 };
 
 __host__ __device__ constexpr int round_up(int a, int b) { return (a + b - 1) / b * b; }
 
 // Shared memory of k_dense_update in units of R.
-template <int P, int T, int NV, typename R>
+template <int P, int T, int NV, typename R, bool VISC>
 struct Smem {
   using S = Shape<P, T>;
-  using W = Split<P, T>;
+  using W = Split<P, T, VISC>;
   static constexpr int VA = 16 / (int)sizeof(R);
   static constexpr int UE = round_up(W::EB * NV, VA);                  // one node of EB elements
   static constexpr int UG = S::Np * UE;                                 // one group of EB elements
@@ -69,7 +78,12 @@ struct Smem {
   // at the front: anchors (double), their fluxes, and two ints per (element, face)
   static constexpr int AN = W::NE * NV * (8 / (int)sizeof(R)), FA = W::NE * 3 * NV;
   static constexpr int FI = (2 * W::NE * S::nlf * 4 + (int)sizeof(R) - 1) / (int)sizeof(R);
-  static constexpr int U = round_up(AN + FA + FI, VA), Gs = U + W::NE / W::EB * UG;
+  static constexpr int U = round_up(AN + FA + FI, VA);
+  // viscous plans: nodal viscous variables [NE][Np][4] and lift [NE][Np][12]; before the points are worked, the
+  // jumps [NE][Nf][12] and their nodal sums [NE][Np][12] where G goes
+  static constexpr int V = U + W::NE / W::EB * UG, LF = V + (VISC ? W::NE * S::Np * 4 : 0);
+  static constexpr int Gs = LF + (VISC ? W::NE * S::Np * 12 : 0);
+  static constexpr int JS = Gs, BS = JS + W::NE * S::Nf * 12, B_END = VISC ? BS + W::NE * S::Np * 12 : 0;
   static constexpr int G = W::NE / W::EB * GG;
   // over G once it is dead: chunk sums, fluxes, face sums, totals, results
   static constexpr int FS = round_up(NV, VA);                          // one row of NV values
@@ -81,7 +95,7 @@ struct Smem {
   static constexpr int Tt = W::one ? Gs : Fl;
   static constexpr int End = Fp + (W::one ? 0 : W::NE * S::Nj * FS);   // P1: no face sums
   static_assert(S::Np <= S::Nf, "the totals take the fluxes' place");
-  static constexpr int total = Gs + G > End ? Gs + G : End;
+  static constexpr int most = Gs + G > End ? Gs + G : End, total = most > B_END ? most : B_END;
 };
 
 // n values at p (16-byte aligned)
@@ -120,12 +134,12 @@ __device__ __forceinline__ void sts16(R* p, const R* r) {
 }
 
 // ------------------------------------------------------------------------------------ element kernel
-template <int P, int T, int NV, typename R>
+template <int P, int T, int NV, typename R, bool VISC>
 __device__ __forceinline__ void update_body(const DevPlan& D, const StatePtrs& St, const FinalizeArgs& A,
                                             const DenseBlock& X, int b, int cta, bool volume_done, R* sm) {
   using S = Shape<P, T>;
-  using W = Split<P, T>;
-  using L = Smem<P, T, NV, R>;
+  using W = Split<P, T, VISC>;
+  using L = Smem<P, T, NV, R, VISC>;
   constexpr int Np = S::Np, Nq = S::Nq, nlf = S::nlf, NE = W::NE, EB = W::EB, EB2 = W::EB2, IB = W::IB;
   double* anchor = reinterpret_cast<double*>(sm);
   R* Fanc = sm + L::AN;                                                // flux of the anchor states
@@ -166,7 +180,76 @@ __device__ __forceinline__ void update_body(const DevPlan& D, const StatePtrs& S
       const int e = t / (Np * NV), i = (t / NV) % Np, v = t % NV;
       if (t < VALS) U[(e / EB) * L::UG + i * L::UE + (e % EB) * NV + v] = x[k];
     }
+    if constexpr (VISC)
+      for (int t = threadIdx.x; t < NE * Np; t += kThreads) {
+        double u[NV], vv[4] = {0.0, 0.0, 0.0, 0.0};
+        if (t / Np < ne) {
+#pragma unroll
+          for (int v = 0; v < NV; ++v) u[v] = Ug[t * NV + v];
+          viscous_vars<NV>(D.ph, u, vv);
+        }
+        sts16<4>(sm + L::V + t * 4, vv);
+      }
     __syncthreads();
+    if constexpr (VISC) {
+      // ---- nodal lift M^-1 sum_f B_f^T jump_f (hybrid/navier_stokes.py:138-188)
+      double* Js = sm + L::JS;
+      double* Bs = sm + L::BS;
+      for (int t = threadIdx.x; t < NE * S::Nf * 12; t += kThreads) {
+        const int e = t / (S::Nf * 12), r = t % (S::Nf * 12);
+        int lf = 0;
+#pragma unroll
+        for (int m = 1; m < nlf; ++m) lf += r >= S::poff(m) * 12;
+        const int nq = S::nq(lf), k = (r - S::poff(lf) * 12) / nq, q = (r - S::poff(lf) * 12) % nq;
+        double x = 0.0;
+        if (e < ne) x = D.face[lf < S::ntri ? 0 : 1].jumpW[face_at(fslot[e * nlf + lf] >> 1, 12, k, nq, q)];
+        Js[(e * S::Nf + S::poff(lf) + q) * 12 + k] = x;
+      }
+      __syncthreads();
+      // thread = (element, node, four of the twelve components)
+      for (int t = threadIdx.x; t < ne * Np * 3; t += kThreads) {
+        const int e = t / (Np * 3), i = t % Np, g = t / Np % 3 * 4;
+        double s[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+        for (int lf = 0; lf < nlf; ++lf) {
+          const int ft = lf < S::ntri ? 0 : 1, nq = S::nq(lf), nfn = S::nfn(lf);
+          const int j = X.finv[ft][fcode[e * nlf + lf] * Np + i];
+          if (j < 0) continue;
+          const double* cB = static_cast<const double*>(X.cB[ft]) + (size_t)fcode[e * nlf + lf] * nq * nfn + j;
+          const double* js = Js + (e * S::Nf + S::poff(lf)) * 12 + g;
+#pragma unroll 4
+          for (int q = 0; q < nq; ++q) {
+            const double bt = __ldg(cB + q * nfn);
+            double x[4];
+            lds16<4>(js + q * 12, x);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) s[k] += bt * x[k];
+          }
+        }
+        sts16<4>(Bs + (e * Np + i) * 12 + g, s);
+      }
+      __syncthreads();
+      for (int t = threadIdx.x; t < ne * Np * 3; t += kThreads) {
+        const int e = t / (Np * 3), i = t % Np, g = t / Np % 3 * 4;
+        const bool aff = B.affine != nullptr && B.affine[e0 + e];
+        const double* Mi = (aff ? B.mref_inv : B.minv + (size_t)(e0 + e) * Np * Np) + i;
+        const double ms = aff ? B.acoef[e0 + e] : 1.0;
+        double s[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 8
+        for (int j = 0; j < Np; ++j) {
+          const double m = __ldg(Mi + j * Np);
+          double x[4];
+          lds16<4>(Bs + (e * Np + j) * 12 + g, x);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) s[k] += m * x[k];
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) s[k] *= ms;
+        sts16<4>(sm + L::LF + (e * Np + i) * 12 + g, s);
+      }
+      for (int t = threadIdx.x; t < (NE - ne) * Np * 12; t += kThreads) sm[L::LF + ne * Np * 12 + t] = 0.0;
+      __syncthreads();
+    }
     for (int t = threadIdx.x; t < NE * 3; t += kThreads) {
       const int d = t % 3;
       const R n[3] = {(R)(d == 0), (R)(d == 1), (R)(d == 2)};
@@ -185,6 +268,10 @@ __device__ __forceinline__ void update_body(const DevPlan& D, const StatePtrs& S
       R acc[EB * NV];
 #pragma unroll
       for (int k = 0; k < EB * NV; ++k) acc[k] = (R)0;
+      double gr[VISC ? 12 : 1], lq[VISC ? 12 : 1];     // reference gradients of v, lift (EB = 1)
+      if constexpr (VISC)
+#pragma unroll
+        for (int k = 0; k < 12; ++k) gr[k] = lq[k] = 0.0;
       const R* Ur = U + g * L::UG;
 #pragma unroll 4
       for (int i = 0; i < Np; ++i) {
@@ -193,6 +280,21 @@ __device__ __forceinline__ void update_body(const DevPlan& D, const StatePtrs& S
         lds16<EB * NV>(Ur + i * L::UE, x);
 #pragma unroll
         for (int k = 0; k < EB * NV; ++k) acc[k] += bq * x[k];
+        if constexpr (VISC) {
+          const double* gd = B.dBq + (size_t)i * 3 * Nq + q;
+          const double d0 = __ldg(gd), d1 = __ldg(gd + Nq), d2 = __ldg(gd + 2 * Nq);
+          double v[4], l[12];
+          lds16<4>(sm + L::V + (g * Np + i) * 4, v);
+          lds16<12>(sm + L::LF + (g * Np + i) * 12, l);
+#pragma unroll
+          for (int m = 0; m < 4; ++m) {
+            gr[m] += d0 * v[m];
+            gr[4 + m] += d1 * v[m];
+            gr[8 + m] += d2 * v[m];
+          }
+#pragma unroll
+          for (int k = 0; k < 12; ++k) lq[k] += bq * l[k];
+        }
       }
       R* Gq = G + g * L::GG + q * L::GQ;
 #pragma unroll
@@ -223,6 +325,32 @@ __device__ __forceinline__ void update_body(const DevPlan& D, const StatePtrs& S
             for (int v = 0; v < NV; ++v)
               out[(r * EB2 + k) * NV + v] = (J[r * 3 + 0] * (F[0][v] - Fa[v]) + J[r * 3 + 1] * (F[1][v] - Fa[NV + v]) +
                                              J[r * 3 + 2] * (F[2][v] - Fa[2 * NV + v])) * wq;
+        }
+        if constexpr (VISC) {
+          // minus the viscous flux of the lifted gradients
+          const int el = g < ne ? g : 0;
+          const size_t e = (size_t)e0 + el;
+          const bool aff = B.affine != nullptr && B.affine[e];
+          const double* Jd = aff ? B.ajinv + e * 9 : B.jinv + e * 9 * Nq + q;
+          const int js = aff ? 1 : Nq;
+          double J[9], grad[12], Uq[NV], Fv[3 * NV];
+#pragma unroll
+          for (int m = 0; m < 9; ++m) J[m] = Jd[m * js];
+          const double wq = aff ? B.wref[q] * B.adet[e] : B.wdet[e * Nq + q];
+#pragma unroll
+          for (int m = 0; m < 4; ++m)
+#pragma unroll
+            for (int d = 0; d < 3; ++d)
+              grad[m * 3 + d] = gr[m] * J[d] + gr[4 + m] * J[3 + d] + gr[8 + m] * J[6 + d] + lq[m * 3 + d];
+#pragma unroll
+          for (int v = 0; v < NV; ++v) Uq[v] = anchor[g * NV + v] + acc[v];
+          const CaseView cv = case_view(D.ph, B.ecase, e);
+          viscous_flux<NV>(D.ph, cv.mu, cv.kappa, Uq, grad, Fv);
+#pragma unroll
+          for (int r = 0; r < 3; ++r)
+#pragma unroll
+            for (int v = 0; v < NV; ++v)
+              out[r * NV + v] -= (J[r * 3] * Fv[v] + J[r * 3 + 1] * Fv[NV + v] + J[r * 3 + 2] * Fv[2 * NV + v]) * wq;
         }
         sts16<EB2 * 3 * NV>(Gq + h * L::GP, out);
       }
@@ -318,6 +446,11 @@ __device__ __forceinline__ void update_body(const DevPlan& D, const StatePtrs& S
       const double* src = fd.fluxI + face_at((size_t)fslot[e * nlf + lf], NV, 0, nq, pt - S::poff(lf));
 #pragma unroll
       for (int v = 0; v < NV; ++v) x[k][v] = src[v * nq];
+      if constexpr (VISC) {
+        const double* vis = fd.fluxV + face_at(fslot[e * nlf + lf] >> 1, NV, 0, nq, pt - S::poff(lf));
+#pragma unroll
+        for (int v = 0; v < NV; ++v) x[k][v] -= vis[v * nq];
+      }
     }
 #pragma unroll
     for (int k = 0; k < FR; ++k) {
@@ -456,8 +589,8 @@ struct UpdateGrid {
   bool volume_done[DGB_MAX_BLOCKS];
 };
 
-template <int P, int NV, typename R>
-__global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) || P == 1 ? 5 : 3)
+template <int P, int NV, typename R, bool VISC>
+__global__ void __launch_bounds__(kThreads, VISC ? 3 : sizeof(R) == sizeof(float) || P == 1 ? 5 : 3)
     k_dense_update(const __grid_constant__ DevPlan D, const StatePtrs St, const __grid_constant__ FinalizeArgs A,
                    const __grid_constant__ DenseTables X, const UpdateGrid L) {
   extern __shared__ __align__(16) unsigned char dyn_smem[];
@@ -465,20 +598,35 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == sizeof(float) || P == 1
   int b = 0;
   while (b + 1 < D.nblocks && (int)blockIdx.x >= L.cta0[b + 1]) ++b;
   const int cta = blockIdx.x - L.cta0[b];
-  if (D.blk[b].type == 0) update_body<P, 0, NV, R>(D, St, A, X.b[b], b, cta, L.volume_done[b], sm);
-  else if (D.blk[b].type == 1) update_body<P, 1, NV, R>(D, St, A, X.b[b], b, cta, L.volume_done[b], sm);
-  else update_body<P, 2, NV, R>(D, St, A, X.b[b], b, cta, L.volume_done[b], sm);
+  if (D.blk[b].type == 0) update_body<P, 0, NV, R, VISC>(D, St, A, X.b[b], b, cta, L.volume_done[b], sm);
+  else if (D.blk[b].type == 1) update_body<P, 1, NV, R, VISC>(D, St, A, X.b[b], b, cta, L.volume_done[b], sm);
+  else update_body<P, 2, NV, R, VISC>(D, St, A, X.b[b], b, cta, L.volume_done[b], sm);
 }
 
 // --------------------------------------------------------------------------------------- face kernel
 // One face type's CTA: kThreads / nq faces, one thread per face point.  The face's nodes on both
 // sides come from the element states into shared memory (minus the side's anchor, node 0).
-template <int P, int FT, int NV, typename R>
+template <int P, int FT, int NV, typename R, bool VISC>
+struct FaceSmem {
+  static constexpr int nq = FT == 0 ? Shape<P, 1>::NQT : Shape<P, 1>::NQQ, nfn = FT == 0 ? Shape<P, 1>::TRI : Shape<P, 1>::QUAD;
+  static_assert(nfn <= nq, "the local lift has one thread per face node");
+  static constexpr int FPC = kThreads / nq, FS = round_up(NV, 16 / (int)sizeof(R));
+  static constexpr int NPM = FT == 0 ? Shape<P, 1>::Np : Shape<P, 0>::Np;      // nodes of the largest element with such faces
+  // in R: anchors (double), face nodes [FPC][2][nfn][FS]; viscous: all nodes' viscous variables [FPC][2][NPM][4],
+  // later the lift's nodal rows b and r [FPC][nfn][12] each, and the jumps [FPC][nq][12]
+  static constexpr int AN = round_up(FPC * 2 * NV * (8 / (int)sizeof(R)), 4), N = AN + FPC * 2 * nfn * FS;
+  static constexpr int V = N, BB = V, RR = BB + FPC * nfn * 12;
+  static constexpr int vis = FPC * 2 * NPM * 4 > FPC * nfn * 24 ? FPC * 2 * NPM * 4 : FPC * nfn * 24;
+  static constexpr int J = V + (VISC ? vis : 0), total = J + (VISC ? FPC * nq * 12 : 0);
+};
+
+template <int P, int FT, int NV, typename R, bool VISC>
 __device__ __forceinline__ void faces_body(const DevPlan& D, const StatePtrs& St, const DenseTables& X, int cta,
-                                           bool store_traces, R* sm) {
-  constexpr int nq = FT == 0 ? Shape<P, 1>::NQT : Shape<P, 1>::NQQ, nfn = FT == 0 ? Shape<P, 1>::TRI : Shape<P, 1>::QUAD;
-  constexpr int FPC = kThreads / nq, FS = round_up(NV, 16 / (int)sizeof(R));
-  __shared__ double anc[FPC * 2 * NV];
+                                           bool store_traces, R* smem) {
+  using L = FaceSmem<P, FT, NV, R, VISC>;
+  constexpr int nq = L::nq, nfn = L::nfn, FPC = L::FPC, FS = L::FS;
+  double* anc = reinterpret_cast<double*>(smem);
+  R* sm = smem + L::AN;
   const FaceDev& fd = D.face[FT];
   const int f0 = cta * FPC, nf = fd.F - f0 < FPC ? fd.F - f0 : FPC;
   for (int t = threadIdx.x; t < nf * 2 * nfn; t += kThreads) {
@@ -497,11 +645,28 @@ __device__ __forceinline__ void faces_body(const DevPlan& D, const StatePtrs& St
     }
     sts16<NV>(sm + t * FS, x);
   }
+  if constexpr (VISC) {
+    for (int t = threadIdx.x; t < nf * 2 * L::NPM; t += kThreads) {
+      const int i = t % L::NPM;
+      const int3 side = X.side[FT][f0 * 2 + t / L::NPM];
+      if (side.x < 0 || i >= D.blk[side.x].Np) continue;
+      const double* un = St.b[side.x] + ((size_t)side.y * D.blk[side.x].Np + i) * NV;
+      double u[NV], vv[4];
+#pragma unroll
+      for (int v = 0; v < NV; ++v) u[v] = un[v];
+      viscous_vars<NV>(D.ph, u, vv);
+      sts16<4>(smem + L::V + t * 4, vv);
+    }
+  }
   __syncthreads();
   const int slot = threadIdx.x / nq, q = threadIdx.x % nq;
   const int f = f0 + slot;
-  if (slot >= nf) return;
-  const int nb = fd.nb[f];
+  const bool live = slot < nf;
+  if (!VISC && !live) return;
+  const int nb = live ? fd.nb[f] : -1;
+  const size_t so = (size_t)f * 2, sn = so + 1;
+  double n[3] = {0.0, 0.0, 0.0}, w = 0.0;
+  double UL[NV], UR[NV];
   auto trace = [&](int side, int blk, int code, double* out) {
     const R* cBt = static_cast<const R*>(X.b[blk].cBt[FT]) + (size_t)code * nfn * nq + q;
     const R* row = sm + (slot * 2 + side) * nfn * FS;
@@ -519,67 +684,209 @@ __device__ __forceinline__ void faces_body(const DevPlan& D, const StatePtrs& St
 #pragma unroll
     for (int v = 0; v < NV; ++v) out[v] = anc[(slot * 2 + side) * NV + v] + (double)acc[v];
   };
-  const double n[3] = {fd.n[face_at(f, 3, 0, nq, q)], fd.n[face_at(f, 3, 1, nq, q)], fd.n[face_at(f, 3, 2, nq, q)]};
-  const double w = fd.w[(size_t)f * nq + q];
-  const size_t so = (size_t)f * 2, sn = so + 1;
-  double UL[NV], UR[NV], Fh[NV], Fa[NV];
-  trace(0, fd.ob[f], fd.oc[f], UL);
-  if (nb >= 0) {
-    trace(1, nb, fd.nc[f], UR);
-  } else if (D.ph.has_boundary) {
-    ghost_state<NV>(D.ph, case_view(D.ph, D.blk[fd.ob[f]].ecase, fd.ol[f]).far, UL, n, fd.tag[f], UR);
-  } else {
+  if (live) {
+    n[0] = fd.n[face_at(f, 3, 0, nq, q)], n[1] = fd.n[face_at(f, 3, 1, nq, q)], n[2] = fd.n[face_at(f, 3, 2, nq, q)];
+    w = fd.w[(size_t)f * nq + q];
+    double Fh[NV], Fa[NV];
+    trace(0, fd.ob[f], fd.oc[f], UL);
+    if (nb >= 0) {
+      trace(1, nb, fd.nc[f], UR);
+    } else if (D.ph.has_boundary) {
+      ghost_state<NV>(D.ph, case_view(D.ph, D.blk[fd.ob[f]].ecase, fd.ol[f]).far, UL, n, fd.tag[f], UR);
+    } else {
 #pragma unroll
-    for (int v = 0; v < NV; ++v) UR[v] = UL[v];
+      for (int v = 0; v < NV; ++v) UR[v] = UL[v];
+    }
+    if (store_traces) {
+#pragma unroll
+      for (int v = 0; v < NV; ++v) fd.trA[face_at(so, NV, v, nq, q)] = UL[v];
+      if (nb >= 0)
+#pragma unroll
+        for (int v = 0; v < NV; ++v) fd.trA[face_at(sn, NV, v, nq, q)] = UR[v];
+    }
+    hllc<NV>(D.ph, UL, UR, n, Fh);
+#pragma unroll
+    for (int side = 0; side < 2; ++side) {
+      if (side == 1 && nb < 0) break;
+      double a[NV];
+#pragma unroll
+      for (int v = 0; v < NV; ++v) a[v] = anc[(slot * 2 + side) * NV + v];
+      normal_flux<NV>(D.ph, a, n, Fa);
+      double* out = fd.fluxI + face_at(side ? sn : so, NV, 0, nq, q);
+#pragma unroll
+      for (int v = 0; v < NV; ++v) out[v * nq] = (Fh[v] - Fa[v]) * w;
+    }
   }
-  if (store_traces) {
+  if constexpr (VISC) {
+    // ---- viscous traces and raw gradients of both sides, the BR2 jump
+    double* jmp = smem + L::J;
+    double gs[2][12], vt[2][4];
 #pragma unroll
-    for (int v = 0; v < NV; ++v) fd.trA[face_at(so, NV, v, nq, q)] = UL[v];
-    if (nb >= 0)
+    for (int s = 0; s < 2; ++s) {
+      if (!live || (s == 1 && nb < 0)) continue;
+      const int blk = s ? nb : fd.ob[f], code = s ? fd.nc[f] : fd.oc[f];
+      const BlockDev& B = D.blk[blk];
+      const int Np = B.Np;
+      const double* Bt = B.trBt[FT] + (size_t)code * Np * nq + q;
+      const double* dBt = B.trdBt[FT] + (size_t)code * Np * 3 * nq + q;
+      const double* row = smem + L::V + (slot * 2 + s) * L::NPM * 4;
+      double gr[12];
 #pragma unroll
-      for (int v = 0; v < NV; ++v) fd.trA[face_at(sn, NV, v, nq, q)] = UR[v];
-  }
-  hllc<NV>(D.ph, UL, UR, n, Fh);
+      for (int k = 0; k < 12; ++k) gr[k] = 0.0;
 #pragma unroll
-  for (int side = 0; side < 2; ++side) {
-    if (side == 1 && nb < 0) break;
-    double a[NV];
+      for (int m = 0; m < 4; ++m) vt[s][m] = 0.0;
+#pragma unroll 4
+      for (int i = 0; i < Np; ++i) {
+        const double bt = __ldg(Bt + i * nq);
+        const double d0 = __ldg(dBt + i * 3 * nq), d1 = __ldg(dBt + (i * 3 + 1) * nq), d2 = __ldg(dBt + (i * 3 + 2) * nq);
+        double v[4];
+        lds16<4>(row + i * 4, v);
 #pragma unroll
-    for (int v = 0; v < NV; ++v) a[v] = anc[(slot * 2 + side) * NV + v];
-    normal_flux<NV>(D.ph, a, n, Fa);
-    double* out = fd.fluxI + face_at(side ? sn : so, NV, 0, nq, q);
+        for (int m = 0; m < 4; ++m) {
+          vt[s][m] += bt * v[m];
+          gr[m] += d0 * v[m];
+          gr[4 + m] += d1 * v[m];
+          gr[8 + m] += d2 * v[m];
+        }
+      }
+      double J[9];
 #pragma unroll
-    for (int v = 0; v < NV; ++v) out[v * nq] = (Fh[v] - Fa[v]) * w;
+      for (int k = 0; k < 9; ++k) J[k] = fd.jinv[face_at(so + s, 9, k, nq, q)];
+#pragma unroll
+      for (int m = 0; m < 4; ++m)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) gs[s][m * 3 + d] = gr[m] * J[d] + gr[4 + m] * J[3 + d] + gr[8 + m] * J[6 + d];
+    }
+    const CaseView cv = case_view(D.ph, D.blk[live ? fd.ob[f] : 0].ecase, live ? fd.ol[f] : 0);
+    if (live) {
+      if (nb < 0) {
+        if (D.ph.has_boundary) viscous_ghost<NV>(D.ph, cv.far, cv.wall_T, UL, n, fd.tag[f], vt[1]);
+        else viscous_vars<NV>(D.ph, UL, vt[1]);
+      }
+      double jr[12];
+#pragma unroll
+      for (int m = 0; m < 4; ++m)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          jr[m * 3 + d] = 0.5 * w * (vt[1][m] - vt[0][m]) * n[d];
+          fd.jumpW[face_at(f, 12, m * 3 + d, nq, q)] = jr[m * 3 + d];
+        }
+      sts16<12>(jmp + (slot * nq + q) * 12, jr);
+    }
+    __syncthreads();
+    // ---- each side's local lift br2 B_f M^-1 B_f^T jump, over the nodes of the face alone (the basis of the
+    // others vanishes there)
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      const bool on = live && (s == 0 || nb >= 0);
+      double* bb = smem + L::BB + slot * nfn * 12;
+      double* rr = smem + L::RR + slot * nfn * 12;
+      const int blk = !on ? 0 : s ? nb : fd.ob[f], code = !on ? 0 : s ? fd.nc[f] : fd.oc[f], el = !on ? 0 : s ? fd.nl[f] : fd.ol[f];
+      const BlockDev& B = D.blk[blk];
+      const DenseBlock& Xb = X.b[blk];
+      if (on && q < nfn) {
+        const double* cB = static_cast<const double*>(Xb.cB[FT]) + (size_t)code * nq * nfn + q;
+        double x[12];
+#pragma unroll
+        for (int k = 0; k < 12; ++k) x[k] = 0.0;
+#pragma unroll 4
+        for (int p = 0; p < nq; ++p) {
+          const double bt = __ldg(cB + p * nfn);
+          double j[12];
+          lds16<12>(jmp + (slot * nq + p) * 12, j);
+#pragma unroll
+          for (int k = 0; k < 12; ++k) x[k] += bt * j[k];
+        }
+        sts16<12>(bb + q * 12, x);
+      }
+      __syncthreads();
+      if (on && q < nfn) {
+        const bool aff = B.affine != nullptr && B.affine[el];
+        const int Np = B.Np;
+        const uint8_t* fn = Xb.fnode[FT] + code * nfn;
+        const double* M = (aff ? B.mref_inv : B.minv + (size_t)el * Np * Np) + fn[q];
+        const double ms = D.ph.br2 * (aff ? B.acoef[el] : 1.0);
+        double x[12];
+#pragma unroll
+        for (int k = 0; k < 12; ++k) x[k] = 0.0;
+#pragma unroll 4
+        for (int p = 0; p < nfn; ++p) {
+          const double m = __ldg(M + (int)fn[p] * Np);
+          double j[12];
+          lds16<12>(bb + p * 12, j);
+#pragma unroll
+          for (int k = 0; k < 12; ++k) x[k] += m * j[k];
+        }
+#pragma unroll
+        for (int k = 0; k < 12; ++k) x[k] *= ms;
+        sts16<12>(rr + q * 12, x);
+      }
+      __syncthreads();
+      if (on) {
+        const double* cBt = static_cast<const double*>(Xb.cBt[FT]) + (size_t)code * nfn * nq + q;
+#pragma unroll 4
+        for (int p = 0; p < nfn; ++p) {
+          const double bt = __ldg(cBt + p * nq);
+          double j[12];
+          lds16<12>(rr + p * 12, j);
+#pragma unroll
+          for (int k = 0; k < 12; ++k) gs[s][k] += bt * j[k];
+        }
+      }
+    }
+    if (!live) return;
+    double Fo[3 * NV];
+    viscous_flux<NV>(D.ph, cv.mu, cv.kappa, UL, gs[0], Fo);
+    if (nb >= 0) {
+      double Fn[3 * NV];
+      viscous_flux<NV>(D.ph, cv.mu, cv.kappa, UR, gs[1], Fn);
+#pragma unroll
+      for (int k = 0; k < 3 * NV; ++k) Fo[k] = 0.5 * (Fo[k] + Fn[k]);
+    }
+    double out[NV];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) out[v] = Fo[v] * n[0] + Fo[NV + v] * n[1] + Fo[2 * NV + v] * n[2];
+    if (nb < 0 && D.ph.has_boundary && tag_in(fd.tag[f], D.ph.wall, D.ph.n_wall)) out[4] = 0.0;
+#pragma unroll
+    for (int v = 0; v < NV; ++v) fd.fluxV[face_at(f, NV, v, nq, q)] = out[v] * w;
   }
 }
 
-template <int P, typename R, int NV>
-__host__ __device__ constexpr int faces_smem() {
-  constexpr int FS = round_up(NV, 16 / (int)sizeof(R));
-  constexpr int t = kThreads / Shape<P, 1>::NQT * 2 * Shape<P, 1>::TRI * FS;
-  constexpr int q = kThreads / Shape<P, 1>::NQQ * 2 * Shape<P, 1>::QUAD * FS;
+template <int P, int NV, typename R, bool VISC>
+constexpr int faces_smem() {
+  constexpr int t = FaceSmem<P, 0, NV, R, VISC>::total, q = FaceSmem<P, 1, NV, R, VISC>::total;
   return t > q ? t : q;
 }
 
-template <int P, int NV, typename R>
-__global__ void __launch_bounds__(kThreads, 4)
+template <int P, int NV, typename R, bool VISC>
+__global__ void __launch_bounds__(kThreads, VISC ? 3 : 4)
     k_dense_faces(const __grid_constant__ DevPlan D, const StatePtrs St, const __grid_constant__ DenseTables X,
                   int tri_ctas, bool store_traces) {
-  __shared__ __align__(16) R sm[faces_smem<P, R, NV>()];
-  if ((int)blockIdx.x < tri_ctas) faces_body<P, 0, NV, R>(D, St, X, blockIdx.x, store_traces, sm);
-  else faces_body<P, 1, NV, R>(D, St, X, blockIdx.x - tri_ctas, store_traces, sm);
+  extern __shared__ __align__(16) unsigned char dyn_smem[];
+  R* sm = reinterpret_cast<R*>(dyn_smem);
+  if ((int)blockIdx.x < tri_ctas) faces_body<P, 0, NV, R, VISC>(D, St, X, blockIdx.x, store_traces, sm);
+  else faces_body<P, 1, NV, R, VISC>(D, St, X, blockIdx.x - tri_ctas, store_traces, sm);
 }
 
 // -------------------------------------------------------------------------------------------- launch
-template <int P, int NV, typename R>
+template <typename K>
+cudaError_t allow_smem(K kernel, size_t smem) {
+  return smem > 40 * 1024 ? cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) : cudaSuccess;
+}
+
+template <int P, int NV, typename R, bool VISC>
 cudaError_t launch_faces(const DevPlan& D, const StatePtrs& S, const DenseTables& T, bool store_traces, cudaStream_t st) {
   constexpr int ft = kThreads / Shape<P, 1>::NQT, fq = kThreads / Shape<P, 1>::NQQ;
+  constexpr size_t smem = sizeof(R) * (size_t)faces_smem<P, NV, R, VISC>();
   const int tri = (D.face[0].F + ft - 1) / ft, quad = (D.face[1].F + fq - 1) / fq;
-  if (tri + quad > 0) k_dense_faces<P, NV, R><<<tri + quad, kThreads, 0, st>>>(D, S, T, tri, store_traces);
+  if (tri + quad == 0) return cudaSuccess;
+  const cudaError_t e = allow_smem(k_dense_faces<P, NV, R, VISC>, smem);
+  if (e != cudaSuccess) return e;
+  k_dense_faces<P, NV, R, VISC><<<tri + quad, kThreads, smem, st>>>(D, S, T, tri, store_traces);
   return cudaGetLastError();
 }
 
-template <int P, int NV, typename R>
+template <int P, int NV, typename R, bool VISC>
 cudaError_t launch_update(const DevPlan& D, const StatePtrs& S, const FinalizeArgs& A, const DenseTables& T,
                           const bool* volume_done, cudaStream_t st) {
   UpdateGrid L;
@@ -587,20 +894,18 @@ cudaError_t launch_update(const DevPlan& D, const StatePtrs& S, const FinalizeAr
   size_t smem = 0;
   for (int b = 0; b < D.nblocks; ++b) {
     const int type = D.blk[b].type;
-    const int ne = type == 0 ? Split<P, 0>::NE : type == 1 ? Split<P, 1>::NE : Split<P, 2>::NE;
-    const size_t need = sizeof(R) * (size_t)(type == 0   ? Smem<P, 0, NV, R>::total
-                                             : type == 1 ? Smem<P, 1, NV, R>::total
-                                                         : Smem<P, 2, NV, R>::total);
+    const int ne = type == 0 ? Split<P, 0, VISC>::NE : type == 1 ? Split<P, 1, VISC>::NE : Split<P, 2, VISC>::NE;
+    const size_t need = sizeof(R) * (size_t)(type == 0   ? Smem<P, 0, NV, R, VISC>::total
+                                             : type == 1 ? Smem<P, 1, NV, R, VISC>::total
+                                                         : Smem<P, 2, NV, R, VISC>::total);
     smem = need > smem ? need : smem;
     L.cta0[b + 1] = L.cta0[b] + (D.blk[b].E + ne - 1) / ne;
     L.volume_done[b] = volume_done != nullptr && volume_done[b];
   }
   if (L.cta0[D.nblocks] == 0) return cudaSuccess;
-  if (smem > 24 * 1024) {                    // the kernel has static shared memory too
-    const cudaError_t e = cudaFuncSetAttribute(k_dense_update<P, NV, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
-  k_dense_update<P, NV, R><<<L.cta0[D.nblocks], kThreads, smem, st>>>(D, S, A, T, L);
+  const cudaError_t e = allow_smem(k_dense_update<P, NV, R, VISC>, smem);
+  if (e != cudaSuccess) return e;
+  k_dense_update<P, NV, R, VISC><<<L.cta0[D.nblocks], kThreads, smem, st>>>(D, S, A, T, L);
   return cudaGetLastError();
 }
 
@@ -619,23 +924,23 @@ DenseShape dense_shape(int P, int type) {
   return P == 1 ? shape_of<1>(type) : P == 2 ? shape_of<2>(type) : shape_of<3>(type);
 }
 
-#define DGB_DENSE_DISPATCH(CALL)                                                                       \
-  if (D.nv == 5) {                                                                                     \
-    if (f32) return D.degree == 1 ? CALL(1, 5, float) : D.degree == 2 ? CALL(2, 5, float) : CALL(3, 5, float);     \
-    return D.degree == 1 ? CALL(1, 5, double) : D.degree == 2 ? CALL(2, 5, double) : CALL(3, 5, double);           \
-  }                                                                                                    \
-  return cudaErrorInvalidValue
+// viscous terms: float64 only (the caller keeps the general kernels for mixed plans)
+#define DGB_DENSE_DISPATCH(CALL)                                                                                   \
+  if (D.nv != 5 || (D.viscous && f32)) return cudaErrorInvalidValue;                                               \
+  if (D.viscous) return D.degree == 1 ? CALL(1, 5, double, true) : D.degree == 2 ? CALL(2, 5, double, true) : CALL(3, 5, double, true); \
+  if (f32) return D.degree == 1 ? CALL(1, 5, float, false) : D.degree == 2 ? CALL(2, 5, float, false) : CALL(3, 5, float, false); \
+  return D.degree == 1 ? CALL(1, 5, double, false) : D.degree == 2 ? CALL(2, 5, double, false) : CALL(3, 5, double, false)
 
 cudaError_t dense_face_flux(const DevPlan& D, const StatePtrs& S, const DenseTables& T, bool f32, bool store_traces,
                             cudaStream_t st) {
-#define DGB_CALL(P, NV, R) (launch_faces<P, NV, R>(D, S, T, store_traces, st))
+#define DGB_CALL(P, NV, R, V) (launch_faces<P, NV, R, V>(D, S, T, store_traces, st))
   DGB_DENSE_DISPATCH(DGB_CALL);
 #undef DGB_CALL
 }
 
 cudaError_t dense_update(const DevPlan& D, const StatePtrs& S, const FinalizeArgs& A, const DenseTables& T, bool f32,
                          const bool* volume_done, cudaStream_t st) {
-#define DGB_CALL(P, NV, R) (launch_update<P, NV, R>(D, S, A, T, volume_done, st))
+#define DGB_CALL(P, NV, R, V) (launch_update<P, NV, R, V>(D, S, A, T, volume_done, st))
   DGB_DENSE_DISPATCH(DGB_CALL);
 #undef DGB_CALL
 }

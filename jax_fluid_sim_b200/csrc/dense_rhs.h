@@ -1,4 +1,4 @@
-// Inviscid right-hand side of the dense blocks in two launches (dense_rhs.cu).
+// Right-hand side of the dense blocks in two launches (dense_rhs.cu).
 #pragma once
 #include <cuda_runtime.h>
 

@@ -662,6 +662,7 @@ static __global__ void k_wall_forces_final(const double* __restrict__ partials, 
 // ---------------------------------------------------------------------------------------------
 struct FinalizeArgs {
   double* out_inv[DGB_MAX_BLOCKS];   // rhs outputs (may be null)
+  int total;                         // out_inv takes the whole residual, formed as one (no stage, no out_vis)
   double* out_vis[DGB_MAX_BLOCKS];
   // fused SSP-RK stage: dst = alpha*base + beta*(cur + dt*(rhs_inv + rhs_vis)); euler = cur + dt*rhs
   int stage;

@@ -403,6 +403,16 @@ class HybridNavierStokesOperator(HybridEulerOperator):
     def rhs(self, states, boundary_state=None):
         if not self.viscous:
             return self.inviscid_rhs(states, boundary_state)
+        if self.precision == "float64":
+            # one residual where the plan's path forms it so; the split residuals' sum elsewhere
+            U = self.to_device(states)
+            self.native.set_boundary(boundary_state)
+            out = {k: torch.empty_like(U[k]) for k in self.names}
+            s_in, s_out = self.native.state(self._blocks(U)), self.native.state(self._blocks(out))
+            rc = N.lib().dgb_rhs_total(self.native.handle, ctypes.byref(s_in), ctypes.byref(s_out), _stream_ptr())
+            if rc != N.UNSUPPORTED:
+                N.check(rc)
+                return out
         inv, vis = self._run_rhs(states, boundary_state, True, True)
         return {k: inv[k] + vis[k] for k in inv}
 
