@@ -710,6 +710,12 @@ int hex_positivity_grid(dgb_plan* p) {
   return DGB_OK;
 }
 
+// Limits of the certificate, with the list for the elements of which (0 or 1).
+CertifyArgs certify_args(const dgb_plan* p, int which) {
+  return CertifyArgs{p->lim.lebesgue, p->lim.density_floor, p->lim.pressure_floor, p->lim.relative_floor,
+                     p->cert_list + (size_t)which * p->dev.blk[0].E, p->cert_count + which};
+}
+
 // Positivity on the sum-factorised path: the certificate pre-pass (one warp per element) lists the
 // elements it cannot clear, and k_hex_positivity limits only those.
 template <int P, int NV>
@@ -717,33 +723,35 @@ int run_positivity_hex(dgb_plan* p, const StatePtrs& S, cudaStream_t st) {
   const size_t sm = sizeof(double) * (size_t)hex_positivity_smem<P, NV>();
   const BlockDev& B = p->dev.blk[0];
   if (B.E == 0) return DGB_OK;
+  const CertifyArgs C = certify_args(p, 0);
   CK(cudaMemsetAsync(p->cert_count, 0, sizeof(int), st));
-  k_certify<NV, HexDims<P>::N3><<<blocks_for(B.E, kThreads / 32), kThreads, 0, st>>>(
-      S.b[0], B.E, p->dev.ph, p->lim.lebesgue, p->lim.density_floor, p->lim.pressure_floor,
-      p->lim.relative_floor, p->cert_list, p->cert_count);
-  k_hex_positivity<P, NV><<<p->pos_grid, kThreads, sm, st>>>(p->dev, S, 0, p->hex_tables, p->lim, p->cert_list,
-                                                             p->cert_count);
+  k_certify<NV, HexDims<P>::N3><<<blocks_for(B.E, kThreads / 32), kThreads, 0, st>>>(S.b[0], B.E, p->dev.ph, C);
+  k_hex_positivity<P, NV><<<p->pos_grid, kThreads, sm, st>>>(p->dev, S, 0, p->hex_tables, p->lim, C.list, C.count);
   CK(cudaGetLastError());
   return DGB_OK;
 }
 
-// The stage blend dst = alpha * base + beta * x followed by positivity on the sum-factorised path,
-// with the blend fused into the certificate pre-pass.
+// Positivity of x, the stage blend dst = alpha * base + beta * x and positivity of dst, on the sum-factorised
+// path, with both certificate pre-passes in the blend.
 template <int P, int NV>
-int run_blend_positivity_hex(dgb_plan* p, const double* base, const double* x, double alpha, double beta, double* dst,
+int run_blend_positivity_hex(dgb_plan* p, const double* base, double* x, double alpha, double beta, double* dst,
                              cudaStream_t st) {
+  constexpr int N3 = HexDims<P>::N3, per = kThreads / 32;
   const BlockDev& B = p->dev.blk[0];
   if (B.E == 0) return DGB_OK;
-  CK(cudaMemsetAsync(p->cert_count, 0, sizeof(int), st));
-  k_blend_certify<NV, HexDims<P>::N3><<<blocks_for(B.E, kThreads / 32), kThreads, 0, st>>>(
-      base, x, alpha, beta, dst, B.E, p->dev.ph, p->lim.lebesgue, p->lim.density_floor, p->lim.pressure_floor,
-      p->lim.relative_floor, p->cert_list, p->cert_count);
-  StatePtrs S;
-  for (int b = 0; b < DGB_MAX_BLOCKS; ++b) S.b[b] = nullptr;
-  S.b[0] = dst;
   const size_t sm = sizeof(double) * (size_t)hex_positivity_smem<P, NV>();
-  k_hex_positivity<P, NV><<<p->pos_grid, kThreads, sm, st>>>(p->dev, S, 0, p->hex_tables, p->lim, p->cert_list,
-                                                             p->cert_count);
+  const CertifyArgs Cx = certify_args(p, 0), Co = certify_args(p, 1);
+  StatePtrs X, O;
+  for (int b = 0; b < DGB_MAX_BLOCKS; ++b) X.b[b] = O.b[b] = nullptr;
+  X.b[0] = x;
+  O.b[0] = dst;
+  const Physics& ph = p->dev.ph;
+  CK(cudaMemsetAsync(p->cert_count, 0, sizeof(int) * 2, st));
+  k_blend_certify<NV, N3, false><<<blocks_for(B.E, per), kThreads, 0, st>>>(base, x, alpha, beta, dst, B.E, ph, Cx, Co);
+  k_hex_positivity<P, NV><<<p->pos_grid, kThreads, sm, st>>>(p->dev, X, 0, p->hex_tables, p->lim, Cx.list, Cx.count);
+  k_blend_certify<NV, N3, true><<<std::min(blocks_for(B.E, per), 148 * 4), kThreads, 0, st>>>(base, x, alpha, beta, dst,
+                                                                                           B.E, ph, Cx, Co);
+  k_hex_positivity<P, NV><<<p->pos_grid, kThreads, sm, st>>>(p->dev, O, 0, p->hex_tables, p->lim, Co.list, Co.count);
   CK(cudaGetLastError());
   return DGB_OK;
 }
@@ -983,13 +991,13 @@ int run_step_mood(dgb_plan* p, const StatePtrs& U0, double dt, dgb_status* statu
     // the subcell update lands in place in the Euler candidate: elements that are neither
     // troubled nor corrected at a face keep theirs without a copy
     if ((rc = run_subcell<NV>(p, *cur[s], p->vis, dt, F, p->eul, st))) return rc;
-    if ((rc = run_positivity<NV>(p, EUL, st))) return rc;
     if (p->hex) {
       rc = p->dev.degree == 1 ? run_blend_positivity_hex<1, NV>(p, U0.b[0], p->eul[0], alphas[s], betas[s], dst[s]->b[0], st)
          : p->dev.degree == 2 ? run_blend_positivity_hex<2, NV>(p, U0.b[0], p->eul[0], alphas[s], betas[s], dst[s]->b[0], st)
                               : run_blend_positivity_hex<3, NV>(p, U0.b[0], p->eul[0], alphas[s], betas[s], dst[s]->b[0], st);
       if (rc) return rc;
     } else {
+      if ((rc = run_positivity<NV>(p, EUL, st))) return rc;
       for (int b = 0; b < P.nblocks; ++b) {
         const size_t n = (size_t)P.blk[b].E * P.blk[b].Np * NV;
         k_blend<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(U0.b[b], p->eul[b], alphas[s], betas[s], dst[s]->b[b], n);
@@ -1537,9 +1545,9 @@ int dgb_plan_finalize(dgb_plan* p) {
     }
   }
   if (p->hex && p->dev.blk[0].E > 0) {
-    CK(cudaMalloc(&p->cert_list, sizeof(int) * (size_t)p->dev.blk[0].E));
+    CK(cudaMalloc(&p->cert_list, sizeof(int) * 2 * (size_t)p->dev.blk[0].E));
     p->allocations.push_back(p->cert_list);
-    CK(cudaMalloc(&p->cert_count, sizeof(int)));
+    CK(cudaMalloc(&p->cert_count, sizeof(int) * 2));
     p->allocations.push_back(p->cert_count);
     const int deg = p->dev.degree;
     rc = NV == 5 ? (deg == 1 ? hex_positivity_grid<1, 5>(p) : deg == 2 ? hex_positivity_grid<2, 5>(p)

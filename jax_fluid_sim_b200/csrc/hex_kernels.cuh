@@ -1056,9 +1056,10 @@ __global__ void __launch_bounds__(kThreads) k_hex_positivity(const DevPlan P_, c
   // clear.  A cleared element keeps its state: its theta is 1, and the reference's
   // mean + 1 * (U - mean) equals U to rounding.  Each CTA loads the tables once and takes the
   // listed elements in a grid stride.
+  const int n = *count;
+  if ((int)blockIdx.x >= n) return;
   load_tables<P>(tables, tb);
   __syncthreads();
-  const int n = *count;
   for (int item = blockIdx.x; item < n; item += gridDim.x) {
     const int e = list[item];
     double* Ug = S.b[b] + (size_t)e * N3 * NV;
@@ -1150,9 +1151,10 @@ __global__ void __launch_bounds__(kThreads) k_hex_troubled(const DevPlan P_, con
   const BlockDev& B = P_.blk[b];
   // The elements are those of list[0, *count): the ones k_hex_sensor neither skipped (predicted)
   // nor certified.  Each CTA loads the tables once and takes the listed elements in a grid stride.
+  const int n = *count;
+  if ((int)blockIdx.x >= n) return;
   load_tables<P>(tables, tb);
   __syncthreads();
-  const int n = *count;
   for (int item = blockIdx.x; item < n; item += gridDim.x) {
     const int e = list[item];
     const double* Ug = S.b[b] + (size_t)e * N3 * NV;
@@ -1232,8 +1234,8 @@ __global__ void __launch_bounds__(kThreads) k_hex_troubled(const DevPlan P_, con
 // Troubled-cell pre-pass, one warp per element: predicted elements are flagged and skipped (as in
 // predicted_skip); an element whose nodal values certify admissible samples and mean
 // (certificate_from_range with the absolute floors) gets its sensor here (the same arithmetic and
-// summation order as k_hex_troubled: the P1 projection by the same pencils, the squares summed
-// per 32 nodes by the same shuffle tree) and its flag; every other element is appended to list
+// summation order as k_hex_troubled: the P1 projection one axis after the other, the squares summed
+// per 32 nodes by the same tree) and its flag; every other element is appended to list
 // for k_hex_troubled.  *count must be zero before the launch.
 template <int P, int NV>
 __global__ void __launch_bounds__(kThreads) k_hex_sensor(const DevPlan P_, const StatePtrs S, int b,
@@ -1242,10 +1244,16 @@ __global__ void __launch_bounds__(kThreads) k_hex_sensor(const DevPlan P_, const
                                                         int* __restrict__ list, int* __restrict__ count) {
   using D = HexDims<P>;
   constexpr int N = D::N, N3 = D::N3;
-  __shared__ double work[kThreads / 32][4 * 2 * N3];   // per warp: Mon, Low, t1, t2
+  constexpr int LD = N + 1 - N % 2, LS = N * N * LD;
+  __shared__ double work[kThreads / 32][2 * 2 * LS];   // per warp: Mon, Low
+  __shared__ int node2lex[N3];                         // (lane-indexed reads of the constant bank are one per lane)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int E = P_.blk[b].E;
   const int e = blockIdx.x * (kThreads / 32) + warp;
+  if (P >= 2) {
+    for (int l = threadIdx.x; l < N3; l += kThreads) node2lex[tables.lex2node[l]] = l;
+    __syncthreads();
+  }
   if (e >= E) return;
   if (pa.mode == 1 && pa.pred && pa.pred[e]) {
     if (lane == 0) {
@@ -1254,50 +1262,83 @@ __global__ void __launch_bounds__(kThreads) k_hex_sensor(const DevPlan P_, const
     }
     return;
   }
-  const double* Ug = S.b[b] + (size_t)e * N3 * NV;
-  double mn[5], mx[5];
-  const bool fin = warp_nodal_range<NV, N3>(Ug, mn, mx);
-  if (!(fin && certificate_from_range(mn, mx, P_.ph, Lc.lebesgue, Lc.density_floor, Lc.pressure_floor, 0.0))) {
+  WarpNodes<NV, N3> un;
+  un.load(S.b[b] + (size_t)e * N3 * NV);
+  if (!un.certified(P_.ph, Lc.lebesgue, Lc.density_floor, Lc.pressure_floor, 0.0)) {
     if (lane == 0) list[atomicAdd(count, 1)] = e;
     return;
   }
-  double* Mon = work[warp];
-  double* Low = Mon + 2 * N3;
-  double* t1 = Low + 2 * N3;
-  double* t2 = t1 + 2 * N3;
-  for (int l = lane; l < N3; l += 32) {
-    double u[NV], W[NV];
-#pragma unroll
-    for (int v = 0; v < NV; ++v) u[v] = Ug[tables.lex2node[l] * NV + v];
-    primitive<NV>(P_.ph, u, W);
-    Mon[l] = W[0];
-    Mon[N3 + l] = W[4];
-  }
-  __syncwarp();
   double value = 0.0;
   if (P >= 2) {
-    warp_tensor3<2, N>(Mon, Low, t1, t2, tables.p1d);
-    // squares of the nodes lane and lane + 32, each set reduced by the block kernel's tree
-    double h[2][4] = {};
+    // (rho, p) at the lexicographic place of each node; lines of N values LD apart, an odd number of values
+    double* Mon = work[warp];
+    double* Low = Mon + 2 * LS;
+#pragma unroll
+    for (int k = 0; k < WarpNodes<NV, N3>::K; ++k) {
+      const int i = k * 32 + lane;
+      if (i < N3) {
+        double W[NV];
+        primitive<NV>(P_.ph, un.u[k], W);
+        const int l = node2lex[i];
+        Mon[l / N * LD + l % N] = W[0];
+        Mon[LS + l / N * LD + l % N] = W[4];
+      }
+    }
+    __syncwarp();
+    // the P1 projection: one axis after the other, a line per lane, in place after the first
+    auto lines = [&](const double* in, int stride, auto&& first) {
+      for (int it = lane; it < 2 * N * N; it += 32) {
+        const int o = it / (N * N) * LS + first(it % (N * N) / N, it % N);
+        double x[N];
+#pragma unroll
+        for (int i = 0; i < N; ++i) x[i] = in[o + i * stride];
+#pragma unroll
+        for (int r = 0; r < N; ++r) {
+          double acc = 0.0;
+#pragma unroll
+          for (int i = 0; i < N; ++i) acc += tables.p1d[r * N + i] * x[i];
+          Low[o + r * stride] = acc;
+        }
+      }
+      __syncwarp();
+    };
+    lines(Mon, 1, [](int z, int y) { return (z * N + y) * LD; });
+    lines(Low, LD, [](int z, int x) { return z * N * LD + x; });
+    lines(Low, N * LD, [](int y, int x) { return y * LD + x; });
+    // squares of the nodes lane and lane + 32 (half), each of the eight sums by the block kernel's tree (lanes 16, 8, 4,
+    // 2, 1 apart); the first three levels halve the sums a lane carries, so 9 values are exchanged
+    // instead of 40.  h[k][half]: k = 0, 1 the differences of rho and p, 2, 3 the values
+    double h[4][2] = {};
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
       const int i = lane + 32 * half;
       if (i < N3) {
-        const double m0 = Mon[i], m1 = Mon[N3 + i];
-        const double d0 = m0 - Low[i], d1 = m1 - Low[N3 + i];
-        h[half][0] += d0 * d0;
-        h[half][1] += d1 * d1;
-        h[half][2] += m0 * m0;
-        h[half][3] += m1 * m1;
+        const int j = i / N * LD + i % N;
+        const double m0 = Mon[j], m1 = Mon[LS + j];
+        const double d0 = m0 - Low[j], d1 = m1 - Low[LS + j];
+        h[0][half] = d0 * d0;
+        h[1][half] = d1 * d1;
+        h[2][half] = m0 * m0;
+        h[3][half] = m1 * m1;
       }
-#pragma unroll
-      for (int k = 0; k < 4; ++k)
-        for (int o = 16; o > 0; o >>= 1) h[half][k] += __shfl_xor_sync(0xffffffff, h[half][k], o);
     }
-    double t[4];
+    const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
+    double g[2][2], f[2];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) t[k] = ((0.0 + h[0][k]) + h[1][k]);
-    const double r0 = t[0] / fmax(t[2], 1.0e-12), r1 = t[1] / fmax(t[3], 1.0e-12);
+    for (int k = 0; k < 2; ++k)
+#pragma unroll
+      for (int half = 0; half < 2; ++half)
+        g[k][half] = (b4 ? h[k + 2][half] : h[k][half]) +
+                     __shfl_xor_sync(0xffffffff, b4 ? h[k][half] : h[k + 2][half], 16);
+#pragma unroll
+    for (int half = 0; half < 2; ++half)
+      f[half] = (b3 ? g[1][half] : g[0][half]) + __shfl_xor_sync(0xffffffff, b3 ? g[0][half] : g[1][half], 8);
+    double s = (b2 ? f[1] : f[0]) + __shfl_xor_sync(0xffffffff, b2 ? f[0] : f[1], 4);
+    s += __shfl_xor_sync(0xffffffff, s, 2);
+    s += __shfl_xor_sync(0xffffffff, s, 1);
+    const double t = s + __shfl_xor_sync(0xffffffff, s, 4);        // both halves: sum of quantity 2 b4 + b3
+    const double r0 = t / fmax(__shfl_xor_sync(0xffffffff, t, 16), 1.0e-12);   // in lanes with b4 = 0
+    const double r1 = __shfl_xor_sync(0xffffffff, r0, 8);
     value = (isnan(r0) || isnan(r1)) ? NAN : fmax(r0, r1);
   }
   if (lane == 0) {
