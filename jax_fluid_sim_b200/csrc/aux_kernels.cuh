@@ -234,6 +234,16 @@ __global__ void __launch_bounds__(kThreads) k_blend_certify(const double* base, 
   }
 }
 
+// BlockDev::elem_code from the faces' records (set-up).
+static __global__ void k_elem_codes(const DevPlan P, int b, uint8_t* __restrict__ out) {
+  const BlockDev& B = P.blk[b];
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= (long long)B.E * B.nlf) return;
+  int ft, f, side;
+  decode_face(B.elem_face[t], ft, f, side);
+  out[t] = (uint8_t)(side == 0 ? P.face[ft].oc[f] : P.face[ft].nc[f]);
+}
+
 // samples = [U at nodes; B U at volume points; Bfs U at face points]  -> S[Ns_total][NV]
 template <int NV>
 __device__ void build_samples(const BlockDev& B, const double* U, double* S) {

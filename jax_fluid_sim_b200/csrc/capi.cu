@@ -1549,6 +1549,15 @@ int dgb_plan_finalize(dgb_plan* p) {
     p->allocations.push_back(p->cert_list);
     CK(cudaMalloc(&p->cert_count, sizeof(int) * 2));
     p->allocations.push_back(p->cert_count);
+    if (p->face_present[1]) {
+      const size_t n = (size_t)p->dev.blk[0].E * p->dev.blk[0].nlf;
+      uint8_t* codes = nullptr;
+      CK(cudaMalloc(&codes, n));
+      p->allocations.push_back(codes);
+      k_elem_codes<<<blocks_for((long)n, kThreads), kThreads>>>(p->dev, 0, codes);
+      CK(cudaGetLastError());
+      p->dev.blk[0].elem_code = codes;
+    }
     const int deg = p->dev.degree;
     rc = NV == 5 ? (deg == 1 ? hex_positivity_grid<1, 5>(p) : deg == 2 ? hex_positivity_grid<2, 5>(p)
                                                               : hex_positivity_grid<3, 5>(p))

@@ -40,6 +40,7 @@ struct BlockDev {
   const double* fsB;      // [Ns][Np]
   const double* p1proj;   // [Np][Np]
   const int32_t* elem_face;  // [E][nlf]
+  const uint8_t* elem_code;  // [E][nlf] orientation code of each face on this element's side (hexahedron plans)
   const double* trB[2];   // per face type: [codes][nq][Np]
   const double* trdB[2];  // per face type: [codes][nq][Np][3]
   // the same tables laid out so that the thread index runs along the fastest axis (coalesced):

@@ -401,7 +401,7 @@ __device__ __forceinline__ void hex_element(const DevPlan& P_, const StatePtrs& 
     int ft, f, side;
     decode_face(B.elem_face[e * 6 + threadIdx.x], ft, f, side);
     fslot[threadIdx.x] = (f * 2 + side) * QF2;
-    fperm[threadIdx.x] = (side == 0 ? fd.oc[f] : fd.nc[f]) * QF2;
+    fperm[threadIdx.x] = B.elem_code[e * 6 + threadIdx.x] * QF2;
     fface[threadIdx.x] = (f << 1) | side;
   }
   for (int l = threadIdx.x; l < N3; l += NT) {
@@ -410,6 +410,25 @@ __device__ __forceinline__ void hex_element(const DevPlan& P_, const StatePtrs& 
     node2lex[node] = l;
   }
   __syncthreads();
+  // what the element reads later, on its way to L2: the faces' jumps and fluxes and the stage's base
+  for (int it = threadIdx.x; it < 6 * 3; it += NT) {
+    const int lf = it % 6, f = fface[lf] >> 1;
+    constexpr int fb = QF2 * (int)sizeof(R);
+    const char* p;
+    int bytes = NV * fb;
+    if (it < 6) {
+      p = (const char*)(sizeof(R) == 4 ? (const void*)fd.fluxI32 : (const void*)fd.fluxI) + (size_t)fslot[lf] * NV * sizeof(R);
+    } else if (!P_.viscous) {
+      break;
+    } else if (it < 12) {
+      p = (const char*)(sizeof(R) == 4 ? (const void*)fd.jumpW32 : (const void*)fd.jumpW) + (size_t)f * 12 * fb;
+      bytes = 12 * fb;
+    } else {
+      p = (const char*)(sizeof(R) == 4 ? (const void*)fd.fluxV32 : (const void*)fd.fluxV) + (size_t)f * NV * fb;
+    }
+    for (int o = 0; o < bytes; o += 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + o));
+  }
+  if (A.stage) prefetch_l2<NT>(A.base[b] + (size_t)e * N3 * NV, N3 * NV * 8);
   if (threadIdx.x < NV) anchor[threadIdx.x] = (R)raw[threadIdx.x];
   if (threadIdx.x == 0)
 #pragma unroll
@@ -423,15 +442,11 @@ __device__ __forceinline__ void hex_element(const DevPlan& P_, const StatePtrs& 
   const float* MT32 = (sizeof(R) == sizeof(float) && B.minv32) ? B.minv32 + (size_t)e * N3 * N3 : nullptr;
   if (!aff) {
     // the element's M^-1, inverse Jacobians and w|det J| on their way to L2 while the nodal work runs
-    auto prefetch = [&](const void* p, int bytes) {
-      for (int o = threadIdx.x * 128; o < bytes; o += NT * 128)
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const char*>(p) + o));
-    };
-    if (MT32) prefetch(MT32, N3 * N3 * 4);
-    else prefetch(MT, N3 * N3 * 8);
-    if (sizeof(R) == sizeof(float) && B.jinv32) prefetch(B.jinv32 + (size_t)e * Q3 * 9, Q3 * 9 * 4);
-    else prefetch(B.jinv + (size_t)e * Q3 * 9, Q3 * 9 * 8);
-    prefetch(B.wdet + (size_t)e * Q3, Q3 * 8);
+    if (MT32) prefetch_l2<NT>(MT32, N3 * N3 * 4);
+    else prefetch_l2<NT>(MT, N3 * N3 * 8);
+    if (sizeof(R) == sizeof(float) && B.jinv32) prefetch_l2<NT>(B.jinv32 + (size_t)e * Q3 * 9, Q3 * 9 * 4);
+    else prefetch_l2<NT>(B.jinv + (size_t)e * Q3 * 9, Q3 * 9 * 8);
+    prefetch_l2<NT>(B.wdet + (size_t)e * Q3, Q3 * 8);
   }
   for (int l = threadIdx.x; l < N3; l += NT) {
     const double* un = raw + lex2node[l] * NV;
@@ -817,6 +832,7 @@ template <int P, int NV, bool SPLIT, typename R>
 __global__ void __launch_bounds__(HexDims<P>::NTE, hex_element_ctas<P, NV, SPLIT, R>())
     k_hex_element(const __grid_constant__ DevPlan P_, const StatePtrs S, const __grid_constant__ HexTablesT<R> tables,
                   const HexCodes codes, const __grid_constant__ FinalizeArgs A) {
+  prefetch_ahead<P, NV, HexDims<P>::NTE>(P_.blk[0], S.b[0]);
   if (A.skip && A.skip[blockIdx.x]) return;     // uniform across the CTA
   hex_element<P, NV, SPLIT, R>(P_, S, tables, codes, A, blockIdx.x);
 }
