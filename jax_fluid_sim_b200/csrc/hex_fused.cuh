@@ -368,6 +368,53 @@ struct HexElemSmem {
   static constexpr int TOTAL = up4(cmax(cmax(B_END, T_END), cmax(G_END, D_END)));
 };
 
+// Sums over the faces of each node: put(c, l, first(c, l) + sum of fv[lf][c][node's place on lf]) for C channels.
+// N = 4: a value per step, its node and places by shifts and masks.  Else a thread keeps one node, whose (at most
+// three) places are found once for its channels: with 3 nodes a side the index arithmetic of every value made the
+// two sums 15 % of the element kernel.  P2 element kernel, a stage: 4k elements 44.2 -> 41.9 us, 13k non-affine
+// 132.6 -> 129.2, 7k with 16 variables 238 -> 229; P3 that way 3,352 -> 3,376 us (202k, mixed), so N = 4 keeps its own.
+template <int N, int C, int FP, int NT, typename R, typename Put, typename First>
+__device__ __forceinline__ void node_faces(const R* fv, Put put, First first) {
+  constexpr int N2 = N * N, N3 = N2 * N, PAD = N == 2 ? 8 : 32;
+  constexpr int G = NT / PAD < 1 ? 1 : NT / PAD > C ? C : NT / PAD, CG = (C + G - 1) / G;      // channels: G groups of CG
+  if constexpr (N == 4) {
+    for (int idx = threadIdx.x; idx < C * N3; idx += NT) {
+      const int c = idx / N3, l = idx % N3;
+      const int xyz[3] = {l % N, (l / N) % N, l / N2};
+      R acc = first(c, l);
+#pragma unroll
+      for (int lf = 0; lf < 6; ++lf) {
+        int a0, end, a1, a2;
+        hex_face_axes(lf, a0, end, a1, a2);
+        if (xyz[a0] == end) acc += fv[(lf * C + c) * FP + xyz[a2] * N + xyz[a1]];
+      }
+      put(c, l, acc);
+    }
+    return;
+  }
+  for (int t = threadIdx.x; t < PAD * G; t += NT) {
+    const int l = t % PAD, c0 = t / PAD * CG;
+    if (l >= N3) continue;
+    const int xyz[3] = {l % N, (l / N) % N, l / N2};
+    int at[6];
+#pragma unroll
+    for (int lf = 0; lf < 6; ++lf) {
+      int a0, end, a1, a2;
+      hex_face_axes(lf, a0, end, a1, a2);
+      at[lf] = xyz[a0] == end ? (lf * C + c0) * FP + xyz[a2] * N + xyz[a1] : -1;
+    }
+#pragma unroll
+    for (int k = 0; k < CG; ++k) {
+      if (C % G != 0 && c0 + k >= C) break;
+      R acc = first(c0 + k, l);
+#pragma unroll
+      for (int lf = 0; lf < 6; ++lf)
+        if (at[lf] >= 0) acc += fv[at[lf] + k * FP];
+      put(c0 + k, l, acc);
+    }
+  }
+}
+
 // Lift + volume + finalize of hexahedron e by one CTA (see the file comment).  SPLIT keeps the inviscid
 // and viscous residuals apart (right-hand-side outputs, the MOOD step's viscous residual).
 template <int P, int NV, bool SPLIT, typename R>
@@ -483,20 +530,11 @@ __device__ __forceinline__ void hex_element(const DevPlan& P_, const StatePtrs& 
     __syncthreads();
     planes<QF, N, FP, FP, NT>(jc, jc, 72, tables.bfT, tables.bfT, threadIdx.x);
     __syncthreads();
-    for (int idx = threadIdx.x; idx < 12 * N3; idx += NT) {
-      const int c = idx / N3, l = idx % N3;
-      const int xyz[3] = {l % N, (l / N) % N, l / N2};
-      R acc = R(0);
-#pragma unroll
-      for (int lf = 0; lf < 6; ++lf) {
-        int a0, end, a1, a2;
-        hex_face_axes(lf, a0, end, a1, a2);
-        if (xyz[a0] == end) acc += jc[(lf * 12 + c) * FP + xyz[a2] * N + xyz[a1]];
-      }
-      // non-affine elements: rows of two 16-byte aligned groups of 6 channels (LR apart) in element
-      // node order, for 16-byte loads in the dense M^-1 (summed in node order)
+    // non-affine elements: rows of two 16-byte aligned groups of 6 channels (LR apart) in element
+    // node order, for 16-byte loads in the dense M^-1 (summed in node order)
+    node_faces<N, 12, FP, NT>(jc, [&](int c, int l, R acc) {
       ball[aff ? c * NS + nod(l) : lex2node[l] * 2 * LR + (c / 6) * LR + c % 6] = acc;
-    }
+    }, [](int, int) { return R(0); });
     __syncthreads();
     if (aff) {
       planes<N, N, PS, PS, NT>(ball, ball, 12 * N, tables.m1i, tables.m1i, threadIdx.x);
@@ -720,21 +758,12 @@ __device__ __forceinline__ void hex_element(const DevPlan& P_, const StatePtrs& 
   // dense M^-1
   constexpr int CSH = L::CSH, CS = L::CS;
   R* RrT = smem + L::RT;
-  for (int idx = threadIdx.x; idx < C * N3; idx += NT) {
-    const int c = idx / N3, l = idx % N3;
-    const int xyz[3] = {l % N, (l / N) % N, l / N2};
-    R acc = Rr[c * NS + nod(l)];
-#pragma unroll
-    for (int lf = 0; lf < 6; ++lf) {
-      int a0, end, a1, a2;
-      hex_face_axes(lf, a0, end, a1, a2);
-      if (xyz[a0] == end) acc += hc[(lf * C + c) * FP + xyz[a2] * N + xyz[a1]];
-    }
+  node_faces<N, C, FP, NT>(hc, [&](int c, int l, R acc) {
     if (aff)
       Rr[c * NS + nod(l)] = acc;
     else
       RrT[lex2node[l] * CS + (c < NV ? c : CSH + c - NV)] = acc;
-  }
+  }, [&](int c, int l) { return Rr[c * NS + nod(l)]; });
   __syncthreads();
   // values idx (node-major, as in memory) of the residuals, inviscid and viscous: coalesced stores
   auto emit = [&](const R* inv, const R* vis, R cf) {
