@@ -440,16 +440,15 @@ def run_ours(args):
         per_stage = 2 * nb + nf                    # traces, face kernel, element kernel
     else:
         per_stage = nb * (4 if (op.native.sum_factorised and op.viscous) else 3) + nf * (2 if op.viscous else 1)
+    hexes = op.native.sum_factorised
     if args.limiter == "mood":
-        per_stage += nb * 6 + nf + nb + 1
+        # detector (with its pre-pass on hexahedra), screen, subcell values, faces and update, the flagged elements'
+        # viscous residual, two positivity passes, the blend (hexahedra: before and after the first of them), reduction
+        per_stage += nb * (2 if hexes else 1) + 4 + (1 if fused and op.viscous else 0) + nb * 2 + nb * (2 if hexes else 1) + 1
         if learned_head:
             per_stage += 3 * nb
     else:
-        per_stage += nb * 2 + 1
-    if op.native.sum_factorised:
-        # the certificate pre-pass before each positivity pass (two per stage with MOOD) and the
-        # sensor pre-pass before the troubled-cell test (MOOD)
-        per_stage += 3 if args.limiter == "mood" else 1
+        per_stage += nb * (2 if hexes else 1) + 1      # positivity (with its certificate pre-pass), reduction
     lim = "MOOD subcell FV (CWENO-Z) + positivity" if args.limiter == "mood" else "positivity limiter"
     prec = ("mixed: float32 arithmetic in the traces, BR2-lift, volume and finalize kernels; float64 state, "
             "face fluxes, limiters and reductions" if head_prec == "mixed" else "plain float64")

@@ -262,8 +262,9 @@ int dgb_wall_forces(dgb_plan* plan, const dgb_state* U, const int32_t* wall_tags
  * launches on state U for each block's threads-per-element width in {16, 32, 64, 128} (best of
  * `reps` runs, one coordinate sweep) and keeps the fastest in the plan.  widths (optional,
  * [3][DGB_MAX_BLOCKS]) receives the choice per kernel (trace, volume, finalize) and block; all
- * zeros on the sum-factorised hexahedron path, whose launches are fixed.  Synchronises the
- * stream. */
+ * zeros on the sum-factorised hexahedron path, whose launches are fixed.  Inviscid plans on the two-launch
+ * dense form have fixed launches too: widths receives the general kernels' defaults, nothing is timed.
+ * Synchronises the stream. */
 int dgb_plan_autotune(dgb_plan* plan, const dgb_state* U, int reps, int* widths, void* stream);
 /* Execution form of the sum-factorised hexahedron right-hand side (no reference counterpart; the
  * results agree to round-off): enable = 1 (the default) runs it as three launches, the traces,

@@ -1,4 +1,5 @@
-// DG residual-and-update kernels for any element type (hexahedron, wedge, tetrahedron; P1-P3).
+// DG residual-and-update kernels for any element type (hexahedron, wedge, tetrahedron; P1-P3): the general form,
+// for split residuals, 16 variables and mixed viscous plans; dense_rhs.cu has the two-launch form of the rest.
 //
 // Pipeline of one right-hand-side evaluation (reference: hybrid/spatial.py:137-249 and
 // hybrid/navier_stokes.py:27-347):

@@ -1,7 +1,7 @@
 // Fused right-hand side of the sum-factorised hexahedron path: three launches per evaluation
 // instead of six.
 //
-//   k_hex_traces   (hex_kernels.cuh, unchanged): face traces of U, of the viscous variables and of
+//   k_hex_traces   (hex_kernels.cuh): face traces of U, of the viscous variables and of
 //                  their raw gradients, per face side.
 //   k_hex_face     one thread per face point, the points of a face in consecutive threads:
 //                  HLLC (or the boundary ghost) minus each side's anchor flux, the BR2 jump,
@@ -12,12 +12,12 @@
 //                  with K = bf m1i bf^T, otherwise a QF^2 x QF^2 operator per element face built
 //                  once from M^-1 (k_hex_lop).  This replaces k_face_flux, the per-face part of
 //                  k_hex_lift and k_face_visc, and the traces are read once.
-//   k_hex_element  one CTA per element: the nodal lift M^-1 sum_f B_f^T jump_f, the volume terms
+//   k_hex_element  one CTA per element (128 threads; one warp at P2): the nodal lift M^-1 sum_f B_f^T jump_f, the volume terms
 //                  (U, grad v and lift at the volume points; inviscid and viscous fluxes), the face
 //                  terms and M^-1 with the stage update.  The lift and the residuals stay in shared
 //                  memory (no nodal-lift or residual buffers in HBM); M^-1 is read by the lift and
 //                  by the final product.
-// Arithmetic and summation order inside each phase are those of the unfused kernels; the local
+// Summation order inside each phase is that of the six-launch kernels; the local
 // lift is summed as one operator instead of three factors, which moves results by round-off.
 #pragma once
 #include "hex_kernels.cuh"

@@ -342,7 +342,8 @@ class HybridEulerOperator:
     def autotune(self, states, boundary_state=None, reps=3):
         """Pick the threads-per-element width of the dense kernels by timing them on ``states``
         (dgb_plan_autotune); returns {kernel: {element_type: width}} (empty on the
-        sum-factorised hexahedron path, whose launches are fixed)."""
+        sum-factorised hexahedron path, whose launches are fixed; the default widths, untimed, where the
+        two-launch form of the dense path runs, csrc/dense_rhs.cu)."""
         U = self.to_device(states)
         self.native.set_boundary(boundary_state)
         widths = np.zeros(3 * N.MAX_BLOCKS, np.int32)
