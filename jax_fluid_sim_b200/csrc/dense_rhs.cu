@@ -19,6 +19,8 @@
 // NV variables of one point while it interpolates, IB nodes x EB2 elements x NV variables of one chunk
 // of points while it sums the residual, with 16-byte shared-memory loads; a table value from L1/L2 then
 // serves EB * NV products instead of NV.  NE is chosen so that both phases fill kThreads.
+// Checked Euler steps of hybrid boxes, general kernels against these two: 16^3 P3 1860 -> 950 us, 32^3 P1
+// 1308 -> 496 us, 23^3 P2 mixed 2776 -> 1436 us.
 // Sums run in the order of the one-value-per-thread form: per output the nodes (points) ascend, and
 // the residual is summed per chunk of points, then over the chunks.
 #include "dense_rhs.h"
