@@ -227,7 +227,7 @@ __device__ __forceinline__ void prefetch_ahead(const BlockDev& B, const double* 
 //    lanes on consecutive planes then fall on distinct banks, with 16-byte accesses; planes of 25 and 9 values
 //    are odd as they are.
 // Per value the sums are those of the pencil form.  P3 element kernel, per element: 8,626 wavefronts with
-// pencil passes and 5,976 with the matrices and paddings alone (float64), 2,690 with the planes in float32.
+// pencil passes, 5,976 with the matrices and paddings alone, 4,117 now (float64; 2,690 in float32).
 template <typename T>
 __host__ __device__ constexpr int plane_stride(int n) { return n == 16 ? (sizeof(T) == 8 ? 18 : 20) : n; }
 
