@@ -560,7 +560,7 @@ int run_rhs_dense(dgb_plan* p, const StatePtrs& S, const FinalizeArgs& A, cudaSt
     auto record = [&](int k) { return ev ? cudaEventRecord(ev[k], st) : cudaSuccess; };
     CK(record(0));
     CK(record(1));                             // the face kernel forms the traces itself
-    CK(dense_face_flux(P, S, p->dense, f32, p->prm.limiter == 2, st));
+    CK(dense_face_flux(P, S, p->dense, f32, A.traces != 0, st));
     CK(record(2));
     CK(record(3));
     for (int b = 0; b < P.nblocks; ++b)
@@ -968,6 +968,7 @@ int run_step_mood(dgb_plan* p, const StatePtrs& U0, double dt, dgb_status* statu
     FinalizeArgs A;
     memset(&A, 0, sizeof(A));
     A.stage = 1;
+    A.traces = 1;                      // k_mood_faces
     A.alpha = alphas[s];
     A.beta = betas[s];
     A.dt = dt;
@@ -1805,6 +1806,7 @@ int dgb_wall_forces(dgb_plan* p, const dgb_state* U, const int32_t* wall_tags, i
   // the face buffers of one right-hand-side evaluation (traces, gradients, BR2 lifts)
   FinalizeArgs A;
   memset(&A, 0, sizeof(A));
+  A.traces = 1;
   const StatePtrs S = to_ptrs(U);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   p->f32_traces = false;

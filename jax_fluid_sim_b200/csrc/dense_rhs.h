@@ -35,7 +35,7 @@ struct DenseShape {
 DenseShape dense_shape(int P, int type);
 
 // rhs of S with the stage update or outputs of A.  store_traces: also write the face traces (the MOOD
-// face kernel reads them).  volume_done[b]: block b's volume residual is already in Rinv.
+// face kernel and the wall forces read them).  volume_done[b]: block b's volume residual is already in Rinv.
 cudaError_t dense_face_flux(const DevPlan& P, const StatePtrs& S, const DenseTables& T, bool f32, bool store_traces,
                             cudaStream_t st);
 cudaError_t dense_update(const DevPlan& P, const StatePtrs& S, const FinalizeArgs& A, const DenseTables& T, bool f32,

@@ -665,6 +665,8 @@ static __global__ void k_wall_forces_final(const double* __restrict__ partials, 
 struct FinalizeArgs {
   double* out_inv[DGB_MAX_BLOCKS];   // rhs outputs (may be null)
   int total;                         // out_inv takes the whole residual, formed as one (no stage, no out_vis)
+  int traces;                        // the caller reads FaceDev::trA afterwards (wall forces, subcell faces): the two-launch
+                                     // dense form, which needs no trace buffer itself, writes it too
   double* out_vis[DGB_MAX_BLOCKS];
   // fused SSP-RK stage: dst = alpha*base + beta*(cur + dt*(rhs_inv + rhs_vis)); euler = cur + dt*rhs
   int stage;
