@@ -398,7 +398,8 @@ int dgb_plan_match_subcell_faces(dgb_plan* plan, int face_type, const int32_t* o
 
 /* HybridSubcellFV.recompute (hybrid/subcell.py:855-950): base state, Euler DG candidate,
  * dt, optional additional rhs (viscous, projected onto the subcells) and troubled flags
- * [E_b] per block (device uint8) -> out (device state).  No positivity limiting. */
+ * [E_b] per block (device uint8) -> out (device state).  No positivity limiting.  out may be the buffers
+ * of base, of the candidate or of additional_rhs (block by block). */
 int dgb_subcell_recompute(dgb_plan* plan, const dgb_state* base, const dgb_state* candidate, double dt,
                           const dgb_state* additional_rhs, uint8_t* const* troubled, const dgb_state* out,
                           void* stream);

@@ -858,8 +858,6 @@ FlagPtrs flag_ptrs(uint8_t* const* f) {
   return out;
 }
 
-// Subcell recompute of the candidate `cand` from the base `cur` (traces of `cur` must be in
-// the face buffers): writes `out`.
 // Lists the troubled elements, the active faces and the elements on them.
 int run_mood_screen(dgb_plan* p, const FlagPtrs& F, cudaStream_t st) {
   const int faces = p->dev.face[0].F + p->dev.face[1].F;
@@ -870,34 +868,41 @@ int run_mood_screen(dgb_plan* p, const FlagPtrs& F, cudaStream_t st) {
   return DGB_OK;
 }
 
-// The subcell recompute of the listed elements, in place on out (the candidate); after run_mood_screen.
+// Subcell recompute of the candidate `cand` from the base `cur` into `out`, after run_mood_screen and with the
+// traces of `cur` in the face buffers.  In place (out is cand) only the listed elements are written; else every
+// element is, and out may be cur's buffer or visc's.
 template <int NV>
-int run_subcell(dgb_plan* p, const StatePtrs& cur, double* const* visc, double dt, const FlagPtrs& F, double* const* out,
-                cudaStream_t st) {
+int run_subcell(dgb_plan* p, const StatePtrs& cur, double* const* cand, double* const* visc, double dt,
+                const FlagPtrs& F, double* const* out, cudaStream_t st) {
   const DevPlan& P = p->dev;
   MoodDev M = p->mood;
   M.recon = p->prm.reconstruction;
-  StatePtrs vis, dst;
+  StatePtrs vis, src, dst;
+  bool in_place = true;
   long elements = 0, faces = (long)P.face[0].F + P.face[1].F;
   size_t sm_fv = 0, sm_up = 0;
   for (int b = 0; b < DGB_MAX_BLOCKS; ++b) {
     vis.b[b] = visc ? visc[b] : nullptr;
+    src.b[b] = cand[b];
     dst.b[b] = out[b];
     if (b >= P.nblocks) continue;
+    in_place &= P.blk[b].E == 0 || cand[b] == out[b];
     const SubcellBlockDev& C = M.blk[b];
     elements += P.blk[b].E;
     sm_fv = std::max(sm_fv, sizeof(double) * (size_t)mood_fv_smem(NV, P.blk[b].Np, C.S, C.NI));
     sm_up = std::max(sm_up, sizeof(double) * (size_t)mood_update_smem(NV, P.blk[b].Np, C.S));
   }
-  if (elements == 0 || faces == 0) return DGB_OK;
+  if (elements == 0) return DGB_OK;
   int rc;
   // about one resident wave of CTAs each
   const int most = (int)std::min(elements, 148L * 6);
   if ((rc = prepare(k_mood_fv<NV>, sm_fv))) return rc;
   k_mood_fv<NV><<<most, kThreads, sm_fv, st>>>(P, M, cur, p->mood_lists);
-  k_mood_faces<NV><<<std::min(blocks_for(faces, kThreads / 32), 148 * 8), kThreads, 0, st>>>(P, M, cur, F, p->mood_lists);
+  if (faces > 0)
+    k_mood_faces<NV><<<std::min(blocks_for(faces, kThreads / 32), 148 * 8), kThreads, 0, st>>>(P, M, cur, F, p->mood_lists);
   if ((rc = prepare(k_mood_update<NV>, sm_up))) return rc;
-  k_mood_update<NV><<<most, kThreads, sm_up, st>>>(P, M, F, vis, dt, dst, p->mood_lists);
+  k_mood_update<NV><<<most, kThreads, sm_up, st>>>(P, M, F, vis, dt, src, dst, p->mood_lists,
+                                                   in_place ? 0u : (unsigned)elements);
   CK(cudaGetLastError());
   return DGB_OK;
 }
@@ -991,7 +996,7 @@ int run_step_mood(dgb_plan* p, const StatePtrs& U0, double dt, dgb_status* statu
     if (vis_after && (rc = run_viscous_flagged<NV>(p, *cur[s], st))) return rc;
     // the subcell update lands in place in the Euler candidate: elements that are neither
     // troubled nor corrected at a face keep theirs without a copy
-    if ((rc = run_subcell<NV>(p, *cur[s], p->vis, dt, F, p->eul, st))) return rc;
+    if ((rc = run_subcell<NV>(p, *cur[s], p->eul, p->vis, dt, F, p->eul, st))) return rc;
     if (p->hex) {
       rc = p->dev.degree == 1 ? run_blend_positivity_hex<1, NV>(p, U0.b[0], p->eul[0], alphas[s], betas[s], dst[s]->b[0], st)
          : p->dev.degree == 2 ? run_blend_positivity_hex<2, NV>(p, U0.b[0], p->eul[0], alphas[s], betas[s], dst[s]->b[0], st)
@@ -1110,14 +1115,10 @@ int run_subcell_api(dgb_plan* p, const dgb_state* base, const dgb_state* cand, d
   double* visp[DGB_MAX_BLOCKS] = {arhs ? arhs->block[0] : nullptr, arhs ? arhs->block[1] : nullptr,
                                   arhs ? arhs->block[2] : nullptr};
   double* outp[DGB_MAX_BLOCKS] = {out->block[0], out->block[1], out->block[2]};
-  // the update is in place on the candidate's copy
-  for (int b = 0; b < P.nblocks; ++b)
-    if (P.blk[b].E > 0 && cand->block[b] != out->block[b])
-      CK(cudaMemcpyAsync(out->block[b], cand->block[b], sizeof(double) * (size_t)P.blk[b].E * P.blk[b].Np * NV,
-                         cudaMemcpyDeviceToDevice, st));
+  double* candp[DGB_MAX_BLOCKS] = {cand->block[0], cand->block[1], cand->block[2]};
   const FlagPtrs F = flag_ptrs(troubled);
   if ((rc = run_mood_screen(p, F, st))) return rc;
-  return run_subcell<NV>(p, S, arhs ? visp : nullptr, dt, F, outp, st);
+  return run_subcell<NV>(p, S, candp, arhs ? visp : nullptr, dt, F, outp, st);
 }
 
 }  // namespace

@@ -13,9 +13,10 @@
 //                  DG-FV coupling subfaces (FV mean on a troubled side, DG value at the
 //                  subface centre otherwise), lanes 16-31 the DG face flux integrated with
 //                  the face rule; stores subface fluxes and (new - old) face flux.
-//   k_mood_update  listed elements, in place.  Troubled: subface fluxes added in local-face order,
+//   k_mood_update  listed elements.  Troubled: subface fluxes added in local-face order,
 //                  FV update (+ projected viscous rhs), bound-limited reconstruction to DG; others:
-//                  the conservative correction from active faces on which they are not troubled.
+//                  the candidate plus the conservative correction from active faces on which they are not
+//                  troubled.  In place on the candidate, or out of place over every element.
 // The lists hold every block's elements (and both face types), so each kernel is one launch whose CTAs
 // take entries in turn.  Before, every kernel was a launch per block with a CTA per element, which on a
 // shocked flow of 202,752 hexahedra (1 % of them troubled) left 99 % of the CTAs to start and return:
@@ -376,23 +377,33 @@ __global__ void __launch_bounds__(kThreads) k_mood_faces(const DevPlan P, const 
 // projection and later its reconstruction rows.
 __host__ __device__ inline int mood_update_smem(int NV, int Np, int S) { return 2 * S * NV + Np * NV + S * Np; }
 
-// The touched elements of out (the candidate): troubled ? bound-limited reconstruction of the FV update :
-// candidate + corrections.
+// out = troubled ? bound-limited reconstruction of the FV update : candidate + corrections.  all = 0: the touched
+// elements, in place (out is the candidate); else every one of the `all` elements.  This kernel is the first to write
+// out, an element once what it reads of that element has been read, so out may also be the base state or visc.
 template <int NV>
 __global__ void __launch_bounds__(kThreads) k_mood_update(const DevPlan P, const MoodDev M, const FlagPtrs Fl,
-                                                         const StatePtrs visc, double dt, const StatePtrs out_,
-                                                         const MoodLists L) {
+                                                         const StatePtrs visc, double dt, const StatePtrs cand_,
+                                                         const StatePtrs out_, const MoodLists L, unsigned all) {
   extern __shared__ double smem[];
   __shared__ double vtot, corr[DGB_MAX_VARS];
-  const unsigned n = L.count[kMoodTouched];
+  const unsigned n = all ? all : L.count[kMoodTouched];
   for (unsigned item = blockIdx.x; item < n; item += gridDim.x) {
-    const int b = L.touched[item] >> 28, e = L.touched[item] & 0xfffffffu;
+    int b = 0, e = (int)item;
+    if (all)
+      for (; e >= P.blk[b].E; ++b) e -= P.blk[b].E;
+    else
+      b = L.touched[item] >> 28, e = L.touched[item] & 0xfffffffu;
     const BlockDev& B = P.blk[b];
     const SubcellBlockDev& C = M.blk[b];
     const int Np = B.Np, Sn = C.S;
     const size_t base = (size_t)e * Np * NV;
     const double* vol = C.vol + (size_t)e * Sn;
+    const double* cand = cand_.b[b];
     double* out = out_.b[b];
+    if (all && !L.mark[b][e]) {
+      for (int idx = threadIdx.x; idx < Np * NV; idx += kThreads) out[base + idx] = cand[base + idx];
+      continue;
+    }
     if (!Fl.f[b][e]) {
       // conservative correction from the active faces, in local-face order
       if (threadIdx.x == 0) {
@@ -413,7 +424,7 @@ __global__ void __launch_bounds__(kThreads) k_mood_update(const DevPlan P, const
         corr[threadIdx.x] = c;
       }
       __syncthreads();
-      for (int idx = threadIdx.x; idx < Np * NV; idx += kThreads) out[base + idx] = out[base + idx] + corr[idx % NV];
+      for (int idx = threadIdx.x; idx < Np * NV; idx += kThreads) out[base + idx] = cand[base + idx] + corr[idx % NV];
       __syncthreads();
       continue;
     }
