@@ -507,11 +507,18 @@ struct Partial {
 // every CTA leaves a partial, and the one that finishes last (by the ticket counter, which wraps to zero for
 // the next launch) reduces them.  A launch per block and one for the final reduction cost about 5 us each
 // on states of any size that stays in L2, a tenth of a small step.
-struct ReduceGrid {
+// Each kind of reduction has partials and a counter of its own, and its CTAs are the same number in every launch
+// of the plan: whatever launches overlap (calls of one plan on two streams, which may spoil one another's result
+// as they always could), each adds `ctas` to a counter that wraps at `ctas`, so it ends at zero and later
+// results are right.
+struct Reduction {
   int cta0[DGB_MAX_BLOCKS + 1];
+  int ctas;                // launched: cta0[nblocks], at least one
+  Partial* partials;       // [ctas]
+  unsigned* ticket;
 };
 
-__device__ __forceinline__ int reduce_block(const ReduceGrid& G, int nblocks) {
+__device__ __forceinline__ int reduce_block(const Reduction& G, int nblocks) {
   int b = 0;
   while (b + 1 < nblocks && (int)blockIdx.x >= G.cta0[b + 1]) ++b;
   return b;
@@ -530,8 +537,8 @@ __device__ __forceinline__ bool last_cta(unsigned* ticket) {
 
 // max over elements of the reference's rate, then dt = clip(cfl / max)
 template <int NV>
-__global__ void __launch_bounds__(kThreads) k_rate(const DevPlan P, const StatePtrs S, const ReduceGrid G, double cp,
-                                                  Partial* partials, unsigned* ticket, double cfl, double* dt_out) {
+__global__ void __launch_bounds__(kThreads) k_rate(const DevPlan P, const StatePtrs S, const Reduction G, double cp,
+                                                  double cfl, double* dt_out) {
   // one warp per element; grid-stride over the block's elements
   const int b = reduce_block(G, P.nblocks);
   const BlockDev& B = P.blk[b];
@@ -580,11 +587,11 @@ __global__ void __launch_bounds__(kThreads) k_rate(const DevPlan P, const StateP
   if (threadIdx.x == 0) {
     double m = red[0];
     for (int k = 1; k < kThreads / 32; ++k) m = fmax(m, red[k]);
-    __stcg(&partials[blockIdx.x].a, m);
+    __stcg(&G.partials[blockIdx.x].a, m);
   }
-  if (!last_cta(ticket)) return;
+  if (!last_cta(G.ticket)) return;
   double m = -INFINITY;
-  for (int i = threadIdx.x; i < (int)gridDim.x; i += kThreads) m = fmax(m, __ldcg(&partials[i].a));
+  for (int i = threadIdx.x; i < (int)gridDim.x; i += kThreads) m = fmax(m, __ldcg(&G.partials[i].a));
   for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffff, m, o));
   if (lane == 0) red[threadIdx.x >> 5] = m;
   __syncthreads();
@@ -596,9 +603,8 @@ __global__ void __launch_bounds__(kThreads) k_rate(const DevPlan P, const StateP
 }
 
 template <int NV>
-__global__ void __launch_bounds__(kThreads) k_adm(const DevPlan P, const StatePtrs S, const ReduceGrid G,
-                                                 Partial* partials, unsigned* ticket, double rho_floor, double p_floor,
-                                                 int combine, dgb_status* status) {
+__global__ void __launch_bounds__(kThreads) k_adm(const DevPlan P, const StatePtrs S, const Reduction G, double rho_floor,
+                                                 double p_floor, int combine, dgb_status* status) {
   const int b = reduce_block(G, P.nblocks);
   const BlockDev& B = P.blk[b];
   const size_t nodes = (size_t)B.E * B.Np;
@@ -639,20 +645,20 @@ __global__ void __launch_bounds__(kThreads) k_adm(const DevPlan P, const StatePt
   };
   reduce();
   if (threadIdx.x == 0) {
-    __stcg(&partials[blockIdx.x].a, rmin);
-    __stcg(&partials[blockIdx.x].b, pmin);
-    __stcg(&partials[blockIdx.x].flag, finite);
+    __stcg(&G.partials[blockIdx.x].a, rmin);
+    __stcg(&G.partials[blockIdx.x].b, pmin);
+    __stcg(&G.partials[blockIdx.x].flag, finite);
   }
-  if (!last_cta(ticket)) return;
+  if (!last_cta(G.ticket)) return;
   rmin = pmin = INFINITY;
   finite = 1, rnan = pnan = 0;
   for (int i = threadIdx.x; i < (int)gridDim.x; i += kThreads) {
-    const double a = __ldcg(&partials[i].a), c = __ldcg(&partials[i].b);
+    const double a = __ldcg(&G.partials[i].a), c = __ldcg(&G.partials[i].b);
     rnan |= isnan(a);
     pnan |= isnan(c);
     rmin = fmin(rmin, a);
     pmin = fmin(pmin, c);
-    finite &= __ldcg(&partials[i].flag);
+    finite &= __ldcg(&G.partials[i].flag);
   }
   reduce();
   if (threadIdx.x != 0) return;

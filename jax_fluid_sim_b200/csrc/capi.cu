@@ -78,9 +78,8 @@ struct dgb_plan {
   // stage buffers for SSP-RK3
   double* stage1[DGB_MAX_BLOCKS] = {nullptr, nullptr, nullptr};
   double* stage2[DGB_MAX_BLOCKS] = {nullptr, nullptr, nullptr};
-  Partial* partials = nullptr;
-  ReduceGrid rate_grid = {}, adm_grid = {};
-  unsigned* ticket = nullptr;          // last_cta's counter
+  // the CFL rate and the admissibility reductions: each its own partials and counter (Reduction)
+  Reduction rate = {}, adm = {};
   double* dt_scratch = nullptr;
   // batched launches of the dense element kernels (all blocks in one grid) and their shared memory
   int num_cases = 0;   // dgb_plan_set_cases
@@ -809,9 +808,8 @@ int run_positivity(dgb_plan* p, const StatePtrs& S, cudaStream_t st) {
 
 template <int NV>
 int run_admissibility(dgb_plan* p, const StatePtrs& S, dgb_status* status, int combine, cudaStream_t st) {
-  const ReduceGrid& G = p->adm_grid;
-  k_adm<NV><<<std::max(1, G.cta0[p->dev.nblocks]), kThreads, 0, st>>>(
-      p->dev, S, G, p->partials, p->ticket, p->lim.adm_density_floor, p->lim.adm_pressure_floor, combine, status);
+  k_adm<NV><<<p->adm.ctas, kThreads, 0, st>>>(p->dev, S, p->adm, p->lim.adm_density_floor, p->lim.adm_pressure_floor,
+                                              combine, status);
   CK(cudaGetLastError());
   return DGB_OK;
 }
@@ -819,8 +817,7 @@ int run_admissibility(dgb_plan* p, const StatePtrs& S, dgb_status* status, int c
 template <int NV>
 int run_stable_dt(dgb_plan* p, const StatePtrs& S, double cfl, double* dt_out, cudaStream_t st) {
   const double cp = p->prm.gamma * p->prm.gas_constant / (p->prm.gamma - 1.0);
-  const ReduceGrid& G = p->rate_grid;
-  k_rate<NV><<<std::max(1, G.cta0[p->dev.nblocks]), kThreads, 0, st>>>(p->dev, S, G, cp, p->partials, p->ticket, cfl, dt_out);
+  k_rate<NV><<<p->rate.ctas, kThreads, 0, st>>>(p->dev, S, p->rate, cp, cfl, dt_out);
   CK(cudaGetLastError());
   return DGB_OK;
 }
@@ -1605,7 +1602,7 @@ int dgb_plan_finalize(dgb_plan* p) {
   // CTAs of the reductions: one warp per element (rate), one thread per node (admissibility), at most eight
   // CTAs per SM over all blocks, shared by the blocks' sizes
   {
-    auto split = [&](ReduceGrid& G, auto work, int per) {
+    auto split = [&](Reduction& G, auto work, int per) -> int {
       long total = 0;
       for (int b = 0; b < p->dev.nblocks; ++b) total += blocks_for(work(p->dev.blk[b]), per);
       const double share = std::min(1.0, 148.0 * 8 / std::max(1L, total));
@@ -1614,18 +1611,16 @@ int dgb_plan_finalize(dgb_plan* p) {
         const int n = blocks_for(work(p->dev.blk[b]), per);
         G.cta0[b + 1] = G.cta0[b] + (n > 0 ? std::max(1, (int)(n * share)) : 0);
       }
-      return G.cta0[p->dev.nblocks];
+      G.ctas = std::max(1, G.cta0[p->dev.nblocks]);
+      CK(cudaMalloc(&G.partials, sizeof(Partial) * (size_t)G.ctas));
+      p->allocations.push_back(G.partials);
+      CK(cudaMalloc(&G.ticket, sizeof(unsigned)));
+      p->allocations.push_back(G.ticket);
+      CK(cudaMemset(G.ticket, 0, sizeof(unsigned)));
+      return DGB_OK;
     };
-    const int n = std::max(split(p->rate_grid, [](const BlockDev& B) { return (long)B.E; }, kThreads / 32),
-                           split(p->adm_grid, [](const BlockDev& B) { return (long)B.E * B.Np; }, kThreads));
-    void* d = nullptr;
-    CK(cudaMalloc(&d, sizeof(Partial) * (size_t)(n + 1)));
-    p->allocations.push_back(d);
-    p->partials = static_cast<Partial*>(d);
-    CK(cudaMalloc(&d, sizeof(unsigned)));
-    p->allocations.push_back(d);
-    CK(cudaMemset(d, 0, sizeof(unsigned)));
-    p->ticket = static_cast<unsigned*>(d);
+    if ((rc = split(p->rate, [](const BlockDev& B) { return (long)B.E; }, kThreads / 32))) return rc;
+    if ((rc = split(p->adm, [](const BlockDev& B) { return (long)B.E * B.Np; }, kThreads))) return rc;
   }
   if ((rc = alloc(p, 1, &p->dt_scratch))) return rc;
   {
