@@ -1667,6 +1667,8 @@ int dgb_plan_finalize(dgb_plan* p) {
       }
     }
   }
+  // set-up kernels and copies ran on the default stream, with which the caller's streams need not synchronise
+  CK(cudaDeviceSynchronize());
   p->finalized = true;
   return DGB_OK;
 }

@@ -1,0 +1,33 @@
+"""What a plan's set-up leaves to its first call: the tables that set-up kernels write on the default stream are
+there for a first right-hand side on a stream that does not synchronise with it."""
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("mu", [0.0, 0.02])
+@pytest.mark.parametrize("mesh", ["box_hex", "mixed_block"])
+def test_first_call_on_another_stream(mesh, mu):
+    import torch
+    from jax_fluid_sim_b200 import (FarfieldWallBoundary, HybridCompressibleSolver, HybridEulerOperator, HybridMesh,
+                                    HybridNavierStokesOperator, meshgen)
+    src = meshgen.mixed_block(jitter=0.1, seed=2) if mesh == "mixed_block" else meshgen.box_hex(
+        (12, 12, 12), hi=(12.0,) * 3, jitter=0.1, seed=3)
+    solver = HybridCompressibleSolver(HybridMesh(src), polynomial_degree=2, dynamic_viscosity=mu)
+    op = (HybridNavierStokesOperator if mu else HybridEulerOperator)(solver)
+    bc = FarfieldWallBoundary(solver, [1.0, 0.4, 0.1, 0.0, 1.0])
+
+    def primitive(x):
+        s = 1.0 + 0.2 * np.sin(1.3 * x[..., 0]) * np.cos(0.7 * x[..., 1])
+        return np.stack([s, 0.5 * s, 0.1 * np.sin(x[..., 2]), 0.0 * s, 1.0 + 0.5 * s], -1)
+
+    U = solver.state_blocks_from_primitive_function(op, primitive)
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        first = op.with_precision("float64").rhs(U, bc)
+    torch.cuda.synchronize()
+    again = op.rhs(U, bc)
+    assert all(torch.equal(first[k], again[k]) for k in again)
