@@ -189,7 +189,8 @@ int upload_by_value(dgb_plan* p, const double* host, size_t rows, int nq, int K,
   if ((rc = upload(p, host, rows * nq * K, out))) return rc;
   if (rows == 0 || nq == 0) return DGB_OK;
   const size_t smem = sizeof(double) * nq * K;
-  if (rows > 0x7fffffff || smem > 48 * 1024) return fail(DGB_ERR_UNSUPPORTED, "per-point table too large");
+  if (rows > 0x7fffffff || smem > 227 * 1024) return fail(DGB_ERR_UNSUPPORTED, "per-point table too large");
+  CK(cudaFuncSetAttribute(k_values_by_row, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   k_values_by_row<<<(unsigned)rows, 128, smem>>>(const_cast<double*>(*out), nq, K);
   CK(cudaGetLastError());
   CK(cudaDeviceSynchronize());

@@ -31,3 +31,27 @@ def test_first_call_on_another_stream(mesh, mu):
     torch.cuda.synchronize()
     again = op.rhs(U, bc)
     assert all(torch.equal(first[k], again[k]) for k in again)
+
+
+@pytest.mark.parametrize("points", [8, 682, 683, 1200])
+def test_volume_rules_of_any_size_are_accepted(points):
+    """A block with more volume points than fit one CTA's default shared memory (683 of 9 values)."""
+    import ctypes
+    from jax_fluid_sim_b200 import _native as N
+    L = N.lib()
+    prm = N.Params()
+    prm.degree, prm.nvars, prm.num_blocks, prm.gamma, prm.gas_constant = 1, 5, 1, 1.4, 1.0
+    handle = ctypes.c_void_p()
+    N.check(L.dgb_plan_create(ctypes.byref(prm), ctypes.byref(handle)))
+    try:
+        arrays = dict(basis=np.ones((points, 8)), basis_grad=np.ones((points, 8, 3)),
+                      inv_jacobian=np.ones((2, points, 3, 3)), wdet=np.ones((2, points)), length=np.ones(2),
+                      face_sample_basis=np.ones((4, 8)), p1_projector=np.eye(8), inv_mass=np.ones((2, 8, 8)))
+        faces = np.arange(12, dtype=np.int32)
+        d = N.BlockDesc(element_type=0, num_elements=2, num_nodes=8, num_qp=points, num_local_faces=6,
+                        elem_face=N.dptr(faces, ctypes.c_int32), num_face_samples=4)
+        for k, a in arrays.items():
+            setattr(d, k, N.dptr(a))
+        N.check(L.dgb_plan_set_block(handle, 0, ctypes.byref(d)))
+    finally:
+        L.dgb_plan_destroy(handle)
