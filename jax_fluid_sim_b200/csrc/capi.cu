@@ -898,9 +898,12 @@ int run_subcell(dgb_plan* p, const StatePtrs& cur, double* const* cand, double* 
   k_mood_fv<NV><<<most, kThreads, sm_fv, st>>>(P, M, cur, p->mood_lists);
   if (faces > 0)
     k_mood_faces<NV><<<std::min(blocks_for(faces, kThreads / 32), 148 * 8), kThreads, 0, st>>>(P, M, cur, F, p->mood_lists);
-  if ((rc = prepare(k_mood_update<NV>, sm_up))) return rc;
-  k_mood_update<NV><<<most, kThreads, sm_up, st>>>(P, M, F, vis, dt, src, dst, p->mood_lists,
-                                                   in_place ? 0u : (unsigned)elements);
+  auto update = [&](auto kernel) -> int {
+    if (int e = prepare(kernel, sm_up)) return e;
+    kernel<<<most, kThreads, sm_up, st>>>(P, M, F, vis, dt, src, dst, p->mood_lists, (unsigned)elements);
+    return DGB_OK;
+  };
+  if ((rc = in_place ? update(k_mood_update<NV, false>) : update(k_mood_update<NV, true>))) return rc;
   CK(cudaGetLastError());
   return DGB_OK;
 }

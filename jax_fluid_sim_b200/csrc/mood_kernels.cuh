@@ -377,19 +377,19 @@ __global__ void __launch_bounds__(kThreads) k_mood_faces(const DevPlan P, const 
 // projection and later its reconstruction rows.
 __host__ __device__ inline int mood_update_smem(int NV, int Np, int S) { return 2 * S * NV + Np * NV + S * Np; }
 
-// out = troubled ? bound-limited reconstruction of the FV update : candidate + corrections.  all = 0: the touched
-// elements, in place (out is the candidate); else every one of the `all` elements.  This kernel is the first to write
-// out, an element once what it reads of that element has been read, so out may also be the base state or visc.
-template <int NV>
+// out = troubled ? bound-limited reconstruction of the FV update : candidate + corrections.  ALL = false: the touched
+// elements, in place (out is the candidate); else every one of the plan's `elements`.  This kernel is the first to
+// write out, an element once what it reads of that element has been read, so out may also be the base state or visc.
+template <int NV, bool ALL>
 __global__ void __launch_bounds__(kThreads) k_mood_update(const DevPlan P, const MoodDev M, const FlagPtrs Fl,
                                                          const StatePtrs visc, double dt, const StatePtrs cand_,
-                                                         const StatePtrs out_, const MoodLists L, unsigned all) {
+                                                         const StatePtrs out_, const MoodLists L, unsigned elements) {
   extern __shared__ double smem[];
   __shared__ double vtot, corr[DGB_MAX_VARS];
-  const unsigned n = all ? all : L.count[kMoodTouched];
+  const unsigned n = ALL ? elements : L.count[kMoodTouched];
   for (unsigned item = blockIdx.x; item < n; item += gridDim.x) {
     int b = 0, e = (int)item;
-    if (all)
+    if constexpr (ALL)
       for (; e >= P.blk[b].E; ++b) e -= P.blk[b].E;
     else
       b = L.touched[item] >> 28, e = L.touched[item] & 0xfffffffu;
@@ -398,9 +398,9 @@ __global__ void __launch_bounds__(kThreads) k_mood_update(const DevPlan P, const
     const int Np = B.Np, Sn = C.S;
     const size_t base = (size_t)e * Np * NV;
     const double* vol = C.vol + (size_t)e * Sn;
-    const double* cand = cand_.b[b];
     double* out = out_.b[b];
-    if (all && !L.mark[b][e]) {
+    const double* cand = ALL ? cand_.b[b] : out;
+    if (ALL && !L.mark[b][e]) {
       for (int idx = threadIdx.x; idx < Np * NV; idx += kThreads) out[base + idx] = cand[base + idx];
       continue;
     }
