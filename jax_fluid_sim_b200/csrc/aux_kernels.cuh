@@ -68,19 +68,34 @@ __device__ __forceinline__ bool certificate_from_range(const double (&mn)[5], co
          (p_lo - tol_p >= fmax(p_floor, rel * pmean_hi + tol_p));
 }
 
-// Smallest and largest value over the warp of each lane's minima and maxima, in every lane: the minima rounded
-// down and the maxima up to float32, as ordered integers through the warp's integer reduction.  The certificate's
-// bounds only widen by that (by less than its own tolerance of 1e-6), and an element it no longer clears gets the full
-// test, so no result depends on the rounding.  10 reductions take the place of 100 shuffles and 50 float64
-// comparisons, which bound these kernels: sensor of 202k P3 elements 353 -> 196 us, certificate of 39k 38 -> 25 us.
+// Smallest and largest value over the warp of each lane's minima and maxima, in every lane, through the warp's
+// integer reduction: a float's or a double's bits, with the lower ones of negative values inverted, order as an
+// integer does.  EXACT: the extreme upper half of the doubles, then the extreme lower half of the lanes that have it.
+// Else the minima rounded down and the maxima up to float32, half the reductions.
+// (Shuffles took 100 of them and 50 float64 comparisons, which bound these kernels.)
+template <bool EXACT>
 __device__ __forceinline__ void warp_range(double (&mn)[5], double (&mx)[5]) {
-  auto ordered = [](int i) { return i ^ ((i >> 31) & 0x7fffffff); };
+  if constexpr (EXACT) {
+    auto ordered = [](long long i) { return i ^ ((i >> 63) & 0x7fffffffffffffffLL); };
+    auto value = [&](int hi, unsigned lo) { return __longlong_as_double(ordered((long long)hi << 32 | lo)); };
 #pragma unroll
-  for (int v = 0; v < 5; ++v) {
-    const int lo = __reduce_min_sync(0xffffffff, ordered(__float_as_int(__double2float_rd(mn[v]))));
-    const int hi = __reduce_max_sync(0xffffffff, ordered(__float_as_int(__double2float_ru(mx[v]))));
-    mn[v] = (double)__int_as_float(ordered(lo));
-    mx[v] = (double)__int_as_float(ordered(hi));
+    for (int v = 0; v < 5; ++v) {
+      const long long a = ordered(__double_as_longlong(mn[v])), b = ordered(__double_as_longlong(mx[v]));
+      const int ah = __reduce_min_sync(0xffffffff, (int)(a >> 32)), bh = __reduce_max_sync(0xffffffff, (int)(b >> 32));
+      const unsigned al = __reduce_min_sync(0xffffffff, (int)(a >> 32) == ah ? (unsigned)a : 0xffffffffu);
+      const unsigned bl = __reduce_max_sync(0xffffffff, (int)(b >> 32) == bh ? (unsigned)b : 0u);
+      mn[v] = value(ah, al);
+      mx[v] = value(bh, bl);
+    }
+  } else {
+    auto ordered = [](int i) { return i ^ ((i >> 31) & 0x7fffffff); };
+#pragma unroll
+    for (int v = 0; v < 5; ++v) {
+      const int lo = __reduce_min_sync(0xffffffff, ordered(__float_as_int(__double2float_rd(mn[v]))));
+      const int hi = __reduce_max_sync(0xffffffff, ordered(__float_as_int(__double2float_ru(mx[v]))));
+      mn[v] = (double)__int_as_float(ordered(lo));
+      mx[v] = (double)__int_as_float(ordered(hi));
+    }
   }
 }
 
@@ -98,31 +113,49 @@ struct WarpNodes {
         for (int v = 0; v < NV; ++v) u[k][v] = Ug[l * NV + v];
     }
   }
-  // whether every value is finite and the certificate clears the element, the same in every lane
-  __device__ __forceinline__ bool certified(const Physics& ph, double L, double rho_floor, double p_floor, double rel) const {
+  // whether every value is finite and the certificate clears the element, the same in every lane: most elements by
+  // their range rounded outward, which contains the exact one and so clears no more than it does; the others by
+  // the exact one, from the values in memory (Ug, as loaded or stored by these lanes), so that no register is kept for it
+  __device__ __forceinline__ bool certified(const double* Ug, const Physics& ph, double L, double rho_floor, double p_floor,
+                                            double rel) const {
     double mn[5], mx[5];
+    auto clear = [&]() {
 #pragma unroll
-    for (int v = 0; v < 5; ++v) {
-      mn[v] = INFINITY;
-      mx[v] = -INFINITY;
-    }
+      for (int v = 0; v < 5; ++v) {
+        mn[v] = INFINITY;
+        mx[v] = -INFINITY;
+      }
+    };
+    auto include = [&](int v, double x) {
+      mn[v] = fmin(mn[v], x);
+      mx[v] = fmax(mx[v], x);
+    };
+    auto cleared = [&]() -> bool {
+      bool ok = false;
+      if ((threadIdx.x & 31) == 0) ok = certificate_from_range(mn, mx, ph, L, rho_floor, p_floor, rel);
+      return __any_sync(0xffffffff, ok);
+    };
     bool fin = true;
+    clear();
 #pragma unroll
     for (int k = 0; k < K; ++k)
       if (k * 32 + (threadIdx.x & 31) < NP)
 #pragma unroll
         for (int v = 0; v < NV; ++v) {
           fin &= isfinite(u[k][v]);
-          if (v < 5) {
-            mn[v] = fmin(mn[v], u[k][v]);
-            mx[v] = fmax(mx[v], u[k][v]);
-          }
+          if (v < 5) include(v, u[k][v]);
         }
     if (!__all_sync(0xffffffff, fin)) return false;
-    warp_range(mn, mx);
-    bool ok = false;
-    if ((threadIdx.x & 31) == 0) ok = certificate_from_range(mn, mx, ph, L, rho_floor, p_floor, rel);
-    return __any_sync(0xffffffff, ok);
+    warp_range<false>(mn, mx);
+    if (cleared()) return true;
+    clear();
+#pragma unroll 1
+    for (int l = threadIdx.x & 31; l < NP; l += 32)
+#pragma unroll
+      for (int v = 0; v < 5; ++v) include(v, Ug[l * NV + v]);
+    __syncwarp();
+    warp_range<true>(mn, mx);
+    return cleared();
   }
 };
 
@@ -194,7 +227,7 @@ __global__ void __launch_bounds__(kThreads) k_certify(const double* __restrict__
   if (e >= E) return;
   WarpNodes<NV, NP> x;
   x.load(U + e * NP * NV);
-  if (!x.certified(ph, C.L, C.rho_floor, C.p_floor, C.rel) && (threadIdx.x & 31) == 0)
+  if (!x.certified(U + e * NP * NV, ph, C.L, C.rho_floor, C.p_floor, C.rel) && (threadIdx.x & 31) == 0)
     C.list[atomicAdd(C.count, 1)] = (int)e;
 }
 
@@ -216,7 +249,7 @@ __global__ void __launch_bounds__(kThreads) k_blend_certify(const double* base, 
     WarpNodes<NV, NP> u, w;
     u.load(x + o);
     w.load(base + o);
-    if (!LIST && !u.certified(ph, Cx.L, Cx.rho_floor, Cx.p_floor, Cx.rel)) {
+    if (!LIST && !u.certified(x + o, ph, Cx.L, Cx.rho_floor, Cx.p_floor, Cx.rel)) {
       if (lane == 0) Cx.list[atomicAdd(Cx.count, 1)] = e;
       continue;
     }
@@ -230,7 +263,7 @@ __global__ void __launch_bounds__(kThreads) k_blend_certify(const double* base, 
           out[o + l * NV + v] = u.u[k][v];
         }
     }
-    if (!u.certified(ph, Co.L, Co.rho_floor, Co.p_floor, Co.rel) && lane == 0) Co.list[atomicAdd(Co.count, 1)] = e;
+    if (!u.certified(out + o, ph, Co.L, Co.rho_floor, Co.p_floor, Co.rel) && lane == 0) Co.list[atomicAdd(Co.count, 1)] = e;
   }
 }
 

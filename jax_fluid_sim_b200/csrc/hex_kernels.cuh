@@ -1287,8 +1287,9 @@ __global__ void __launch_bounds__(kThreads) k_hex_sensor(const DevPlan P_, const
     return;
   }
   WarpNodes<NV, N3> un;
-  un.load(S.b[b] + (size_t)e * N3 * NV);
-  if (!un.certified(P_.ph, Lc.lebesgue, Lc.density_floor, Lc.pressure_floor, 0.0)) {
+  const double* Ug = S.b[b] + (size_t)e * N3 * NV;
+  un.load(Ug);
+  if (!un.certified(Ug, P_.ph, Lc.lebesgue, Lc.density_floor, Lc.pressure_floor, 0.0)) {
     if (lane == 0) list[atomicAdd(count, 1)] = e;
     return;
   }
