@@ -15,6 +15,7 @@
 #include <stdint.h>
 
 #include "../../include/dgb200.h"
+#include "quotient.h"
 
 namespace dgb {
 
@@ -93,20 +94,22 @@ __device__ __forceinline__ void conserved(const Physics& ph, const T* W, T* U) {
   for (int s = 5; s < NV; ++s) U[s] = mul(rho, W[s]);
 }
 
-// Primitive state [rho, u, v, w, p] for the fluxes, with inv = 1 / max(rho, floor).  In float64 the quotients are
-// products with inv (one unit in the last place from the divided ones): a face point's fluxes held 21 divisions,
-// a quarter of the face kernels' instructions, and hold 5 this way.  Limiters and detectors, whose thresholds
-// the reference's divided values meet, take primitive().
+// Primitive state [rho, u, v, w, p] for the fluxes, with inv = 1 / max(rho, floor).  In float64 the quotients come
+// from that one division (quotient(): the same values as primitive()'s).  A face point's fluxes held 21 divisions, a
+// quarter of the face kernels' instructions, and hold 5 this way.
 template <int NV, typename T>
 __device__ __forceinline__ void flux_primitive(const Physics& ph, const T* U, T* W, T& inv) {
   if constexpr (sizeof(T) == sizeof(double)) {
-    inv = T(1) / fmax(U[0], T(kRhoFloor));
+    const T srho = fmax(U[0], T(kRhoFloor));
+    inv = T(1) / srho;
+    const T m2 = add(add(mul(U[1], U[1]), mul(U[2], U[2])), mul(U[3], U[3])), h = mul(T(0.5), m2);
+    // with |m|^2 finite the momenta are below 1.4e154, and their quotients finite
+    const bool refine = refinable(h, srho, inv);
     W[0] = U[0];
-    W[1] = mul(U[1], inv);
-    W[2] = mul(U[2], inv);
-    W[3] = mul(U[3], inv);
-    const T m2 = add(add(mul(U[1], U[1]), mul(U[2], U[2])), mul(U[3], U[3]));
-    W[4] = mul(T(ph.gamma - 1.0), sub(U[4], mul(mul(T(0.5), m2), inv)));
+    W[1] = quotient(U[1], srho, inv, refine);
+    W[2] = quotient(U[2], srho, inv, refine);
+    W[3] = quotient(U[3], srho, inv, refine);
+    W[4] = mul(T(ph.gamma - 1.0), sub(U[4], quotient(h, srho, inv, refine)));
   } else {
     T full[NV];
     primitive<NV>(ph, U, full);
@@ -158,15 +161,15 @@ template <int NV>
 __device__ __forceinline__ void hllc_star(const Physics& ph, const double* U, const double* W, double s, double sm,
                                           const double* n, double* S) {
   const double un = W[1] * n[0] + W[2] * n[1] + W[3] * n[2];
-  const double rden = 1.0 / safe_signed(s - sm);
-  const double comp = (s - un) * rden;
+  const double den = safe_signed(s - sm), rden = 1.0 / den;
+  const double comp = quotient(s - un, den, rden);     // (a result that is not finite goes to the Rusanov flux)
   const double rs = W[0] * comp;
   S[0] = rs;
   S[1] = rs * (W[1] + (sm - un) * n[0]);
   S[2] = rs * (W[2] + (sm - un) * n[1]);
   S[3] = rs * (W[3] + (sm - un) * n[2]);
   const double ps = W[4] + W[0] * (s - un) * (sm - un);
-  S[4] = ((s - un) * U[4] - W[4] * un + ps * sm) * rden;
+  S[4] = quotient((s - un) * U[4] - W[4] * un + ps * sm, den, rden);
 #pragma unroll
   for (int v = 5; v < NV; ++v) S[v] = U[v] * comp;
 }
@@ -189,8 +192,9 @@ __device__ void hllc(const Physics& ph, const double* UL, const double* UR, cons
   const double rl = WL[0], rr = WR[0], pl = WL[4], pr = WR[4];
   const double unl = WL[1] * n[0] + WL[2] * n[1] + WL[3] * n[2];
   const double unr = WR[1] * n[0] + WR[2] * n[1] + WR[3] * n[2];
-  const double cl = sqrt(fmax(ph.gamma * pl * il, 0.0));
-  const double cr = sqrt(fmax(ph.gamma * pr * ir, 0.0));
+  const double dl = fmax(rl, kRhoFloor), dr = fmax(rr, kRhoFloor), gl = ph.gamma * pl, gr = ph.gamma * pr;
+  const double cl = sqrt(fmax(quotient(gl, dl, il, refinable(gl, dl, il)), 0.0));
+  const double cr = sqrt(fmax(quotient(gr, dr, ir, refinable(gr, dr, ir)), 0.0));
   const double sl = fmin(unl - cl, unr - cr);
   const double sr = fmax(unl + cl, unr + cr);
   const double den = rl * (sl - unl) - rr * (sr - unr);
@@ -245,7 +249,8 @@ __device__ __forceinline__ void viscous_vars(const Physics& ph, const double* U,
   out[0] = W[1];
   out[1] = W[2];
   out[2] = W[3];
-  out[3] = W[4] * inv * (1.0 / ph.R);
+  const double den = fmax(W[0], kRhoFloor) * ph.R, rden = inv * (1.0 / ph.R);
+  out[3] = quotient(W[4], den, rden, refinable(W[4], den, rden));
 }
 
 // Ghost [u, v, w, T] for the viscous traces (boundary.py:74-102).
