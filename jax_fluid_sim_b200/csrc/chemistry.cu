@@ -1,5 +1,5 @@
-// Finite-rate chemistry: operator-split point-implicit reaction advance, one thread per
-// solution node, float64 throughout.
+// Finite-rate chemistry: operator-split point-implicit reaction advance, four lanes per solution node, and the
+// rates alone, one thread per sample; float64 throughout.
 //
 // Follows the reference's hybrid/chemistry package:
 //   nasa.py:47-118          NASA-7 cp/R, h/RT, s/R with T clamped to each species' range
@@ -38,7 +38,13 @@
 //    e(T) converges quadratically, so the remaining iterations of the fixed count change T
 //    only in its last bits;
 //  - in the same way a node keeps its state once a Newton iteration has moved each density by at most
-//    1e-13 of it and T by at most 1e-13 T: the next update would be of the order of the square of that.
+//    1e-13 of it and T by at most 1e-13 T.  T is inverted after the densities, outside the Jacobian, so the iterations
+//    converge linearly: an iteration shrinks the change by 1e-3 in the median and by 0.13 in the slowest hot nodes, so
+//    that the remaining ones would still move a density by at most 1e-13 0.13 / 0.87 = 1.5e-14 of it, within the
+//    round-off that every further iteration leaves anew.  Root mean square of a node's largest error in any density, against
+//    the converged iterations in extended precision, after the stop and after all 12 (after 11 and 13): hot mixtures 1.087e-14 and
+//    1.085e-14 (1.079, 1.083), at a tenth of the step 4.37e-15 and 4.40e-15, free stream 3.071e-14 and 3.073e-14,
+//    behind a Mach 8 shock 1.394e-14 and 1.399e-14 (1.411, 1.406).
 //    A warp stops when its eight nodes have.  Nodes whose iterations do not settle that far (I - dt J
 //    ill-conditioned) run the whole count;
 //  - with one temperature (T_v = T) the three controlling temperatures of a reaction, floored at 10 K,
@@ -208,12 +214,12 @@ __device__ void rates(const Tables& M, const Slots<NS>& sl, const double (&rho)[
     const double Tr = jmax(select_T(R.rmode, T, T), 10.0);
     double dG = 0.0;
     if (Tr == Tg) {
-    #pragma unroll 1
-  for (int k = 0; k < R.nd; ++k) dG += R.d_nu[k] * sl.g(R.d_sp[k]);
+#pragma unroll 1
+      for (int k = 0; k < R.nd; ++k) dG += R.d_nu[k] * sl.g(R.d_sp[k]);
     } else {
       const TPow tr = tpow(Tr);
-    #pragma unroll 1
-  for (int k = 0; k < R.nd; ++k) dG += R.d_nu[k] * g_RT(M, R.d_sp[k], tr);
+#pragma unroll 1
+      for (int k = 0; k < R.nd; ++k) dG += R.d_nu[k] * g_RT(M, R.d_sp[k], tr);
     }
     const double base = Tr == Tg ? base_g : kPStd / (kRUniv * Tr);
     const double conv = R.dn == 0.0 ? 1.0 : (R.dn == 1.0 ? base : (R.dn == -1.0 ? 1.0 / base : pow(base, R.dn)));
@@ -606,7 +612,10 @@ __global__ void __launch_bounds__(kReactThreads, 3)
       }
       a[s][NS] = -(rho[s] - r0[s] - dtp * w);
     }
-    // ---- LU with partial pivoting: the pivot is the largest entry of the column to 16 bits
+    // ---- LU with partial pivoting: the pivot is the largest entry of the column to 16 bits of the mantissa, so that
+    // one integer maximum finds value and row.  Which of two entries that agree to 1.5e-5 is the pivot enters no value:
+    // the factors stay below 1 + 1.5e-5 instead of 1.  The largest by all bits took 6 % longer (54,000 nodes: 1628 ->
+    // 1731 us) and left the same states bit for bit.
     unsigned used = 0;                                   // slots of this lane that have been pivot rows
 #pragma unroll
     for (int s = 0; s < SLOTS; ++s) used |= row.q[s] < NS ? 0u : 1u << s;
