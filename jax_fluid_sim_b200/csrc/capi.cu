@@ -217,9 +217,11 @@ StatePtrs to_ptrs(const dgb_state* s) {
   return out;
 }
 
+// Allows a launch smem bytes of dynamic shared memory.  Without the attribute a CTA has 48 KB in all, of which the
+// kernels' static arrays take up to 8 KB.
 template <typename K>
 int prepare(K kernel, size_t smem) {
-  if (smem > 48 * 1024) CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (smem > 40 * 1024) CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   return DGB_OK;
 }
 
