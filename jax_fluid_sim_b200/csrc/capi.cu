@@ -6,6 +6,7 @@
 
 #include <string>
 #include <algorithm>
+#include <functional>
 #include <vector>
 
 #include "aux_kernels.cuh"
@@ -119,6 +120,9 @@ struct dgb_plan {
   bool mood_ready = false;
   MoodLists mood_lists = {};
   size_t mood_marks = 0;
+  // dynamic shared memory of k_mood_fv and k_mood_update, and the CTAs of each that are resident at once
+  size_t mood_smem_fv = 0, mood_smem_up = 0;
+  int mood_ctas_fv = 0, mood_ctas_up = 0;
   uint8_t* flags[DGB_MAX_BLOCKS] = {nullptr, nullptr, nullptr};
   // learned troubled-cell predictor (dgb_plan_set_predictor)
   int pred_mode = 0;
@@ -868,6 +872,26 @@ int run_mood_screen(dgb_plan* p, const FlagPtrs& F, cudaStream_t st) {
   return DGB_OK;
 }
 
+// Shared memory and resident CTAs of the subcell kernels, over the plan's blocks (set-up).
+template <int NV>
+int mood_grids(dgb_plan* p) {
+  for (int b = 0; b < p->dev.nblocks; ++b) {
+    const SubcellBlockDev& C = p->mood.blk[b];
+    const int Np = p->dev.blk[b].Np;
+    p->mood_smem_fv = std::max(p->mood_smem_fv, sizeof(double) * (size_t)mood_fv_smem(NV, Np, C.S, C.NI));
+    p->mood_smem_up = std::max(p->mood_smem_up, sizeof(double) * (size_t)mood_update_smem(NV, Np, C.S));
+  }
+  int rc, dev = 0, sms = 0, n = 0;
+  if ((rc = prepare(k_mood_fv<NV>, p->mood_smem_fv)) || (rc = prepare(k_mood_update<NV, false>, p->mood_smem_up))) return rc;
+  CK(cudaGetDevice(&dev));
+  CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_mood_fv<NV>, kThreads, p->mood_smem_fv));
+  p->mood_ctas_fv = std::max(n, 1) * sms;
+  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_mood_update<NV, false>, kThreads, p->mood_smem_up));
+  p->mood_ctas_up = std::max(n, 1) * sms;
+  return DGB_OK;
+}
+
 // Subcell recompute of the candidate `cand` from the base `cur` into `out`, after run_mood_screen and with the
 // traces of `cur` in the face buffers.  In place (out is cand) only the listed elements are written; else every
 // element is, and out may be cur's buffer or visc's.
@@ -880,29 +904,28 @@ int run_subcell(dgb_plan* p, const StatePtrs& cur, double* const* cand, double* 
   StatePtrs vis, src, dst;
   bool in_place = true;
   long elements = 0, faces = (long)P.face[0].F + P.face[1].F;
-  size_t sm_fv = 0, sm_up = 0;
   for (int b = 0; b < DGB_MAX_BLOCKS; ++b) {
     vis.b[b] = visc ? visc[b] : nullptr;
     src.b[b] = cand[b];
     dst.b[b] = out[b];
     if (b >= P.nblocks) continue;
     in_place &= P.blk[b].E == 0 || cand[b] == out[b];
-    const SubcellBlockDev& C = M.blk[b];
     elements += P.blk[b].E;
-    sm_fv = std::max(sm_fv, sizeof(double) * (size_t)mood_fv_smem(NV, P.blk[b].Np, C.S, C.NI));
-    sm_up = std::max(sm_up, sizeof(double) * (size_t)mood_update_smem(NV, P.blk[b].Np, C.S));
   }
   if (elements == 0) return DGB_OK;
   int rc;
-  // about one resident wave of CTAs each
-  const int most = (int)std::min(elements, 148L * 6);
+  // one resident wave each, whose CTAs take the listed elements in turn: with a CTA per SM more than fit, the last
+  // ones start when the others end, and a long list takes as long as two waves (12,776 P3 hexahedra, all troubled: recompute
+  // 2.03 ms with six CTAs per SM for the five that fit, 1.59 ms with those)
+  const size_t sm_fv = p->mood_smem_fv, sm_up = p->mood_smem_up;
   if ((rc = prepare(k_mood_fv<NV>, sm_fv))) return rc;
-  k_mood_fv<NV><<<most, kThreads, sm_fv, st>>>(P, M, cur, p->mood_lists);
+  k_mood_fv<NV><<<(int)std::min<long>(elements, p->mood_ctas_fv), kThreads, sm_fv, st>>>(P, M, cur, p->mood_lists);
   if (faces > 0)
     k_mood_faces<NV><<<std::min(blocks_for(faces, kThreads / 32), 148 * 8), kThreads, 0, st>>>(P, M, cur, F, p->mood_lists);
   auto update = [&](auto kernel) -> int {
     if (int e = prepare(kernel, sm_up)) return e;
-    kernel<<<most, kThreads, sm_up, st>>>(P, M, F, vis, dt, src, dst, p->mood_lists, (unsigned)elements);
+    kernel<<<(int)std::min<long>(elements, p->mood_ctas_up), kThreads, sm_up, st>>>(P, M, F, vis, dt, src, dst,
+                                                                                  p->mood_lists, (unsigned)elements);
     return DGB_OK;
   };
   if ((rc = in_place ? update(k_mood_update<NV, false>) : update(k_mood_update<NV, true>))) return rc;
@@ -1119,6 +1142,27 @@ int run_subcell_api(dgb_plan* p, const dgb_state* base, const dgb_state* cand, d
                                   arhs ? arhs->block[2] : nullptr};
   double* outp[DGB_MAX_BLOCKS] = {out->block[0], out->block[1], out->block[2]};
   double* candp[DGB_MAX_BLOCKS] = {cand->block[0], cand->block[1], cand->block[2]};
+  // the candidate is copied to out first and updated in place, unless out shares memory with what is still to be
+  // read, or every element has a CTA of the update anyway, whose own copy saves the launch (1,216 P3 hexahedra on
+  // 740 CTAs: 52 us instead of 57 with none troubled, but 97 instead of 87 with 1 %; 12,776: 149 instead of 123)
+  long elements = 0;
+  bool shared = false;
+  for (int b = 0; b < P.nblocks; ++b) {
+    elements += P.blk[b].E;
+    const size_t n = (size_t)P.blk[b].E * P.blk[b].Np * NV;
+    for (int c = 0; c < P.nblocks; ++c) {
+      const size_t m = (size_t)P.blk[c].E * P.blk[c].Np * NV;
+      for (const double* in : {S.b[c], visp[c], c == b ? nullptr : candp[c]})
+        shared |= in && std::less<>()(in, outp[b] + n) && std::less<>()(outp[b], in + m);
+    }
+  }
+  if (!shared && elements > p->mood_ctas_up)
+    for (int b = 0; b < P.nblocks; ++b)
+      if (P.blk[b].E > 0 && candp[b] != outp[b]) {
+        CK(cudaMemcpyAsync(outp[b], candp[b], sizeof(double) * (size_t)P.blk[b].E * P.blk[b].Np * NV,
+                           cudaMemcpyDeviceToDevice, st));
+        candp[b] = outp[b];
+      }
   const FlagPtrs F = flag_ptrs(troubled);
   if ((rc = run_mood_screen(p, F, st))) return rc;
   return run_subcell<NV>(p, S, candp, arhs ? visp : nullptr, dt, F, outp, st);
@@ -2093,6 +2137,7 @@ int dgb_plan_enable_mood(dgb_plan* p) {
       mark += p->dev.blk[b].E;
     }
   }
+  if ((rc = NV == 5 ? mood_grids<5>(p) : mood_grids<16>(p))) return rc;
   for (double*& d : p->sub_bdc) {    // the boundary subface centres were only needed for matching
     cudaFree(d);
     d = nullptr;

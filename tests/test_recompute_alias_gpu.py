@@ -1,7 +1,8 @@
 """dgb_subcell_recompute into the buffers of its own inputs: the result in a buffer of its own, in the
 candidate's, in the base state's and in the additional right-hand side's is the same bit for bit (each element is
 written last, from what has been read; the work lists' order enters no result), and the inputs that are not the output
-keep their values.  From no troubled element to all of them, on a mesh of every element type and on hexahedra."""
+keep their values.  From no troubled element to all of them, on a mesh of every element type and on hexahedra, fewer and
+more than one wave of CTAs (out of place, large candidates are copied first)."""
 
 import ctypes
 
@@ -13,14 +14,14 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("share", [0.0, 0.4, 1.0])
 @pytest.mark.parametrize("degree", [1, 2, 3])
-@pytest.mark.parametrize("mesh", ["mixed_block", "box_hex"])
+@pytest.mark.parametrize("mesh", ["mixed_block", "box_hex", "large_box_hex"])
 def test_output_in_an_input_buffer(mesh, degree, share):
     import torch
     from jax_fluid_sim_b200 import (FarfieldWallBoundary, HybridCompressibleSolver, HybridMesh, HybridNavierStokesOperator,
                                     HybridSubcellFV, meshgen)
     from jax_fluid_sim_b200 import _native as N
     src = meshgen.mixed_block(jitter=0.1, seed=2) if mesh == "mixed_block" else meshgen.box_hex(
-        (4, 3, 2), hi=(4.0, 3.0, 2.0), jitter=0.1, seed=3)
+        (4, 3, 2) if mesh == "box_hex" else (12, 12, 12), hi=(4.0, 3.0, 2.0), jitter=0.1, seed=3)
     solver = HybridCompressibleSolver(HybridMesh(src), polynomial_degree=degree, dynamic_viscosity=0.02)
     op = HybridNavierStokesOperator(solver)
     fv = HybridSubcellFV(op)
