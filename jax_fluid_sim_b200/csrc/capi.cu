@@ -89,10 +89,11 @@ struct dgb_plan {
   size_t force_partials_n = 0;
   ElemLaunch launch_tr, launch_vol, launch_fin, launch_tr64;
   size_t smem_tr = 0, smem_vol = 0, smem_fin = 0, smem_tr64 = 0;
-  // two-launch inviscid right-hand side of the dense path (dense_rhs.cu); faces_regular: every local
-  // face of the block has the face type its element type gives it
+  // two-launch right-hand side of the dense path (dense_rhs.cu), built by dgb_plan_finalize.  faces_regular: every
+  // local face of the block has the face type its element type gives it; shapes of the trace tables per face type
   DenseTables dense = {};
-  bool faces_regular[DGB_MAX_BLOCKS] = {false, false, false};
+  bool faces_regular[DGB_MAX_BLOCKS] = {false, false, false}, all_affine[DGB_MAX_BLOCKS] = {false, false, false};
+  int trace_codes[DGB_MAX_BLOCKS][2] = {}, trace_nq[DGB_MAX_BLOCKS][2] = {};
   size_t smem_pos[DGB_MAX_BLOCKS], smem_troubled[DGB_MAX_BLOCKS];
   // sum-factorised hexahedron path (single hexahedron block)
   bool hex = false;
@@ -197,7 +198,6 @@ int upload_by_value(dgb_plan* p, const double* host, size_t rows, int nq, int K,
   CK(cudaFuncSetAttribute(k_values_by_row, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   k_values_by_row<<<(unsigned)rows, 128, smem>>>(const_cast<double*>(*out), nq, K);
   CK(cudaGetLastError());
-  CK(cudaDeviceSynchronize());
   return DGB_OK;
 }
 
@@ -325,14 +325,24 @@ int upload_real(dgb_plan* p, const std::vector<double>& v, const void** out) {
   return rc;
 }
 
-// The face-node tables of one block and face type (DenseBlock) from its trace table B
-// [codes][nq][np]: the nodes whose basis does not vanish on the face.  Left empty (and with it the
-// two-launch form off) when the shapes or the number of such nodes are not those of the element type.
-int dense_trace_tables(dgb_plan* p, int b, int ft, int ncodes, int nq, int np, const double* B) {
+// The two sides of each face in one record (DenseTables::side; set-up).
+__global__ void k_face_sides(const FaceDev fd, int3* __restrict__ out) {
+  const int f = blockIdx.x * blockDim.x + threadIdx.x;
+  if (f >= fd.F) return;
+  out[2 * f] = make_int3(fd.ob[f], fd.ol[f], fd.oc[f]);
+  out[2 * f + 1] = make_int3(fd.nb[f], fd.nl[f], fd.nc[f]);
+}
+
+// The face-node tables of one block and face type (DenseBlock) from its trace table [codes][nq][np]: the nodes
+// whose basis does not vanish on the face.  Left empty (and with it the two-launch form off) when the shapes or the
+// number of such nodes are not those of the element type.
+int dense_trace_tables(dgb_plan* p, int b, int ft) {
   const BlockDev& blk = p->dev.blk[b];
-  if (p->dev.degree < 1 || p->dev.degree > 3 || blk.type < 0 || blk.type > 2 || !B) return DGB_OK;
+  const int ncodes = p->trace_codes[b][ft], nq = p->trace_nq[b][ft], np = blk.Np;
   const DenseShape s = dense_shape(p->dev.degree, blk.type);
-  if (np != s.Np || nq != s.nq[ft]) return DGB_OK;
+  if (!blk.trB[ft] || np != s.Np || nq != s.nq[ft]) return DGB_OK;
+  std::vector<double> B((size_t)ncodes * nq * np);
+  CK(cudaMemcpy(B.data(), blk.trB[ft], sizeof(double) * B.size(), cudaMemcpyDeviceToHost));
   const int nfn = s.nfn[ft];
   std::vector<uint8_t> node((size_t)ncodes * nfn);
   std::vector<int8_t> inv((size_t)ncodes * np, -1);
@@ -395,8 +405,8 @@ size_t dense_layout(const dgb_plan* p, ElemLaunch& L, DenseKind kind, size_t rs)
 // Completes the two-launch form (dense_rhs.cu) where every block has its shapes and tables.
 int dense_finish(dgb_plan* p) {
   p->dense.ready = false;
-  if (p->hex || p->dev.nv != 5 || p->dev.degree < 1 || p->dev.degree > 3) return DGB_OK;
   const bool f32 = p->prm.precision == 1;
+  if (p->hex || p->dev.nv != 5 || p->dev.degree < 1 || p->dev.degree > 3 || (f32 && p->dev.viscous)) return DGB_OK;
   for (int b = 0; b < p->dev.nblocks; ++b) {
     const BlockDev& B = p->dev.blk[b];
     DenseBlock& X = p->dense.b[b];
@@ -404,6 +414,9 @@ int dense_finish(dgb_plan* p) {
     if (B.E == 0) continue;
     const DenseShape s = dense_shape(p->dev.degree, B.type);
     const bool tri = B.type != 0, quad = B.type != 2;
+    int rc;
+    if (tri && (rc = dense_trace_tables(p, b, 0))) return rc;
+    if (quad && (rc = dense_trace_tables(p, b, 1))) return rc;
     if (B.Np != s.Np || B.Nq != s.Nq || B.nlf != s.nlf || !p->faces_regular[b] || !B.Bt || !B.dBi || !B.dBq || !B.jinv ||
         !B.wdet || (tri && !X.cB[0]) || (quad && !X.cB[1]))
       return DGB_OK;
@@ -414,16 +427,26 @@ int dense_finish(dgb_plan* p) {
     X.mref = B.mref_inv;
     if (f32) {
       float* f;
-      int rc;
       if ((rc = to_float32(p, B.Bt, (size_t)B.Np * B.Nq, &f))) return rc;
       X.Bt = f;
       if ((rc = to_float32(p, B.dBi, (size_t)B.Nq * 3 * B.Np, &f))) return rc;
       X.dBi = f;
-      if ((rc = to_float32(p, B.minv, (size_t)B.E * B.Np * B.Np, &f))) return rc;
+      f = nullptr;                     // affine elements take mref
+      if (!p->all_affine[b] && (rc = to_float32(p, B.minv, (size_t)B.E * B.Np * B.Np, &f))) return rc;
       X.minv = f;
       if ((rc = to_float32(p, B.mref_inv, (size_t)B.Np * B.Np, &f))) return rc;
       X.mref = f;
     }
+  }
+  for (int ft = 0; ft < 2; ++ft) {
+    if (!p->face_present[ft]) continue;
+    const FaceDev& F = p->dev.face[ft];
+    void* d = nullptr;
+    CK(cudaMalloc(&d, sizeof(int3) * 2 * (size_t)F.F));
+    p->allocations.push_back(d);
+    k_face_sides<<<blocks_for(F.F, kThreads), kThreads>>>(F, static_cast<int3*>(d));
+    CK(cudaGetLastError());
+    p->dense.side[ft] = static_cast<const int3*>(d);
   }
   p->dense.ready = true;
   return DGB_OK;
@@ -1322,13 +1345,6 @@ int dgb_plan_set_faces(dgb_plan* p, const dgb_face_desc* d) {
   if ((rc = upload_by_value(p, d->normals, n, (int)nq, 3, &F.n))) return rc;
   if ((rc = upload(p, d->weights, n * nq, &F.w))) return rc;
   if ((rc = upload_by_value(p, d->side_inv_jacobian, n * 2, (int)nq, 9, &F.jinv))) return rc;
-  // the two sides of each face in one record (dense_rhs.cu)
-  std::vector<int3> side(2 * n);
-  for (size_t f = 0; f < n; ++f) {
-    side[2 * f] = make_int3(d->owner_block[f], d->owner_local[f], d->owner_code[f]);
-    side[2 * f + 1] = make_int3(d->nbr_block[f], d->nbr_local[f], d->nbr_code[f]);
-  }
-  if ((rc = upload(p, side.data(), side.size(), &p->dense.side[d->face_type]))) return rc;
   p->face_present[d->face_type] = n > 0;
   return DGB_OK;
 }
@@ -1355,7 +1371,8 @@ int dgb_plan_set_trace(dgb_plan* p, int etype, int ftype, int ncodes, int nq, in
       if ((rc = upload(p, bt.data(), bt.size(), &blk.trBt[ftype]))) return rc;
       if ((rc = upload(p, dt.data(), dt.size(), &blk.trdBt[ftype]))) return rc;
     }
-    if ((rc = dense_trace_tables(p, b, ftype, ncodes, nq, np, B))) return rc;
+    p->trace_codes[b][ftype] = ncodes;
+    p->trace_nq[b][ftype] = nq;
     found = 1;
   }
   if (!found) return fail(DGB_ERR_ARGUMENT, "trace table for an element type without a block");
@@ -1539,6 +1556,7 @@ int dgb_plan_set_block_affine(dgb_plan* p, int b, const uint8_t* affine, const d
   if ((rc = upload(p, det, (size_t)B.E, &B.adet))) return rc;
   if ((rc = upload(p, ref_weights, (size_t)B.Nq, &B.wref))) return rc;
   if ((rc = upload(p, ref_inv_mass, (size_t)B.Np * B.Np, &B.mref_inv))) return rc;
+  p->all_affine[b] = std::all_of(affine, affine + B.E, [](uint8_t a) { return a != 0; });
   return DGB_OK;
 }
 
