@@ -247,6 +247,9 @@ int dgb_rhs(dgb_plan* plan, const dgb_state* U, const dgb_state* inviscid_out,
  * form: Euler plans, the fused hexahedron form, the two-launch dense form (5 variables); else
  * DGB_ERR_UNSUPPORTED. */
 int dgb_rhs_total(dgb_plan* plan, const dgb_state* U, const dgb_state* out, void* stream);
+/* 1 if dgb_rhs_total takes this plan, 0 if not (DGB_ERR_UNSUPPORTED); fixed once the plan is finalized, but for
+ * dgb_plan_set_fused. */
+int dgb_rhs_total_supported(dgb_plan* plan);
 /* Physical coordinates of every face point, [F][nq][3] for one face type (the moment arms of
  * dgb_wall_forces). */
 int dgb_plan_set_face_points(dgb_plan* plan, int face_type, const double* points);

@@ -154,6 +154,7 @@ def lib():
                                 P_double, P_double, P_double, P_double, P_double, P_double],
             "dgb_plan_destroy": [c_void_p],
             "dgb_plan_update_params": [c_void_p, ctypes.POINTER(Params)],
+            "dgb_rhs_total_supported": [c_void_p],
             "dgb_rhs_total": [c_void_p, ctypes.POINTER(State), ctypes.POINTER(State), c_void_p],
             "dgb_rhs": [c_void_p, ctypes.POINTER(State), ctypes.POINTER(State), ctypes.POINTER(State), c_void_p],
             "dgb_stable_dt": [c_void_p, ctypes.POINTER(State), c_double, c_void_p, c_void_p],

@@ -1808,12 +1808,16 @@ int dgb_rhs(dgb_plan* p, const dgb_state* U, const dgb_state* inv_out, const dgb
   return p->dev.nv == 5 ? run_rhs<5>(p, S, A, st) : run_rhs<16>(p, S, A, st);
 }
 
+int dgb_rhs_total_supported(dgb_plan* p) {
+  if (int rc = check_ready(p)) return rc;
+  // mixed plans form the residuals apart (dgb_rhs); Euler plans have one
+  return p->prm.precision == 0 && (!p->dev.viscous || (p->hex ? p->fused : p->dense.ready));
+}
+
 int dgb_rhs_total(dgb_plan* p, const dgb_state* U, const dgb_state* out, void* stream) {
   int rc;
   if ((rc = check_ready(p)) || (rc = check_state(p, U, "U")) || (rc = check_state(p, out, "out"))) return rc;
-  if (p->prm.precision == 1) return fail(DGB_ERR_UNSUPPORTED, "mixed plans form the residuals apart (dgb_rhs)");
-  if (p->dev.viscous && !(p->hex ? p->fused : p->dense.ready))
-    return fail(DGB_ERR_UNSUPPORTED, "this plan forms the residuals apart (dgb_rhs)");
+  if (!dgb_rhs_total_supported(p)) return fail(DGB_ERR_UNSUPPORTED, "this plan forms the residuals apart (dgb_rhs)");
   FinalizeArgs A;
   memset(&A, 0, sizeof(A));
   A.total = 1;

@@ -134,6 +134,7 @@ class NativePlan:
         self.affine = bool(affine)
         N.check(L.dgb_plan_finalize(handle))
         self.fused = True          # the plan's default form of the hexahedron right-hand side
+        self.single_residual = N.lib().dgb_rhs_total_supported(handle) == 1
         self._pushed = self._snapshot()
 
     def enable_mood(self, coupling="reference", tables="device"):
@@ -231,6 +232,7 @@ class NativePlan:
         sum-factorised hexahedron right-hand side (``dgb_plan_set_fused``)."""
         N.check(N.lib().dgb_plan_set_fused(self.handle, int(bool(enable))))
         self.fused = bool(enable)
+        self.single_residual = N.lib().dgb_rhs_total_supported(self.handle) == 1
 
     def device_errors(self, reset=True):
         """Error bits recorded on the device by kernels with bounded waits (0: none)."""
@@ -404,14 +406,14 @@ class HybridNavierStokesOperator(HybridEulerOperator):
     def rhs(self, states, boundary_state=None):
         if not self.viscous:
             return self.inviscid_rhs(states, boundary_state)
-        if self.precision == "float64":
+        if self.native.single_residual:
             # one residual where the plan's path forms it so; the split residuals' sum elsewhere
             U = self.to_device(states)
             self.native.set_boundary(boundary_state)
             out = {k: torch.empty_like(U[k]) for k in self.names}
             s_in, s_out = self.native.state(self._blocks(U)), self.native.state(self._blocks(out))
             rc = N.lib().dgb_rhs_total(self.native.handle, ctypes.byref(s_in), ctypes.byref(s_out), _stream_ptr())
-            if rc != N.UNSUPPORTED:
+            if rc != N.UNSUPPORTED:      # (the form was changed through the handle)
                 N.check(rc)
                 return out
         inv, vis = self._run_rhs(states, boundary_state, True, True)

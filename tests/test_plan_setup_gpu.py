@@ -55,3 +55,26 @@ def test_volume_rules_of_any_size_are_accepted(points):
         N.check(L.dgb_plan_set_block(handle, 0, ctypes.byref(d)))
     finally:
         L.dgb_plan_destroy(handle)
+
+
+def test_split_residuals_are_the_only_outputs_allocated():
+    """A plan that forms the residuals apart (the six-launch hexahedron form) allocates them and their sum, three
+    states, and no output for the single residual that it does not have; switching the form back takes that one."""
+    import torch
+    from jax_fluid_sim_b200 import HybridCompressibleSolver, HybridMesh, HybridNavierStokesOperator, meshgen
+    solver = HybridCompressibleSolver(HybridMesh(meshgen.box_hex((16, 16, 16), hi=(1.0,) * 3, jitter=0.1, seed=3)),
+                                      polynomial_degree=2, dynamic_viscosity=0.02)
+    op = HybridNavierStokesOperator(solver)
+    U = solver.state_blocks_from_primitive_function(
+        op, lambda x: np.stack([1.0 + 0.1 * np.sin(x[..., 0]), 0.3 + 0 * x[..., 0], 0 * x[..., 1], 0 * x[..., 2],
+                                1.0 + 0 * x[..., 0]], -1))
+    state = sum(v.numel() * 8 for v in U.values())
+    for fused, states in ((True, 1), (False, 3), (True, 1)):
+        op.native.set_fused(fused)
+        op.rhs(U)
+        torch.cuda.synchronize()
+        torch.cuda.reset_peak_memory_stats()
+        before = torch.cuda.memory_allocated()
+        R = op.rhs(U)
+        assert torch.cuda.max_memory_allocated() - before < (states + 0.5) * state
+        del R
