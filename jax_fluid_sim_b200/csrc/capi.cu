@@ -138,7 +138,6 @@ struct dgb_plan {
   double* unl[DGB_MAX_BLOCKS] = {nullptr, nullptr, nullptr};
   double* eul[DGB_MAX_BLOCKS] = {nullptr, nullptr, nullptr};
   double* vis[DGB_MAX_BLOCKS] = {nullptr, nullptr, nullptr};
-  double* rec[DGB_MAX_BLOCKS] = {nullptr, nullptr, nullptr};
   // tensor-core (tcgen05) inviscid volume kernel of the dense blocks (dgb_plan_set_tensor_cores)
   TcShape tc[DGB_MAX_BLOCKS];
   float* tc_image[DGB_MAX_BLOCKS] = {nullptr, nullptr, nullptr};
@@ -2125,7 +2124,6 @@ int dgb_plan_enable_mood(dgb_plan* p) {
     if ((rc = alloc(p, state, &p->unl[b]))) return rc;
     if ((rc = alloc(p, state, &p->eul[b]))) return rc;
     if ((rc = alloc(p, state, &p->vis[b]))) return rc;
-    if ((rc = alloc(p, state, &p->rec[b]))) return rc;
   }
   for (int ft = 0; ft < 2; ++ft) {
     if (!p->face_present[ft]) continue;

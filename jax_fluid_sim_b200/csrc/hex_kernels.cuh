@@ -326,17 +326,6 @@ __device__ __forceinline__ void tensor2(const T* in, T* out, T* t, const T* M1, 
   __syncthreads();
 }
 
-// Gather the N^2 slab of face (a0, end) from lexicographic nodal data X[c][N^3] into slab[c][j2][j1].
-template <int C, int N, typename T>
-__device__ __forceinline__ void face_slab(const T* X, T* slab, int a0, int end, int a1, int a2) {
-  for (int idx = threadIdx.x; idx < C * N * N; idx += kThreads) {
-    const int j1 = idx % N, j2 = (idx / N) % N, c = idx / (N * N);
-    // 1-D node 0 sits at xi=0, node 1 at xi=1
-    const int l = end * axis_stride<N>(a0) + j1 * axis_stride<N>(a1) + j2 * axis_stride<N>(a2);
-    slab[idx] = X[c * N * N * N + l];
-  }
-}
-
 // --------------------------------------------------------------------------------------------
 // Shared-memory layouts (doubles) of the hex element kernels; each kernel has its own.
 constexpr int cmax(int a, int b) { return a > b ? a : b; }
@@ -348,7 +337,6 @@ struct HexSmem {
   static constexpr int N = D::N, Q = D::Q, QF = D::QF, N2 = D::N2, N3 = D::N3, Q3 = D::Q3, QF2 = D::QF2;
   // table size in R, rounded up to 16 bytes so that the arrays after the tables stay 16-byte aligned
   static constexpr int T = (int)((sizeof(HexTablesT<R>) + 15) / 16 * 16 / sizeof(R));
-  static constexpr int MS = N3 + 1;                 // padded row stride of the staged M^-1 (transposed)
   // traces: U, v, then the six faces' slabs, contraction scratch, face values and tangential derivatives
   static constexpr int TR_U = 0, TR_V = TR_U + NV * N3, TR_W = (TR_V + 4 * N3 + 3) / 4 * 4;
   // slabs [CH][FP] (the face values of U and dv/dn take their place), the face values of v [24][FP] and the
@@ -389,16 +377,6 @@ __device__ __forceinline__ void load_tables(const HexTables& src, HexTablesT<flo
   float* d = reinterpret_cast<float*>(dst);
   for (int i = threadIdx.x; i < kHexTableValues; i += kThreads) d[i] = (float)s[i];
   for (int i = threadIdx.x; i < 64; i += kThreads) dst->lex2node[i] = src.lex2node[i];
-}
-
-// Stage M^-1 of one element transposed into shared memory, in lexicographic node order:
-// Mt[lj * MS + li] = M^-1[node(li)][node(lj)].  Global reads are coalesced rows.
-template <int N3, int MS>
-__device__ __forceinline__ void stage_minv(const double* Mg, const int* lex2node, const int* node2lex, double* Mt) {
-  for (int idx = threadIdx.x; idx < N3 * N3; idx += kThreads) {
-    const int i = idx / N3, j = idx % N3;          // element node indices
-    Mt[node2lex[j] * MS + node2lex[i]] = Mg[idx];
-  }
 }
 
 // --------------------------------------------------------------------------------------------
