@@ -175,8 +175,8 @@ def stage_bytes_fused(op, nv, split, sizeof=8):
     """Algorithmic HBM bytes per launch of the fused sum-factorised hex right-hand side (traces,
     face kernel, element kernel; every input read once, every output written once).  The face
     kernel is reported as the "face_flux" stage and the element kernel (nodal lift, volume terms,
-    face terms, M^-1 and the outputs) as the "volume" stage.  Mixed-precision plans read float32
-    copies of M^-1 and of the per-point inverse Jacobians."""
+    face terms, M^-1 and the outputs) as the "volume" stage.  Mixed-precision plans hold M^-1, the inverse
+    Jacobians, the lift operators, the viscous traces, the face fluxes and the jumps in float32."""
     out = dict.fromkeys(STAGES, 0)
     visc = op.viscous
     msz = 4 if op.precision == "mixed" else sizeof
@@ -186,12 +186,15 @@ def stage_bytes_fused(op, nv, split, sizeof=8):
     Ed = E - Ea
     fp = op.plan.faces["quad"]
     nqf = fp.nq
-    out["traces"] = sizeof * E * (nv * Np + nlf * nqf * (nv + (16 if visc else 0))) + (msz * E * nlf * nqf * 9 if visc else 0)
-    per_point = 2 * nv + 4 + 2 * nv + ((2 * 4 + 2 * 12 + 12 + nv) if visc else 0)
-    out["face_flux"] = fp.F * (sizeof * nqf * per_point + 8) + (sizeof * Ed * nlf * nqf * nqf if visc else 0)
+    # U in; per face point U out (float64), v and its gradients out, inverse Jacobian in
+    out["traces"] = E * (sizeof * (nv * Np + nlf * nqf * nv) + (msz * nlf * nqf * (16 + 9) if visc else 0))
+    # per face point: both sides' U, n and w in (float64); both sides' inviscid fluxes out, both sides' v and
+    # gradients in, jumps and viscous flux out
+    out["face_flux"] = fp.F * (nqf * (sizeof * (2 * nv + 4) + msz * (2 * nv + ((2 * 16 + 12 + nv) if visc else 0))) + 8)
+    out["face_flux"] += msz * Ed * nlf * nqf * nqf if visc else 0
     outputs = (2 if split else 1) * nv * Np
-    out["volume"] = (sizeof * E * (nv * Np + outputs + nlf * nqf * ((12 + 2 * nv) if visc else nv))
-                     + msz * Ed * (10 * Nq + Np * Np) + sizeof * 11 * Ea)
+    out["volume"] = (E * (sizeof * (nv * Np + outputs) + msz * nlf * nqf * ((12 + 2 * nv) if visc else nv))
+                     + Ed * (msz * (9 * Nq + Np * Np) + sizeof * Nq) + sizeof * 11 * Ea)
     return out
 
 

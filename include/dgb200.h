@@ -266,7 +266,9 @@ int dgb_wall_forces(dgb_plan* plan, const dgb_state* U, const int32_t* wall_tags
  * `reps` runs, one coordinate sweep) and keeps the fastest in the plan.  widths (optional,
  * [3][DGB_MAX_BLOCKS]) receives the choice per kernel (trace, volume, finalize) and block; all
  * zeros on the sum-factorised hexahedron path, whose launches are fixed.  Inviscid plans on the two-launch
- * dense form have fixed launches too: widths receives the general kernels' defaults, nothing is timed.
+ * dense form have fixed launches too: widths receives the general kernels' defaults, nothing is timed.  Viscous
+ * float64 plans on that form take it for whole residuals and steps without MOOD; their widths are those of the
+ * separate right-hand sides and of MOOD steps.
  * Synchronises the stream. */
 int dgb_plan_autotune(dgb_plan* plan, const dgb_state* U, int reps, int* widths, void* stream);
 /* Execution form of the sum-factorised hexahedron right-hand side (no reference counterpart; the

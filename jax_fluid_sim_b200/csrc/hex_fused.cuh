@@ -12,8 +12,8 @@
 //                  with K = bf m1i bf^T, otherwise a QF^2 x QF^2 operator per element face built
 //                  once from M^-1 (k_hex_lop).  This replaces k_face_flux, the per-face part of
 //                  k_hex_lift and k_face_visc, and the traces are read once.
-//   k_hex_element  one CTA per element (128 threads; one warp at P2): the nodal lift M^-1 sum_f B_f^T jump_f, the volume terms
-//                  (U, grad v and lift at the volume points; inviscid and viscous fluxes), the face
+//   k_hex_element  one CTA per element (128 threads at P3, one warp at P1 and P2): the nodal lift
+//                  M^-1 sum_f B_f^T jump_f, the volume terms (U, grad v and lift at the volume points; inviscid and viscous fluxes), the face
 //                  terms and M^-1 with the stage update.  The lift and the residuals stay in shared
 //                  memory (no nodal-lift or residual buffers in HBM); M^-1 is read by the lift and
 //                  by the final product.

@@ -51,7 +51,6 @@ struct HexDims {
   static constexpr int Q = P == 1 ? 2 : (P == 2 ? 3 : 5);
   static constexpr int QF = P == 1 ? 2 : (P == 2 ? 3 : 4);
   static constexpr int N3 = N * N * N, Q3 = Q * Q * Q, N2 = N * N, QF2 = QF * QF;
-  // CTA size of the traces and element kernels (one element each)
   // CTA sizes of the traces and element kernels (one element each).  A phase of a P2 element has 9 to 90 items:
   // at 128 threads the warps mostly waited for one another at the barriers.  Element kernel of 12,776 P2
   // hexahedra (float64) at 128, 64, 32 threads: 779, 537, 454 us; traces 193, 192, 206.  A P3 element fills

@@ -344,8 +344,10 @@ class HybridEulerOperator:
     def autotune(self, states, boundary_state=None, reps=3):
         """Pick the threads-per-element width of the dense kernels by timing them on ``states``
         (dgb_plan_autotune); returns {kernel: {element_type: width}} (empty on the
-        sum-factorised hexahedron path, whose launches are fixed; the default widths, untimed, where the
-        two-launch form of the dense path runs, csrc/dense_rhs.cu)."""
+        sum-factorised hexahedron path, whose launches are fixed; the default widths, untimed, for inviscid
+        operators on the two-launch form of the dense path, csrc/dense_rhs.cu).  Viscous float64 operators on
+        that form take it for whole residuals and for steps without MOOD: their widths are those of the separate
+        right-hand sides and of MOOD steps."""
         U = self.to_device(states)
         self.native.set_boundary(boundary_state)
         widths = np.zeros(3 * N.MAX_BLOCKS, np.int32)
