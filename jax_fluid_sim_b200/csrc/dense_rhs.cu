@@ -10,7 +10,7 @@
 //                    stage update, with everything between them in shared memory.
 //
 // The residual of a 4^3 P2 hybrid box with viscous terms took nine launches and three additions of the
-// split residuals, 122 us, and takes these two, 49 us.  Split residuals (MOOD, the separate right-hand
+// split residuals, 122 us, and takes these two, 51 us.  Split residuals (MOOD, the separate right-hand
 // sides) and mixed viscous plans keep the general kernels of dg_kernels.cuh.
 //
 // The element kernel is bound by the operand loads of its contractions, not by their arithmetic: with
@@ -19,8 +19,11 @@
 // NV variables of one point while it interpolates, IB nodes x EB2 elements x NV variables of one chunk
 // of points while it sums the residual, with 16-byte shared-memory loads; a table value from L1/L2 then
 // serves EB * NV products instead of NV.  NE is chosen so that both phases fill kThreads.
-// Checked Euler steps of hybrid boxes, general kernels against these two: 16^3 P3 1860 -> 950 us, 32^3 P1
-// 1308 -> 496 us, 23^3 P2 mixed 2776 -> 1436 us.
+// Checked Euler steps of hybrid boxes, general kernels against these two: 16^3 P3 1860 -> 952 us, 32^3 P1
+// 1308 -> 499 us, 23^3 P2 mixed 2776 -> 1433 us.
+// A nodal value that is not finite reaches a neighbour through the faces that the node lies on; the general kernels
+// multiply it by the zeros of the other faces' tables as well, so it is a ring of elements further after a step.  Either
+// way the element itself is not finite and the step's status refuses the state.
 // Sums run in the order of the one-value-per-thread form: per output the nodes (points) ascend, and
 // the residual is summed per chunk of points, then over the chunks.
 #include "dense_rhs.h"
